@@ -233,7 +233,7 @@ struct Buf {
         return p;
     }
 };
-Buf b_tab, b_A, b_md, b_ld, b_tr, b_res, b_st;
+Buf b_tab, b_A, b_md, b_ld, b_tr, b_res, b_st, b_work;
 
 } // namespace
 
@@ -287,8 +287,9 @@ int capc_batch(double R, double d, int n, const double *q, int nq, char DN, int 
         COUNT_LAUNCH(1);
         CK(cudaGetLastError());
         launch_stats(nullptr, nt, n, d_A, n, mstride, d_md, mode, d_tr, d_res, d_st, st);
-        launch_cholesky(nt, n, d_A, n, mstride, d_st, d_ld, st);
-        launch_final(nt, n, d_ld, d_tr, d_st, d_res, mode, st);
+        void *d_work = b_work.get(cholesky_work_bytes(nt, n));
+        launch_cholesky(nt, n, d_A, n, mstride, d_st, d_md, d_ld, d_work, st);
+        launch_final(nt, n, d_ld, d_work, d_tr, d_st, d_res, mode, st);
         CK(cudaMemcpyAsync(res.data(), d_res, (size_t)nt * sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(hst.data(), d_st, (size_t)nt * sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));

@@ -111,7 +111,11 @@ void launch_elem_ff(const Task *tasks, const int *tlist, int nlist, int ldim, co
 // one sum of squares per task (launch_sweep_ff), otherwise k_elem_ff's per-warp partials
 void launch_stats_ff(const int *tlist, int nlist, int ldim, const double *diag, const float *part, int mode, double *trace,
                      double *result, int *status, cudaStream_t st, bool part_per_task = false);
-void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, double *logdiag, cudaStream_t st);
+// FP64 form: A (lower triangle, FP64) is converted to fixed point in place and factored; mdiag: M_ii
+// (n per task); logdet: ceil(n / 64) partial sums per task; work: cholesky_work_bytes
+size_t cholesky_work_bytes(int ntask, int n);
+void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, double *logdet,
+                     void *work, cudaStream_t st);
 size_t mixed_work_bytes(int ntask, int n);
 // live CUDA-event timing of the tcgen05 trailing update (mixed.cu)
 void kernel_timer_enable(bool on);
@@ -123,7 +127,8 @@ enum { MIXED_SCHED_IMAGES = 0, MIXED_SCHED_REGSTAGE = 1, MIXED_SCHED_PER_TILE = 
 void launch_cholesky_mixed(int ntask, int n, const double *A, size_t lda, size_t mstride, int *status, float *S, size_t sstride,
                            const double *mdiag, const double *trace, double *result, int mode, cudaStream_t st, bool tc,
                            bool convert, void *work, int sched);
-void launch_final(int ntask, int n, const double *logdiag, const double *trace, int *status, double *result, int mode, cudaStream_t st);
+void launch_final(int ntask, int n, const double *logdet, const void *work, const double *trace, int *status, double *result, int mode,
+                  cudaStream_t st);
 
 // HODLR log-determinants of the listed tasks (hodlr.cu), elements on demand; the diagonal of
 // M alone for the trace rule; workspace bytes for nbatch matrices.  mx == nullptr: the I

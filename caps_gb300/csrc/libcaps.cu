@@ -535,7 +535,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
                           + (size_t)nu_stride * sizeof(double2) + (size_t)3 * L * sizeof(sd) + (size_t)dim * 8
                           + (size_t)2 * 256 * nu_stride * 12  // partial sums, up to 256 warps
                           + (size_t)(4 * (caps->ldim + 4096)) * sizeof(double4) // p tables
-                          + (mixed && !hodlr ? mixed_work_bytes(1, dim) : 0);   // diagonal-block inverses, panel images
+                          + (hodlr ? 0 : mixed && !O.square ? mixed_work_bytes(1, dim) : cholesky_work_bytes(1, dim)); // diagonal-block inverses, panel images
     size_t budget = (size_t)(0.70 * (double)(freeb + g_eng.A.bytes + g_eng.I.bytes + g_eng.partM.bytes + g_eng.partE.bytes + g_eng.S32.bytes
                                              + g_eng.a12.bytes + g_eng.part.bytes + g_eng.B.bytes + g_eng.hwork.bytes
                                              + g_eng.seed.bytes + g_eng.mwork.bytes));
@@ -816,8 +816,9 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
                                   schedule_for(caps->precision, dim));
         } else if (O.factor) {
             double *d_ld = (double *)g_eng.logdiag.get((size_t)nt * dim * sizeof(double));
-            launch_cholesky(nt, dim, d_A, lda, mstride, d_status, d_ld, st);
-            launch_final(nt, dim, d_ld, d_trace, d_status, d_res, O.mode, st);
+            void *d_work = g_eng.mwork.get(cholesky_work_bytes(nt, dim));
+            launch_cholesky(nt, dim, d_A, lda, mstride, d_status, d_dg, d_ld, d_work, st);
+            launch_final(nt, dim, d_ld, d_work, d_trace, d_status, d_res, O.mode, st);
         }
         CK(cudaEventRecord(g_eng.ev[8], st));
 

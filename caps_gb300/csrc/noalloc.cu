@@ -170,7 +170,10 @@ extern "C" int caps_logdetD_noalloc(caps_t *self, double xi_, int m, double *log
     double *d_pM = C.take<double>((size_t)2 * max_warps * nu_stride);
     int *d_pE = C.take<int>((size_t)2 * max_warps * nu_stride);
     sd *d_K = C.take<sd>((size_t)2 * nu_stride);
-    sd *d_I = C.take<sd>((size_t)2 * L * L);
+    // the I table; the factorisation's workspace takes its place once the elements are formed
+    const size_t i_bytes = (size_t)2 * L * L * sizeof(sd), w_bytes = cholesky_work_bytes(1, dim);
+    unsigned char *d_Iw = C.take<unsigned char>(i_bytes > w_bytes ? i_bytes : w_bytes);
+    sd *d_I = (sd *)d_Iw;
     double *d_A = C.take<double>((size_t)dim * dim);
     double *d_ld = C.take<double>(dim);
     double *d_md = C.take<double>(dim);
@@ -207,8 +210,8 @@ extern "C" int caps_logdetD_noalloc(caps_t *self, double xi_, int m, double *log
     launch_elem(d_task, nullptr, 1, ldim, d_I, d_Sa, d_Sb, d_uv, d_A, dim, (size_t)dim * dim, d_md, d_status, st, false);
     const int mode = self->detalg == DETALG_HODLR ? 1 : 0;
     launch_stats(nullptr, 1, dim, d_A, dim, (size_t)dim * dim, d_md, mode, d_trace, d_res, d_status, st);
-    launch_cholesky(1, dim, d_A, dim, (size_t)dim * dim, d_status, d_ld, st);
-    launch_final(1, dim, d_ld, d_trace, d_status, d_res, mode, st);
+    launch_cholesky(1, dim, d_A, dim, (size_t)dim * dim, d_status, d_md, d_ld, d_Iw, st);
+    launch_final(1, dim, d_ld, d_Iw, d_trace, d_status, d_res, mode, st);
     int status = 0;
     double r = NAN;
     NA_CK(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, st));

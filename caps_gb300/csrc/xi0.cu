@@ -140,7 +140,7 @@ struct Xi0Buf {
         return (T *)p;
     }
 };
-static struct { Xi0Buf I, ratio, f, m, lmin, status, A, ld, md, tr, res; } g_x0;
+static struct { Xi0Buf I, ratio, f, m, lmin, status, A, ld, md, tr, res, work; } g_x0;
 static std::mutex g_xi0_mu;
 
 // I_nu for nu = 0 .. numax and ratio_l, f_l for l = 0 .. lmax of the plasma xi=0 block,
@@ -201,8 +201,9 @@ int logdetD0_batch(caps_t *self, const int *ms, int n, int which, double *out, d
     CK(cudaGetLastError());
     const int mode = self->detalg == DETALG_HODLR ? 1 : 0;
     launch_stats(nullptr, n, ldim, d_A, ldim, mstride, d_md, mode, d_tr, d_res, d_status, st);
-    launch_cholesky(n, ldim, d_A, ldim, mstride, d_status, d_ld, st);
-    launch_final(n, ldim, d_ld, d_tr, d_status, d_res, mode, st);
+    void *d_work = g_x0.work.get<unsigned char>(cholesky_work_bytes(n, ldim));
+    launch_cholesky(n, ldim, d_A, ldim, mstride, d_status, d_md, d_ld, d_work, st);
+    launch_final(n, ldim, d_ld, d_work, d_tr, d_status, d_res, mode, st);
     std::vector<int> hs(n);
     CK(cudaMemcpy(out, d_res, n * sizeof(double), cudaMemcpyDeviceToHost));
     CK(cudaMemcpy(hs.data(), d_status, n * sizeof(int), cudaMemcpyDeviceToHost));
