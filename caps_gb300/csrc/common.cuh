@@ -134,4 +134,26 @@ enum : int {
     ST_ERR_RANGE = 512,    // mixed form: a factor entry |x| >= 4, outside the range of the FP16 panel images
 };
 
+// compensated sum: two-sum (exact), the error terms summed beside
+struct CSum {
+    double s = 0.0, c = 0.0;
+    CAPS_DEV void add(double y, double yc)
+    {
+        const double t = s + y, bb = t - s;
+        c += ((s - (t - bb)) + (y - bb)) + yc;
+        s = t;
+    }
+};
+// this warp's share of the sum of v[0..n) over all threads of the block (valid in every lane)
+CAPS_DEV CSum csum_warp(const double *v, int n)
+{
+    CSum a;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) a.add(v[i], 0.0);
+    for (int o = 16; o > 0; o >>= 1) {
+        const double s = __shfl_xor_sync(0xffffffffu, a.s, o), c = __shfl_xor_sync(0xffffffffu, a.c, o);
+        a.add(s, c);
+    }
+    return a;
+}
+
 } // namespace capsgpu

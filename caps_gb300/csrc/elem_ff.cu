@@ -218,8 +218,8 @@ __global__ void __launch_bounds__(EB) k_diag_ff(const Task *tasks, int ntask, in
     diag[(size_t)task * n + 2 * a + 1] = fe_to_double(MM);
 }
 
-// per task (tlist[blockIdx.x], or blockIdx.x without a list): Kahan trace of M over its
-// FP64 diagonal (index order, misc.c:26), the Frobenius norm from the element partials
+// per task (tlist[blockIdx.x], or blockIdx.x without a list; 256 threads): compensated trace of
+// M over its FP64 diagonal, the Frobenius norm from the element partials
 // (fixed order), and the reference's shortcut decision: |tr| < 1e-8 -> -tr; dense modes:
 // Mercator when its error bound is below 1e-8 relative; otherwise factorise.  Without
 // partials (part == nullptr) only the trace rule is applied: a matrix it does not decide
@@ -248,28 +248,15 @@ __global__ void k_stats_ff(const int *tlist, int nlist, int ldim, const double *
             __syncthreads();
         }
     }
-    if (threadIdx.x >= 32) return;
-    // Kahan trace (misc.c:26) over the diagonal, split across the 32 lanes of warp 0: lane l
-    // sums the l-th contiguous chunk, lane 0 then adds the 32 compensated partials in order
-    const double *dg = diag + (size_t)task * n;
-    const int lane = threadIdx.x, per = (n + 31) / 32;
-    double tr = 0.0, c = 0.0;
-    for (int i = lane * per; i < min(n, (lane + 1) * per); i++) {
-        const double y = dg[i] - c;
-        const double t = tr + y;
-        c = (t - tr) - y;
-        tr = t;
-    }
-    const double partial = tr - c;
-    tr = 0.0;
-    c = 0.0;
-    for (int l = 0; l < 32; l++) {
-        const double y = __shfl_sync(0xffffffffu, partial, l) - c;
-        const double t = tr + y;
-        c = (t - tr) - y;
-        tr = t;
-    }
-    if (lane != 0) return;
+    // trace of M over its FP64 diagonal, compensated (see k_stats)
+    __shared__ double rs[8], rc[8];
+    const CSum w = csum_warp(diag + (size_t)task * n, n);
+    if ((threadIdx.x & 31) == 0) { rs[threadIdx.x >> 5] = w.s; rc[threadIdx.x >> 5] = w.c; }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    CSum all;
+    for (int k = 0; k < 8; k++) all.add(rs[k], rc[k]);
+    const double tr = all.s + all.c;
     trace_out[task] = tr;
     if (status[task] & ~0xF) { result[task] = NAN; return; }
     if (fabs(tr) < 1e-8) { result[task] = -tr; status[task] = ST_TRACE; return; }
