@@ -658,7 +658,8 @@ __global__ void k_elem(const Task *tasks, const int *tlist, int nlist, int ldim,
 // column; mode 1 read it too, 5 ms for 24 matrices of dimension 2100).
 constexpr int ST_NT = 512;
 __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, int n, const double *A, size_t lda, size_t mat_stride, int mode,
-                                                 const double *mdiag, double *trace_out, double *result, int *status)
+                                                 const double *mdiag, double *trace_out, double *result, int *status, const double *frop,
+                                                 int nfro)
 {
     if ((int)blockIdx.x >= nlist) return;
     const int task = tlist ? tlist[blockIdx.x] : (int)blockIdx.x;
@@ -667,7 +668,7 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
     const double *md = mdiag + (size_t)task * n;
     const CSum tr = csum_warp(md, n);
     if (lane == 0) { rs[warp] = tr.s; rc[warp] = tr.c; }
-    if (A && mode == 0) {
+    if (A && mode == 0 && !frop) {
         // sum of squares of M: diagonal once, strict lower twice (M is symmetric)
         const double *Am = A + (size_t)task * mat_stride;
         double s = 0.0;
@@ -693,7 +694,10 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
     if (!A) return;
     if (mode == 0) {
         double fro2 = 0.0;
-        for (int w = 0; w < ST_NT / 32; w++) fro2 += red[w];
+        if (frop)
+            for (int w = 0; w < nfro; w++) fro2 += frop[(size_t)task * nfro + w];
+        else
+            for (int w = 0; w < ST_NT / 32; w++) fro2 += red[w];
         const double fro = sqrt(fro2);
         if (fro < 1) {
             const double merc = -t - fro2 / 2;
@@ -886,10 +890,10 @@ void launch_elem(const Task *tasks, const int *tlist, int nlist, int ldim, const
 }
 
 void launch_stats(const int *tlist, int nlist, int n, const double *A, size_t lda, size_t mat_stride, const double *mdiag, int mode,
-                  double *trace, double *result, int *status, cudaStream_t st)
+                  double *trace, double *result, int *status, cudaStream_t st, const double *fro, int nfro)
 {
     if (nlist <= 0) return;
-    k_stats<<<nlist, ST_NT, 0, st>>>(tlist, nlist, n, A, lda, mat_stride, mode, mdiag, trace, result, status);
+    k_stats<<<nlist, ST_NT, 0, st>>>(tlist, nlist, n, A, lda, mat_stride, mode, mdiag, trace, result, status, fro, nfro);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }

@@ -129,6 +129,21 @@ template <int NC> CAPS_DEV void fold_group(uint32_t taddr, int s, long long (&v)
 // ---------------------------------------------------------------------------
 // FP64 -> fixed point, in place (lower triangle)
 // ---------------------------------------------------------------------------
+// scale exponent of a matrix whose largest diagonal entry is mx: none below 2, else a power of four
+CAPS_DEV int fix_sexp(double mx) { return mx >= 2.0 ? min(2 * ((ilogb(mx) + 2) / 2), 400) : 0; }
+
+// for producers that write fixed point themselves: the exponents alone, one warp per task
+__global__ void k_fix_scale(const int *tlist, int nlist, int n, const double *mdiag, FixInfo *info)
+{
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (b >= nlist) return;
+    const int task = tlist ? tlist[b] : b;
+    double mx = 0.0;
+    for (int i = lane; i < n; i += 32) mx = fmax(mx, 1.0 - mdiag[(size_t)task * n + i]);
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) info[task].sexp = fix_sexp(mx);
+}
+
 // grid (ceil(n / 8), ntask), 256 threads: 8 columns per block
 __global__ void __launch_bounds__(256) k_fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, const int *status,
                                                      const double *mdiag, FixInfo *info)
@@ -142,8 +157,7 @@ __global__ void __launch_bounds__(256) k_fix_convert(int ntask, int n, double *A
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
     __syncthreads();
     for (int w = 0; w < 8; w++) mx = fmax(mx, red[w]);
-    int sexp = 0;
-    if (mx >= 2.0) sexp = min(2 * ((ilogb(mx) + 2) / 2), 400);
+    const int sexp = fix_sexp(mx);
     if (blockIdx.x == 0 && threadIdx.x == 0) info[task].sexp = sexp;
     const double sc = ldexp(1.0, FQ - sexp);
     for (int c = blockIdx.x * 8; c < min(n, (int)blockIdx.x * 8 + 8); c++) {
@@ -690,7 +704,7 @@ static FixWork fix_work(int ntask, void *work)
 }
 
 void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, double *logdet, void *work,
-                     cudaStream_t st)
+                     cudaStream_t st, bool fixed)
 {
     static bool attr = false;
     static int sms = 148;
@@ -706,8 +720,10 @@ void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, in
     const FixWork wk = fix_work(ntask, work);
     long long *S = reinterpret_cast<long long *>(A);
     // grid y is at most 65535: every caller's chunk is
-    k_fix_convert<<<dim3((n + 7) / 8, ntask), 256, 0, st>>>(ntask, n, A, lda, mstride, status, mdiag, wk.info);
-    COUNT_LAUNCH(1);
+    if (!fixed) {
+        k_fix_convert<<<dim3((n + 7) / 8, ntask), 256, 0, st>>>(ntask, n, A, lda, mstride, status, mdiag, wk.info);
+        COUNT_LAUNCH(1);
+    }
     for (int k0 = 0; k0 < n; k0 += NB) {
         k_fix_potf2<<<ntask, 256, POTF2_SMEM, st>>>(ntask, n, k0, S, lda, mstride, status, wk, logdet);
         COUNT_LAUNCH(1);
@@ -725,6 +741,14 @@ void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, in
         k_fix_syrk<<<dim3(items, ntask), SY_THREADS, SY_SMEM, st>>>(ntask, n, t0, chunk, S, lda, mstride, status, wk);
         COUNT_LAUNCH(1);
     }
+    CK(cudaGetLastError());
+}
+
+void launch_fix_scale(const int *tlist, int nlist, int n, const double *mdiag, void *work, cudaStream_t st)
+{
+    if (nlist <= 0) return;
+    k_fix_scale<<<(nlist + 3) / 4, 128, 0, st>>>(tlist, nlist, n, mdiag, (FixInfo *)work);
+    COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }
 

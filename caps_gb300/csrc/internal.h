@@ -79,7 +79,8 @@ void launch_elem(const Task *tasks, const int *tlist, int nlist, int ldim, const
                  double *A, size_t lda, size_t mat_stride, double *mdiag, int *status, cudaStream_t st, bool diag_only);
 // shortcut decision of the listed tasks; A == nullptr: the trace rule alone, undecided tasks keep status 0
 void launch_stats(const int *tlist, int nlist, int n, const double *A, size_t lda, size_t mat_stride, const double *mdiag, int mode,
-                  double *trace, double *result, int *status, cudaStream_t st);
+                  double *trace, double *result, int *status, cudaStream_t st, const double *fro = nullptr, int nfro = 0);
+// (fro: nfro sums of squares of M per task instead of the matrix; A is then only tested for nullptr)
 // mixed form: elements in float-float straight into the FP32 delta matrix (elem_ff.cu)
 size_t elem_ff_part_floats(int ldim);
 // float-float copies of the scale factors (Saf, Sbf: L ffe per task; uvf: L float4 per task)
@@ -115,7 +116,21 @@ void launch_stats_ff(const int *tlist, int nlist, int ldim, const double *diag, 
 // (n per task); logdet: ceil(n / 64) partial sums per task; work: cholesky_work_bytes
 size_t cholesky_work_bytes(int ntask, int n);
 void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, double *logdet,
-                     void *work, cudaStream_t st);
+                     void *work, cudaStream_t st, bool fixed = false);
+// fixed: the matrix is in fixed point already (units 2^(sexp - 60), launch_sweep64), its exponents
+// written by launch_fix_scale: two ints per task at the start of the workspace, sexp the first
+void launch_fix_scale(const int *tlist, int nlist, int n, const double *mdiag, void *work, cudaStream_t st);
+// FP64 form: M by the I recurrence from q-sum seeds (sweep64.cu).  launch_diag64: the band seeds
+// and M_ii; launch_sweep64: the rest of the seeds and 1 - M of the listed tasks in fixed point, P
+// CTAs per matrix (sweep64_parts); fro != nullptr: P sums of squares of M per task
+size_t seed64_bytes(int ldim, int ntask);
+size_t sweep64_work_bytes(int ldim, int nlist, int P);
+int sweep64_parts(int ldim, int nlist);
+void launch_diag64(const Task *tasks, int ntask, int ldim, const sd *K, int nu_stride, const double *lft, const double4 *ptab, int pstride,
+                   const sd *Sa, const sd *Sb, const double2 *uv, void *seed, double *mdiag, int *status, cudaStream_t st);
+void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, int P, const sd *K, int nu_stride, const double *lft,
+                    const double4 *ptab, int pstride, const sd *Sa, const sd *Sb, void *seed, const double *mdiag, const int *info,
+                    void *work, long long *A, size_t mstride, double *fro, int *status, cudaStream_t st);
 size_t mixed_work_bytes(int ntask, int n);
 // live CUDA-event timing of the tcgen05 trailing update (mixed.cu)
 void kernel_timer_enable(bool on);

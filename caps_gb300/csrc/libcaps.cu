@@ -105,7 +105,7 @@ struct Engine {
     cudaStream_t side = nullptr;          // Mie coefficients and scale factors, beside setup and K
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     double *d_lfac = nullptr;
-    DevBuf tasks, edges, coef, partM, partE, K, I, Sa, Sb, uv, A, logdiag, trace, result, status, mie_a, mie_b, xi, eps, lft, xtab, ptab, S32, ptabf, a12, gm, glmin, Saf, Sbf, uvf, part, diag, groups, B, diag2, mwork, a12t, coefF, tlist, groups2, glist2, KP, KPe, hwork, seed;
+    DevBuf tasks, edges, coef, partM, partE, K, I, Sa, Sb, uv, A, logdiag, trace, result, status, mie_a, mie_b, xi, eps, lft, xtab, ptab, S32, ptabf, a12, gm, glmin, Saf, Sbf, uvf, part, diag, groups, B, diag2, mwork, a12t, coefF, tlist, groups2, glist2, KP, KPe, hwork, seed, sw64, fro;
     std::vector<double> host_pinned_dummy;
     double timings[6] = {0, 0, 0, 0, 0, 0};
     double timings_cum[6] = {0, 0, 0, 0, 0, 0};
@@ -511,16 +511,18 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     // ... and, where the window fits its shared-memory ring, M comes from the I recurrence seeded
     // by 4 L q-sums per matrix (sweep.cu) instead of the q-sums of every pair
     const bool sweep = ff_elem && sweep_fits(ldim);
+    // the FP64 form's dense matrices by the same recurrence in FP64 (sweep64.cu), into fixed point
+    const bool sweep64 = !mixed && O.factor && !O.square && !O.M_out && !hodlr;
     // chunk size from free memory.  The budget counts the large work buffers held from earlier
     // batches as free for this one: true while batches keep one shape, each buffer serving the
     // same array again; when the shape (dimension, precision, path) changes they are released
     // first, since a buffer the new path does not use would stay held beside the new ones
     // (every batch ends synchronised with the device, so none is in use)
     const uint64_t shape = ((uint64_t)dim << 16) | (uint64_t)mixed | (uint64_t)hodlr << 1 | (uint64_t)sweep << 2 |
-                           (uint64_t)ff_elem << 3 | (uint64_t)O.square << 4 | (uint64_t)O.M_out << 5 | (uint64_t)O.factor << 6;
+                           (uint64_t)ff_elem << 3 | (uint64_t)O.square << 4 | (uint64_t)(O.M_out != nullptr) << 5 | (uint64_t)O.factor << 6 | (uint64_t)sweep64 << 7;
     if (g_eng.shape != shape) {
         for (DevBuf *b : {&g_eng.A, &g_eng.I, &g_eng.partM, &g_eng.partE, &g_eng.S32, &g_eng.a12, &g_eng.part, &g_eng.B,
-                          &g_eng.hwork, &g_eng.seed, &g_eng.mwork})
+                          &g_eng.hwork, &g_eng.seed, &g_eng.mwork, &g_eng.sw64})
             b->release();
         g_eng.shape = shape;
     }
@@ -529,6 +531,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     const size_t mat_bytes = O.square ? 16 : ff_elem ? 4 + 1 : (caps->precision == CAPS_PREC_MIXED ? 12 : 8);
     const size_t dense_bytes = hodlr ? hodlr_work_bytes(ldim, 1)
                              : sweep ? (size_t)dim * dim * 4 + seed_bytes(ldim, 1)
+                             : sweep64 ? (size_t)dim * dim * 8 + seed64_bytes(ldim, 1) + sweep64_work_bytes(ldim, 1, 1)
                                      : (size_t)dim * dim * mat_bytes + (size_t)2 * L * L * sizeof(sd)
                                            + (size_t)L * (L + 1) / 2 * 32; // a_0..a_2 table (one row per task)
     const size_t per_task = dense_bytes + (size_t)2 * nu_stride * sizeof(sd)
@@ -538,7 +541,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
                           + (hodlr ? 0 : mixed && !O.square ? mixed_work_bytes(1, dim) : cholesky_work_bytes(1, dim)); // diagonal-block inverses, panel images
     size_t budget = (size_t)(0.70 * (double)(freeb + g_eng.A.bytes + g_eng.I.bytes + g_eng.partM.bytes + g_eng.partE.bytes + g_eng.S32.bytes
                                              + g_eng.a12.bytes + g_eng.part.bytes + g_eng.B.bytes + g_eng.hwork.bytes
-                                             + g_eng.seed.bytes + g_eng.mwork.bytes));
+                                             + g_eng.seed.bytes + g_eng.mwork.bytes + g_eng.sw64.bytes));
     int chunk = (int)std::max<size_t>(1, std::min<size_t>(budget / per_task, 65535));
     chunk = std::min(chunk, n);
 
@@ -642,9 +645,9 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         CK(cudaEventRecord(g_eng.ev[2], st));
         CK(cudaStreamWaitEvent(st, g_eng.ev_join, 0)); // Mie and scale factors from here on
 
-        sd *d_I = (hodlr || sweep) ? nullptr : (sd *)g_eng.I.get((size_t)nt * 2 * L * L * sizeof(sd));
+        sd *d_I = (hodlr || sweep || sweep64) ? nullptr : (sd *)g_eng.I.get((size_t)nt * 2 * L * L * sizeof(sd));
         double4 *d_ptab = (double4 *)g_eng.ptab.get((size_t)nt * 2 * pstride * sizeof(double4));
-        void *d_a12 = (hodlr || sweep) ? nullptr : g_eng.a12.get(a12_bytes(ldim, ngroup));
+        void *d_a12 = (hodlr || sweep || sweep64) ? nullptr : g_eng.a12.get(a12_bytes(ldim, ngroup));
         // a_0..a_2 per m; the mixed form's trace rule first needs only the band of each m
         void *d_a12t = nullptr;
         if (caps->precision == CAPS_PREC_MIXED) {
@@ -652,7 +655,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             // on demand)
             d_a12t = g_eng.a12t.get(a12_tab_bytes(ldim, ngroup));
             launch_a12_mixed(d_gm, d_glm, ngroup, ldim, d_lft, d_a12, d_a12t, st, true, nullptr, (hodlr || ff_elem) ? 0 : -1);
-        } else if (!hodlr)
+        } else if (!hodlr && !sweep64)
             launch_a12(d_gm, d_glm, ngroup, ldim, d_lft, d_a12, st);
         const size_t lda = dim, mstride = (size_t)dim * dim;
         double *d_trace = (double *)g_eng.trace.get(nt * sizeof(double));
@@ -754,6 +757,16 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             CK(cudaEventRecord(g_eng.ev[4], st));
             undecided();
             CK(cudaEventRecord(g_eng.ev[5], st));
+        } else if (sweep64) {
+            // M_ii from the band of q-sums, the trace rule; the undecided matrices by the recurrence
+            launch_ptab(d_tasks, nt, d_ptab, pstride, st);
+            d_seed = g_eng.seed.get(seed64_bytes(ldim, nt));
+            launch_diag64(d_tasks, nt, ldim, d_K, nu_stride, d_lft, d_ptab, pstride, d_Sa, d_Sb, d_uv, d_seed, d_dg, d_status, st);
+            CK(cudaEventRecord(g_eng.ev[3], st));
+            launch_stats(nullptr, nt, dim, nullptr, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st);
+            CK(cudaEventRecord(g_eng.ev[4], st));
+            undecided();
+            CK(cudaEventRecord(g_eng.ev[5], st));
         } else {
             launch_ptab(d_tasks, nt, d_ptab, pstride, st);
             if (diag_first) {
@@ -784,6 +797,16 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             float *d_part = (float *)g_eng.part.get((size_t)nt * elem_ff_part_floats(ldim) * sizeof(float));
             launch_elem_ff(d_tasks, d_list, nlist, ldim, d_Saf, d_Sbf, d_uvf, d_I, d_S, mstride, d_dg, d_part, d_status, st);
             launch_stats_ff(d_list, nlist, ldim, d_dg, d_part, O.mode, d_trace, d_res, d_status, st);
+        } else if (sweep64) {
+            d_A = (double *)g_eng.A.get((size_t)nt * mstride * sizeof(double));
+            void *d_work = g_eng.mwork.get(cholesky_work_bytes(nt, dim));
+            const int P = sweep64_parts(ldim, nlist);
+            double *d_fro = O.mode == 0 ? (double *)g_eng.fro.get((size_t)nt * P * sizeof(double)) : nullptr;
+            launch_fix_scale(d_list, nlist, dim, d_dg, d_work, st);
+            launch_sweep64(d_tasks, d_list, nlist, ldim, P, d_K, nu_stride, d_lft, d_ptab, pstride, d_Sa, d_Sb, d_seed, d_dg,
+                           (const int *)d_work, g_eng.sw64.get(sweep64_work_bytes(ldim, nlist, P)), (long long *)d_A, mstride, d_fro,
+                           d_status, st);
+            launch_stats(d_list, nlist, dim, d_A, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st, d_fro, P);
         } else {
             d_A = (double *)g_eng.A.get((size_t)nt * mstride * sizeof(double));
             launch_elem(d_tasks, d_list, nlist, ldim, d_I, d_Sa, d_Sb, d_uv, d_A, lda, mstride, d_dg, d_status, st, false);
@@ -817,7 +840,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         } else if (O.factor) {
             double *d_ld = (double *)g_eng.logdiag.get((size_t)nt * dim * sizeof(double));
             void *d_work = g_eng.mwork.get(cholesky_work_bytes(nt, dim));
-            launch_cholesky(nt, dim, d_A, lda, mstride, d_status, d_dg, d_ld, d_work, st);
+            launch_cholesky(nt, dim, d_A, lda, mstride, d_status, d_dg, d_ld, d_work, st, sweep64);
             launch_final(nt, dim, d_ld, d_work, d_trace, d_status, d_res, O.mode, st);
         }
         CK(cudaEventRecord(g_eng.ev[8], st));
