@@ -668,7 +668,12 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
     const double *md = mdiag + (size_t)task * n;
     const CSum tr = csum_warp(md, n);
     if (lane == 0) { rs[warp] = tr.s; rc[warp] = tr.c; }
-    if (A && mode == 0 && !frop) {
+    if (mode == 0 && frop) {
+        double s = 0.0;
+        for (int i = threadIdx.x; i < nfro; i += ST_NT) s += frop[(size_t)task * nfro + i];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) red[warp] = s;
+    } else if (A && mode == 0) {
         // sum of squares of M: diagonal once, strict lower twice (M is symmetric)
         const double *Am = A + (size_t)task * mat_stride;
         double s = 0.0;
@@ -694,10 +699,7 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
     if (!A) return;
     if (mode == 0) {
         double fro2 = 0.0;
-        if (frop)
-            for (int w = 0; w < nfro; w++) fro2 += frop[(size_t)task * nfro + w];
-        else
-            for (int w = 0; w < ST_NT / 32; w++) fro2 += red[w];
+        for (int w = 0; w < ST_NT / 32; w++) fro2 += red[w];
         const double fro = sqrt(fro2);
         if (fro < 1) {
             const double merc = -t - fro2 / 2;

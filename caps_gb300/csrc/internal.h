@@ -121,14 +121,14 @@ void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, in
 // written by launch_fix_scale: two ints per task at the start of the workspace, sexp the first
 void launch_fix_scale(const int *tlist, int nlist, int n, const double *mdiag, void *work, cudaStream_t st);
 // FP64 form: M by the I recurrence from q-sum seeds (sweep64.cu).  launch_diag64: the band seeds
-// and M_ii; launch_sweep64: the rest of the seeds and 1 - M of the listed tasks in fixed point, P
-// CTAs per matrix (sweep64_parts); fro != nullptr: P sums of squares of M per task
+// and M_ii; launch_sweep64: the rest of the seeds and 1 - M of the listed tasks in fixed point;
+// fro != nullptr: sweep64_nfro sums of squares of M per task
 size_t seed64_bytes(int ldim, int ntask);
-size_t sweep64_work_bytes(int ldim, int nlist, int P);
-int sweep64_parts(int ldim, int nlist);
+size_t sweep64_work_bytes(int ldim, int nlist);
+int sweep64_nfro(int ldim);
 void launch_diag64(const Task *tasks, int ntask, int ldim, const sd *K, int nu_stride, const double *lft, const double4 *ptab, int pstride,
                    const sd *Sa, const sd *Sb, const double2 *uv, void *seed, double *mdiag, int *status, cudaStream_t st);
-void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, int P, const sd *K, int nu_stride, const double *lft,
+void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, const sd *K, int nu_stride, const double *lft,
                     const double4 *ptab, int pstride, const sd *Sa, const sd *Sb, void *seed, const double *mdiag, const int *info,
                     void *work, long long *A, size_t mstride, double *fro, int *status, cudaStream_t st);
 size_t mixed_work_bytes(int ntask, int n);

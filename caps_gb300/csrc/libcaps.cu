@@ -531,7 +531,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     const size_t mat_bytes = O.square ? 16 : ff_elem ? 4 + 1 : (caps->precision == CAPS_PREC_MIXED ? 12 : 8);
     const size_t dense_bytes = hodlr ? hodlr_work_bytes(ldim, 1)
                              : sweep ? (size_t)dim * dim * 4 + seed_bytes(ldim, 1)
-                             : sweep64 ? (size_t)dim * dim * 8 + seed64_bytes(ldim, 1) + sweep64_work_bytes(ldim, 1, 1)
+                             : sweep64 ? (size_t)dim * dim * 8 + seed64_bytes(ldim, 1) + sweep64_work_bytes(ldim, 1)
                                      : (size_t)dim * dim * mat_bytes + (size_t)2 * L * L * sizeof(sd)
                                            + (size_t)L * (L + 1) / 2 * 32; // a_0..a_2 table (one row per task)
     const size_t per_task = dense_bytes + (size_t)2 * nu_stride * sizeof(sd)
@@ -800,13 +800,13 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         } else if (sweep64) {
             d_A = (double *)g_eng.A.get((size_t)nt * mstride * sizeof(double));
             void *d_work = g_eng.mwork.get(cholesky_work_bytes(nt, dim));
-            const int P = sweep64_parts(ldim, nlist);
-            double *d_fro = O.mode == 0 ? (double *)g_eng.fro.get((size_t)nt * P * sizeof(double)) : nullptr;
+            const int nfro = sweep64_nfro(ldim);
+            double *d_fro = O.mode == 0 ? (double *)g_eng.fro.get((size_t)nt * nfro * sizeof(double)) : nullptr;
             launch_fix_scale(d_list, nlist, dim, d_dg, d_work, st);
-            launch_sweep64(d_tasks, d_list, nlist, ldim, P, d_K, nu_stride, d_lft, d_ptab, pstride, d_Sa, d_Sb, d_seed, d_dg,
-                           (const int *)d_work, g_eng.sw64.get(sweep64_work_bytes(ldim, nlist, P)), (long long *)d_A, mstride, d_fro,
+            launch_sweep64(d_tasks, d_list, nlist, ldim, d_K, nu_stride, d_lft, d_ptab, pstride, d_Sa, d_Sb, d_seed, d_dg,
+                           (const int *)d_work, g_eng.sw64.get(sweep64_work_bytes(ldim, nlist)), (long long *)d_A, mstride, d_fro,
                            d_status, st);
-            launch_stats(d_list, nlist, dim, d_A, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st, d_fro, P);
+            launch_stats(d_list, nlist, dim, d_A, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st, d_fro, nfro);
         } else {
             d_A = (double *)g_eng.A.get((size_t)nt * mstride * sizeof(double));
             launch_elem(d_tasks, d_list, nlist, ldim, d_I, d_Sa, d_Sb, d_uv, d_A, lda, mstride, d_dg, d_status, st, false);

@@ -8,14 +8,14 @@
 // moving away from the diagonal; against q-sums of every pair log det changes by 1e-13 relative
 // at most (tests/test_gpu_sweep64.py), the size of the q-sums' own rounding.
 //
-// One CTA takes a range of rows of one matrix.  Where a batch has fewer matrices than the
-// chip has SMs, the rows are split over P CTAs of about equal numbers of pairs; each but the first
-// starts from the q-sums of two whole rows (ldim more q-sums per CTA).
-//
-// What bounds it: the FP64 pipe, two operations per clock and SM.  The row factors dA, dB of
-// the elements are folded into the coefficients of their row (J' = dA J costs what J does) and
-// the column factors into tables, so that a pair takes 8 operations in the recurrence and 20 in
-// its four elements; conversion to fixed point is integer work.
+// Two kernels, both bound by the FP64 pipe (two operations per clock and SM).  k_rec64 fills the
+// table T row by row, 4 operations per entry and polarisation, one CTA per matrix and range of
+// rows: a range but the first starts from the q-sums of two whole rows, and the number of ranges
+// depends on ldim alone, so that a matrix has the same value in every batch.  k_elem64 forms
+// the elements of all pairs at once: the row factors dA, dB are folded into the coefficients of
+// their row (J' = dA J costs what J does) and the column factors into tables, 20 operations for
+// the four elements of a pair; conversion to fixed point is integer work.  For a perfectly
+// reflecting plate T_TE = -T_TM, and only T_TM is formed.
 #include "common.cuh"
 #include "internal.h"
 #include "qsum64.cuh"
@@ -30,20 +30,18 @@ CAPS_DEV int col64(const Task &T)
     return T.lmin - 1 >= mm ? 0 : 1;
 }
 
-// first element row (1 .. ldim) of part q of P: equal numbers of pairs
-__host__ __device__ inline int sweep64_row(int q, int P, int ldim)
-{
-    if (q <= 0) return 1;
-    if (q >= P) return ldim + 1;
-    const int x = 1 + (int)(ldim * sqrt((double)q / P));
-    return x < 5 ? 5 : x;
-}
+// ranges of rows of T: part q of P forms rows (row(q), row(q + 1)], row(0) = -1, of about equal
+// numbers of pairs; parts q >= 1 start from the q-sums of rows row(q) - 1 and row(q)
+__host__ __device__ inline int rec64_row(int q, int P, int L) { return q <= 0 ? -1 : q >= P ? L - 1 : (int)(L * sqrt((double)q / P)); }
+// A part of 512 rows takes 0.25 ms at row 512 and 1 ms at row 2048 of a matrix; its two rows of
+// q-sums cost about as much as 100 rows
+__host__ __device__ inline int rec64_parts(int ldim) { return ldim < 1024 ? 1 : ldim / 512; }
 
 // ---------------------------------------------------------------------------
 // seeds
 // ---------------------------------------------------------------------------
 // seed[((task * 2 + pol) * SEED_KINDS + kind) * L + w]: the pair (w, w), (w+1, w), (w+2, w) or (w, c);
-// rows[(((b * (P - 1) + q - 1) * 2 + i) * 2 + pol) * L + y]: T rows x_q - 1 + i of listed task b, y <= row
+// rows[(((b * (P - 1) + q - 1) * 2 + i) * 2 + pol) * L + y]: row(q) - 1 + i of listed task b, y <= row
 // grid (ceil(L / 128) * (2 + 2 (P - 1)), nlist), one pair per thread; kind0 and kind1 first
 __global__ void __launch_bounds__(128) k_seed64(const Task *tasks, const int *tlist, int nlist, int ldim, int P, int kind0, int kind1,
                                                 const sd *__restrict__ K, int nu_stride, const double *__restrict__ lft,
@@ -66,7 +64,7 @@ __global__ void __launch_bounds__(128) k_seed64(const Task *tasks, const int *tl
         oE = seed + ((size_t)(task * 2 + 0) * SEED_KINDS + kind) * L + w;
     } else {
         const int q = (part - 2) / 2 + 1, i = (part - 2) & 1;
-        a1 = sweep64_row(q, P, ldim) - 1 + i;
+        a1 = rec64_row(q, P, L) - 1 + i;
         const size_t o = ((((size_t)blockIdx.y * (P - 1) + q - 1) * 2 + i) * 2) * L + w;
         oT = rows + o + L;
         oE = rows + o;
@@ -165,10 +163,84 @@ __global__ void __launch_bounds__(256) k_sweep64_tab(const Task *tasks, const in
 }
 
 // ---------------------------------------------------------------------------
-// the sweep
+// the table
 // ---------------------------------------------------------------------------
-constexpr int S64_NT = 256, S64_NW = S64_NT / 32, S64_CH = 30, S64_RING = 4;
+// T(r, y), y <= r, of listed task b at tt[((b * 2 + pol) * L + y) * L + r] (column y of the triangle
+// contiguous, the order in which k_elem64 reads it)
+constexpr int R64_NT = 256, R64_RING = 4;
 
+// grid nlist * P.  The ring of four rows (TE then TM, L + 2 values each) is in shared memory, or
+// in global memory (ring != nullptr) where it does not fit; one barrier per row.
+__global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *tlist, int nlist, int ldim, int P,
+                                                  const sd *__restrict__ seed, const sd *__restrict__ rows, const double *__restrict__ tab,
+                                                  const int *__restrict__ ktab, double *tt, const int *status, double *ring)
+{
+    extern __shared__ __align__(16) double r64_sm[];
+    const int L = ldim + 2, LP = L + 2;
+    const int b = blockIdx.x / P, q = P - 1 - (int)blockIdx.x % P;
+    if (b >= nlist) return;
+    const int task = tlist ? tlist[b] : b;
+    if (status[task] & ~0xF) return; // no status changes in this launch: uniform
+    const Task &T = tasks[task];
+    const int c = col64(T), r1 = rec64_row(q + 1, P, L);
+    const bool te = !T.is_pr;
+    double *R = ring ? ring + (size_t)blockIdx.x * R64_RING * 2 * LP : r64_sm;
+    auto rowp = [&](int r) { return R + (size_t)((r & 3) * 2) * LP; };
+    const double *W = tab + (size_t)b * W_FIELDS * L;
+    auto F = [&](int f, int w) { return __ldg(W + (size_t)f * L + w); };
+    const int *kt = ktab + (size_t)b * L;
+    auto sp = [&](int pol, int kind) { return seed + ((size_t)(task * 2 + pol) * SEED_KINDS + kind) * L; };
+    double *tE = tt + (size_t)b * 2 * L * L, *tT = tE + (size_t)L * L;
+    const int tid = threadIdx.x;
+    int r = 0;
+    if (q > 0) { // the two rows before the range, from their q-sums
+        r = rec64_row(q, P, L) + 1;
+        for (int i = 0; i < 2; i++) {
+            const int rr = r - 2 + i;
+            const sd *src = rows + ((((size_t)b * (P - 1) + q - 1) * 2 + i) * 2) * L;
+            double *D = rowp(rr);
+            for (int y = tid; y <= rr; y += R64_NT) {
+                const int k = kt[rr] + kt[y];
+                const double vE = y < c ? 0.0 : sd_scaled(src[y], k), vT = y < c ? 0.0 : sd_scaled(src[L + y], k);
+                D[y] = vE;
+                D[LP + y] = vT;
+            }
+        }
+        __syncthreads();
+    }
+    for (; r <= r1; r++) {
+        double *D = rowp(r);
+        // rows before the first are never read: y >= c + 1 and y <= r - 2 need r >= 3
+        const double *P1 = rowp(r + 3), *P2 = rowp(r + 2); // rows r - 1, r - 2
+        const double R1 = F(W_R1, r), R2 = F(W_R2, r);
+        for (int y = tid; y <= r; y += R64_NT) {
+            double vE = 0.0, vT = 0.0;
+            if (y >= c) {
+                if (y == r || y == r - 1 || y == c) {
+                    const int kind = y == r ? SEED_D0 : (y == r - 1 ? SEED_D1 : SEED_COL), wi = kind == SEED_COL ? r : y;
+                    const int k = kt[r] + kt[y];
+                    vE = sd_scaled(sp(0, kind)[wi], k);
+                    vT = sd_scaled(sp(1, kind)[wi], k);
+                } else {
+                    const double Cp = F(W_CP, y), Cm = F(W_CM, y);
+                    vT = fma(R1, fma(Cp, P1[LP + y + 1], Cm * P1[LP + y - 1]), R2 * P2[LP + y]);
+                    if (te) vE = fma(R1, fma(Cp, P1[y + 1], Cm * P1[y - 1]), R2 * P2[y]);
+                }
+            }
+            D[LP + y] = vT;
+            tT[(size_t)y * L + r] = vT;
+            if (te) {
+                D[y] = vE;
+                tE[(size_t)y * L + r] = vE;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// elements
+// ---------------------------------------------------------------------------
 // v in units of 2^-q, rounded, saturated at +-2^62 (integer work only)
 CAPS_DEV long long to_fix(double v, int q, bool &bad)
 {
@@ -183,172 +255,110 @@ CAPS_DEV long long to_fix(double v, int q, bool &bad)
     return b < 0 ? -mnt : mnt;
 }
 
-// grid nlist * P.  The ring of four rows (TE then TM, L + 2 values each) is in shared memory, or
-// in global memory (ring != nullptr) where it does not fit.  Row r of T, a barrier, the elements
-// of row r - 1: 30 columns per pass of 32 lanes, J of the neighbours by shuffles.
+// grid (ceil(ldim / E64_X), ceil(ldim / E64_Y), nlist), E64_X threads: thread x (window index 1 ..
+// ldim, a row of 2x2 blocks) walks E64_Y columns y <= x with T and J of the columns y - 1, y, y + 1 in
+// registers; consecutive threads write consecutive rows of the column-major matrix.
+constexpr int E64_X = 64, E64_Y = 16;
 template <bool FRO>
-__global__ void __launch_bounds__(S64_NT) k_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, int P,
-                                                    const sd *__restrict__ seed, const sd *__restrict__ rows, const double *__restrict__ tab,
-                                                    const int *__restrict__ ktab, const double *__restrict__ mdiag, const int *info,
-                                                    long long *A, size_t mstride, double *fro_out, int *status, double *ring)
+__global__ void __launch_bounds__(E64_X) k_elem64(const Task *tasks, const int *tlist, int nlist, int ldim, const double *__restrict__ tt,
+                                                  const double *__restrict__ tab, const double *__restrict__ mdiag, const int *info,
+                                                  long long *A, size_t mstride, double *fro_out, int *status)
 {
-    extern __shared__ __align__(16) double s64_sm[];
-    const int L = ldim + 2, n = 2 * ldim, LP = L + 2;
-    const int b = blockIdx.x / P, q = P - 1 - (int)blockIdx.x % P;
+    const int L = ldim + 2, n = 2 * ldim;
+    const int b = blockIdx.z;
     if (b >= nlist) return;
     const int task = tlist ? tlist[b] : b;
-    __shared__ int s_st;
-    if (threadIdx.x == 0) s_st = status[task];
-    __syncthreads();
-    if (s_st & ~0xF) return;
-    const Task &T = tasks[task];
-    const int mt = T.m, c = col64(T);
-    const int x0 = sweep64_row(q, P, ldim), x1 = sweep64_row(q + 1, P, ldim);
-    double *R = ring ? ring + (size_t)blockIdx.x * S64_RING * 2 * LP : s64_sm;
-    auto rowp = [&](int r) { return R + (size_t)((r & 3) * 2) * LP; };
-    const double *W = tab + (size_t)b * W_FIELDS * L;
-    auto F = [&](int f, int w) { return __ldg(W + (size_t)f * L + w); };
-    const int *kt = ktab + (size_t)b * L;
-    auto sp = [&](int pol, int kind) { return seed + ((size_t)(task * 2 + pol) * SEED_KINDS + kind) * L; };
-    const int fq = 60 - info[2 * task];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    long long *Am = A + (size_t)task * mstride;
-    const double *md = mdiag + (size_t)task * n;
-    bool bad = false;
+    const int x = blockIdx.x * E64_X + threadIdx.x + 1, y0 = blockIdx.y * E64_Y + 1;
     double fro = 0.0;
-    int r = 0;
-    if (q > 0) { // rows x0 - 1 and x0 from their q-sums
-        for (int i = 0; i < 2; i++) {
-            const int rr = x0 - 1 + i;
-            const sd *src = rows + ((((size_t)b * (P - 1) + q - 1) * 2 + i) * 2) * L;
-            double *D = rowp(rr), *D1 = rowp(rr - 1);
-            for (int y = tid; y <= rr; y += S64_NT) {
-                const int k = kt[rr] + kt[y];
-                const double vE = y < c ? 0.0 : sd_scaled(src[y], k), vT = y < c ? 0.0 : sd_scaled(src[L + y], k);
-                D[y] = vE;
-                D[LP + y] = vT;
-                if (i == 1 && y == rr - 1) { D1[rr] = vE; D1[LP + rr] = vT; }
-            }
-        }
-        r = x0 + 1;
-        __syncthreads();
-    }
-    for (; r <= x1 && r < L; r++) {
-        double *D = rowp(r);
-        // rows before the first are never read: y >= c + 1 and y <= r - 2 need r >= 3
-        double *P1 = rowp(r + 3), *P2 = rowp(r + 2); // rows r - 1, r - 2
-        const double R1 = F(W_R1, r), R2 = F(W_R2, r);
-        for (int y = tid; y <= r; y += S64_NT) {
-            double vE = 0.0, vT = 0.0;
-            if (y >= c) {
-                if (y == r || y == r - 1 || y == c) {
-                    const int kind = y == r ? SEED_D0 : (y == r - 1 ? SEED_D1 : SEED_COL), wi = kind == SEED_COL ? r : y;
-                    const int k = kt[r] + kt[y];
-                    vE = sd_scaled(sp(0, kind)[wi], k);
-                    vT = sd_scaled(sp(1, kind)[wi], k);
-                } else {
-                    const double Cp = F(W_CP, y), Cm = F(W_CM, y);
-                    vE = fma(R1, fma(Cp, P1[y + 1], Cm * P1[y - 1]), R2 * P2[y]);
-                    vT = fma(R1, fma(Cp, P1[LP + y + 1], Cm * P1[LP + y - 1]), R2 * P2[LP + y]);
+    if (y0 <= min((int)(blockIdx.x + 1) * E64_X, ldim)) { // uniform: some thread of the block has y0 <= x
+        bool bad = false;
+        if (x <= ldim && y0 <= x) {
+            const Task &T = tasks[task];
+            const int mt = T.m;
+            const bool pr = T.is_pr;
+            const double *W = tab + (size_t)b * W_FIELDS * L;
+            auto F = [&](int f, int w) { return __ldg(W + (size_t)f * L + w); };
+            const double *tE = tt + (size_t)b * 2 * L * L, *tT = tE + (size_t)L * L;
+            // T(u, v) for any order of u and v
+            auto TV = [&](const double *t, int u, int v) { return u >= v ? t[(size_t)v * L + u] : t[(size_t)u * L + v]; };
+            const int fq = 60 - info[2 * task];
+            const double dA = F(W_DA, x), dB = F(W_DB, x), mA = F(W_A, x), mB = F(W_B, x);
+            const double UxA = F(W_UA, x), VxA = F(W_VA, x), UxB = F(W_UB, x), VxB = F(W_VB, x);
+            // of column v: T_TM, T_TE at x, and J'_TM = dA(x) J_TM, J'_TE = dB(x) J_TE with
+            // J(x, v) = Um(x) T(x-1, v) - Vp(x) T(x+1, v)
+            struct Col { double T, E, JT, JE; };
+            auto col = [&](int v) {
+                Col q{TV(tT, x, v), 0.0, 0.0, 0.0};
+                q.E = pr ? -q.T : TV(tE, x, v);
+                if (mt > 0) {
+                    const double a = TV(tT, x - 1, v), d = TV(tT, x + 1, v);
+                    q.JT = fma(UxA, a, VxA * d);
+                    q.JE = pr ? -fma(UxB, a, VxB * d) : fma(UxB, TV(tE, x - 1, v), VxB * TV(tE, x + 1, v));
                 }
-            }
-            D[y] = vE;
-            D[LP + y] = vT;
-            // T(r, r-1) and T(r, r-2) past the diagonals of rows r-1 and r-2
-            if (y == r - 1) { P1[r] = vE; P1[LP + r] = vT; }
-            if (y == r - 2) { P2[r] = vE; P2[LP + r] = vT; }
-        }
-        __syncthreads();
-        const int x = r - 1;
-        if (x < x0) continue; // uniform
-        const double *Rm = rowp(x + 3), *R0 = rowp(x), *Rp = rowp(x + 1);
-        const double dA = F(W_DA, x), dB = F(W_DB, x), mA = F(W_A, x), mB = F(W_B, x);
-        const double UxA = F(W_UA, x), VxA = F(W_VA, x), UxB = F(W_UB, x), VxB = F(W_VB, x);
-        const int r0 = 2 * (x - 1);
-        for (int k = warp; k * S64_CH <= x; k += S64_NW) {
-            const int y = k * S64_CH - 1 + lane;
-            // J'_TM = dA(x) J_TM, J'_TE = dB(x) J_TE with J(x, y) = Um(x) T(x-1, y) - Vp(x) T(x+1, y)
-            double JT = 0.0, JE = 0.0;
-            if (mt > 0 && y >= 0 && y <= x + 1) {
-                JT = fma(UxA, Rm[LP + y], VxA * Rp[LP + y]);
-                JE = fma(UxB, Rm[y], VxB * Rp[y]);
-            }
-            const double JTm = __shfl_up_sync(0xffffffffu, JT, 1), JTp = __shfl_down_sync(0xffffffffu, JT, 1);
-            const double JEm = __shfl_up_sync(0xffffffffu, JE, 1), JEp = __shfl_down_sync(0xffffffffu, JE, 1);
-            if (lane == 0 || lane == 31 || y < 1 || y > x) continue;
-            const double tT = R0[LP + y], tE = R0[y];
-            double ee, mm, em = 0.0, me = 0.0;
-            if (mt == 0) {
-                ee = dA * F(W_DA, y) * tT;
-                mm = -(dB * F(W_DB, y) * tE);
-            } else {
-                // EE = dA dA [B_TM - m^2 T_TE], MM = dB dB [m^2 T_TM - B_TE], B(x, y) = Um(y) J(x, y-1) - Vp(y) J(x, y+1)
-                const double yUA = F(W_UA, y), yVA = F(W_VA, y), yA = F(W_A, y), yUB = F(W_UB, y), yVB = F(W_VB, y), yB = F(W_B, y);
-                const double hE = fma(yUB, R0[y - 1], yVB * R0[y + 1]), hT = fma(yUA, R0[LP + y - 1], yVA * R0[LP + y + 1]);
-                ee = fma(yUA, JTm, fma(yVA, JTp, -(mA * (yA * tE))));
-                mm = fma(mB, yB * tT, -fma(yUB, JEm, yVB * JEp));
-                em = fma(mA, hE, -(yB * JT)); // m dA(x) dB(y) [H_TE - J_TM]
-                me = fma(-mB, hT, yA * JE);   // m dB(x) dA(y) [J_TE - H_TM]
-            }
-            const int c0 = 2 * (y - 1);
-            long long *col = Am + (size_t)c0 * n + r0;
-            if (y != x) {
-                *reinterpret_cast<longlong2 *>(col) = make_longlong2(-to_fix(ee, fq, bad), -to_fix(me, fq, bad));
-                *reinterpret_cast<longlong2 *>(col + n) = make_longlong2(-to_fix(em, fq, bad), -to_fix(mm, fq, bad));
-                if (FRO) fro += 2.0 * (fma(ee, ee, me * me) + fma(mm, mm, em * em));
-            } else {
-                // the diagonal from M_ii, which the trace is taken from too
-                const double dee = md[r0], dmm = md[r0 + 1];
-                const long long one = 1LL << fq;
-                *reinterpret_cast<longlong2 *>(col) = make_longlong2(one - to_fix(dee, fq, bad), -to_fix(me, fq, bad));
-                col[n + 1] = one - to_fix(dmm, fq, bad);
-                if (FRO) fro += fma(dee, dee, dmm * dmm) + 2.0 * me * me;
+                return q;
+            };
+            const int y1 = min(min(y0 + E64_Y - 1, ldim), x);
+            Col cm = col(y0 - 1), c0 = col(y0);
+            long long *Am = A + (size_t)task * mstride + (size_t)2 * (y0 - 1) * n + 2 * (x - 1);
+            for (int y = y0; y <= y1; y++, Am += 2 * (size_t)n) {
+                const Col cp = col(y + 1);
+                double ee, mm, em = 0.0, me = 0.0;
+                if (mt == 0) {
+                    ee = dA * F(W_DA, y) * c0.T;
+                    mm = -(dB * F(W_DB, y) * c0.E);
+                } else {
+                    // EE = dA dA [B_TM - m^2 T_TE], MM = dB dB [m^2 T_TM - B_TE], B(x, y) = Um(y) J(x, y-1) - Vp(y) J(x, y+1)
+                    const double yUA = F(W_UA, y), yVA = F(W_VA, y), yA = F(W_A, y), yUB = F(W_UB, y), yVB = F(W_VB, y), yB = F(W_B, y);
+                    ee = fma(yUA, cm.JT, fma(yVA, cp.JT, -(mA * (yA * c0.E))));
+                    mm = fma(mB, yB * c0.T, -fma(yUB, cm.JE, yVB * cp.JE));
+                    // em = m dA(x) dB(y) [H_TE - J_TM], me = m dB(x) dA(y) [J_TE - H_TM], H(x, y) = Um(y) T(x, y-1) - Vp(y) T(x, y+1)
+                    em = fma(mA, fma(yUB, cm.E, yVB * cp.E), -(yB * c0.JT));
+                    me = fma(-mB, fma(yUA, cm.T, yVA * cp.T), yA * c0.JE);
+                }
+                if (y != x) {
+                    *reinterpret_cast<longlong2 *>(Am) = make_longlong2(-to_fix(ee, fq, bad), -to_fix(me, fq, bad));
+                    *reinterpret_cast<longlong2 *>(Am + n) = make_longlong2(-to_fix(em, fq, bad), -to_fix(mm, fq, bad));
+                    if (FRO) fro += 2.0 * (fma(ee, ee, me * me) + fma(mm, mm, em * em));
+                } else {
+                    // the diagonal from M_ii, which the trace is taken from too
+                    const double dee = mdiag[(size_t)task * n + 2 * (x - 1)], dmm = mdiag[(size_t)task * n + 2 * (x - 1) + 1];
+                    const long long one = 1LL << fq;
+                    *reinterpret_cast<longlong2 *>(Am) = make_longlong2(one - to_fix(dee, fq, bad), -to_fix(me, fq, bad));
+                    Am[n + 1] = one - to_fix(dmm, fq, bad);
+                    if (FRO) fro += fma(dee, dee, dmm * dmm) + 2.0 * me * me;
+                }
+                cm = c0;
+                c0 = cp;
             }
         }
+        if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status + task, ST_ERR_NONFINITE);
     }
-    if (FRO) { // per-CTA sums, added by the statistics kernel in order
-        __shared__ double red[S64_NW];
+    if (FRO) { // per-block sums, added by the statistics kernel in order
+        __shared__ double red[E64_X / 32];
         for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
-        if (lane == 0) red[warp] = fro;
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = fro;
         __syncthreads();
-        if (tid == 0) {
-            double s = 0.0;
-            for (int w = 0; w < S64_NW; w++) s += red[w];
-            fro_out[(size_t)task * P + q] = s;
-        }
+        if (threadIdx.x == 0) fro_out[((size_t)task * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = red[0] + red[1];
     }
-    if (__syncthreads_or(bad) && tid == 0) atomicOr(status + task, ST_ERR_NONFINITE);
 }
 
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-static size_t s64_ring_bytes(int ldim) { return (size_t)S64_RING * 2 * (ldim + 4) * sizeof(double); }
-static bool s64_ring_fits(int ldim) { return s64_ring_bytes(ldim) <= 220 * 1024; }
+static size_t r64_ring_bytes(int ldim) { return (size_t)R64_RING * 2 * (ldim + 4) * sizeof(double); }
+static bool r64_ring_fits(int ldim) { return r64_ring_bytes(ldim) <= 220 * 1024; }
 
 size_t seed64_bytes(int ldim, int ntask) { return (size_t)ntask * 2 * SEED_KINDS * (ldim + 2) * sizeof(sd); }
 
-size_t sweep64_work_bytes(int ldim, int nlist, int P)
-{
-    const size_t L = ldim + 2;
-    size_t b = (size_t)nlist * (P - 1) * 4 * L * sizeof(sd) + (size_t)nlist * L * (W_FIELDS * sizeof(double) + sizeof(int)) + 512;
-    if (!s64_ring_fits(ldim)) b += (size_t)nlist * P * s64_ring_bytes(ldim);
-    return b;
-}
+int sweep64_nfro(int ldim) { return ((ldim + E64_X - 1) / E64_X) * ((ldim + E64_Y - 1) / E64_Y); }
 
-// CTAs per matrix: about one per SM in all, at least 16 rows per part and at most 16 parts (each
-// starts from the q-sums of two rows).  One matrix of ldim 140: 2 parts 0.36 ms for seeds and
-// sweep, 8 parts 0.15, the q-sums and elements of every pair 0.15; 32 matrices of ldim 350: 4 parts
-// 0.6, every pair 2.3 ms
-int sweep64_parts(int ldim, int nlist)
+// T, the column tables, rows of q-sums, k, the ring
+size_t sweep64_work_bytes(int ldim, int nlist)
 {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    }
-    return max(1, min(min(16, ldim / 16), sms / max(nlist, 1)));
+    const size_t L = ldim + 2, P = rec64_parts(ldim);
+    size_t b = (size_t)nlist * L * (2 * L * sizeof(double) + W_FIELDS * sizeof(double) + (P - 1) * 4 * sizeof(sd) + sizeof(int)) + 512;
+    if (!r64_ring_fits(ldim)) b += (size_t)nlist * P * r64_ring_bytes(ldim);
+    return b;
 }
 
 static void seed64(const Task *tasks, const int *tlist, int nlist, int ldim, int P, int k0, int k1, const sd *K, int nu_stride,
@@ -369,34 +379,32 @@ void launch_diag64(const Task *tasks, int ntask, int ldim, const sd *K, int nu_s
     CK(cudaGetLastError());
 }
 
-void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, int P, const sd *K, int nu_stride, const double *lft,
+void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, const sd *K, int nu_stride, const double *lft,
                     const double4 *ptab, int pstride, const sd *Sa, const sd *Sb, void *seed, const double *mdiag, const int *info,
                     void *work, long long *A, size_t mstride, double *fro, int *status, cudaStream_t st)
 {
     if (nlist <= 0) return;
     const size_t L = ldim + 2;
-    double *tab = (double *)work; // 16-byte multiples: W_FIELDS is even
+    const int P = rec64_parts(ldim);
+    double *tt = (double *)work, *tab = tt + (size_t)nlist * 2 * L * L; // 16-byte multiples: W_FIELDS is even
     sd *rows = (sd *)(tab + nlist * W_FIELDS * L);
     int *kt = (int *)(rows + (size_t)nlist * (P - 1) * 4 * L);
     const size_t ring_off = ((char *)(kt + nlist * L) - (char *)work + 255) & ~(size_t)255;
-    const bool fits = s64_ring_fits(ldim);
+    const bool fits = r64_ring_fits(ldim);
     double *ring = fits ? nullptr : (double *)((char *)work + ring_off);
-    const size_t sm = fits ? s64_ring_bytes(ldim) : 0;
+    const size_t sm = fits ? r64_ring_bytes(ldim) : 0;
     static size_t attr = 0;
     if (sm > attr) {
-        CK(cudaFuncSetAttribute(k_sweep64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        CK(cudaFuncSetAttribute(k_sweep64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        CK(cudaFuncSetAttribute(k_rec64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         attr = sm;
     }
     seed64(tasks, tlist, nlist, ldim, P, SEED_D1, SEED_COL, K, nu_stride, lft, ptab, pstride, seed, rows, status, st);
     k_sweep64_tab<<<nlist, 256, 0, st>>>(tasks, tlist, nlist, ldim, (const sd *)seed, Sa, Sb, tab, kt);
-    if (fro)
-        k_sweep64<true><<<nlist * P, S64_NT, sm, st>>>(tasks, tlist, nlist, ldim, P, (const sd *)seed, rows, tab, kt, mdiag, info, A,
-                                                       mstride, fro, status, ring);
-    else
-        k_sweep64<false><<<nlist * P, S64_NT, sm, st>>>(tasks, tlist, nlist, ldim, P, (const sd *)seed, rows, tab, kt, mdiag, info, A,
-                                                        mstride, fro, status, ring);
-    COUNT_LAUNCH(2);
+    k_rec64<<<nlist * P, R64_NT, sm, st>>>(tasks, tlist, nlist, ldim, P, (const sd *)seed, rows, tab, kt, tt, status, ring);
+    const dim3 g((ldim + E64_X - 1) / E64_X, (ldim + E64_Y - 1) / E64_Y, nlist);
+    if (fro) k_elem64<true><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, mdiag, info, A, mstride, fro, status);
+    else k_elem64<false><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, mdiag, info, A, mstride, fro, status);
+    COUNT_LAUNCH(3);
     CK(cudaGetLastError());
 }
 
