@@ -502,9 +502,15 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     // HODLR semantics: the HODLR path (elements on demand) where it applies; the FP64 form
     // takes it from CAPS_HODLR_AUTO_DIM on, the mixed form from CAPS_HODLR_AUTO_DIM_MIXED on
     const bool mixed = caps->precision == CAPS_PREC_MIXED;
+    auto auto_hodlr = [&]() {
+        if (mixed) return dim >= CAPS_HODLR_AUTO_DIM_MIXED;
+        if (dim < CAPS_HODLR_LOW_MEM_DIM || dim >= CAPS_HODLR_AUTO_DIM) return dim >= CAPS_HODLR_AUTO_DIM;
+        size_t f = 0, t = 0;
+        CK(cudaMemGetInfo(&f, &t));
+        return (size_t)dim * dim * 8 + cholesky_work_bytes(1, dim) > (f + g_eng.A.bytes + g_eng.hwork.bytes) / 2;
+    };
     const bool hodlr = O.factor && !O.square && !O.M_out && !O.force_dense && caps->detalg == DETALG_HODLR &&
-                       (caps->path == CAPS_PATH_HODLR ||
-                        (caps->path == CAPS_PATH_AUTO && dim >= (mixed ? CAPS_HODLR_AUTO_DIM_MIXED : CAPS_HODLR_AUTO_DIM)));
+                       (caps->path == CAPS_PATH_HODLR || (caps->path == CAPS_PATH_AUTO && auto_hodlr()));
     // mixed precision without a dense-M request: elements go straight into the FP32 delta
     // matrix (no FP64 matrix)
     const bool ff_elem = mixed && O.factor && !O.M_out && !O.square && !hodlr;

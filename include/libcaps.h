@@ -188,21 +188,24 @@ void caps_integrate_plasma_free(integration_plasma_t *self);                    
 int caps_logdetD_batch(caps_t *self, const double *xi_, const int *m, int n, double *out, int *status);
 
 /* precision of the factorisation */
-#define CAPS_PREC_FP64  0  /* plain FP64 Cholesky */
+#define CAPS_PREC_FP64  0  /* FP64 elements, Cholesky in 64-bit fixed point */
 #define CAPS_PREC_MIXED 1  /* tensor-core factorisation + FP64 log-det correction */
 int caps_gpu_set_precision(caps_t *self, int precision);
 
 /* determinant path of an FP64 caps object with DETALG_HODLR (the default): a HODLR
  * factorisation with the elements evaluated on demand (src/libhodlr, matrix.c:125-147) or the
  * dense batched Cholesky with the same result rules.  Automatic: HODLR from dimension
- * CAPS_HODLR_AUTO_DIM on (where sampling the off-diagonal blocks needs fewer q-sums than the
- * dense I table).  The mixed form takes HODLR only when asked (CAPS_PATH_HODLR or the
+ * CAPS_HODLR_AUTO_DIM on, and from CAPS_HODLR_LOW_MEM_DIM on where half the free device memory
+ * does not hold one dense matrix.  Measured on the GB300, ms for 4 matrices (dense, HODLR):
+ * dimension 5000 26, 397; 8000 64, 581; 12000 163, 1116; 20000 628, 1652; dense grows with the
+ * third power of the dimension, HODLR with less than the second, so they meet near 32000.  The mixed form takes HODLR only when asked (CAPS_PATH_HODLR or the
  * autotuner); its sampled elements then come from the float-float q-sums, its compression and
  * factorisation stay FP64.  Returns 1, or 0 for an unknown path. */
 #define CAPS_PATH_AUTO  0
 #define CAPS_PATH_HODLR 1
 #define CAPS_PATH_DENSE 2
-#define CAPS_HODLR_AUTO_DIM 4000
+#define CAPS_HODLR_AUTO_DIM 32000
+#define CAPS_HODLR_LOW_MEM_DIM 4000
 #define CAPS_HODLR_AUTO_DIM_MIXED 1000000000 /* the mixed form factors densely unless asked */
 int caps_gpu_set_path(caps_t *self, int path);
 
