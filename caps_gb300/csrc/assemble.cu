@@ -1,7 +1,7 @@
 // assemble.cu -- FP64 assembly of the round-trip matrices M(xi,m) of a batch.
 //
 // Phases (each one launch over the whole batch):
-//   k_setup   per task: K panel grid and the degree-recurrence coefficients
+//   k_coef    per m: the degree-recurrence coefficients
 //   k_mie     per (xi, l): log|a_l|, log|b_l|                     (libcaps.c:485-602)
 //   k_scale   per (task, l): symmetric scale factors sqrt(Lambda a_l), u(l), v(l)
 //   k_ktab    per (task, 32 quadrature nodes): all K_{nu,p} partial sums
@@ -20,38 +20,21 @@
 
 namespace capsgpu {
 
-__constant__ double c_glx[GLN];
-__constant__ double c_glw[GLN];
-
-void upload_gauss_legendre(const double *x, const double *w)
-{
-    CK(cudaMemcpyToSymbol(c_glx, x, GLN * sizeof(double)));
-    CK(cudaMemcpyToSymbol(c_glw, w, GLN * sizeof(double)));
-}
-
 // ---------------------------------------------------------------------------
-// setup: quadrature grid + recurrence coefficients for every task
+// degree recurrence coefficients, once per distinct m
 // ---------------------------------------------------------------------------
-__global__ void k_setup(Task *tasks, int ntask, double *edges, int max_panels, double2 *coefAB, int nu_stride,
-                        double c_width, int *status)
+// A_nu = (2nu+1)/(nu-mu+1), B_nu = (nu+mu)/(nu-mu+1): P_{nu+1} = A x P_nu - B P_{nu-1}, entry i = nu - mu
+// of group g, in FP64 or (mixed form) float-float
+__global__ void k_coef(const int *group_m, int ngroup, int nu_stride, double2 *coefAB, float4 *coefF)
 {
-    const int task = blockIdx.x;
-    if (task >= ntask) return;
-    Task &T = tasks[task];
-    if (threadIdx.x < 32) { // warp 0 builds the grid
-        KGridParams P = kgrid_default();
-        P.c_width = c_width;
-        const int np = kgrid_build_warp(T.alpha, T.mu, T.s, T.nu_max, P, edges + (size_t)task * (max_panels + 1), max_panels);
-        if (threadIdx.x == 0) {
-            if (np < 0) { T.npanel = 0; status[task] |= ST_ERR_GRID; }
-            else T.npanel = np;
-        }
-    }
-    // A_nu = (2nu+1)/(nu-mu+1), B_nu = (nu+mu)/(nu-mu+1): P_{nu+1} = A x P_nu - B P_{nu-1}
-    const int nnu = T.nu_max - T.mu + 1;
-    for (int i = threadIdx.x; i < nnu; i += blockDim.x) {
-        const double nu = T.mu + i, d = 1.0 / (i + 1.0);
-        coefAB[(size_t)task * nu_stride + i] = make_double2((2 * nu + 1) * d, (nu + T.mu) * d);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, g = blockIdx.y;
+    if (i >= nu_stride || g >= ngroup) return;
+    const int mu = 2 * max(group_m[g], 1);
+    const double nu = mu + i, d = 1.0 / (i + 1.0), a = (2 * nu + 1) * d, b = (nu + mu) * d;
+    if (coefAB) coefAB[(size_t)g * nu_stride + i] = make_double2(a, b);
+    if (coefF) {
+        const ff x = ff_from_d(a), y = ff_from_d(b);
+        coefF[(size_t)g * nu_stride + i] = make_float4(x.h, x.l, y.h, y.l);
     }
 }
 
@@ -93,19 +76,52 @@ __global__ void k_scale(const Task *tasks, int ntask, int ldim, const double *ln
 }
 
 // ---------------------------------------------------------------------------
-// K integrals on the shared panel grid
+// K integrals on the shared nodes
 // ---------------------------------------------------------------------------
-// One warp owns 32 nodes (two panels).  Each lane runs the degree recurrence of
-// P_nu^mu at its node; at every degree the warp aligns the lane values to the
-// warp-maximum binary exponent and parks them in shared memory; every 32
-// degrees lane r folds row r with the node weights (times the Fresnel
+// One warp owns 32 nodes.  Each lane runs the degree recurrence of P_nu^mu at its node; at every
+// degree the warp aligns the lane values to the warp-maximum binary exponent and parks them in
+// shared memory; every 32 degrees lane r folds row r with the node weights (times the Fresnel
 // coefficient of each node) into the partial K sum of degree nu0+r.
-constexpr int KT_WARPS = 8;
+//
+// FP64 form: 5 FP64 operations per node and degree at two per clock and SM; the nodes of kgrid.cuh
+// are a fifth of the Gauss-Legendre panels' (R/L = 100 free energy: K 18.8 -> 8.1 ms), aligning once per 16
+// degrees without FP64 comparisons and one warp per CTA left 3.3 ms.
+
+// node j of task T: x, the binary exponent E and the mantissas WTM, WTE of its weight, e^{-alpha x}
+// (x^2-1)^{-s} times the start P_mu^mu = (2mu-1)!! sinh^mu t of the recurrence and r_p
+template <bool PR> CAPS_DEV void k_node(const Task &T, int j, const double *lfac_tab, double &x, int &E, double &WTM, double &WTE)
+{
+    const double w = T.kw0 + j * KG_H, z = w / T.kc;
+    // u = c log(1 + e^z), du/dw = 1 / (1 + e^-z)
+    const double ez = exp(-fabs(z));
+    const double u = T.kc * (fmax(z, 0.0) + log1p(ez)), up = (z >= 0 ? 1.0 : ez) / (1.0 + ez);
+    const double xm = u * u / (4 * T.alpha);                  // x - 1
+    x = 1.0 + xm;
+    const double lsh = 0.5 * log(xm * (x + 1.0));             // log sinh t
+    const double ldf = lfac(lfac_tab, 2 * T.mu) - T.mu * LN2 - lfac(lfac_tab, T.mu);
+    const double lc = log(KG_H * u * up / (2 * T.alpha)) - T.alpha * x + (T.mu - 2 * T.s) * lsh + ldf;
+    const double fl = floor(lc * INV_LN2);
+    const double f = exp(lc - fl * LN2);
+    E = (int)fl;
+    double rTE = -1.0, rTM = 1.0;
+    if (!PR) { // Fresnel at k = xi_ sinh t  (libcaps.c:616)
+        const double eps = T.epsm1_plate;
+        const double y = eps / (x * x);
+        const double bm1 = y / (sqrt(1 + y) + 1);
+        rTE = -bm1 / (2 + bm1);
+        rTM = (eps - bm1) / (eps + 2 + bm1);
+    }
+    WTM = f * rTM;
+    WTE = f * rTE;
+}
+
+// one warp per CTA, so that a small batch's warps spread over the SMs and their FP64 pipes (24
+// matrices of dimension 2100: eight warps per CTA 1.54 ms, one 0.99)
+constexpr int KT_WARPS = 1, KT_ALIGN = 16;
 
 template <bool PR>
 __global__ void __launch_bounds__(KT_WARPS * 32)
-k_ktab(const Task *tasks, const double *edges, int max_panels, const double2 *coefAB, int nu_stride,
-       const double *lfac_tab, double *partM, int *partE, int max_warps)
+k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lfac_tab, double *partM, int *partE, int max_warps)
 {
     extern __shared__ double smem[];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -117,73 +133,57 @@ k_ktab(const Task *tasks, const double *edges, int max_panels, const double2 *co
     const int task = blockIdx.y;
     const Task T = tasks[task];
     const int warp = blockIdx.x * KT_WARPS + wib;
-    const int nwarp = (T.npanel + 1) / 2;
-    if (warp >= nwarp) return;
-
-    const int panel = warp * 2 + (lane >> 4), j = lane & 15;
-    const bool valid = panel < T.npanel;
+    if (warp * 32 >= T.nnode) return;
+    const bool valid = warp * 32 + lane < T.nnode;
     double x = 1.0, WTM = 0.0, WTE = 0.0;
     int E = -(1 << 29);
-    if (valid) {
-        const double *ed = edges + (size_t)task * (max_panels + 1);
-        const double a = ed[panel], b = ed[panel + 1];
-        const double h = 0.5 * (b - a), c = 0.5 * (a + b);
-        const double t = c + h * c_glx[j], w = h * c_glw[j];
-        const double sh = sinh(t);
-        x = cosh(t);
-        // log of node weight times e^{-alpha x} sinh^{mu+1-2s} t (2mu-1)!!
-        const double ldf = lfac(lfac_tab, 2 * T.mu) - T.mu * LN2 - lfac(lfac_tab, T.mu);
-        const double lc = log(w) - T.alpha * x + (T.mu + 1 - 2 * T.s) * log(sh) + ldf;
-        const double fl = floor(lc * INV_LN2);
-        const double f = exp(lc - fl * LN2);
-        E = (int)fl;
-        double rTE = -1.0, rTM = 1.0;
-        if (!PR) { // Fresnel at k = xi_ sinh t  (libcaps.c:616)
-            const double eps = T.epsm1_plate;
-            const double y = eps / (x * x);
-            const double bm1 = y / (sqrt(1 + y) + 1);
-            rTE = -bm1 / (2 + bm1);
-            rTM = (eps - bm1) / (eps + 2 + bm1);
-        }
-        WTM = f * rTM;
-        WTE = f * rTE;
-    }
+    if (valid) k_node<PR>(T, warp * 32 + lane, lfac_tab, x, E, WTM, WTE);
     wTM[lane] = WTM;
     wTE[lane] = WTE;
 
     double pp = 0.0, pc = valid ? 1.0 : 0.0;
     const int nnu = T.nu_max - T.mu + 1;
-    const double2 *ab = coefAB + (size_t)task * nu_stride;
+    const double2 *ab = coefAB + (size_t)T.mgroup * nu_stride;
     const size_t pTM = ((size_t)(task * 2 + 1) * max_warps + warp) * nu_stride;
     const size_t pTE = ((size_t)(task * 2 + 0) * max_warps + warp) * nu_stride;
 
     for (int base = 0; base < nnu; base += 32) {
         const int rows = min(32, nnu - base);
-        for (int r = 0; r < rows; r++) {
-            const int e = (pc != 0.0) ? expo(pc) + E : -(1 << 29);
-            const int emax = __reduce_max_sync(0xffffffffu, e);
-            buf[r * 33 + lane] = (pc != 0.0 && e - emax > -1000) ? shift2(pc, E - emax) : 0.0;
-            if (lane == 0) rowE[r] = emax;
-            const double2 c = __ldg(ab + base + r);
-            const double pn = fma(c.x * x, pc, -c.y * pp);
-            pp = pc;
-            pc = pn;
-            if (fabs(pc) > 0x1p600) { pc *= 0x1p-600; pp *= 0x1p-600; E += 600; }
+        for (int half = 0; half < 32; half += KT_ALIGN) {
+            // the lane values aligned to the largest of the warp, for KT_ALIGN degrees at once: a value
+            // grows by (A x)^16 < 2^900 meanwhile (x < 2^50), and one that starts 2^1000 below stays below
+            const int ex = (int)((__double_as_longlong(pc) >> 52) & 0x7ff), k = ex ? ex - 1023 : 0;
+            pc = shift2(pc, -k);
+            pp = shift2(pp, -k);
+            E += k;
+            const int emax = __reduce_max_sync(0xffffffffu, ex ? E : -(1 << 29));
+            const int d = max(E - emax, -1023);
+            if (lane < KT_ALIGN) rowE[half + lane] = emax;
+#pragma unroll
+            for (int r = 0; r < KT_ALIGN; r++) {
+                if (half + r < rows) { // uniform
+                    buf[(half + r) * 33 + lane] = shift2(pc, d);
+                    const double2 c = __ldg(ab + base + half + r);
+                    const double pn = fma(c.x * x, pc, -c.y * pp);
+                    pp = pc;
+                    pc = pn;
+                }
+            }
         }
         __syncwarp();
         if (lane < rows) {
-            double sTM = 0.0, sTE = 0.0;
+            double sM[2] = {0.0, 0.0}, sE[2] = {0.0, 0.0}; // two chains each: the additions' latency
             const double *row = buf + lane * 33;
 #pragma unroll 8
             for (int l = 0; l < 32; l++) {
                 const double v = row[l];
-                sTM = fma(v, wTM[l], sTM);
-                if (!PR) sTE = fma(v, wTE[l], sTE);
+                sM[l & 1] = fma(v, wTM[l], sM[l & 1]);
+                if (!PR) sE[l & 1] = fma(v, wTE[l], sE[l & 1]);
             }
-            partM[pTM + base + lane] = sTM;
+            partM[pTM + base + lane] = sM[0] + sM[1];
             partE[pTM + base + lane] = rowE[lane];
             if (!PR) {
-                partM[pTE + base + lane] = sTE;
+                partM[pTE + base + lane] = sE[0] + sE[1];
                 partE[pTE + base + lane] = rowE[lane];
             }
         }
@@ -198,19 +198,9 @@ k_ktab(const Task *tasks, const double *edges, int max_panels, const double2 *co
 // the sums do not cancel; the upward recurrence (dominant solution) loses at most a bit
 // per step to its subtraction.  The node weights are still formed once per node in FP64.
 // Partials: float-float (h, l) times 2^partE.
-__global__ void k_coef_ff(int ntask, int nu_stride, const double2 *coefAB, float4 *coefF)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, task = blockIdx.y;
-    if (i >= nu_stride || task >= ntask) return;
-    const double2 c = coefAB[(size_t)task * nu_stride + i];
-    const ff a = ff_from_d(c.x), b = ff_from_d(c.y);
-    coefF[(size_t)task * nu_stride + i] = make_float4(a.h, a.l, b.h, b.l);
-}
-
 template <bool PR>
 __global__ void __launch_bounds__(KT_WARPS * 32)
-k_ktab_ff(const Task *tasks, const double *edges, int max_panels, const float4 *coefF, int nu_stride, const double *lfac_tab,
-          float2 *partF, int *partE, int max_warps)
+k_ktab_ff(const Task *tasks, const float4 *coefF, int nu_stride, const double *lfac_tab, float2 *partF, int *partE, int max_warps)
 {
     extern __shared__ double smem[];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -222,42 +212,23 @@ k_ktab_ff(const Task *tasks, const double *edges, int max_panels, const float4 *
     const int task = blockIdx.y;
     const Task T = tasks[task];
     const int warp = blockIdx.x * KT_WARPS + wib;
-    const int nwarp = (T.npanel + 1) / 2;
-    if (warp >= nwarp) return;
-
-    const int panel = warp * 2 + (lane >> 4), j = lane & 15;
-    const bool valid = panel < T.npanel;
+    if (warp * 32 >= T.nnode) return;
+    const bool valid = warp * 32 + lane < T.nnode;
     ff x{1.0f, 0.0f}, WTM{0.0f, 0.0f}, WTE{0.0f, 0.0f};
     int E = -(1 << 29);
     if (valid) {
-        const double *ed = edges + (size_t)task * (max_panels + 1);
-        const double a = ed[panel], b = ed[panel + 1];
-        const double h = 0.5 * (b - a), c = 0.5 * (a + b);
-        const double t = c + h * c_glx[j], w = h * c_glw[j];
-        const double sh = sinh(t), xd = cosh(t);
-        const double ldf = lfac(lfac_tab, 2 * T.mu) - T.mu * LN2 - lfac(lfac_tab, T.mu);
-        const double lc = log(w) - T.alpha * xd + (T.mu + 1 - 2 * T.s) * log(sh) + ldf;
-        const double fl = floor(lc * INV_LN2);
-        const double f = exp(lc - fl * LN2);
-        E = (int)fl;
-        double rTE = -1.0, rTM = 1.0;
-        if (!PR) { // Fresnel at k = xi_ sinh t  (libcaps.c:616)
-            const double eps = T.epsm1_plate;
-            const double y = eps / (xd * xd);
-            const double bm1 = y / (sqrt(1 + y) + 1);
-            rTE = -bm1 / (2 + bm1);
-            rTM = (eps - bm1) / (eps + 2 + bm1);
-        }
+        double xd, tm, te;
+        k_node<PR>(T, warp * 32 + lane, lfac_tab, xd, E, tm, te);
         x = ff_from_d(xd);
-        WTM = ff_from_d(f * rTM);
-        WTE = ff_from_d(f * rTE);
+        WTM = ff_from_d(tm);
+        WTE = ff_from_d(te);
     }
     wTM[lane] = make_float2(WTM.h, WTM.l);
     wTE[lane] = make_float2(WTE.h, WTE.l);
 
     ff pp{0.0f, 0.0f}, pc{valid ? 1.0f : 0.0f, 0.0f};
     const int nnu = T.nu_max - T.mu + 1;
-    const float4 *ab = coefF + (size_t)task * nu_stride;
+    const float4 *ab = coefF + (size_t)T.mgroup * nu_stride;
     const size_t pTM = ((size_t)(task * 2 + 1) * max_warps + warp) * nu_stride;
     const size_t pTE = ((size_t)(task * 2 + 0) * max_warps + warp) * nu_stride;
 
@@ -316,7 +287,7 @@ __global__ void k_kred_ff(const Task *tasks, int ntask, const float2 *partF, con
     const Task &T = tasks[task];
     const int nnu = T.nu_max - T.mu + 1;
     if (i >= nnu) return;
-    const int nwarp = (T.npanel + 1) / 2;
+    const int nwarp = (T.nnode + 31) / 32;
     ffe kp[2];
     for (int p = 1; p >= 0; p--) {
         if (p == 0 && T.is_pr) { // K_TE = -K_TM for perfect reflectors (integration.c:638)
@@ -357,7 +328,7 @@ __global__ void k_kred(const Task *tasks, int ntask, const double *partM, const 
     const Task &T = tasks[task];
     const int nnu = T.nu_max - T.mu + 1;
     if (i >= nnu) return;
-    const int nwarp = (T.npanel + 1) / 2;
+    const int nwarp = (T.nnode + 31) / 32;
     for (int p = 1; p >= 0; p--) {
         sd *out = K + (size_t)(task * 2 + p) * nu_stride + i;
         if (p == 0 && T.is_pr) { // K_TE = -K_TM for perfect reflectors (integration.c:638)
@@ -656,7 +627,7 @@ __global__ void k_elem(const Task *tasks, const int *tlist, int nlist, int ldim,
 // dimension 280 and 0.5 ms at 2100, against about 10 us here, and loses no less.  The Frobenius norm
 // decides the Mercator shortcut alone, so only mode 0 reads the matrix for it (warp per
 // column; mode 1 read it too, 5 ms for 24 matrices of dimension 2100).
-constexpr int ST_NT = 512;
+constexpr int ST_NT = 512; // at most; a quarter as many where n is small (a warp's sum takes 35 FP64 operations)
 __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, int n, const double *A, size_t lda, size_t mat_stride, int mode,
                                                  const double *mdiag, double *trace_out, double *result, int *status, const double *frop,
                                                  int nfro)
@@ -670,14 +641,14 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
     if (lane == 0) { rs[warp] = tr.s; rc[warp] = tr.c; }
     if (mode == 0 && frop) {
         double s = 0.0;
-        for (int i = threadIdx.x; i < nfro; i += ST_NT) s += frop[(size_t)task * nfro + i];
+        for (int i = threadIdx.x; i < nfro; i += blockDim.x) s += frop[(size_t)task * nfro + i];
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) red[warp] = s;
     } else if (A && mode == 0) {
         // sum of squares of M: diagonal once, strict lower twice (M is symmetric)
         const double *Am = A + (size_t)task * mat_stride;
         double s = 0.0;
-        for (int j = warp; j < n; j += ST_NT / 32) {
+        for (int j = warp; j < n; j += blockDim.x / 32) {
             const double *col = Am + (size_t)j * lda;
             double a = 0.0;
 #pragma unroll 4
@@ -691,7 +662,7 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
     __syncthreads();
     if (threadIdx.x != 0) return;
     CSum all;
-    for (int w = 0; w < ST_NT / 32; w++) all.add(rs[w], rc[w]);
+    for (int w = 0; w < (int)blockDim.x / 32; w++) all.add(rs[w], rc[w]);
     const double t = all.s + all.c;
     trace_out[task] = t;
     if (status[task] & ~0xF) { result[task] = NAN; return; }
@@ -699,7 +670,7 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
     if (!A) return;
     if (mode == 0) {
         double fro2 = 0.0;
-        for (int w = 0; w < ST_NT / 32; w++) fro2 += red[w];
+        for (int w = 0; w < (int)blockDim.x / 32; w++) fro2 += red[w];
         const double fro = sqrt(fro2);
         if (fro < 1) {
             const double merc = -t - fro2 / 2;
@@ -713,13 +684,21 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-void launch_setup(Task *tasks, int ntask, double *edges, int max_panels, double2 *coefAB, int nu_stride, double c_width,
-                  int *status, cudaStream_t st)
+void launch_coef(const int *group_m, int ngroup, int nu_stride, double2 *coefAB, float4 *coefF, cudaStream_t st)
 {
-    k_setup<<<ntask, 256, 0, st>>>(tasks, ntask, edges, max_panels, coefAB, nu_stride, c_width, status);
+    k_coef<<<dim3((nu_stride + 127) / 128, ngroup), 128, 0, st>>>(group_m, ngroup, nu_stride, coefAB, coefF);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }
+
+void set_k_nodes(Task &T, double left)
+{
+    const KGrid g = kgrid(T.alpha, T.mu, T.nu_max, T.epsm1_plate, left);
+    T.kw0 = g.w0;
+    T.kc = g.c;
+    T.nnode = g.n;
+}
+double k_left(int mu, int s) { return kgrid_left(mu, s); }
 
 void launch_mie(const double *xi, const double *epsm1, int nxi, double LbyR, int lmax, double *lna, double *lnb, cudaStream_t st)
 {
@@ -740,8 +719,8 @@ void launch_scale(const Task *tasks, int ntask, int ldim, const double *lna, con
 
 size_t ktab_smem_bytes() { return (size_t)KT_WARPS * (32 * 33 + 64) * sizeof(double) + KT_WARPS * 32 * sizeof(int); }
 
-void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double *edges, int max_panels, const double2 *coefAB,
-                 int nu_stride, const double *lfac_tab, double *partM, int *partE, cudaStream_t st)
+void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double2 *coefAB, int nu_stride, const double *lfac_tab,
+                 double *partM, int *partE, cudaStream_t st)
 {
     static bool attr_set = false;
     const size_t sm = ktab_smem_bytes();
@@ -751,8 +730,8 @@ void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const dou
         attr_set = true;
     }
     dim3 g((max_warps + KT_WARPS - 1) / KT_WARPS, ntask);
-    if (pr) k_ktab<true><<<g, KT_WARPS * 32, sm, st>>>(tasks, edges, max_panels, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
-    else k_ktab<false><<<g, KT_WARPS * 32, sm, st>>>(tasks, edges, max_panels, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
+    if (pr) k_ktab<true><<<g, KT_WARPS * 32, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
+    else k_ktab<false><<<g, KT_WARPS * 32, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }
@@ -823,8 +802,8 @@ void launch_ptab_groups(const int *group_m, int ngroup, float4 *ptabf, int pstri
     CK(cudaGetLastError());
 }
 
-void launch_ktab_ff(bool pr, const Task *tasks, int ntask, int max_warps, const double *edges, int max_panels, const double2 *coefAB,
-                    float4 *coefF, int nu_stride, const double *lfac_tab, float2 *partF, int *partE, cudaStream_t st)
+void launch_ktab_ff(bool pr, const Task *tasks, int ntask, int max_warps, const float4 *coefF, int nu_stride, const double *lfac_tab,
+                    float2 *partF, int *partE, cudaStream_t st)
 {
     static bool attr_set = false;
     const size_t sm = ktab_smem_bytes();
@@ -833,12 +812,10 @@ void launch_ktab_ff(bool pr, const Task *tasks, int ntask, int max_warps, const 
         CK(cudaFuncSetAttribute(k_ktab_ff<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         attr_set = true;
     }
-    dim3 gc((nu_stride + 127) / 128, ntask);
-    k_coef_ff<<<gc, 128, 0, st>>>(ntask, nu_stride, coefAB, coefF);
     dim3 g((max_warps + KT_WARPS - 1) / KT_WARPS, ntask);
-    if (pr) k_ktab_ff<true><<<g, KT_WARPS * 32, sm, st>>>(tasks, edges, max_panels, coefF, nu_stride, lfac_tab, partF, partE, max_warps);
-    else k_ktab_ff<false><<<g, KT_WARPS * 32, sm, st>>>(tasks, edges, max_panels, coefF, nu_stride, lfac_tab, partF, partE, max_warps);
-    COUNT_LAUNCH(2);
+    if (pr) k_ktab_ff<true><<<g, KT_WARPS * 32, sm, st>>>(tasks, coefF, nu_stride, lfac_tab, partF, partE, max_warps);
+    else k_ktab_ff<false><<<g, KT_WARPS * 32, sm, st>>>(tasks, coefF, nu_stride, lfac_tab, partF, partE, max_warps);
+    COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }
 
@@ -895,7 +872,7 @@ void launch_stats(const int *tlist, int nlist, int n, const double *A, size_t ld
                   double *trace, double *result, int *status, cudaStream_t st, const double *fro, int nfro)
 {
     if (nlist <= 0) return;
-    k_stats<<<nlist, ST_NT, 0, st>>>(tlist, nlist, n, A, lda, mat_stride, mode, mdiag, trace, result, status, fro, nfro);
+    k_stats<<<nlist, mode == 0 || n > 1024 ? ST_NT : ST_NT / 4, 0, st>>>(tlist, nlist, n, A, lda, mat_stride, mode, mdiag, trace, result, status, fro, nfro);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }

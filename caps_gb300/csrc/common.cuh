@@ -20,9 +20,6 @@ constexpr double LOGPI = 1.14472988584940017414;
 constexpr double HALF_LOG_2PI = 0.91893853320467274178;
 constexpr double PI = 3.14159265358979323846;
 
-// number of Gauss-Legendre nodes per panel of the K quadrature
-constexpr int GLN = 16;
-
 struct sd { double m; int e; };   // value = m * 2^e
 
 // per (m, l1 >= l2) pair: a_1, a_2 and a_0 = a0m 2^a0e of the I q-sum
@@ -116,7 +113,8 @@ struct Task {
     int nu_max;          // largest degree of K needed: 2 (lmin+ldim)
     int xi_index;        // row of the Mie table
     int is_pr;           // plate is a perfect reflector: K_TE = -K_TM
-    int npanel;          // number of quadrature panels of K
+    int nnode;           // quadrature nodes of K (kgrid.cuh): w = kw0 + j KG_H
+    double kw0, kc;      // first node, width of the map's bend
     int mgroup;          // row of the per-m table of a_0, a_1, a_2 in the current chunk
 };
 

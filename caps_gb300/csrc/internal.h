@@ -27,21 +27,24 @@ struct Counters { long long launches = 0, h2d = 0, d2h = 0, nfactor = 0, nmat = 
 extern Counters g_counters;
 #define COUNT_LAUNCH(n) (::capsgpu::g_counters.launches += (n))
 
-void upload_gauss_legendre(const double *x, const double *w);
-void launch_setup(Task *tasks, int ntask, double *edges, int max_panels, double2 *coefAB, int nu_stride, double c_width,
-                  int *status, cudaStream_t st);
+// quadrature nodes of K (kgrid.cuh) into a task whose other fields are set; k_left: their left end,
+// which depends on m alone
+double k_left(int mu, int s);
+void set_k_nodes(Task &T, double left);
+// degree-recurrence coefficients per distinct m (FP64, float-float; either may be nullptr)
+void launch_coef(const int *group_m, int ngroup, int nu_stride, double2 *coefAB, float4 *coefF, cudaStream_t st);
 void launch_mie(const double *xi, const double *epsm1, int nxi, double LbyR, int lmax, double *lna, double *lnb, cudaStream_t st);
 void launch_scale(const Task *tasks, int ntask, int ldim, const double *lna, const double *lnb, int lmax, const double *lfac_tab,
                   sd *Sa, sd *Sb, double2 *uv, cudaStream_t st);
 size_t ktab_smem_bytes();
-void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double *edges, int max_panels, const double2 *coefAB,
-                 int nu_stride, const double *lfac_tab, double *partM, int *partE, cudaStream_t st);
+void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double2 *coefAB, int nu_stride, const double *lfac_tab,
+                 double *partM, int *partE, cudaStream_t st);
 void launch_kred(const Task *tasks, int ntask, int max_nnu, const double *partM, const int *partE, int max_warps, int nu_stride,
                  sd *K, int *status, cudaStream_t st);
 // mixed form: the K integrals in float-float
 struct ffe;
-void launch_ktab_ff(bool pr, const Task *tasks, int ntask, int max_warps, const double *edges, int max_panels, const double2 *coefAB,
-                    float4 *coefF, int nu_stride, const double *lfac_tab, float2 *partF, int *partE, cudaStream_t st);
+void launch_ktab_ff(bool pr, const Task *tasks, int ntask, int max_warps, const float4 *coefF, int nu_stride, const double *lfac_tab,
+                    float2 *partF, int *partE, cudaStream_t st);
 // KP, KPe: TM and TE of one (task, nu) under one exponent, the table the q-sums read
 void launch_kred_ff(const Task *tasks, int ntask, int max_nnu, const float2 *partF, const int *partE, int max_warps, int nu_stride,
                     float4 *KP, int *KPe, int *status, cudaStream_t st);

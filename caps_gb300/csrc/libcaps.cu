@@ -105,7 +105,7 @@ struct Engine {
     cudaStream_t side = nullptr;          // Mie coefficients and scale factors, beside setup and K
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     double *d_lfac = nullptr;
-    DevBuf tasks, edges, coef, partM, partE, K, I, Sa, Sb, uv, A, logdiag, trace, result, status, mie_a, mie_b, xi, eps, lft, xtab, ptab, S32, ptabf, a12, gm, glmin, Saf, Sbf, uvf, part, diag, groups, B, diag2, mwork, a12t, coefF, tlist, groups2, glist2, KP, KPe, hwork, seed, sw64, fro;
+    DevBuf tasks, coef, partM, partE, K, I, Sa, Sb, uv, A, logdiag, trace, result, status, mie_a, mie_b, xi, eps, lft, xtab, ptab, S32, ptabf, a12, gm, glmin, Saf, Sbf, uvf, part, diag, groups, B, diag2, mwork, a12t, coefF, tlist, groups2, glist2, KP, KPe, hwork, seed, sw64, fro;
     std::vector<double> host_pinned_dummy;
     double timings[6] = {0, 0, 0, 0, 0, 0};
     double timings_cum[6] = {0, 0, 0, 0, 0, 0};
@@ -146,22 +146,6 @@ static void engine_init()
     std::call_once(g_tab_once, init_host_tables);
     CK(cudaMalloc(&g_eng.d_lfac, 1024 * sizeof(double)));
     CK(cudaMemcpy(g_eng.d_lfac, h_lfac_tab, 1024 * sizeof(double), cudaMemcpyHostToDevice));
-    // Gauss-Legendre nodes on [-1,1] by Newton iteration on P_GLN
-    double x[GLN], w[GLN];
-    for (int i = 0; i < GLN; i++) {
-        double z = cos(PI * (i + 0.75) / (GLN + 0.5)), pp = 0;
-        for (int it = 0; it < 100; it++) {
-            double p1 = 1, p2 = 0;
-            for (int j = 1; j <= GLN; j++) { double p3 = p2; p2 = p1; p1 = ((2 * j - 1) * z * p2 - (j - 1) * p3) / j; }
-            pp = GLN * (z * p1 - p2) / (z * z - 1);
-            const double z1 = z;
-            z = z1 - p1 / pp;
-            if (fabs(z - z1) < 1e-16) break;
-        }
-        x[i] = z;
-        w[i] = 2 / ((1 - z * z) * pp * pp);
-    }
-    upload_gauss_legendre(x, w);
     for (int i = 0; i < Engine::NEV; i++) CK(cudaEventCreate(&g_eng.ev[i]));
     g_eng.ready = true;
 }
@@ -432,13 +416,6 @@ static void d2h(void *dst, const void *src, size_t bytes, cudaStream_t st)
     g_counters.d2h += (long long)bytes;
 }
 
-// panel width of the K quadrature grid in units of the local peak width: the accuracy of K
-// (|d log K| ~ 1e-13 against an adaptive quadrature) is the same from 1 to 3; the FP64 form
-// keeps 2, the mixed form, where K is a fifth of a free energy's time, takes 3 (a third
-// fewer nodes)
-static const double KGRID_WIDTH = 2.0, KGRID_WIDTH_MIXED = 3.0;
-static const int MAX_PANELS = 2048;
-
 static int lmin_of(const caps_t *c, int m)
 {
     size_t lo, hi;
@@ -465,7 +442,8 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     for (int i = 0; i < n; i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return ms[a] != ms[b] ? ms[a] < ms[b] : xi_[a] < xi_[b]; });
     std::vector<Task> tasks(n);
-    int lmax_mie = 1;
+    int lmax_mie = 1, max_nodes = 1;
+    double left = 0;
     for (int i = 0; i < n; i++) {
         const int src = order[i];
         auto it = xi_index.find(xi_[src]);
@@ -491,7 +469,9 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         T.nu_max = 2 * (T.lmin + ldim);
         T.xi_index = ix;
         T.is_pr = is_pr ? 1 : 0;
-        T.npanel = 0;
+        if (i == 0 || T.m != tasks[i - 1].m) left = k_left(T.mu, T.s);
+        set_k_nodes(T, left);
+        max_nodes = std::max(max_nodes, T.nnode);
         lmax_mie = std::max(lmax_mie, T.lmin + ldim);
     }
     const int nxi = (int)xis.size();
@@ -542,7 +522,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
                                            + (size_t)L * (L + 1) / 2 * 32; // a_0..a_2 table (one row per task)
     const size_t per_task = dense_bytes + (size_t)2 * nu_stride * sizeof(sd)
                           + (size_t)nu_stride * sizeof(double2) + (size_t)3 * L * sizeof(sd) + (size_t)dim * 8
-                          + (size_t)2 * 256 * nu_stride * 12  // partial sums, up to 256 warps
+                          + (size_t)2 * ((max_nodes + 31) / 32) * nu_stride * 12 // partial K sums per warp
                           + (size_t)(4 * (caps->ldim + 4096)) * sizeof(double4) // p tables
                           + (hodlr ? 0 : mixed && !O.square ? mixed_work_bytes(1, dim) : cholesky_work_bytes(1, dim)); // diagonal-block inverses, panel images
     size_t budget = (size_t)(0.70 * (double)(freeb + g_eng.A.bytes + g_eng.I.bytes + g_eng.partM.bytes + g_eng.partE.bytes + g_eng.S32.bytes
@@ -610,16 +590,11 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         h2d(d_sub, sub.data(), nsub * sizeof(int4), st);
         int *d_status = (int *)g_eng.status.get(nt * sizeof(int));
         CK(cudaMemsetAsync(d_status, 0, nt * sizeof(int), st));
-        double *d_edges = (double *)g_eng.edges.get((size_t)nt * (MAX_PANELS + 1) * sizeof(double));
-        double2 *d_coef = (double2 *)g_eng.coef.get((size_t)nt * nu_stride * sizeof(double2));
-        launch_setup(d_tasks, nt, d_edges, MAX_PANELS, d_coef, nu_stride,
-                     caps->precision == CAPS_PREC_MIXED ? KGRID_WIDTH_MIXED : KGRID_WIDTH, d_status, st);
-        // panel counts decide the size of the partial-sum buffers
-        std::vector<Task> tback(nt);
-        d2h(tback.data(), d_tasks, nt * sizeof(Task), st);
-        CK(cudaStreamSynchronize(st));
-        int max_warps = 1;
-        for (auto &T : tback) max_warps = std::max(max_warps, (T.npanel + 1) / 2);
+        const bool mixed = caps->precision == CAPS_PREC_MIXED;
+        double2 *d_coef = mixed ? nullptr : (double2 *)g_eng.coef.get((size_t)ngroup * nu_stride * sizeof(double2));
+        float4 *d_coefF = mixed ? (float4 *)g_eng.coefF.get((size_t)ngroup * nu_stride * sizeof(float4)) : nullptr;
+        launch_coef(d_gm, ngroup, nu_stride, d_coef, d_coefF, st);
+        const int max_warps = (max_nodes + 31) / 32;
         sd *d_Sa = (sd *)g_eng.Sa.get((size_t)nt * L * sizeof(sd));
         sd *d_Sb = (sd *)g_eng.Sb.get((size_t)nt * L * sizeof(sd));
         double2 *d_uv = (double2 *)g_eng.uv.get((size_t)nt * L * sizeof(double2));
@@ -631,7 +606,6 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
 
         double *d_pM = (double *)g_eng.partM.get((size_t)nt * 2 * max_warps * nu_stride * sizeof(double));
         int *d_pE = (int *)g_eng.partE.get((size_t)nt * 2 * max_warps * nu_stride * sizeof(int));
-        const bool mixed = caps->precision == CAPS_PREC_MIXED;
         sd *d_K = nullptr;
         float4 *d_KP = nullptr;
         int *d_KPe = nullptr;
@@ -639,13 +613,11 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             // mixed form: float-float K, TM and TE paired, the table the q-sums read
             d_KP = (float4 *)g_eng.KP.get((size_t)nt * nu_stride * sizeof(float4));
             d_KPe = (int *)g_eng.KPe.get((size_t)nt * nu_stride * sizeof(int));
-            float4 *d_coefF = (float4 *)g_eng.coefF.get((size_t)nt * nu_stride * sizeof(float4));
-            launch_ktab_ff(is_pr, d_tasks, nt, max_warps, d_edges, MAX_PANELS, d_coef, d_coefF, nu_stride, g_eng.d_lfac,
-                           (float2 *)d_pM, d_pE, st);
+            launch_ktab_ff(is_pr, d_tasks, nt, max_warps, d_coefF, nu_stride, g_eng.d_lfac, (float2 *)d_pM, d_pE, st);
             launch_kred_ff(d_tasks, nt, nnu_max, (const float2 *)d_pM, d_pE, max_warps, nu_stride, d_KP, d_KPe, d_status, st);
         } else {
             d_K = (sd *)g_eng.K.get((size_t)nt * 2 * nu_stride * sizeof(sd));
-            launch_ktab(is_pr, d_tasks, nt, max_warps, d_edges, MAX_PANELS, d_coef, nu_stride, g_eng.d_lfac, d_pM, d_pE, st);
+            launch_ktab(is_pr, d_tasks, nt, max_warps, d_coef, nu_stride, g_eng.d_lfac, d_pM, d_pE, st);
             launch_kred(d_tasks, nt, nnu_max, d_pM, d_pE, max_warps, nu_stride, d_K, d_status, st);
         }
         CK(cudaEventRecord(g_eng.ev[2], st));

@@ -11,7 +11,7 @@
 //
 // Limits (rejected with an error code and a message, never truncated):
 //   ldim <= 512 (matrix dimension <= 1024), lmin + ldim <= 2048, and at most
-//   256 quadrature panels for the K integrals.
+//   4096 quadrature nodes for the K integrals.
 //
 // The scratch array is shared by all calls and keeps the last call's contents;
 // everything that must start at zero is cleared at the start of each call.
@@ -20,13 +20,12 @@
 //
 // Set-up: the first call on a device (with that device current) resolves the
 // device address of the scratch array with cudaGetSymbolAddress and uploads
-// the log n! and Gauss-Legendre constants to fixed device symbols.  Make that
+// the log n! constants to a fixed device symbol.  Make that
 // first call before any stream capture begins.
 //
 // It runs the same kernels as caps_logdetD, with the same HODLR/LU semantics
 // of caps_t::detalg, on the legacy default stream.  The call synchronises the
-// host with that stream twice (once to read the quadrature panel count, once for
-// the result) and copies the result to the caller's host double.  Rejected input
+// host with that stream once, for the result, and copies the result to the caller's host double.  Rejected input
 // and failed CUDA API calls return a negative code with a message; a kernel
 // launch that fails aborts the process, as every launch of the library does.
 #include <cmath>
@@ -41,7 +40,7 @@ using namespace capsgpu;
 #define NOALLOC_SCRATCH_BYTES (32u << 20)
 #define NOALLOC_MAX_LDIM 512
 #define NOALLOC_MAX_LWINDOW 2048
-#define NOALLOC_MAX_PANELS 256
+#define NOALLOC_MAX_NODES 4096
 #define NOALLOC_MAX_DEVICES 64
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
@@ -74,22 +73,6 @@ static int noalloc_setup(int dev)
     for (int n = 0; n < 1024; n++) tab[n] = lgamma(n + 1.0);
     if (cudaMemcpyToSymbol(g_noalloc_lfac, tab, sizeof tab) != cudaSuccess)
         return noalloc_fail(-3, "upload of the log n! table failed");
-    // Gauss-Legendre nodes of the K panels (Newton iteration on P_GLN)
-    double x[GLN], w[GLN];
-    for (int i = 0; i < GLN; i++) {
-        double z = cos(PI * (i + 0.75) / (GLN + 0.5)), pp = 0;
-        for (int it = 0; it < 100; it++) {
-            double p1 = 1, p2 = 0;
-            for (int j = 1; j <= GLN; j++) { double p3 = p2; p2 = p1; p1 = ((2 * j - 1) * z * p2 - (j - 1) * p3) / j; }
-            pp = GLN * (z * p1 - p2) / (z * z - 1);
-            const double z1 = z;
-            z = z1 - p1 / pp;
-            if (fabs(z - z1) < 1e-16) break;
-        }
-        x[i] = z;
-        w[i] = 2 / ((1 - z * z) * pp * pp);
-    }
-    upload_gauss_legendre(x, w);
     g_lfac_ptr[dev] = (double *)lf;
     g_scratch_ptr[dev] = p;
     return 0;
@@ -153,22 +136,23 @@ extern "C" int caps_logdetD_noalloc(caps_t *self, double xi_, int m, double *log
     const int lmax_mie = lmin + ldim;
     const int lmax_all = lmin + ldim + 2;
     const int nlf = 4 * lmax_all + 8, nx = 2 * lmax_all + 8, pstride = 2 * lmax_all + 8;
-    const int max_warps = NOALLOC_MAX_PANELS / 2;
+    set_k_nodes(T, k_left(T.mu, T.s));
+    if (T.nnode > NOALLOC_MAX_NODES) return noalloc_fail(-2, "the K quadrature needs more than 4096 nodes for this (xi, m)");
+    const int cap_warps = NOALLOC_MAX_NODES / 32, max_warps = (T.nnode + 31) / 32;
 
     Carve C{(unsigned char *)g_scratch_ptr[dev]};
     Task *d_task = C.take<Task>(1);
     int *d_status = C.take<int>(1);
     double *d_xi = C.take<double>(1), *d_eps = C.take<double>(1);
     double *d_lna = C.take<double>(lmax_mie + 1), *d_lnb = C.take<double>(lmax_mie + 1);
-    double *d_edges = C.take<double>(NOALLOC_MAX_PANELS + 1);
     double2 *d_coef = C.take<double2>(nu_stride);
     sd *d_Sa = C.take<sd>(L), *d_Sb = C.take<sd>(L);
     double2 *d_uv = C.take<double2>(L);
     double *d_lft = C.take<double>(nlf);
     double2 *d_xtab = C.take<double2>(nx);
     double4 *d_ptab = C.take<double4>((size_t)2 * pstride);
-    double *d_pM = C.take<double>((size_t)2 * max_warps * nu_stride);
-    int *d_pE = C.take<int>((size_t)2 * max_warps * nu_stride);
+    double *d_pM = C.take<double>((size_t)2 * cap_warps * nu_stride);
+    int *d_pE = C.take<int>((size_t)2 * cap_warps * nu_stride);
     sd *d_K = C.take<sd>((size_t)2 * nu_stride);
     // the I table; the factorisation's workspace takes its place once the elements are formed
     const size_t i_bytes = (size_t)2 * L * L * sizeof(sd), w_bytes = cholesky_work_bytes(1, dim);
@@ -183,7 +167,7 @@ extern "C" int caps_logdetD_noalloc(caps_t *self, double xi_, int m, double *log
     // (k_kred has read the partials before k_a12 writes the table, both on one stream);
     // otherwise nu_stride is small and the table gets a region of its own
     void *d_a12 = d_pM;
-    if (a12_bytes(ldim, 1) > (size_t)2 * max_warps * nu_stride * sizeof(double)) d_a12 = C.take<unsigned char>(a12_bytes(ldim, 1));
+    if (a12_bytes(ldim, 1) > (size_t)2 * cap_warps * nu_stride * sizeof(double)) d_a12 = C.take<unsigned char>(a12_bytes(ldim, 1));
     if (!C.ok) return noalloc_fail(-2, "workspace of this geometry exceeds the 32 MiB scratch array");
 
     // only the status word must start at zero; every other piece is written before it is read
@@ -192,18 +176,14 @@ extern "C" int caps_logdetD_noalloc(caps_t *self, double xi_, int m, double *log
     NA_CK(cudaMemcpyAsync(d_xi, &T.xi_, sizeof(double), cudaMemcpyHostToDevice, st));
     NA_CK(cudaMemcpyAsync(d_eps, &T.epsm1_sphere, sizeof(double), cudaMemcpyHostToDevice, st));
     launch_mie(d_xi, d_eps, 1, self->LbyR, lmax_mie, d_lna, d_lnb, st);
-    launch_setup(d_task, 1, d_edges, NOALLOC_MAX_PANELS, d_coef, nu_stride, 2.0, d_status, st);
-    Task back;
-    NA_CK(cudaMemcpyAsync(&back, d_task, sizeof back, cudaMemcpyDeviceToHost, st));
-    NA_CK(cudaStreamSynchronize(st));
-    if (back.npanel == 0) return noalloc_fail(-2, "the K quadrature needs more than 256 panels for this (xi, m)");
     launch_scale(d_task, 1, ldim, d_lna, d_lnb, lmax_mie, g_lfac_ptr[dev], d_Sa, d_Sb, d_uv, st);
     launch_tables(g_lfac_ptr[dev], d_lft, nlf, d_xtab, nx, st);
-    launch_ktab(T.is_pr != 0, d_task, 1, max_warps, d_edges, NOALLOC_MAX_PANELS, d_coef, nu_stride, g_lfac_ptr[dev], d_pM, d_pE, st);
-    launch_kred(d_task, 1, nnu, d_pM, d_pE, max_warps, nu_stride, d_K, d_status, st);
     const int gm_h[2] = {m, lmin};
     NA_CK(cudaMemcpyAsync(d_gm, &gm_h[0], sizeof(int), cudaMemcpyHostToDevice, st));
     NA_CK(cudaMemcpyAsync(d_glm, &gm_h[1], sizeof(int), cudaMemcpyHostToDevice, st));
+    launch_coef(d_gm, 1, nu_stride, d_coef, nullptr, st);
+    launch_ktab(T.is_pr != 0, d_task, 1, max_warps, d_coef, nu_stride, g_lfac_ptr[dev], d_pM, d_pE, st);
+    launch_kred(d_task, 1, nnu, d_pM, d_pE, max_warps, nu_stride, d_K, d_status, st);
     launch_a12(d_gm, d_glm, 1, ldim, d_lft, d_a12, st);
     launch_ptab(d_task, 1, d_ptab, pstride, st);
     launch_itab(d_task, nullptr, 1, ldim, d_K, nu_stride, d_lft, d_xtab, d_ptab, pstride, d_I, d_status, st, d_a12, false);
