@@ -15,7 +15,8 @@
 //    products with i + j > 6 are below 2^-60 and left out, so the error of a product is that
 //    of the last digit, 2^-54 per factor -- an FP64 sum of 64 products has 2^-53 of its
 //    partial sums at every step.
-//  * the 64 x 64 diagonal blocks (factor and inverse) run on the integer pipes: a number is
+//  * the 64 x 64 diagonal blocks (factor and inverse) are taken in FP32 and corrected to 2^-54 by a
+//    few such products (k_fix_potf2); blocks where that fails run on the integer pipes: a number is
 //    h 2^30 + l, and a product needs three 32 x 32 -> 64 bit multiply-adds (h h, h l, l h).
 //
 // Per 64 columns three launches over the batch: k_fix_potf2 (diagonal block, W = L_kk^-1 as digit
@@ -34,6 +35,7 @@ namespace capsgpu {
 constexpr int NB = 64;
 constexpr int FQ = 60;                       // fixed point: value = integer 2^-60
 constexpr int ND = 6, NG = 7;                // digits of a factor, accumulators (i + j = 0..6)
+constexpr int SY_G0 = 4;                     // accumulators of a first part, see k_fix_syrk
 constexpr int IMG_BLK = NB * NB * 2;         // bytes of one digit of one 64 x 64 block
 constexpr int FIX_WAIT_ITERS = 1 << 22;      // polls of a bounded mbarrier wait
 
@@ -86,42 +88,45 @@ CAPS_DEV void split8(const long long (&x)[8], uint4 (&d)[ND])
     for (int i = 0; i < ND; i++) d[i] = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
 }
 
-// the MMAs of group s = i + j of one 128 x 64 tile, K = 64: A digits 16 KB apart, B digits 8 KB
-CAPS_DEV void mma_group(uint32_t acc, uint32_t a, uint32_t b, int s)
+// the digit products of one 128 x 64 tile, K = 64, of groups G0 .. G1 - 1, accumulator g at tmem + 64 g: NA
+// digits of A (ASTEP bytes apart) and NBD digits of B (one block apart); alo, blo: low descriptor
+// words of digit 0.  Unrolled, so that every descriptor is a sum with a constant.  Two parts, groups
+// 0..SY_G0 - 1 and the rest, are handed to the folding warps one after the other.
+template <int NA, int NBD, int ASTEP, int G0, int G1> CAPS_DEV void mma_groups(uint32_t tmem, uint32_t alo, uint32_t blo)
 {
-    constexpr uint32_t idesc = umma::idesc_f16(128, 64);
-    bool first = true;
-    for (int i = s > ND - 1 ? s - ND + 1 : 0; i <= s && i < ND; i++) {
-        const uint32_t ai = a + i * 2 * IMG_BLK, bj = b + (s - i) * IMG_BLK;
+    constexpr uint32_t idesc = umma::idesc_f16(128, 64), hi = umma::desc_hi(1024);
 #pragma unroll
-        for (int ks = 0; ks < 4; ks++) {
-            umma::mma_f16(acc, umma::desc_kmajor(ai + ks * 256, 128, 1024), umma::desc_kmajor(bj + ks * 256, 128, 1024), idesc, !first);
-            first = false;
-        }
+    for (int g = G0; g < G1; g++) {
+        const int i0 = g > NBD - 1 ? g - NBD + 1 : 0, i1 = g < NA - 1 ? g : NA - 1;
+#pragma unroll
+        for (int i = 0; i < NA; i++)
+            if (i >= i0 && i <= i1) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ks++) {
+                    const uint32_t d = tmem + g * NB, a = alo + i * (ASTEP / 16) + ks * 16, b = blo + (g - i) * (IMG_BLK / 16) + ks * 16;
+                    if (i == i0 && ks == 0) umma::mma_f16_lo<0>(d, a, b, hi, idesc);
+                    else umma::mma_f16_lo<1>(d, a, b, hi, idesc);
+                }
+            }
     }
 }
 
-// NC columns of group s of this warp's lanes folded into v (units of 2^-60 once s = 0 is in);
-// groups come in the order s = 6, 5, ..., 0, of weight 2^(44 - 9 s)
+// NC columns of group s of this warp's lanes folded into v: groups come in the order s = 0, 1, ..., 6 and
+// each weighs 2^-9 of the one before, v = 512 v + g up to s = 5 (units of 2^-61; |v| < 2), then
+// units of 2^-60.  One piece of code for all groups: unrolled, its first pass through the instruction cache
+// cost more than the work.
 template <int NC> CAPS_DEV void fold_group(uint32_t taddr, int s, long long (&v)[NC])
 {
 #pragma unroll
     for (int h = 0; h < NC / 16; h++) {
         float f[16];
         umma::ld16(taddr + h * 16, f);
+        if (s < 6) { // uniform
 #pragma unroll
-        for (int c = 0; c < 16; c++) {
-            const int g = __float2int_rn(f[c]);
-            long long &a = v[h * 16 + c];
-            switch (s) { // uniform, constant after unrolling
-            case 6: a = g; break;
-            case 5: a += (long long)g * 512; break;
-            case 4: a = (a + (long long)g * 262144 + 512) >> 10; break;
-            case 3: a += (long long)g * (1 << 17); break;
-            case 2: a += (long long)g * (1 << 26); break;
-            case 1: a += (long long)((unsigned long long)(unsigned)(g * 8) << 32); break;
-            default: a += (long long)((unsigned long long)(unsigned)(g * 4096) << 32); break;
-            }
+            for (int c = 0; c < 16; c++) v[h * 16 + c] = v[h * 16 + c] * 512 + __float2int_rn(f[c]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 16; c++) v[h * 16 + c] = (v[h * 16 + c] + ((__float2int_rn(f[c]) + 256) >> 9) + 1) >> 1;
         }
     }
 }
@@ -214,45 +219,36 @@ CAPS_DEV long long fix_rsqrt(long long d, int &k)
     return ((long long)R << 29) + (__mul64hi((long long)((unsigned long long)R << 32), c << 4) >> 3);
 }
 
-// one CTA of 256 threads per matrix.  L_kk and W = L_kk^-1 of the 64 x 64 block at k0 (past the
-// matrix: the identity), W as digit images in the operand layout, sum of log L_jj into
-// logdet[task * nbk + block].
-//
-// In 16-column sub-panels.  Warps 0..2: every warp holds the sub-panel's 16 diagonal rows in
-// lanes 0..15 (all three compute them alike, so no warp waits for another) and 16 of the up to 48
-// rows below in lanes 16..31, a row of 16 entries in registers; column j's entries reach the
-// warp by shuffles.  Then all warps apply the rank-16 update to the rest of the triangle, in
-// 2 x 2 tiles.  W: the four 16 x 16 diagonal blocks by substitution, one lane per column, then
-// X_ij = -X_ii sum_k L_ik X_kj by distance from the diagonal.  Bound by the pivot chain (about
-// 200 clocks per column: reciprocal square root, product, shuffle, multiply-add) and the
-// 32-bit multipliers.
 constexpr int PP = NB + 1;
-__global__ void __launch_bounds__(256) k_fix_potf2(int ntask, int n, int k0, const long long *S, size_t lda, size_t mstride, int *status,
-                                                   FixWork wk, double *logdet)
+constexpr int PF_NT = 512;
+
+// The block in limbs throughout, for blocks that k_fix_potf2 cannot take (ill conditioned beyond FP32, or
+// not positive definite): L_kk by 16-column sub-panels, then W; about 80 us.  T, W: [64][PP] integers, Y:
+// 3 x [16][17] limb pairs; on return W holds L_kk^-1 in units of 2^-wq (returned), *logs the sum of log
+// L_jj over the first nb columns, *bad whether a pivot was not positive.  All threads.
+//
+// Warps 0..2: every warp holds the sub-panel's 16 diagonal rows in lanes 0..15 (all three compute
+// them alike, so no warp waits for another) and 16 of the up to 48 rows below in lanes 16..31.
+// Then all warps apply the rank-16 update to the rest of the triangle, in 2 x 2 tiles.  W: the
+// four 16 x 16 diagonal blocks by substitution, one lane per column, then X_ij = -X_ii sum_k L_ik
+// X_kj by distance from the diagonal.
+__device__ __noinline__ int potf2_limbs(const long long *Sm, size_t lda, int nb, long long *T, long long *W, int2 *Y, double *logs, bool *isbad)
 {
-    const int task = blockIdx.x;
-    if (task >= ntask || status[task] != ST_FACTOR) return;
-    extern __shared__ __align__(16) unsigned char pf_sm[];
-    long long *T = reinterpret_cast<long long *>(pf_sm);   // [64][PP]: the block, then L as limbs (int2)
-    long long *W = T + NB * PP;                            // [64][PP]: W, units of 2^-wq
-    int2 *Y = reinterpret_cast<int2 *>(W + NB * PP);       // [48][17] x 3 blocks: sums of a distance, as limbs
     __shared__ long long piv[NB], inv[NB];
     __shared__ int invk[NB];
-    __shared__ unsigned long long smax;
     __shared__ double slog[2];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nb = min(NB, n - k0);
-    const long long *Sm = S + (size_t)task * mstride + (size_t)k0 * lda + k0;
+    __syncthreads(); // the shared memory is free
     {
-        long long v[16];
+        long long v[NB * NB / PF_NT];
 #pragma unroll
-        for (int u = 0; u < 16; u++) {
-            const int e = tid + 256 * u, c = e >> 6, r = e & 63;
+        for (int u = 0; u < NB * NB / PF_NT; u++) {
+            const int e = tid + PF_NT * u, c = e >> 6, r = e & 63;
             v[u] = (r >= c && r < nb && c < nb) ? Sm[(size_t)c * lda + r] : (r == c ? 1LL << FQ : 0LL);
         }
 #pragma unroll
-        for (int u = 0; u < 16; u++) {
-            const int e = tid + 256 * u, c = e >> 6, r = e & 63;
+        for (int u = 0; u < NB * NB / PF_NT; u++) {
+            const int e = tid + PF_NT * u, c = e >> 6, r = e & 63;
             T[r * PP + c] = v[u];
         }
     }
@@ -299,7 +295,7 @@ __global__ void __launch_bounds__(256) k_fix_potf2(int ntask, int n, int k0, con
         }
         __syncthreads();
         const int c0 = o + PB, t2 = (NB - c0) / 2; // 2 x 2 tiles: rows and columns c0 + i, c0 + i + t2
-        for (int e = tid; e < t2 * (t2 + 1) / 2; e += 256) {
+        for (int e = tid; e < t2 * (t2 + 1) / 2; e += PF_NT) {
             int ti = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
             while ((ti + 1) * (ti + 2) / 2 <= e) ti++;
             while (ti * (ti + 1) / 2 > e) ti--;
@@ -334,7 +330,6 @@ __global__ void __launch_bounds__(256) k_fix_potf2(int ntask, int n, int k0, con
     int wq = 57;
 #pragma unroll 1
     for (;; wq -= 12) {
-        if (tid == 0) smax = 0;
         __syncthreads();
         const float lim = ldexpf(1.0f, 61 - wq - 1); // limbs need |w| < 2^(61 - wq)
         bool over = false;
@@ -364,7 +359,7 @@ __global__ void __launch_bounds__(256) k_fix_potf2(int ntask, int n, int k0, con
         __syncthreads();
         for (int dl = 1; dl < 4; dl++) {
             const int np = 4 - dl;
-            for (int e = tid; e < np * 256; e += 256) {
+            for (int e = tid; e < np * 256; e += PF_NT) {
                 const int p = e >> 8, r = (e >> 4) & 15, c = e & 15, i = p + dl;
                 long long sum = 0;
                 for (int k = p; k < i; k++) {
@@ -377,7 +372,7 @@ __global__ void __launch_bounds__(256) k_fix_potf2(int ntask, int n, int k0, con
                 Y[(p * 16 + r) * 17 + c] = limbs(sum);
             }
             __syncthreads();
-            for (int e = tid; e < np * 256; e += 256) {
+            for (int e = tid; e < np * 256; e += PF_NT) {
                 const int p = e >> 8, r = (e >> 4) & 15, c = e & 15, i = p + dl;
                 LAcc t;
                 float ap = 0.0f;
@@ -394,109 +389,513 @@ __global__ void __launch_bounds__(256) k_fix_potf2(int ntask, int n, int k0, con
         }
         if (!__syncthreads_or(over) || wq <= 33) break;
     }
-    unsigned long long mx = 0;
-    for (int e = tid; e < NB * NB; e += 256) {
-        const int r = e >> 6, c = e & 63;
-        if (c <= r) {
-            const long long v = W[r * PP + c];
-            mx = max(mx, (unsigned long long)(v < 0 ? -v : v));
-        }
-    }
-    atomicMax(&smax, mx);
     __syncthreads();
-    // image: W 2^-wexp in units of 2^-60, below 3.9 (the top digit stays below 1024)
-    int wexp = 0;
-    while (wexp < 40 && ldexp((double)smax, -wq - wexp) > 3.9) wexp++;
-    unsigned char *img = wk.wimg(task, n);
-    const int sh = FQ - wq - wexp;
-    for (int e = tid; e < NB * 8; e += 256) {
-        const int j = e & 63, kc = e >> 6;
+    *logs = 0.5 * (slog[0] + slog[1]);
+    *isbad = __syncthreads_or(bad) != 0;
+    return wq;
+}
+
+// ---- the block in FP32 and one correction ----
+// L_kk and W = L_kk^-1 of the 64 x 64 block at k0 (past the matrix: the identity), W as digit images in
+// the operand layout, sum of log L_jj into logdet[task * nbk + block]; one CTA per matrix.
+//
+// A factor in 64-bit arithmetic is a chain of 64 long steps (about 1000 clocks each in limbs, more on
+// the FP64 pipe).  Instead W0 ~ L^-1 is taken from an FP32 Cholesky (a chain of 64 steps of about 90
+// clocks) and corrected by products that the tensor cores form to 2^-54:
+//   E = W0 S W0^T - I                             (|E| ~ 1e-6),
+//   I + E = (I + Y)(I + Y)^T, Y = F(E) - F(P P^T), P = F(E) the lower triangle with half the diagonal
+//                                                 (left out: third order in E),
+//   L^-1 = (I + Y)^-1 W0 = W0 - Z W0, Z = Y - P^2,
+//   log L_jj = log(1 + Y_jj) - log W0_jj.
+// W0 has three digits (27 bits), so that the products take 17 MMAs per 16 columns instead of 26; P P^T
+// and P^2 are of second order and FP32 suffices.  Where E is not small (|E| > 2^-18, beyond which its third
+// order shows; a block of condition above about 50) or FP32 finds no factor, potf2_limbs takes the
+// block.
+//
+// 512 threads.  The FP32 part runs on the block augmented by the identity in panels of 8 columns (three
+// warps hold a panel's 8 diagonal rows and 24 of the others each; two barriers per panel), so that its
+// code is short: fully unrolled 32 x 32 steps spent most of their time fetching instructions (50 us a
+// block; 82 us with the 64-bit limbs).  64 rows use lanes 0..63 of tensor memory, so the warps of lane
+// quadrants 0 and 1 fold, 16 columns each; warps 2 and 3 take the logarithms of W0_jj meanwhile.
+constexpr int PF_W0 = ND * IMG_BLK, PF_WT = PF_W0 + 3 * IMG_BLK, PF_F = PF_WT + 3 * IMG_BLK, PF_SMEM = PF_F + 2 * NB * PP * 4; // 130 KB
+static_assert(NB * PP * 16 + 3 * 16 * 17 * 8 <= PF_SMEM, "potf2_limbs fits");
+
+// F: the block (lower triangle) in FP32, replaced by L; X: W0 = L^-1, all 64 x 64; rinv: scratch of 64.  Begins
+// and ends with a barrier; false where a pivot is not above 1e-6 (in the three panel warps).
+CAPS_DEV bool pf_factor32(float *F, float *X, float *rinv)
+{
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    bool ok = true;
+    for (int e = tid; e < NB * NB; e += PF_NT) X[(e >> 6) * PP + (e & 63)] = (e >> 6) == (e & 63) ? 1.0f : 0.0f;
+    __syncthreads();
+#pragma unroll 1
+    for (int p = 0; p <= 8; p++) {
+        const int o = p * 8, q = o - 8;
+        if (warp < 3 && p < 8) {
+            const int row = lane < 8 ? o + lane : o + warp * 24 + lane;
+            const bool live = row < NB;
+            float a[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) a[c] = live ? F[row * PP + o + c] : 0.0f;
+            asm volatile("bar.sync 1, 96;" ::: "memory"); // the three warps have read the diagonal rows
+            float rv = 0.0f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float d = __shfl_sync(0xffffffffu, a[j], j);
+                ok &= d > 1e-6f;
+                const float r = rsqrtf(fmaxf(d, 1e-6f));
+                if (lane == j) rv = r;
+                a[j] *= r;
+#pragma unroll
+                for (int c = j + 1; c < 8; c++) a[c] = fmaf(-a[j], __shfl_sync(0xffffffffu, a[j], c), a[c]);
+            }
+            if (live && (warp == 0 || lane >= 8))
+#pragma unroll
+                for (int c = 0; c < 8; c++) F[row * PP + o + c] = a[c];
+            if (warp == 0 && lane < 8) rinv[o + lane] = rv;
+        } else if (warp >= 4 && warp < 6 && p > 0) { // rows q .. q + 7 of X, one column per thread
+            const int c = tid - 128;
+            float x[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                float t = X[(q + i) * PP + c];
+#pragma unroll
+                for (int k = 0; k < i; k++) t = fmaf(-F[(q + i) * PP + q + k], x[k], t);
+                x[i] = t * rinv[q + i];
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) X[(q + i) * PP + c] = x[i];
+        }
+        __syncthreads();
+        // 2 x 2 tiles: of the block's rest with panel p, then of X below row o with panel p - 1
+        const int ts = p < 8 ? (56 - o) / 2 : 0, ns = ts * (ts + 1) / 2, nx = p > 0 ? (NB - o) / 2 * (o / 2) : 0;
+        for (int e = tid; e < ns + nx; e += PF_NT) {
+            const float *x0, *y0;
+            float *out;
+            int ys, yk; // y of column j at y0[j * ys + k * yk]
+            bool diag = false;
+            if (e < ns) {
+                int ti = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
+                while ((ti + 1) * (ti + 2) / 2 <= e) ti++;
+                while (ti * (ti + 1) / 2 > e) ti--;
+                const int tj = e - ti * (ti + 1) / 2, rr = o + 8 + 2 * ti, cc = o + 8 + 2 * tj;
+                x0 = F + rr * PP + o;
+                y0 = F + cc * PP + o;
+                ys = PP;
+                yk = 1;
+                out = F + rr * PP + cc;
+                diag = ti == tj;
+            } else {
+                const int t = e - ns, w = o / 2, rr = o + 2 * (t / w), cc = 2 * (t % w);
+                x0 = F + rr * PP + q;
+                y0 = X + q * PP + cc;
+                ys = 1;
+                yk = PP;
+                out = X + rr * PP + cc;
+            }
+            float s00 = 0, s01 = 0, s10 = 0, s11 = 0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float u0 = x0[k], u1 = x0[PP + k], w0 = y0[k * yk], w1 = y0[ys + k * yk];
+                s00 = fmaf(u0, w0, s00);
+                s01 = fmaf(u0, w1, s01);
+                s10 = fmaf(u1, w0, s10);
+                s11 = fmaf(u1, w1, s11);
+            }
+            out[0] -= s00;
+            if (!diag) out[1] -= s01;
+            out[PP] -= s10;
+            out[PP + 1] -= s11;
+        }
+        __syncthreads();
+    }
+    return ok;
+}
+
+// eight FP32 numbers times 2^18 as FP16 high and low parts
+CAPS_DEV void split_half(const float (&x)[8], uint4 &h, uint4 &l)
+{
+    unsigned hw[4], lw[4];
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        const float a = x[2 * p] * 0x1p18f, b = x[2 * p + 1] * 0x1p18f;
+        const __half2 hh = __floats2half2_rn(a, b);
+        const __half2 ll = __floats2half2_rn(a - __low2float(hh), b - __high2float(hh));
+        hw[p] = *reinterpret_cast<const unsigned *>(&hh);
+        lw[p] = *reinterpret_cast<const unsigned *>(&ll);
+    }
+    h = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+    l = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+}
+
+// one thread of warp 15 issues, warps of quadrants 0 and 1 fold; see k_fix_potf2
+struct PfCtx {
+    uint64_t *sfull; // two mbarriers
+    uint32_t tmem;
+    int n0, n1;      // their completed phases
+    bool live;       // no wait has run out
+};
+// D = A B^T of 64 x 64 blocks with NA and NBD digits into v (folding warps: row quad * 32 + lane, columns part * 16
+// + c).  Begins with a barrier: the digits are written, the accumulators free.
+template <int NA, int NBD> CAPS_DEV void pf_product(uint32_t a, uint32_t b, long long (&v)[16], PfCtx &C)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, part = warp >> 2;
+    umma::fence_smem_async();
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    if (warp == 15) {
+        if (lane == 0) {
+            mma_groups<NA, NBD, IMG_BLK, 0, SY_G0>(C.tmem, umma::desc_lo(a, 128), umma::desc_lo(b, 128));
+            umma::commit(&C.sfull[0]);
+            mma_groups<NA, NBD, IMG_BLK, SY_G0, NG>(C.tmem, umma::desc_lo(a, 128), umma::desc_lo(b, 128));
+            umma::commit(&C.sfull[1]);
+        }
+        __syncwarp();
+    } else if (quad < 2) {
+#pragma unroll
+        for (int c = 0; c < 16; c++) v[c] = 0;
+#pragma unroll 1
+        for (int g = 0; g < NG; g++) {
+            if (g == 0 || g == SY_G0) {
+                C.live = C.live && umma::mbar_wait(&C.sfull[g ? 1 : 0], (g ? C.n1 : C.n0) & 1, FIX_WAIT_ITERS);
+                C.live = __all_sync(0xffffffffu, C.live);
+                umma::fence_after();
+            }
+            if (C.live) fold_group(C.tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
+        }
+        umma::fence_before();
+    }
+    C.n0++;
+    C.n1++;
+}
+
+// digits of this warp's 16 columns of a folded product into an image
+CAPS_DEV void pf_store(const long long (&v)[16], unsigned char *img)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3, part = warp >> 2;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
         long long x[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int c = kc * 8 + u;
-            const long long v = c <= j ? W[j * PP + c] : 0;
-            x[u] = sh >= 0 ? v << sh : (v + (1LL << (-sh - 1))) >> -sh;
-        }
+        for (int u = 0; u < 8; u++) x[u] = v[q * 8 + u];
         uint4 d[ND];
         split8(x, d);
 #pragma unroll
-        for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(img + i * IMG_BLK + img_off(j, kc)) = d[i];
-    }
-    const int anybad = __syncthreads_or(bad);
-    if (tid == 0) {
-        wk.info[task].wexp = wexp;
-        logdet[(size_t)task * fix_nbk(n) + k0 / NB] = 0.5 * (slog[0] + slog[1]);
-        if (anybad) atomicOr(status + task, ST_ERR_PIVOT);
+        for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(img + i * IMG_BLK + img_off(quad * 32 + lane, part * 2 + q)) = d[i];
     }
 }
-constexpr int POTF2_SMEM = NB * PP * 16 + 3 * 16 * 17 * 8;
+
+__global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0, const long long *S, size_t lda, size_t mstride, int *status,
+                                                        FixWork wk, double *logdet)
+{
+    const int task = blockIdx.x;
+    if (task >= ntask || status[task] != ST_FACTOR) return;
+    extern __shared__ __align__(1024) unsigned char pf_sm[];
+    float *F = reinterpret_cast<float *>(pf_sm + PF_F), *X = F + NB * PP;
+    int *W27 = reinterpret_cast<int *>(X); // W0 2^-wexp in units of 2^-26
+    __shared__ float rinv[NB];
+    __shared__ uint64_t sfull[2], drain;
+    __shared__ uint32_t tslot;
+    __shared__ int s_ok, s_max, s_emax;
+    __shared__ double slog[2];
+    __shared__ long long sy;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, part = warp >> 2;
+    const bool folds = quad < 2;
+    const int nb = min(NB, n - k0);
+    const long long *Sm = S + (size_t)task * mstride + (size_t)k0 * lda + k0;
+    constexpr float Q2F = 0x1p-60f;
+    const int er = tid & 63, ek = tid >> 6; // this thread's row and chunk of 8 columns of an image
+    {
+        long long x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) { // the symmetric block, the identity past the matrix
+            const int c = ek * 8 + u, hi = max(er, c), lo = min(er, c);
+            x[u] = hi < nb ? Sm[(size_t)lo * lda + hi] : (er == c ? 1LL << FQ : 0LL);
+        }
+        if (tid == 0) {
+            umma::mbar_init(&sfull[0], 1);
+            umma::mbar_init(&sfull[1], 1);
+            umma::mbar_init(&drain, 1);
+            s_ok = 1;
+            s_max = s_emax = 0;
+            sy = 0;
+        }
+        if (warp == 15) umma::alloc(&tslot, 512);
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (ek * 8 + u <= er) F[er * PP + ek * 8 + u] = (float)x[u] * Q2F;
+        uint4 d[ND];
+        split8(x, d);
+#pragma unroll
+        for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(pf_sm + i * IMG_BLK + img_off(er, ek)) = d[i];
+    }
+    if (!pf_factor32(F, X, rinv)) s_ok = 0; // its barriers publish s_ok's first value; the ones below this
+    {
+        float mx = 0.0f;
+#pragma unroll
+        for (int u = 0; u < 8; u++) mx = fmaxf(mx, fabsf(X[er * PP + ek * 8 + u]));
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (lane == 0) atomicMax(&s_max, __float_as_int(mx)); // non-negative floats order as integers; NaN is large
+    }
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    const float w0max = __int_as_float(s_max);
+    bool ok = s_ok && w0max < 1e6f; // uniform
+    int wexp = 0;
+    while (wexp < 24 && w0max > 3.9f * (float)(1 << wexp)) wexp++;
+    PfCtx C{sfull, tslot, 0, 0, true};
+    if (ok) {
+        const float sc = (float)(1 << 26) / (float)(1 << wexp);
+        const uint32_t base = umma::smem_u32(pf_sm);
+        // W0 in place as integers of 27 bits, then its digits, by rows and by columns
+#pragma unroll
+        for (int u = 0; u < 8; u++) W27[er * PP + ek * 8 + u] = __float2int_rn(X[er * PP + ek * 8 + u] * sc);
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            long long x[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) x[u] = (long long)(t ? W27[(ek * 8 + u) * PP + er] : W27[er * PP + ek * 8 + u]) << (FQ - 26);
+            uint4 d[ND];
+            split8(x, d); // the last three digits are zero
+#pragma unroll
+            for (int i = 0; i < 3; i++) *reinterpret_cast<uint4 *>(pf_sm + (t ? PF_WT : PF_W0) + i * IMG_BLK + img_off(er, ek)) = d[i];
+        }
+        long long v[16];
+        // T = W0 S, in the digits' place afterwards
+        pf_product<3, ND>(base + PF_W0, base, v, C);
+        if (folds) pf_store(v, pf_sm);
+        if (warp == 2 || warp == 3) { // logarithms of W0_jj on warps that neither fold nor issue
+            const int j = (warp - 2) * 32 + lane;
+            const double w = (double)W27[j * PP + j] * pow2i(wexp - 26);
+            double lw = j < nb ? (w > 0.5 && w < 2.0 ? log1p(w - 1.0) : log(w)) : 0.0;
+            for (int o = 16; o > 0; o >>= 1) lw += __shfl_xor_sync(0xffffffffu, lw, o);
+            if (lane == 0) slog[warp - 2] = lw;
+        }
+        // E = T W0^T - I; P = F(E) in FP32 in place of L
+        pf_product<ND, 3>(base, base + PF_W0, v, C);
+        const int row = quad * 32 + lane, c0 = part * 16;
+        if (folds) {
+            int mx = 0;
+#pragma unroll
+            for (int c = 0; c < 16; c++) {
+                v[c] = (v[c] << (2 * wexp)) - (row == c0 + c ? 1LL << FQ : 0LL);
+                const float e = (float)v[c] * Q2F;
+                F[row * PP + c0 + c] = row > c0 + c ? e : row == c0 + c ? 0.5f * e : 0.0f;
+                mx = max(mx, __float_as_int(fabsf(e)));
+            }
+            for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            if (lane == 0) atomicMax(&s_emax, mx);
+        }
+        __syncthreads(); // the MMAs have read T: P's parts take its place (rows high, low, columns high, low)
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            float x[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) x[u] = t ? F[(ek * 8 + u) * PP + er] : F[er * PP + ek * 8 + u];
+            uint4 h, l;
+            split_half(x, h, l);
+            *reinterpret_cast<uint4 *>(pf_sm + (2 * t) * IMG_BLK + img_off(er, ek)) = h;
+            *reinterpret_cast<uint4 *>(pf_sm + (2 * t + 1) * IMG_BLK + img_off(er, ek)) = l;
+        }
+        const float emax = __int_as_float(s_emax);
+        // P P^T and P^2, scaled by 2^36: high high + high low + low high
+        umma::fence_smem_async();
+        umma::fence_before();
+        __syncthreads();
+        umma::fence_after();
+        if (warp == 15) {
+            if (lane == 0) {
+                constexpr uint32_t idesc = umma::idesc_f16(128, 64), hi = umma::desc_hi(1024);
+                const uint32_t ph = umma::desc_lo(base, 128), pl = ph + IMG_BLK / 16;
+#pragma unroll
+                for (int t = 0; t < 2; t++) {
+                    const uint32_t qh = ph + t * 2 * IMG_BLK / 16, ql = qh + IMG_BLK / 16, d = C.tmem + t * NB;
+#pragma unroll
+                    for (int ks = 0; ks < 4; ks++) {
+                        if (ks == 0) umma::mma_f16_lo<0>(d, ph, ql, hi, idesc);
+                        else umma::mma_f16_lo<1>(d, ph + ks * 16, ql + ks * 16, hi, idesc);
+                        umma::mma_f16_lo<1>(d, pl + ks * 16, qh + ks * 16, hi, idesc);
+                        umma::mma_f16_lo<1>(d, ph + ks * 16, qh + ks * 16, hi, idesc);
+                    }
+                }
+                umma::commit(&sfull[0]);
+            }
+            __syncwarp();
+        } else if (folds) {
+            C.live = C.live && umma::mbar_wait(&sfull[0], C.n0 & 1, FIX_WAIT_ITERS);
+            C.live = __all_sync(0xffffffffu, C.live);
+            umma::fence_after();
+            if (C.live) {
+                float gg[16], pp[16];
+                umma::ld16(C.tmem + ((uint32_t)(quad * 32) << 16) + c0, gg);
+                umma::ld16(C.tmem + ((uint32_t)(quad * 32) << 16) + NB + c0, pp);
+                long long ysum = 0;
+#pragma unroll
+                for (int c = 0; c < 16; c++) {
+                    // Z = F(E) - F(P P^T) - P^2; log(1 + y) = y - y^2 / 2 + y^3 / 3 of Y's diagonal
+                    const bool dg = row == c0 + c;
+                    const long long e = dg ? v[c] >> 1 : v[c];
+                    const float g = dg ? 0.5f * gg[c] : gg[c];
+                    if (dg && row < nb) {
+                        const float y = (float)e * Q2F;
+                        ysum = e - __float2ll_rn(g * 0x1p24f + y * y * (0.5f - 0.33333333f * y) * 0x1p60f);
+                    }
+                    v[c] = row >= c0 + c ? e - __float2ll_rn((g + pp[c]) * 0x1p24f) : 0;
+                }
+                if (ysum) atomicAdd(reinterpret_cast<unsigned long long *>(&sy), (unsigned long long)ysum);
+                pf_store(v, pf_sm); // Z's digits; every MMA so far has completed
+            }
+            umma::fence_before();
+        }
+        C.n0++;
+        // W = W0 - Z W0, its digits straight to the image (below 4: the top digit stays below 1024)
+        pf_product<ND, 3>(base, base + PF_WT, v, C);
+        if (folds) {
+#pragma unroll
+            for (int c = 0; c < 16; c++) v[c] = ((long long)W27[row * PP + c0 + c] << (FQ - 26)) - v[c];
+            if (C.live) pf_store(v, wk.wimg(task, n));
+        }
+        ok = emax < 0x1p-18f;
+    }
+    if (!__syncthreads_and(C.live)) {
+        if (tid == 0) atomicOr(status + task, ST_ERR_WAIT);
+        if (tid == 15 * 32) { // the MMAs issued before the failure complete before the tensor memory goes
+            umma::commit(&drain);
+            umma::mbar_wait(&drain, 0, FIX_WAIT_ITERS);
+        }
+    } else if (ok) {
+        if (tid == 0) {
+            wk.info[task].wexp = wexp;
+            logdet[(size_t)task * fix_nbk(n) + k0 / NB] = (double)sy * 0x1p-60 - (slog[0] + slog[1]);
+        }
+    } else {
+        double lg;
+        bool bad;
+        long long *T = reinterpret_cast<long long *>(pf_sm), *W = T + NB * PP;
+        const int wq = potf2_limbs(Sm, lda, nb, T, W, reinterpret_cast<int2 *>(W + NB * PP), &lg, &bad);
+        __shared__ unsigned long long smax;
+        if (tid == 0) smax = 0;
+        __syncthreads();
+        unsigned long long mx = 0;
+        for (int e = tid; e < NB * NB; e += PF_NT) {
+            const int r = e >> 6, c = e & 63;
+            if (c <= r) {
+                const long long w = W[r * PP + c];
+                mx = max(mx, (unsigned long long)(w < 0 ? -w : w));
+            }
+        }
+        atomicMax(&smax, mx);
+        __syncthreads();
+        int we = 0;
+        while (we < 40 && (float)smax * exp2f((float)(-wq - we)) > 3.9f) we++;
+        unsigned char *img = wk.wimg(task, n);
+        const int sh = FQ - wq - we;
+        for (int e = tid; e < NB * 8; e += PF_NT) {
+            const int j = e & 63, kc = e >> 6;
+            long long x[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int c = kc * 8 + u;
+                const long long w = c <= j ? W[j * PP + c] : 0;
+                x[u] = sh >= 0 ? w << sh : (w + (1LL << (-sh - 1))) >> -sh;
+            }
+            uint4 d[ND];
+            split8(x, d);
+#pragma unroll
+            for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(img + i * IMG_BLK + img_off(j, kc)) = d[i];
+        }
+        if (tid == 0) {
+            wk.info[task].wexp = we;
+            logdet[(size_t)task * fix_nbk(n) + k0 / NB] = lg;
+            if (bad) atomicOr(status + task, ST_ERR_PIVOT);
+        }
+    }
+    umma::fence_before();
+    __syncthreads();
+    if (warp == 15) {
+        umma::fence_after();
+        umma::dealloc(C.tmem, 512);
+    }
+}
 
 // ---------------------------------------------------------------------------
 // panel solve: X = S W^T for 128 rows below the diagonal block
 // ---------------------------------------------------------------------------
-// grid (ceil(rows / 128), ntask), 256 threads, 144 KB of shared memory.  The threads split the
+// grid (ceil(rows / 128), ntask), 512 threads, 144 KB of shared memory.  The threads split the
 // rows of S into digits while the digits of W arrive by bulk copies; one thread issues the
-// MMAs of each group, and all warps fold the accumulators (lane quadrant warp mod 4, 32 of
-// the 64 columns), split X and store its images.  Rows past n are zero.
+// MMAs of each group, and all warps fold the accumulators (lane quadrant warp mod 4, 16 of
+// the 64 columns), split X and store its images.  Rows past n are zero.  Bound by its latencies (loads, 104
+// MMAs, fold): with 256 threads and the loads in four rounds 45 us for 336 CTAs.
+constexpr int TR_NT = 512;
 constexpr int TR_A = ND * 2 * IMG_BLK, TR_B = ND * IMG_BLK; // 96 KB, 48 KB
 constexpr int TR_SMEM = TR_A + TR_B;
-__global__ void __launch_bounds__(256) k_fix_trsm(int ntask, int n, int k0, const long long *S, size_t lda, size_t mstride, int *status,
-                                                  FixWork wk)
+__global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, const long long *S, size_t lda, size_t mstride, int *status,
+                                                    FixWork wk)
 {
     const int task = blockIdx.y;
     if (task >= ntask || (status[task] & ~ST_ERR_WAIT) != ST_FACTOR) return; // a wait error of this launch is masked: uniform per block
     extern __shared__ __align__(1024) unsigned char tr_sm[];
-    __shared__ uint64_t wfull, gfull[NG];
+    __shared__ uint64_t wfull, gfull[2];
     __shared__ uint32_t tslot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = k0 + NB + blockIdx.x * 128;
-    if (warp == 0) umma::alloc(&tslot, 512);
-    if (tid == 0) {
-        umma::mbar_init(&wfull, 1);
-        for (int g = 0; g < NG; g++) umma::mbar_init(&gfull[g], 1);
-        umma::mbar_arrive_tx(&wfull, TR_B);
-        umma::bulk_g2s(tr_sm + TR_A, wk.wimg(task, n), TR_B, &wfull);
-    }
     const long long *Sm = S + (size_t)task * mstride;
     {
-        const int r = tid & 127, R = row0 + r;
-        for (int kc = tid >> 7; kc < 8; kc += 2) {
-            long long x[8];
+        const int r = tid & 127, R = row0 + r, kc = tid >> 7; // chunks kc and kc + 4 of 8 columns
+        long long x[16];
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = R < n ? Sm[(size_t)(k0 + kc * 8 + u) * lda + R] : 0;
+        for (int u = 0; u < 16; u++) x[u] = R < n ? Sm[(size_t)(k0 + (kc + (u >> 3) * 4) * 8 + (u & 7)) * lda + R] : 0;
+        if (warp == 0) umma::alloc(&tslot, 512);
+        if (tid == 0) {
+            umma::mbar_init(&wfull, 1);
+            for (int g = 0; g < 2; g++) umma::mbar_init(&gfull[g], 1);
+            umma::mbar_arrive_tx(&wfull, TR_B);
+            umma::bulk_g2s(tr_sm + TR_A, wk.wimg(task, n), TR_B, &wfull);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            long long y[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) y[u] = x[h * 8 + u];
             uint4 d[ND];
-            split8(x, d);
+            split8(y, d);
 #pragma unroll
-            for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(tr_sm + i * 2 * IMG_BLK + img_off(r, kc)) = d[i];
+            for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(tr_sm + i * 2 * IMG_BLK + img_off(r, kc + h * 4)) = d[i];
         }
     }
     umma::fence_smem_async();
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
-    const uint32_t tmem = tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tslot, 0);
     const bool have = umma::mbar_wait(&wfull, 0, FIX_WAIT_ITERS);
     if (!have && tid == 0) atomicOr(status + task, ST_ERR_WAIT);
     bool ok = have;
     if (warp == 0 && have) {
+        const uint32_t a = umma::desc_lo(umma::smem_u32(tr_sm), 128), b = a + TR_A / 16;
         if (lane == 0) {
-            const uint32_t a = umma::smem_u32(tr_sm), b = a + TR_A;
-            for (int g = 0; g < NG; g++) {
-                mma_group(tmem + g * NB, a, b, NG - 1 - g);
-                umma::commit(&gfull[g]);
-            }
+            mma_groups<ND, ND, 2 * IMG_BLK, 0, SY_G0>(tmem, a, b);
+            umma::commit(&gfull[0]);
+            mma_groups<ND, ND, 2 * IMG_BLK, SY_G0, NG>(tmem, a, b);
+            umma::commit(&gfull[1]);
         }
         __syncwarp();
     }
-    const int quad = warp & 3, half = warp >> 2;
-    long long v[32];
+    const int quad = warp & 3, part = warp >> 2;
+    long long v[16];
 #pragma unroll
+    for (int c = 0; c < 16; c++) v[c] = 0;
+#pragma unroll 1
     for (int g = 0; g < NG; g++) {
-        ok = ok && umma::mbar_wait(&gfull[g], 0, FIX_WAIT_ITERS);
-        ok = __all_sync(0xffffffffu, ok);
-        umma::fence_after();
-        if (ok) fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + half * 32, NG - 1 - g, v);
+        if (g == 0 || g == SY_G0) {
+            ok = ok && umma::mbar_wait(&gfull[g ? 1 : 0], 0, FIX_WAIT_ITERS);
+            ok = __all_sync(0xffffffffu, ok);
+            umma::fence_after();
+        }
+        if (ok) fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
     }
     if (ok) {
         const int wexp = wk.info[task].wexp;
@@ -504,20 +903,20 @@ __global__ void __launch_bounds__(256) k_fix_trsm(int ntask, int n, int k0, cons
         const size_t dst = (size_t)(fix_nbk(n) + 1) * IMG_BLK;          // digit to digit
         unsigned char *img = wk.ximg(task, n) + (size_t)blk * IMG_BLK;
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < 2; q++) {
             long long x[8];
 #pragma unroll
             for (int u = 0; u < 8; u++) x[u] = v[q * 8 + u] << wexp;
             uint4 d[ND];
             split8(x, d);
 #pragma unroll
-            for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(img + i * dst + img_off(r & 63, half * 4 + q)) = d[i];
+            for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(img + i * dst + img_off(r & 63, part * 2 + q)) = d[i];
         }
     } else if (lane == 0)
         atomicOr(status + task, ST_ERR_WAIT);
-    // a group's wait that ran out leaves its MMAs in flight: wait for the last of them (bounded)
+    // a wait that ran out leaves MMAs in flight: wait for the last of them (bounded)
     // before the tensor memory goes
-    if (tid == 0 && have && !ok) umma::mbar_wait(&gfull[NG - 1], 0, FIX_WAIT_ITERS);
+    if (tid == 0 && have && !ok) umma::mbar_wait(&gfull[1], 0, FIX_WAIT_ITERS);
     umma::fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -532,11 +931,10 @@ __global__ void __launch_bounds__(256) k_fix_trsm(int ntask, int n, int k0, cons
 // A CTA takes one pair of row blocks (128 rows) against up to `chunk` 64-column blocks: the rows'
 // digits (96 KB) stay in shared memory, the columns' (48 KB) come in two stages.  Warp 16 copies,
 // warp 17 issues the MMAs (104 of 128 x 64 x 16 per tile), warps 0..15 fold and update S (lane
-// quadrant warp mod 4, 16 of the 64 columns).  The 512
-// columns of tensor memory are a ring of eight 64-column slots; a tile takes seven in turn, one
-// per group, and a slot is free again once the epilogue has folded it, so that the MMAs of the
-// next tile run under the epilogue of this one.
-constexpr int SY_EPI = 16, SY_THREADS = (SY_EPI + 2) * 32, SY_SLOTS = 8;
+// quadrant warp mod 4, 16 of the 64 columns).  The accumulators are handed over in two parts, groups 0..3 (40
+// MMAs) and 4..6 (64), each folded while the MMAs of the other run (with a hand-over per group and a
+// ring of eight accumulators the hand-overs alone took 2.6 us per tile).
+constexpr int SY_EPI = 16, SY_THREADS = (SY_EPI + 2) * 32;
 constexpr int SY_SMEM = TR_A + 2 * TR_B; // 192 KB
 __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, int t0, int chunk, long long *S, size_t lda, size_t mstride,
                                                             int *status, FixWork wk)
@@ -554,7 +952,7 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
     if (p < 0) return;
     const int j0 = it * chunk, j1 = min(j0 + chunk, min(2 * p + 2, nbt));
     extern __shared__ __align__(1024) unsigned char sy_sm[];
-    __shared__ uint64_t afull, bfull[2], bempty[2], sfull[SY_SLOTS], sempty[SY_SLOTS], drain;
+    __shared__ uint64_t afull, bfull[2], bempty[2], sfull[2], sempty[2], drain;
     __shared__ uint32_t tslot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) umma::alloc(&tslot, 512);
@@ -563,8 +961,6 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
         for (int i = 0; i < 2; i++) {
             umma::mbar_init(&bfull[i], 1);
             umma::mbar_init(&bempty[i], 1);
-        }
-        for (int i = 0; i < SY_SLOTS; i++) {
             umma::mbar_init(&sfull[i], 1);
             umma::mbar_init(&sempty[i], SY_EPI);
         }
@@ -573,44 +969,42 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
-    const uint32_t tmem = tslot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tslot, 0);
     if (warp < SY_EPI) {
         const int quad = warp & 3, part = warp >> 2;
         const int R = t0 + p * 128 + quad * 32 + lane;
         long long *Sm = S + (size_t)task * mstride + R;
-        int use = 0;
         for (int j = j0; j < j1; j++) {
             const int c0 = t0 + j * NB + part * 16;
             const int jm = R < n ? min(n - c0, R - c0 + 1) : 0; // columns c0 .. c0 + jm - 1 of this row
-            long long *dst = Sm + (size_t)c0 * lda;
+            unsigned long long *dst = reinterpret_cast<unsigned long long *>(Sm + (size_t)c0 * lda);
             long long v[16];
-            bool ok = true;
 #pragma unroll
-            for (int g = 0; g < NG; g++, use++) {
-                const int slot = use % SY_SLOTS;
-                ok = ok && umma::mbar_wait(&sfull[slot], (use / SY_SLOTS) & 1, FIX_WAIT_ITERS);
+            for (int c = 0; c < 16; c++) v[c] = 0;
+            bool ok = true;
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                ok = ok && umma::mbar_wait(&sfull[h], (j - j0) & 1, FIX_WAIT_ITERS);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 umma::fence_after();
-                fold_group(tmem + ((uint32_t)(quad * 32) << 16) + slot * NB + part * 16, NG - 1 - g, v);
+#pragma unroll 1
+                for (int g = h ? SY_G0 : 0; g < (h ? NG : SY_G0); g++)
+                    fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
                 umma::fence_before();
                 __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(&sempty[slot])) : "memory");
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(&sempty[h])) : "memory");
             }
             if (!ok) {
                 if (lane == 0) atomicOr(status + task, ST_ERR_WAIT);
                 break;
             }
-            // the accumulators are free: these loads and stores run under the next tile's MMAs
+            // the subtraction as an atomic add at the L2 cache: exact in integers, and no load's latency
+            // stands between the accumulators and the next tile (loads and stores: 287 us for the second
+            // panel of 24 matrices of dimension 2100)
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                long long cur[8];
-#pragma unroll
-                for (int c = 0; c < 8; c++) cur[c] = h * 8 + c < jm ? dst[(size_t)(h * 8 + c) * lda] : 0;
-#pragma unroll
-                for (int c = 0; c < 8; c++)
-                    if (h * 8 + c < jm) dst[(size_t)(h * 8 + c) * lda] = cur[c] - v[h * 8 + c];
-            }
+            for (int c = 0; c < 16; c++)
+                if (c < jm) atomicAdd(dst + (size_t)c * lda, 0ULL - (unsigned long long)v[c]);
         }
     } else if (warp == SY_EPI) {
         if (lane == 0) {
@@ -636,20 +1030,20 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
                 if (last[s] >= 0) umma::mbar_wait(&bfull[s], last[s] & 1, FIX_WAIT_ITERS);
         }
     } else if (lane == 0) {
-        const uint32_t a = umma::smem_u32(sy_sm);
+        const uint32_t a = umma::desc_lo(umma::smem_u32(sy_sm), 128);
         bool ok = umma::mbar_wait(&afull, 0, FIX_WAIT_ITERS);
-        int use = 0;
         for (int j = j0; ok && j < j1; j++) {
             const int q = j - j0, s = q & 1, u = q >> 1;
             ok = umma::mbar_wait(&bfull[s], u & 1, FIX_WAIT_ITERS);
             umma::fence_after();
-            for (int g = 0; ok && g < NG; g++, use++) {
-                const int slot = use % SY_SLOTS;
-                if (use >= SY_SLOTS) ok = umma::mbar_wait(&sempty[slot], (use / SY_SLOTS - 1) & 1, FIX_WAIT_ITERS);
+            for (int h = 0; ok && h < 2; h++) {
+                if (q > 0) ok = umma::mbar_wait(&sempty[h], (q - 1) & 1, FIX_WAIT_ITERS);
                 if (!ok) break;
                 umma::fence_after();
-                mma_group(tmem + slot * NB, a, a + TR_A + s * TR_B, NG - 1 - g);
-                umma::commit(&sfull[slot]);
+                const uint32_t b = a + (TR_A + s * TR_B) / 16;
+                if (h == 0) mma_groups<ND, ND, 2 * IMG_BLK, 0, SY_G0>(tmem, a, b);
+                else mma_groups<ND, ND, 2 * IMG_BLK, SY_G0, NG>(tmem, a, b);
+                umma::commit(&sfull[h]);
             }
             umma::commit(&bempty[s]);
         }
@@ -709,7 +1103,7 @@ void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, in
     static bool attr = false;
     static int sms = 148;
     if (!attr) {
-        CK(cudaFuncSetAttribute(k_fix_potf2, cudaFuncAttributeMaxDynamicSharedMemorySize, POTF2_SMEM));
+        CK(cudaFuncSetAttribute(k_fix_potf2, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
         CK(cudaFuncSetAttribute(k_fix_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, TR_SMEM));
         CK(cudaFuncSetAttribute(k_fix_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, SY_SMEM));
         int dev = 0;
@@ -725,11 +1119,11 @@ void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, in
         COUNT_LAUNCH(1);
     }
     for (int k0 = 0; k0 < n; k0 += NB) {
-        k_fix_potf2<<<ntask, 256, POTF2_SMEM, st>>>(ntask, n, k0, S, lda, mstride, status, wk, logdet);
+        k_fix_potf2<<<ntask, PF_NT, PF_SMEM, st>>>(ntask, n, k0, S, lda, mstride, status, wk, logdet);
         COUNT_LAUNCH(1);
         const int t0 = k0 + NB, rest = n - t0;
         if (rest <= 0) break;
-        k_fix_trsm<<<dim3((rest + 127) / 128, ntask), 256, TR_SMEM, st>>>(ntask, n, k0, S, lda, mstride, status, wk);
+        k_fix_trsm<<<dim3((rest + 127) / 128, ntask), TR_NT, TR_SMEM, st>>>(ntask, n, k0, S, lda, mstride, status, wk);
         COUNT_LAUNCH(1);
         // tiles per CTA: about three CTAs per SM where the batch is small, at most 8 tiles
         const int nbt = (rest + NB - 1) / NB, np = (nbt + 1) / 2;

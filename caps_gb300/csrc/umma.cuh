@@ -62,6 +62,19 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
                  "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
+// the two words of a K-major descriptor: the low one holds the address (16-byte units) and lbo, so that
+// a byte offset o moves it by o / 16; the high one (sbo, version) stays the same.  A single thread
+// issues all MMAs of a CTA, and forming 64-bit descriptors in a loop took it longer (150 clocks per
+// MMA) than the tensor cores take for a 128 x 64 x 16 one (51; 128 x 128 x 16: 66)
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr, uint32_t lbo) { return (saddr >> 4) | (lbo >> 4) << 16; }
+__host__ __device__ constexpr uint32_t desc_hi(uint32_t sbo) { return (sbo >> 4) | 1u << 14; }
+template <uint32_t ACC>
+__device__ __forceinline__ void mma_f16_lo(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t hi, uint32_t idesc)
+{
+    asm volatile("{\n\t.reg .b64 a, b;\n\t.reg .pred p;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}" ::"r"(tmem_d),
+                 "r"(alo), "r"(blo), "r"(hi), "r"(idesc), "n"(ACC));
+}
 // arrive on the mbarrier once every MMA issued so far by this thread has completed
 __device__ __forceinline__ void commit(uint64_t *mbar)
 {
