@@ -45,9 +45,12 @@ __host__ __device__ inline int fix_nbk(int n) { return (n + NB - 1) / NB; }
 __host__ __device__ inline size_t fix_ximg_bytes(int n) { return (size_t)(fix_nbk(n) + 1) * ND * IMG_BLK; }
 __host__ __device__ inline size_t fix_task_bytes(int n) { return (size_t)ND * IMG_BLK + fix_ximg_bytes(n); }
 struct FixInfo { int sexp, wexp; };          // A 2^-sexp is factored; W 2^-wexp is in the image
+// first[task * (nbk + 1) + block]: the first digit of the current panel's X that is not zero in the whole 64-row
+// block (block counted below the diagonal block; NG: none)
 struct FixWork {
     unsigned char *img;
     FixInfo *info;
+    int *first;
     __host__ __device__ unsigned char *wimg(int task, int n) const { return img + (size_t)task * fix_task_bytes(n); }
     __host__ __device__ unsigned char *ximg(int task, int n) const { return wimg(task, n) + (size_t)ND * IMG_BLK; }
 };
@@ -57,6 +60,20 @@ struct FixWork {
 CAPS_DEV int img_off(int row, int kcore) { return (row >> 3) * 1024 + kcore * 128 + (row & 7) * 16; }
 
 // ---- digits ----
+// the magnitude of x (units of 2^-60) as digits see it, in units of 2^-53: its bit length bounds the digits
+// that are not zero (k digits hold +-255 (512^k - 1) / 511)
+CAPS_DEV unsigned long long digit_mag(long long x)
+{
+    const long long y = (x + 64) >> 7;
+    return (unsigned long long)(y < 0 ? -y : y);
+}
+// first digit that may be nonzero, from the bitwise or of magnitudes; NG: none is
+CAPS_DEV int first_digit(unsigned long long any)
+{
+    const int bits = 64 - __clzll((long long)any);
+    return bits == 0 ? NG : bits <= 8 ? 5 : bits <= 16 ? 4 : bits <= 25 ? 3 : bits <= 34 ? 2 : bits <= 43 ? 1 : 0;
+}
+
 // eight numbers (units of 2^-60, |x| < 4) to six 16-byte vectors of FP16 digits
 CAPS_DEV void split8(const long long (&x)[8], uint4 (&d)[ND])
 {
@@ -108,6 +125,30 @@ template <int NA, int NBD, int ASTEP, int G0, int G1> CAPS_DEV void mma_groups(u
                     else umma::mma_f16_lo<1>(d, a, b, hi, idesc);
                 }
             }
+    }
+}
+
+// the same for groups g0 .. g1 - 1 and ND x ND digits of which the first fa of A and fb of B are zero: their
+// products are left out, and groups below fa + fb have none.  Entries of the factor fall off so fast
+// away from the diagonal that of all products in the trailing updates of a free energy's matrices
+// (R/L = 50) 5 % are left, and a third of the tiles have any.
+CAPS_DEV void mma_nonzero(uint32_t tmem, uint32_t alo, uint32_t blo, int fa, int fb, int g0, int g1)
+{
+    constexpr uint32_t idesc = umma::idesc_f16(128, 64), hi = umma::desc_hi(1024);
+    for (int g = max(g0, fa + fb); g < g1; g++) {
+        const int i0 = max(fa, g - (ND - 1)), i1 = min(ND - 1, g - fb);
+        uint32_t a = alo + i0 * (2 * IMG_BLK / 16), b = blo + (g - i0) * (IMG_BLK / 16);
+        const uint32_t d = tmem + g * NB;
+        umma::mma_f16_lo<0>(d, a, b, hi, idesc);
+#pragma unroll
+        for (int ks = 1; ks < 4; ks++) umma::mma_f16_lo<1>(d, a + ks * 16, b + ks * 16, hi, idesc);
+#pragma unroll 1
+        for (int i = i0 + 1; i <= i1; i++) {
+            a += 2 * IMG_BLK / 16;
+            b -= IMG_BLK / 16;
+#pragma unroll
+            for (int ks = 0; ks < 4; ks++) umma::mma_f16_lo<1>(d, a + ks * 16, b + ks * 16, hi, idesc);
+        }
     }
 }
 
@@ -438,16 +479,24 @@ CAPS_DEV bool pf_factor32(float *F, float *X, float *rinv)
 #pragma unroll
             for (int c = 0; c < 8; c++) a[c] = live ? F[row * PP + o + c] : 0.0f;
             asm volatile("bar.sync 1, 96;" ::: "memory"); // the three warps have read the diagonal rows
-            float rv = 0.0f;
+            // every lane keeps the panel's pivots, so that none is broadcast: the chain of a column is a
+            // reciprocal square root (2^-22, as good as the factor needs), a product, a shuffle and an fma
+            float rv = 0.0f, d[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) d[j] = __shfl_sync(0xffffffffu, a[j], j);
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const float d = __shfl_sync(0xffffffffu, a[j], j);
-                ok &= d > 1e-6f;
-                const float r = rsqrtf(fmaxf(d, 1e-6f));
+                ok &= d[j] > 1e-6f;
+                float r;
+                asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(fmaxf(d[j], 1e-6f)));
                 if (lane == j) rv = r;
                 a[j] *= r;
 #pragma unroll
-                for (int c = j + 1; c < 8; c++) a[c] = fmaf(-a[j], __shfl_sync(0xffffffffu, a[j], c), a[c]);
+                for (int c = j + 1; c < 8; c++) {
+                    const float y = __shfl_sync(0xffffffffu, a[j], c);
+                    a[c] = fmaf(-a[j], y, a[c]);
+                    d[c] = fmaf(-y, y, d[c]);
+                }
             }
             if (live && (warp == 0 || lane >= 8))
 #pragma unroll
@@ -468,45 +517,46 @@ CAPS_DEV bool pf_factor32(float *F, float *X, float *rinv)
         }
         __syncthreads();
         // 2 x 2 tiles: of the block's rest with panel p, then of X below row o with panel p - 1
-        const int ts = p < 8 ? (56 - o) / 2 : 0, ns = ts * (ts + 1) / 2, nx = p > 0 ? (NB - o) / 2 * (o / 2) : 0;
-        for (int e = tid; e < ns + nx; e += PF_NT) {
-            const float *x0, *y0;
-            float *out;
-            int ys, yk; // y of column j at y0[j * ys + k * yk]
-            bool diag = false;
-            if (e < ns) {
-                int ti = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
-                while ((ti + 1) * (ti + 2) / 2 <= e) ti++;
-                while (ti * (ti + 1) / 2 > e) ti--;
-                const int tj = e - ti * (ti + 1) / 2, rr = o + 8 + 2 * ti, cc = o + 8 + 2 * tj;
-                x0 = F + rr * PP + o;
-                y0 = F + cc * PP + o;
-                ys = PP;
-                yk = 1;
-                out = F + rr * PP + cc;
-                diag = ti == tj;
-            } else {
-                const int t = e - ns, w = o / 2, rr = o + 2 * (t / w), cc = 2 * (t % w);
-                x0 = F + rr * PP + q;
-                y0 = X + q * PP + cc;
-                ys = 1;
-                yk = PP;
-                out = X + rr * PP + cc;
-            }
-            float s00 = 0, s01 = 0, s10 = 0, s11 = 0;
+        const int ts = p < 8 ? (56 - o) / 2 : 0, ns = ts * (ts + 1) / 2;
+        // (two loops with constant strides: one loop over both kinds took twice as long)
+        for (int e = tid; e < ns; e += PF_NT) {
+            int ti = (int)((sqrtf(8.0f * e + 1.0f) - 1.0f) * 0.5f);
+            ti += (ti + 1) * (ti + 2) / 2 <= e;
+            ti -= ti * (ti + 1) / 2 > e;
+            const int tj = e - ti * (ti + 1) / 2, rr = o + 8 + 2 * ti, cc = o + 8 + 2 * tj;
+            const float *x0 = F + rr * PP + o, *y0 = F + cc * PP + o;
+            float *out = F + rr * PP + cc, s00 = 0, s01 = 0, s10 = 0, s11 = 0;
 #pragma unroll
             for (int k = 0; k < 8; k++) {
-                const float u0 = x0[k], u1 = x0[PP + k], w0 = y0[k * yk], w1 = y0[ys + k * yk];
-                s00 = fmaf(u0, w0, s00);
-                s01 = fmaf(u0, w1, s01);
-                s10 = fmaf(u1, w0, s10);
-                s11 = fmaf(u1, w1, s11);
+                s00 = fmaf(x0[k], y0[k], s00);
+                s01 = fmaf(x0[k], y0[PP + k], s01);
+                s10 = fmaf(x0[PP + k], y0[k], s10);
+                s11 = fmaf(x0[PP + k], y0[PP + k], s11);
             }
             out[0] -= s00;
-            if (!diag) out[1] -= s01;
+            if (ti != tj) out[1] -= s01;
             out[PP] -= s10;
             out[PP + 1] -= s11;
         }
+        // columns in pairs by lane, rows by warp, from the last warp on (the first have the block's tiles)
+        const int cc = 2 * lane;
+        if (cc < o)
+            for (int rr = o + 2 * (PF_NT / 32 - 1 - warp); rr < NB; rr += PF_NT / 16) {
+                const float *x0 = F + rr * PP + q, *y0 = X + q * PP + cc;
+                float *out = X + rr * PP + cc, s00 = 0, s01 = 0, s10 = 0, s11 = 0;
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const float w0 = y0[k * PP], w1 = y0[k * PP + 1];
+                    s00 = fmaf(x0[k], w0, s00);
+                    s01 = fmaf(x0[k], w1, s01);
+                    s10 = fmaf(x0[PP + k], w0, s10);
+                    s11 = fmaf(x0[PP + k], w1, s11);
+                }
+                out[0] -= s00;
+                out[1] -= s01;
+                out[PP] -= s10;
+                out[PP + 1] -= s11;
+            }
         __syncthreads();
     }
     return ok;
@@ -607,11 +657,12 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
     constexpr float Q2F = 0x1p-60f;
     const int er = tid & 63, ek = tid >> 6; // this thread's row and chunk of 8 columns of an image
     {
-        long long x[8];
+        // the lower triangle (the identity past the matrix), mirrored in shared memory
+        long long x[8], *tmp = reinterpret_cast<long long *>(pf_sm + PF_W0); // [64][PP]
 #pragma unroll
-        for (int u = 0; u < 8; u++) { // the symmetric block, the identity past the matrix
-            const int c = ek * 8 + u, hi = max(er, c), lo = min(er, c);
-            x[u] = hi < nb ? Sm[(size_t)lo * lda + hi] : (er == c ? 1LL << FQ : 0LL);
+        for (int u = 0; u < 8; u++) {
+            const int c = ek * 8 + u;
+            x[u] = c <= er && er < nb ? Sm[(size_t)c * lda + er] : (er == c ? 1LL << FQ : 0LL);
         }
         if (tid == 0) {
             umma::mbar_init(&sfull[0], 1);
@@ -623,8 +674,17 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
         }
         if (warp == 15) umma::alloc(&tslot, 512);
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (ek * 8 + u <= er) F[er * PP + ek * 8 + u] = (float)x[u] * Q2F;
+        for (int u = 0; u < 8; u++) {
+            const int c = ek * 8 + u;
+            if (c <= er) {
+                F[er * PP + c] = (float)x[u] * Q2F;
+                tmp[er * PP + c] = x[u];
+                tmp[c * PP + er] = x[u];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = tmp[er * PP + ek * 8 + u];
         uint4 d[ND];
         split8(x, d);
 #pragma unroll
@@ -741,9 +801,9 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
                     const float g = dg ? 0.5f * gg[c] : gg[c];
                     if (dg && row < nb) {
                         const float y = (float)e * Q2F;
-                        ysum = e - __float2ll_rn(g * 0x1p24f + y * y * (0.5f - 0.33333333f * y) * 0x1p60f);
+                        ysum = e - __float2int_rn(g * 0x1p24f + y * y * (0.5f - 0.33333333f * y) * 0x1p60f);
                     }
-                    v[c] = row >= c0 + c ? e - __float2ll_rn((g + pp[c]) * 0x1p24f) : 0;
+                    v[c] = row >= c0 + c ? e - __float2int_rn((g + pp[c]) * 0x1p24f) : 0; // below 2^30 for |E| < 2^-18
                 }
                 if (ysum) atomicAdd(reinterpret_cast<unsigned long long *>(&sy), (unsigned long long)ysum);
                 pf_store(v, pf_sm); // Z's digits; every MMA so far has completed
@@ -839,15 +899,31 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
     if (task >= ntask || (status[task] & ~ST_ERR_WAIT) != ST_FACTOR) return; // a wait error of this launch is masked: uniform per block
     extern __shared__ __align__(1024) unsigned char tr_sm[];
     __shared__ uint64_t wfull, gfull[2];
-    __shared__ uint32_t tslot;
+    __shared__ uint32_t tslot, s_any[2][3]; // or of the magnitudes' low and high words: S, X of both row blocks
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = k0 + NB + blockIdx.x * 128;
+    int *first = wk.first + (size_t)task * (fix_nbk(n) + 1) + blockIdx.x * 2;
     const long long *Sm = S + (size_t)task * mstride;
     {
         const int r = tid & 127, R = row0 + r, kc = tid >> 7; // chunks kc and kc + 4 of 8 columns
         long long x[16];
 #pragma unroll
         for (int u = 0; u < 16; u++) x[u] = R < n ? Sm[(size_t)(k0 + (kc + (u >> 3) * 4) * 8 + (u & 7)) * lda + R] : 0;
+        if (tid < 6) s_any[tid & 1][tid >> 1] = 0;
+        __syncthreads();
+        unsigned long long any = 0;
+#pragma unroll
+        for (int u = 0; u < 16; u++) any |= digit_mag(x[u]);
+        const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)any), hi = __reduce_or_sync(0xffffffffu, (unsigned)(any >> 32));
+        if (lane == 0 && (lo | hi)) {
+            atomicOr(&s_any[0][0], lo);
+            atomicOr(&s_any[1][0], hi);
+        }
+        __syncthreads();
+        if ((s_any[0][0] | s_any[1][0]) == 0) { // S has no digit here: X = 0
+            if (tid < 2) first[tid] = NG;
+            return;
+        }
         if (warp == 0) umma::alloc(&tslot, 512);
         if (tid == 0) {
             umma::mbar_init(&wfull, 1);
@@ -874,12 +950,13 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
     const bool have = umma::mbar_wait(&wfull, 0, FIX_WAIT_ITERS);
     if (!have && tid == 0) atomicOr(status + task, ST_ERR_WAIT);
     bool ok = have;
+    const int fa = first_digit((unsigned long long)s_any[1][0] << 32 | s_any[0][0]);
     if (warp == 0 && have) {
         const uint32_t a = umma::desc_lo(umma::smem_u32(tr_sm), 128), b = a + TR_A / 16;
         if (lane == 0) {
-            mma_groups<ND, ND, 2 * IMG_BLK, 0, SY_G0>(tmem, a, b);
+            mma_nonzero(tmem, a, b, fa, 0, 0, SY_G0);
             umma::commit(&gfull[0]);
-            mma_groups<ND, ND, 2 * IMG_BLK, SY_G0, NG>(tmem, a, b);
+            mma_nonzero(tmem, a, b, fa, 0, SY_G0, NG);
             umma::commit(&gfull[1]);
         }
         __syncwarp();
@@ -895,31 +972,48 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
             ok = __all_sync(0xffffffffu, ok);
             umma::fence_after();
         }
-        if (ok) fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
+        if (ok && g >= fa) fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
     }
+    const int wexp = wk.info[task].wexp, rb = quad >> 1; // rb: row block of the pair
+    {
+        unsigned long long any = 0;
+#pragma unroll
+        for (int c = 0; c < 16; c++) {
+            v[c] <<= wexp;
+            any |= digit_mag(v[c]);
+        }
+        const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)any), hi = __reduce_or_sync(0xffffffffu, (unsigned)(any >> 32));
+        if (lane == 0 && (lo | hi)) {
+            atomicOr(&s_any[0][1 + rb], lo);
+            atomicOr(&s_any[1][1 + rb], hi);
+        }
+    }
+    umma::fence_before();
+    __syncthreads();
+    if (tid < 2) first[tid] = first_digit((unsigned long long)s_any[1][1 + tid] << 32 | s_any[0][1 + tid]);
     if (ok) {
-        const int wexp = wk.info[task].wexp;
-        const int r = quad * 32 + lane, blk = blockIdx.x * 2 + (r >> 6); // row block below the diagonal block
+        const int r = quad * 32 + lane, blk = blockIdx.x * 2 + rb; // row block below the diagonal block
+        // digits that are zero in both blocks of the pair are not read
+        const int f = first_digit((unsigned long long)(s_any[1][1] | s_any[1][2]) << 32 | (s_any[0][1] | s_any[0][2]));
         const size_t dst = (size_t)(fix_nbk(n) + 1) * IMG_BLK;          // digit to digit
         unsigned char *img = wk.ximg(task, n) + (size_t)blk * IMG_BLK;
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             long long x[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = v[q * 8 + u] << wexp;
+            for (int u = 0; u < 8; u++) x[u] = v[q * 8 + u];
             uint4 d[ND];
             split8(x, d);
 #pragma unroll
-            for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(img + i * dst + img_off(r & 63, part * 2 + q)) = d[i];
+            for (int i = 0; i < ND; i++)
+                if (i >= f) *reinterpret_cast<uint4 *>(img + i * dst + img_off(r & 63, part * 2 + q)) = d[i];
         }
     } else if (lane == 0)
         atomicOr(status + task, ST_ERR_WAIT);
     // a wait that ran out leaves MMAs in flight: wait for the last of them (bounded)
     // before the tensor memory goes
     if (tid == 0 && have && !ok) umma::mbar_wait(&gfull[1], 0, FIX_WAIT_ITERS);
-    umma::fence_before();
-    __syncthreads();
-    if (warp == 0) {
+    if (warp == 0) { // every warp has read its accumulators (the barrier above)
         umma::fence_after();
         umma::dealloc(tmem, 512);
     }
@@ -951,6 +1045,12 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
     }
     if (p < 0) return;
     const int j0 = it * chunk, j1 = min(j0 + chunk, min(2 * p + 2, nbt));
+    // first nonzero digits of the rows and of column block j; tiles without a product are skipped
+    const int *first = wk.first + (size_t)task * (fix_nbk(n) + 1);
+    const int fa = 2 * p + 1 < nbt ? min(first[2 * p], first[2 * p + 1]) : first[2 * p];
+    bool any = false;
+    for (int j = j0; j < j1; j++) any |= fa + first[j] < NG;
+    if (!any) return; // uniform: nothing writes first in this launch
     extern __shared__ __align__(1024) unsigned char sy_sm[];
     __shared__ uint64_t afull, bfull[2], bempty[2], sfull[2], sempty[2], drain;
     __shared__ uint32_t tslot;
@@ -974,7 +1074,10 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
         const int quad = warp & 3, part = warp >> 2;
         const int R = t0 + p * 128 + quad * 32 + lane;
         long long *Sm = S + (size_t)task * mstride + R;
+        int q = 0; // tiles so far
         for (int j = j0; j < j1; j++) {
+            const int s0 = fa + first[j];
+            if (s0 >= NG) continue;
             const int c0 = t0 + j * NB + part * 16;
             const int jm = R < n ? min(n - c0, R - c0 + 1) : 0; // columns c0 .. c0 + jm - 1 of this row
             unsigned long long *dst = reinterpret_cast<unsigned long long *>(Sm + (size_t)c0 * lda);
@@ -984,12 +1087,12 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
             bool ok = true;
 #pragma unroll 1
             for (int h = 0; h < 2; h++) {
-                ok = ok && umma::mbar_wait(&sfull[h], (j - j0) & 1, FIX_WAIT_ITERS);
+                ok = ok && umma::mbar_wait(&sfull[h], q & 1, FIX_WAIT_ITERS);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 umma::fence_after();
 #pragma unroll 1
-                for (int g = h ? SY_G0 : 0; g < (h ? NG : SY_G0); g++)
+                for (int g = max(s0, h ? SY_G0 : 0); g < (h ? NG : SY_G0); g++)
                     fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
                 umma::fence_before();
                 __syncwarp();
@@ -1005,24 +1108,28 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
 #pragma unroll
             for (int c = 0; c < 16; c++)
                 if (c < jm) atomicAdd(dst + (size_t)c * lda, 0ULL - (unsigned long long)v[c]);
+            q++;
         }
     } else if (warp == SY_EPI) {
         if (lane == 0) {
             const unsigned char *img = wk.ximg(task, n);
             const size_t dstep = (size_t)(fix_nbk(n) + 1) * IMG_BLK;
-            umma::mbar_arrive_tx(&afull, TR_A);
-            for (int i = 0; i < ND; i++) umma::bulk_g2s(sy_sm + i * 2 * IMG_BLK, img + i * dstep + (size_t)2 * p * IMG_BLK, 2 * IMG_BLK, &afull);
-            int last[2] = {-1, -1};
+            umma::mbar_arrive_tx(&afull, (ND - fa) * 2 * IMG_BLK);
+            for (int i = fa; i < ND; i++) umma::bulk_g2s(sy_sm + i * 2 * IMG_BLK, img + i * dstep + (size_t)2 * p * IMG_BLK, 2 * IMG_BLK, &afull);
+            int last[2] = {-1, -1}, q = 0;
             for (int j = j0; j < j1; j++) {
-                const int q = j - j0, s = q & 1, u = q >> 1;
+                const int fb = first[j];
+                if (fa + fb >= NG) continue;
+                const int s = q & 1, u = q >> 1;
                 if (u > 0 && !umma::mbar_wait(&bempty[s], (u - 1) & 1, FIX_WAIT_ITERS)) {
                     atomicOr(status + task, ST_ERR_WAIT);
                     break;
                 }
-                umma::mbar_arrive_tx(&bfull[s], TR_B);
-                for (int i = 0; i < ND; i++)
+                umma::mbar_arrive_tx(&bfull[s], (ND - fb) * IMG_BLK);
+                for (int i = fb; i < ND; i++)
                     umma::bulk_g2s(sy_sm + TR_A + s * TR_B + i * IMG_BLK, img + i * dstep + (size_t)j * IMG_BLK, IMG_BLK, &bfull[s]);
                 last[s] = u;
+                q++;
             }
             // no copy may be in flight when the CTA leaves
             umma::mbar_wait(&afull, 0, FIX_WAIT_ITERS);
@@ -1032,8 +1139,9 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
     } else if (lane == 0) {
         const uint32_t a = umma::desc_lo(umma::smem_u32(sy_sm), 128);
         bool ok = umma::mbar_wait(&afull, 0, FIX_WAIT_ITERS);
-        for (int j = j0; ok && j < j1; j++) {
-            const int q = j - j0, s = q & 1, u = q >> 1;
+        for (int j = j0, q = 0; ok && j < j1; j++) {
+            const int fb = first[j], s = q & 1, u = q >> 1;
+            if (fa + fb >= NG) continue;
             ok = umma::mbar_wait(&bfull[s], u & 1, FIX_WAIT_ITERS);
             umma::fence_after();
             for (int h = 0; ok && h < 2; h++) {
@@ -1041,11 +1149,11 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
                 if (!ok) break;
                 umma::fence_after();
                 const uint32_t b = a + (TR_A + s * TR_B) / 16;
-                if (h == 0) mma_groups<ND, ND, 2 * IMG_BLK, 0, SY_G0>(tmem, a, b);
-                else mma_groups<ND, ND, 2 * IMG_BLK, SY_G0, NG>(tmem, a, b);
+                mma_nonzero(tmem, a, b, fa, fb, h ? SY_G0 : 0, h ? NG : SY_G0);
                 umma::commit(&sfull[h]);
             }
             umma::commit(&bempty[s]);
+            q++;
         }
         if (!ok) atomicOr(status + task, ST_ERR_WAIT);
         // every MMA this thread issued completes before the CTA frees tensor memory
@@ -1085,16 +1193,16 @@ __global__ void k_final(int ntask, int n, const double *logdet, const FixInfo *i
     result[task] = ld;
 }
 
-size_t cholesky_work_bytes(int ntask, int n)
-{
-    const size_t info = ((size_t)ntask * sizeof(FixInfo) + 255) & ~(size_t)255;
-    return info + (size_t)ntask * fix_task_bytes(n);
-}
+// the exponents first (launch_fix_scale), then the digit table, then the images
+static size_t fix_info_bytes(int ntask) { return ((size_t)ntask * sizeof(FixInfo) + 255) & ~(size_t)255; }
+static size_t fix_first_bytes(int ntask, int n) { return ((size_t)ntask * (fix_nbk(n) + 1) * sizeof(int) + 255) & ~(size_t)255; }
 
-static FixWork fix_work(int ntask, void *work)
+size_t cholesky_work_bytes(int ntask, int n) { return fix_info_bytes(ntask) + fix_first_bytes(ntask, n) + (size_t)ntask * fix_task_bytes(n); }
+
+static FixWork fix_work(int ntask, int n, void *work)
 {
-    const size_t info = ((size_t)ntask * sizeof(FixInfo) + 255) & ~(size_t)255;
-    return FixWork{(unsigned char *)work + info, (FixInfo *)work};
+    unsigned char *w = (unsigned char *)work;
+    return FixWork{w + fix_info_bytes(ntask) + fix_first_bytes(ntask, n), (FixInfo *)w, (int *)(w + fix_info_bytes(ntask))};
 }
 
 void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, double *logdet, void *work,
@@ -1111,7 +1219,7 @@ void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, in
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         attr = true;
     }
-    const FixWork wk = fix_work(ntask, work);
+    const FixWork wk = fix_work(ntask, n, work);
     long long *S = reinterpret_cast<long long *>(A);
     // grid y is at most 65535: every caller's chunk is
     if (!fixed) {

@@ -91,9 +91,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *mbar, uint32_t parity, int m
 {
     uint32_t done = 0;
     for (int it = 0; it < max_iter && !done; it++)
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(done)
-                     : "r"(smem_u32(mbar)), "r"(parity)
+                     : "r"(smem_u32(mbar)), "r"(parity), "r"(10000)
                      : "memory");
     return done != 0;
 }

@@ -36,3 +36,20 @@ def test_batches(count):
     assert (status < 16).all()
     for k in {0, count // 2, count - 1}:
         assert got[k] == c.logdetD(xi[k], 2)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-3, 1e-8, 1e-14])
+def test_small_entries(scale):
+    """matrices whose factor has whole blocks of zero digits (they are skipped), down to M below the last
+    digit: high frequencies, against the oracle relative to the value"""
+    import caps_gb300 as cg
+    from oracle import binding as ob
+    R, L, ldim = 40e-6, 1e-6, 150
+    c = cg.Caps(R, L, ldim=ldim, detalg=cg.DETALG_HODLR)
+    # log det falls like e^{-2 xi L/c}: the decay that scales it by `scale`
+    xi = (1 + R / L) / 2 * (0.5 - np.log(scale))
+    got, status = c.logdetD_batch([xi, xi, xi], [0, 1, 4])
+    assert (status < 16).all()
+    for m, v in zip((0, 1, 4), got):
+        want = ob.logdetD(R, L, ldim, xi, m)
+        assert abs(v - want) <= 1e-10 * abs(want) + 3e-14, (xi, m, v, want)
