@@ -106,9 +106,10 @@ __global__ void k_diag64(const Task *tasks, int ntask, int ldim, const sd *__res
 // per-window tables
 // ---------------------------------------------------------------------------
 // per listed task and window index: Cp, Cm of the recurrence; R1 = 1 / Cp(w - 1), R2 = -Cm(w - 1) R1
-// of row w; UA = Um dA, VA = -Vp dA, A = m dA and the same with dB; dA, dB.  tab[(b * W_FIELDS + field) * L + w], so that consecutive lanes read
+// of row w; UA = Um dA, VA = -Vp dA, A = m dA and the same with dB; dA, dB; the scaled seeds of row w:
+// T(w, w), T(w, w - 1), T(w, c), TE and TM each.  tab[(b * W_FIELDS + field) * L + w], so that consecutive lanes read
 // consecutive entries
-enum { W_CP, W_CM, W_R1, W_R2, W_UA, W_VA, W_A, W_UB, W_VB, W_B, W_DA, W_DB, W_FIELDS };
+enum { W_CP, W_CM, W_R1, W_R2, W_UA, W_VA, W_A, W_UB, W_VB, W_B, W_DA, W_DB, W_SEED, W_FIELDS = W_SEED + 6 };
 
 // m 2^e as a double; below the normal range 0, above it infinite
 CAPS_DEV double sd_scaled(sd v, int k)
@@ -155,7 +156,14 @@ __global__ void __launch_bounds__(256) k_sweep64_tab(const Task *tasks, const in
         }
         const double um = (l + 1.0) * cm, vp = l * cp, m = T.m;
         const double dA = sd_scaled(Sa[(size_t)task * L + w], -kw), dB = sd_scaled(Sb[(size_t)task * L + w], -kw);
-        const double f[W_FIELDS] = {cp, cm, r1, r2, um * dA, -vp * dA, m * dA, um * dB, -vp * dB, m * dB, dA, dB};
+        double f[W_FIELDS] = {cp, cm, r1, r2, um * dA, -vp * dA, m * dA, um * dB, -vp * dB, m * dB, dA, dB};
+#pragma unroll
+        for (int pol = 0; pol < 2; pol++) {
+            const sd *sp = seed + (size_t)(task * 2 + pol) * SEED_KINDS * L;
+            f[W_SEED + pol] = w >= c ? sd_scaled(sp[SEED_D0 * L + w], 2 * kw) : 0.0;
+            f[W_SEED + 2 + pol] = w > c ? sd_scaled(sp[SEED_D1 * L + w - 1], kw + k64(d0, w - 1, c)) : 0.0;
+            f[W_SEED + 4 + pol] = w >= c ? sd_scaled(sp[SEED_COL * L + w], kw + k64(d0, c, c)) : 0.0;
+        }
 #pragma unroll
         for (int i = 0; i < W_FIELDS; i++) t[(size_t)i * L] = f[i];
         ktab[(size_t)blockIdx.x * L + w] = kw;
@@ -170,9 +178,13 @@ __global__ void __launch_bounds__(256) k_sweep64_tab(const Task *tasks, const in
 constexpr int R64_NT = 256, R64_RING = 4;
 
 // grid nlist * P.  The ring of four rows (TE then TM, L + 2 values each) is in shared memory, or
-// in global memory (ring != nullptr) where it does not fit; one barrier per row.
+// in global memory (ring != nullptr) where it does not fit; one barrier per row.  Rows are a serial chain, so
+// nothing but the ring, three dependent FP64 operations and the barrier stands in it: a thread keeps the
+// coefficients of its first columns in registers, and the next row's seeds and factors are loaded a row
+// ahead (with all of them loaded in the row, 2 us a row; now ROWTIME).
+constexpr int R64_KEEP = 3; // columns per thread with coefficients in registers
 __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *tlist, int nlist, int ldim, int P,
-                                                  const sd *__restrict__ seed, const sd *__restrict__ rows, const double *__restrict__ tab,
+                                                  const sd *__restrict__ rows, const double *__restrict__ tab,
                                                   const int *__restrict__ ktab, double *tt, const int *status, double *ring)
 {
     extern __shared__ __align__(16) double r64_sm[];
@@ -189,7 +201,6 @@ __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *
     const double *W = tab + (size_t)b * W_FIELDS * L;
     auto F = [&](int f, int w) { return __ldg(W + (size_t)f * L + w); };
     const int *kt = ktab + (size_t)b * L;
-    auto sp = [&](int pol, int kind) { return seed + ((size_t)(task * 2 + pol) * SEED_KINDS + kind) * L; };
     double *tE = tt + (size_t)b * 2 * L * L, *tT = tE + (size_t)L * L;
     const int tid = threadIdx.x;
     int r = 0;
@@ -208,21 +219,34 @@ __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *
         }
         __syncthreads();
     }
+    __shared__ double ahead[2][8]; // of the next row: its seeds (W_SEED ..), R1, R2
+    auto fetch = [&](int row) {
+        if (tid < 8 && row < L) ahead[row & 1][tid] = F(tid < 6 ? W_SEED + tid : W_R1 + tid - 6, row);
+    };
+    double cp[R64_KEEP], cm[R64_KEEP];
+#pragma unroll
+    for (int i = 0; i < R64_KEEP; i++) {
+        const int y = tid + i * R64_NT;
+        cp[i] = y < L ? F(W_CP, y) : 0.0;
+        cm[i] = y < L ? F(W_CM, y) : 0.0;
+    }
+    fetch(r);
+    __syncthreads();
     for (; r <= r1; r++) {
+        fetch(r + 1);
         double *D = rowp(r);
         // rows before the first are never read: y >= c + 1 and y <= r - 2 need r >= 3
         const double *P1 = rowp(r + 3), *P2 = rowp(r + 2); // rows r - 1, r - 2
-        const double R1 = F(W_R1, r), R2 = F(W_R2, r);
-        for (int y = tid; y <= r; y += R64_NT) {
+        const double *sr = ahead[r & 1];
+        const double R1 = sr[6], R2 = sr[7];
+        auto column = [&](int y, double Cp, double Cm) {
             double vE = 0.0, vT = 0.0;
             if (y >= c) {
                 if (y == r || y == r - 1 || y == c) {
-                    const int kind = y == r ? SEED_D0 : (y == r - 1 ? SEED_D1 : SEED_COL), wi = kind == SEED_COL ? r : y;
-                    const int k = kt[r] + kt[y];
-                    vE = sd_scaled(sp(0, kind)[wi], k);
-                    vT = sd_scaled(sp(1, kind)[wi], k);
+                    const int k = y == r ? 0 : y == r - 1 ? 2 : 4;
+                    vE = sr[k];
+                    vT = sr[k + 1];
                 } else {
-                    const double Cp = F(W_CP, y), Cm = F(W_CM, y);
                     vT = fma(R1, fma(Cp, P1[LP + y + 1], Cm * P1[LP + y - 1]), R2 * P2[LP + y]);
                     if (te) vE = fma(R1, fma(Cp, P1[y + 1], Cm * P1[y - 1]), R2 * P2[y]);
                 }
@@ -233,7 +257,11 @@ __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *
                 D[y] = vE;
                 tE[(size_t)y * L + r] = vE;
             }
-        }
+        };
+#pragma unroll
+        for (int i = 0; i < R64_KEEP; i++)
+            if (tid + i * R64_NT <= r) column(tid + i * R64_NT, cp[i], cm[i]);
+        for (int y = tid + R64_KEEP * R64_NT; y <= r; y += R64_NT) column(y, F(W_CP, y), F(W_CM, y));
         __syncthreads();
     }
 }
@@ -400,7 +428,7 @@ void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, co
     }
     seed64(tasks, tlist, nlist, ldim, P, SEED_D1, SEED_COL, K, nu_stride, lft, ptab, pstride, seed, rows, status, st);
     k_sweep64_tab<<<nlist, 256, 0, st>>>(tasks, tlist, nlist, ldim, (const sd *)seed, Sa, Sb, tab, kt);
-    k_rec64<<<nlist * P, R64_NT, sm, st>>>(tasks, tlist, nlist, ldim, P, (const sd *)seed, rows, tab, kt, tt, status, ring);
+    k_rec64<<<nlist * P, R64_NT, sm, st>>>(tasks, tlist, nlist, ldim, P, rows, tab, kt, tt, status, ring);
     const dim3 g((ldim + E64_X - 1) / E64_X, (ldim + E64_Y - 1) / E64_Y, nlist);
     if (fro) k_elem64<true><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, mdiag, info, A, mstride, fro, status);
     else k_elem64<false><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, mdiag, info, A, mstride, fro, status);
