@@ -3,10 +3,10 @@
 // Network: 5 inputs -> 64 -> 64 -> 64 -> 1, SiLU activations, FP32.  Inputs are
 // the normalised features (log R/L, 2 xi L/c, m/sqrt(R/L), omega_p, gamma) built by the
 // caller.  Hand-written kernels:
-//   k_mlp_fwdbwd  one CTA of 64 threads (one per neuron) walks a slice of the
-//                 batch: forward pass, MSE loss, backward pass; per-CTA gradient
-//                 partials are kept in shared memory (each thread owns the rows of
-//                 its neuron, so no atomics) and written out per CTA;
+//   k_mlp_fwdbwd  one CTA of 256 threads walks a slice of the batch 16 samples at a
+//                 time: forward pass, MSE loss, backward pass; a thread owns one
+//                 neuron for four samples in the passes and 16 weights of each square
+//                 layer in the gradient (in registers, so no atomics), written out per CTA;
 //   k_mlp_reduce  fixed-order sum of the CTA partials (deterministic gradients);
 //   k_mlp_adam    Adam update, one thread per parameter;
 //   k_mlp_fwd     inference.
@@ -29,94 +29,219 @@ constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + HN * NIN, OFF_W2 = OFF_B1 + HN, OFF_
 
 __device__ __forceinline__ float sig(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// forward (and optionally backward) of the samples [blockIdx.x*per, ...); y == nullptr: inference only
-__global__ void __launch_bounds__(HN) k_mlp_fwdbwd(const float *__restrict__ P, const float *__restrict__ X, const float *__restrict__ Y,
-                                                   int n, int per, float *out, float *gpart, float *lpart)
+// shared memory in floats: parameters (rows of the square layers padded to 65), then per layer the
+// activations of 16 samples, [neuron][sample]
+constexpr int SB = 16, MLP_NT = 256;
+constexpr int SW1 = 0, SW2 = SW1 + HN * NIN, SW3 = SW2 + HN * (HN + 1), SB1 = SW3 + HN * (HN + 1), SB2 = SB1 + HN, SB3 = SB2 + HN,
+              SW4 = SB3 + HN, SH1 = SW4 + HN + 4, SH2 = SH1 + HN * SB, SH3 = SH2 + HN * SB, SD3 = SH3 + HN * SB, SD2 = SD3 + HN * SB,
+              SX = SD2 + HN * SB, SRED = SX + NIN * SB, SMEMF = SRED + 8 * 4 + 2 * SB;
+static_assert(SH1 % 4 == 0 && SX % 4 == 0, "vector loads of four samples");
+
+// forward (and optionally backward) of the samples [blockIdx.x*per, ...); y == nullptr: inference only.
+// Bound by latency (2600 samples: 163 CTAs of one batch): one sample after the other with a thread per neuron took
+// 150 us, 16 at once take 24 (loss, gradient and prediction of 2600 samples, copies included: 0.378 -> 0.121 ms).
+__global__ void __launch_bounds__(MLP_NT) k_mlp_fwdbwd(const float *__restrict__ P, const float *__restrict__ X, const float *__restrict__ Y,
+                                                       int n, int per, float *out, float *gpart, float *lpart)
 {
-    extern __shared__ float sm[];
-    float *w = sm;                      // parameters
-    float *g = sm + NPARAM;             // gradient accumulators (backward only)
-    float *h1 = g + (Y ? NPARAM : 0), *h2 = h1 + HN, *h3 = h2 + HN, *d3 = h3 + HN, *d2 = d3 + HN, *red = d2 + HN;
-    const int j = threadIdx.x;
-    for (int i = j; i < NPARAM; i += HN) { w[i] = P[i]; if (Y) g[i] = 0.0f; }
-    __syncthreads();
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, j = tid & 63, q = tid >> 6, lane = tid & 31, warp = tid >> 5; // neuron, group of four samples
+    for (int i = tid; i < NPARAM; i += MLP_NT) {
+        const float w = P[i];
+        if (i < OFF_B1) sm[SW1 + i] = w;
+        else if (i < OFF_W2) sm[SB1 + i - OFF_B1] = w;
+        else if (i < OFF_B2) sm[SW2 + (i - OFF_W2) / HN * (HN + 1) + (i - OFF_W2) % HN] = w;
+        else if (i < OFF_W3) sm[SB2 + i - OFF_B2] = w;
+        else if (i < OFF_B3) sm[SW3 + (i - OFF_W3) / HN * (HN + 1) + (i - OFF_W3) % HN] = w;
+        else if (i < OFF_W4) sm[SB3 + i - OFF_B3] = w;
+        else sm[SW4 + i - OFF_W4] = w; // W4, b4
+    }
     const int s0 = blockIdx.x * per, s1 = min(n, s0 + per);
     float loss = 0.0f;
-    for (int s = s0; s < s1; s++) {
-        const float *x = X + (size_t)s * NIN;
-        float z1 = w[OFF_B1 + j];
+    // this thread's gradients: W2[j][16 q ..], W3[j][16 q ..]; q = 0: W1[j], b1..b3[j], W4[j]; thread 0: b4
+    float g2[16], g3[16], g1[NIN], gb1 = 0, gb2 = 0, gb3 = 0, gw4 = 0, gb4 = 0;
 #pragma unroll
-        for (int c = 0; c < NIN; c++) z1 = fmaf(w[OFF_W1 + j * NIN + c], x[c], z1);
-        const float s1g = sig(z1);
-        h1[j] = z1 * s1g;
-        __syncthreads();
-        float z2 = w[OFF_B2 + j];
-        for (int k = 0; k < HN; k++) z2 = fmaf(w[OFF_W2 + j * HN + k], h1[k], z2);
-        const float s2g = sig(z2);
-        h2[j] = z2 * s2g;
-        __syncthreads();
-        float z3 = w[OFF_B3 + j];
-        for (int k = 0; k < HN; k++) z3 = fmaf(w[OFF_W3 + j * HN + k], h2[k], z3);
-        const float s3g = sig(z3);
-        h3[j] = z3 * s3g;
-        // output: b4 + sum_j W4[j] h3[j]  (fixed-order reduction through shared memory)
-        red[j] = w[OFF_W4 + j] * h3[j];
-        __syncthreads();
-        for (int st = HN / 2; st > 0; st >>= 1) {
-            if (j < st) red[j] += red[j + st];
-            __syncthreads();
-        }
-        const float yhat = red[0] + w[OFF_B4];
-        __syncthreads();
-        if (!Y) {
-            if (j == 0) out[s] = yhat;
-            continue;
-        }
-        const float r = yhat - Y[s];
-        loss += r * r;
-        const float d4 = 2.0f * r / n;          // d loss / d yhat, loss = mean (yhat - y)^2
-        // layer 4
-        g[OFF_W4 + j] += d4 * h3[j];
-        if (j == 0) g[OFF_B4] += d4;
-        const float dz3 = d4 * w[OFF_W4 + j] * s3g * (1.0f + z3 * (1.0f - s3g));
-        d3[j] = dz3;
-        __syncthreads();
-        for (int k = 0; k < HN; k++) g[OFF_W3 + j * HN + k] += dz3 * h2[k];
-        g[OFF_B3 + j] += dz3;
-        float a2 = 0.0f;
-        for (int i = 0; i < HN; i++) a2 = fmaf(w[OFF_W3 + i * HN + j], d3[i], a2);
-        const float dz2 = a2 * s2g * (1.0f + z2 * (1.0f - s2g));
-        d2[j] = dz2;
-        __syncthreads();
-        for (int k = 0; k < HN; k++) g[OFF_W2 + j * HN + k] += dz2 * h1[k];
-        g[OFF_B2 + j] += dz2;
-        float a1 = 0.0f;
-        for (int i = 0; i < HN; i++) a1 = fmaf(w[OFF_W2 + i * HN + j], d2[i], a1);
-        const float dz1 = a1 * s1g * (1.0f + z1 * (1.0f - s1g));
+    for (int k = 0; k < 16; k++) g2[k] = g3[k] = 0.0f;
 #pragma unroll
-        for (int c = 0; c < NIN; c++) g[OFF_W1 + j * NIN + c] += dz1 * x[c];
-        g[OFF_B1 + j] += dz1;
+    for (int c = 0; c < NIN; c++) g1[c] = 0.0f;
+    auto vec = [&](int layer, int k, int s) { return *reinterpret_cast<const float4 *>(sm + layer + k * SB + s); };
+    for (int base = s0; base < s1; base += SB) {
+        __syncthreads(); // the parameters are in; the last batch's activations have been read
+        if (tid < SB * NIN) {
+            const int s = tid / NIN, c = tid % NIN;
+            sm[SX + c * SB + s] = X[(size_t)min(base + s, s1 - 1) * NIN + c]; // past the end: the last sample again, with d = 0
+        }
         __syncthreads();
+        float sg1[4], z1[4], sg2[4], z2[4], sg3[4], z3[4], h[4];
+        // one layer: z = W h + b for four samples, h' = z sig(z)
+        auto act = [&](int layer, const float (&z)[4], float (&sg)[4]) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                sg[i] = sig(z[i]);
+                h[i] = z[i] * sg[i];
+            }
+            *reinterpret_cast<float4 *>(sm + layer + j * SB + 4 * q) = make_float4(h[0], h[1], h[2], h[3]);
+        };
+        auto dot = [&](const float *w, int step, int layer, float z0, float (&z)[4]) {
+            z[0] = z[1] = z[2] = z[3] = z0;
+#pragma unroll 16
+            for (int k = 0; k < HN; k++) {
+                const float a = w[k * step];
+                const float4 v = vec(layer, k, 4 * q);
+                z[0] = fmaf(a, v.x, z[0]);
+                z[1] = fmaf(a, v.y, z[1]);
+                z[2] = fmaf(a, v.z, z[2]);
+                z[3] = fmaf(a, v.w, z[3]);
+            }
+        };
+        z1[0] = z1[1] = z1[2] = z1[3] = sm[SB1 + j];
+#pragma unroll
+        for (int c = 0; c < NIN; c++) {
+            const float a = sm[SW1 + j * NIN + c];
+            const float4 v = vec(SX, c, 4 * q);
+            z1[0] = fmaf(a, v.x, z1[0]);
+            z1[1] = fmaf(a, v.y, z1[1]);
+            z1[2] = fmaf(a, v.z, z1[2]);
+            z1[3] = fmaf(a, v.w, z1[3]);
+        }
+        act(SH1, z1, sg1);
+        __syncthreads();
+        dot(sm + SW2 + j * (HN + 1), 1, SH1, sm[SB2 + j], z2);
+        act(SH2, z2, sg2);
+        __syncthreads();
+        dot(sm + SW3 + j * (HN + 1), 1, SH2, sm[SB3 + j], z3);
+        act(SH3, z3, sg3);
+        // output: b4 + sum_j W4[j] h3[j], over the two warps of a group of samples
+        const float w4 = sm[SW4 + j];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float t = w4 * h[i];
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == 0) sm[SRED + warp * 4 + i] = t;
+        }
+        __syncthreads();
+        if (tid < SB) {
+            const int s = base + tid;
+            const float yhat = sm[SRED + (tid >> 2) * 8 + (tid & 3)] + sm[SRED + (tid >> 2) * 8 + 4 + (tid & 3)] + sm[SW4 + HN];
+            if (!Y) {
+                if (s < s1) out[s] = yhat;
+            } else {
+                const float e = s < s1 ? yhat - Y[s] : 0.0f;
+                sm[SRED + 32 + tid] = 2.0f * e / n; // d loss / d yhat, loss = mean (yhat - y)^2
+                sm[SRED + 32 + SB + tid] = e * e;
+            }
+        }
+        if (!Y) continue;
+        __syncthreads();
+        float d4[4], dz[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) d4[i] = sm[SRED + 32 + 4 * q + i];
+        if (tid == 0)
+            for (int s = 0; s < SB; s++) {
+                loss += sm[SRED + 32 + SB + s];
+                gb4 += sm[SRED + 32 + s];
+            }
+#pragma unroll
+        for (int i = 0; i < 4; i++) dz[i] = d4[i] * w4 * sg3[i] * (1.0f + z3[i] * (1.0f - sg3[i]));
+        *reinterpret_cast<float4 *>(sm + SD3 + j * SB + 4 * q) = make_float4(dz[0], dz[1], dz[2], dz[3]);
+        __syncthreads();
+        // gradient of a square layer: G[j][16 q + k] += sum_s d[j][s] h[16 q + k][s]
+        auto outer = [&](int dl, int hl, float (&g)[16]) {
+            float d[SB];
+#pragma unroll
+            for (int s = 0; s < SB; s += 4) {
+                const float4 v = vec(dl, j, s);
+                d[s] = v.x; d[s + 1] = v.y; d[s + 2] = v.z; d[s + 3] = v.w;
+            }
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+#pragma unroll
+                for (int s = 0; s < SB; s += 4) {
+                    const float4 v = vec(hl, 16 * q + k, s);
+                    g[k] = fmaf(d[s], v.x, g[k]);
+                    g[k] = fmaf(d[s + 1], v.y, g[k]);
+                    g[k] = fmaf(d[s + 2], v.z, g[k]);
+                    g[k] = fmaf(d[s + 3], v.w, g[k]);
+                }
+            float t = 0.0f;
+#pragma unroll
+            for (int s = 0; s < SB; s++) t += d[s];
+            return t;
+        };
+        const float t3 = outer(SD3, SH2, g3);
+        float a[4];
+        dot(sm + SW3 + j, HN + 1, SD3, 0.0f, a); // a2 = W3^T d3
+#pragma unroll
+        for (int i = 0; i < 4; i++) dz[i] = a[i] * sg2[i] * (1.0f + z2[i] * (1.0f - sg2[i]));
+        *reinterpret_cast<float4 *>(sm + SD2 + j * SB + 4 * q) = make_float4(dz[0], dz[1], dz[2], dz[3]);
+        if (q == 0) {
+            gb3 += t3;
+#pragma unroll
+            for (int s = 0; s < SB; s++) gw4 = fmaf(sm[SRED + 32 + s], sm[SH3 + j * SB + s], gw4);
+        }
+        __syncthreads();
+        const float t2 = outer(SD2, SH1, g2);
+        dot(sm + SW2 + j, HN + 1, SD2, 0.0f, a); // a1 = W2^T d2
+#pragma unroll
+        for (int i = 0; i < 4; i++) dz[i] = a[i] * sg1[i] * (1.0f + z1[i] * (1.0f - sg1[i]));
+        __syncthreads(); // d3 has been read: d1 takes its place
+        *reinterpret_cast<float4 *>(sm + SD3 + j * SB + 4 * q) = make_float4(dz[0], dz[1], dz[2], dz[3]);
+        __syncthreads();
+        if (q == 0) {
+            gb2 += t2;
+#pragma unroll
+            for (int s = 0; s < SB; s++) {
+                const float d = sm[SD3 + j * SB + s];
+                gb1 += d;
+#pragma unroll
+                for (int c = 0; c < NIN; c++) g1[c] = fmaf(d, sm[SX + c * SB + s], g1[c]);
+            }
+        }
     }
     if (!Y) return;
-    for (int i = j; i < NPARAM; i += HN) gpart[(size_t)blockIdx.x * NPARAM + i] = g[i];
-    if (j == 0) lpart[blockIdx.x] = loss;
+    float *g = gpart + (size_t)blockIdx.x * NPARAM;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+        g[OFF_W2 + j * HN + 16 * q + k] = g2[k];
+        g[OFF_W3 + j * HN + 16 * q + k] = g3[k];
+    }
+    if (q == 0) {
+#pragma unroll
+        for (int c = 0; c < NIN; c++) g[OFF_W1 + j * NIN + c] = g1[c];
+        g[OFF_B1 + j] = gb1;
+        g[OFF_B2 + j] = gb2;
+        g[OFF_B3 + j] = gb3;
+        g[OFF_W4 + j] = gw4;
+    }
+    if (tid == 0) {
+        g[OFF_B4] = gb4;
+        lpart[blockIdx.x] = loss;
+    }
 }
 
-__global__ void k_mlp_reduce(const float *gpart, const float *lpart, int nblk, float *grad, float *loss, int n)
+// grid ceil(NPARAM / 32): 32 parameters by 8 slices of the CTAs each, slices added in order; the loss by
+// one more block
+__global__ void __launch_bounds__(256) k_mlp_reduce(const float *gpart, const float *lpart, int nblk, float *grad, float *loss, int n)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < NPARAM) {
-        float s = 0.0f;
-        for (int b = 0; b < nblk; b++) s += gpart[(size_t)b * NPARAM + i];
+    __shared__ float part[8][33];
+    const int c = threadIdx.x & 31, sl = threadIdx.x >> 5, i = blockIdx.x * 32 + c;
+    const bool is_loss = blockIdx.x == gridDim.x - 1;
+    const int per = (nblk + 7) / 8, b1 = min(nblk, (sl + 1) * per);
+    float s = 0.0f;
+    if (is_loss) {
+        if (c == 0)
+            for (int b = sl * per; b < b1; b++) s += lpart[b];
+    } else if (i < NPARAM)
+        for (int b = sl * per; b < b1; b++) s += gpart[(size_t)b * NPARAM + i];
+    part[sl][c] = s;
+    __syncthreads();
+    if (sl) return;
+    for (int k = 1; k < 8; k++) s += part[k][c];
+    if (is_loss) {
+        if (c == 0) *loss = s / n;
+    } else if (i < NPARAM)
         grad[i] = s;
-    }
-    if (i == 0) {
-        float s = 0.0f;
-        for (int b = 0; b < nblk; b++) s += lpart[b];
-        *loss = s / n;
-    }
 }
+constexpr int MLP_RED_GRID = (NPARAM + 31) / 32 + 1;
 
 __global__ void k_mlp_adam(float *P, const float *grad, float *m1, float *m2, int t, float lr)
 {
@@ -154,8 +279,9 @@ static void mlp_reserve(caps_mlp_t *m, size_t n)
 
 static int mlp_blocks(int n, int *per)
 {
-    const int nblk = std::max(1, std::min(304, (n + 15) / 16));
-    *per = (n + nblk - 1) / nblk;
+    // whole batches of SB samples per CTA, at most two CTAs per SM
+    const int nb = (n + SB - 1) / SB, nblk = std::max(1, std::min(304, nb));
+    *per = (nb + nblk - 1) / nblk * SB;
     return (n + *per - 1) / *per;
 }
 
@@ -169,7 +295,7 @@ static void mlp_reserve_blocks(caps_mlp_t *m, size_t nblk)
     }
 }
 
-static size_t mlp_smem(bool train) { return (size_t)(NPARAM * (train ? 2 : 1) + 6 * HN) * sizeof(float); }
+static constexpr size_t MLP_SMEM = SMEMF * sizeof(float);
 
 extern "C" int caps_mlp_nparams(void) { return NPARAM; }
 
@@ -196,7 +322,7 @@ extern "C" caps_mlp_t *caps_mlp_create(unsigned seed)
     CK(cudaMemset(m->M2, 0, NPARAM * sizeof(float)));
     static bool attr = false;
     if (!attr) {
-        CK(cudaFuncSetAttribute(k_mlp_fwdbwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_smem(true)));
+        CK(cudaFuncSetAttribute(k_mlp_fwdbwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MLP_SMEM));
         attr = true;
     }
     return m;
@@ -218,9 +344,9 @@ static double mlp_fwdbwd(caps_mlp_t *m, int n)
     int per;
     const int nblk = mlp_blocks(n, &per);
     mlp_reserve_blocks(m, nblk);
-    k_mlp_fwdbwd<<<nblk, HN, mlp_smem(true)>>>(m->P, m->X, m->Y, n, per, nullptr, m->gpart, m->lpart);
+    k_mlp_fwdbwd<<<nblk, MLP_NT, MLP_SMEM>>>(m->P, m->X, m->Y, n, per, nullptr, m->gpart, m->lpart);
     COUNT_LAUNCH(1);
-    k_mlp_reduce<<<(NPARAM + 255) / 256, 256>>>(m->gpart, m->lpart, nblk, m->G, m->loss, n);
+    k_mlp_reduce<<<MLP_RED_GRID, 256>>>(m->gpart, m->lpart, nblk, m->G, m->loss, n);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
     float l;
@@ -250,8 +376,8 @@ extern "C" double caps_mlp_train(caps_mlp_t *m, const float *X, const float *y, 
     for (int e = 0; e < epochs; e++) {
         // full-batch Adam; cosine-decayed step size
         const float lr_e = lr * 0.5f * (1.0f + cosf(3.14159265f * e / epochs)) + 1e-5f;
-        k_mlp_fwdbwd<<<nblk, HN, mlp_smem(true)>>>(m->P, m->X, m->Y, n, per, nullptr, m->gpart, m->lpart);
-        k_mlp_reduce<<<(NPARAM + 255) / 256, 256>>>(m->gpart, m->lpart, nblk, m->G, m->loss, n);
+        k_mlp_fwdbwd<<<nblk, MLP_NT, MLP_SMEM>>>(m->P, m->X, m->Y, n, per, nullptr, m->gpart, m->lpart);
+        k_mlp_reduce<<<MLP_RED_GRID, 256>>>(m->gpart, m->lpart, nblk, m->G, m->loss, n);
         k_mlp_adam<<<(NPARAM + 255) / 256, 256>>>(m->P, m->G, m->M1, m->M2, ++m->t, lr_e);
         COUNT_LAUNCH(3);
     }
@@ -269,7 +395,7 @@ extern "C" void caps_mlp_predict(caps_mlp_t *m, const float *X, int n, float *y)
     CK(cudaMemcpy(m->X, X, (size_t)n * NIN * sizeof(float), cudaMemcpyHostToDevice));
     int per;
     const int nblk = mlp_blocks(n, &per);
-    k_mlp_fwdbwd<<<nblk, HN, mlp_smem(false)>>>(m->P, m->X, nullptr, n, per, m->out, nullptr, nullptr);
+    k_mlp_fwdbwd<<<nblk, MLP_NT, MLP_SMEM>>>(m->P, m->X, nullptr, n, per, m->out, nullptr, nullptr);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
     CK(cudaMemcpy(y, m->out, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost));
