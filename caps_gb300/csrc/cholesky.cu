@@ -25,85 +25,12 @@
 // (ST_ERR_PIVOT) and its result becomes NaN; nothing traps.  A matrix whose diagonal exceeds 2
 // (M with large negative diagonal entries) is scaled by a power of four on conversion.
 #include "common.cuh"
+#include "fix.cuh"
 #include "internal.h"
 #include "umma.cuh"
 #include <algorithm>
-#include <cuda_fp16.h>
 
 namespace capsgpu {
-
-constexpr int NB = 64;
-constexpr int FQ = 60;                       // fixed point: value = integer 2^-60
-constexpr int ND = 6, NG = 7;                // digits of a factor, accumulators (i + j = 0..6)
-constexpr int SY_G0 = 4;                     // accumulators of a first part, see k_fix_syrk
-constexpr int IMG_BLK = NB * NB * 2;         // bytes of one digit of one 64 x 64 block
-constexpr int FIX_WAIT_ITERS = 1 << 22;      // polls of a bounded mbarrier wait
-
-// per-task workspace: W image, X image (one digit after the other, a spare row block so that a
-// pair of row blocks can always be read), exponents
-__host__ __device__ inline int fix_nbk(int n) { return (n + NB - 1) / NB; }
-__host__ __device__ inline size_t fix_ximg_bytes(int n) { return (size_t)(fix_nbk(n) + 1) * ND * IMG_BLK; }
-__host__ __device__ inline size_t fix_task_bytes(int n) { return (size_t)ND * IMG_BLK + fix_ximg_bytes(n); }
-struct FixInfo { int sexp, wexp; };          // A 2^-sexp is factored; W 2^-wexp is in the image
-// first[task * (nbk + 1) + block]: the first digit of the current panel's X that is not zero in the whole 64-row
-// block (block counted below the diagonal block; NG: none)
-struct FixWork {
-    unsigned char *img;
-    FixInfo *info;
-    int *first;
-    __host__ __device__ unsigned char *wimg(int task, int n) const { return img + (size_t)task * fix_task_bytes(n); }
-    __host__ __device__ unsigned char *ximg(int task, int n) const { return wimg(task, n) + (size_t)ND * IMG_BLK; }
-};
-
-// byte offset of element (row, k) inside one digit of a 64-row block: the operand layout of
-// umma.cuh (8 x 16-byte core matrices), k innermost, 1024 bytes per 8 rows
-CAPS_DEV int img_off(int row, int kcore) { return (row >> 3) * 1024 + kcore * 128 + (row & 7) * 16; }
-
-// ---- digits ----
-// the magnitude of x (units of 2^-60) as digits see it, in units of 2^-53: its bit length bounds the digits
-// that are not zero (k digits hold +-255 (512^k - 1) / 511)
-CAPS_DEV unsigned long long digit_mag(long long x)
-{
-    const long long y = (x + 64) >> 7;
-    return (unsigned long long)(y < 0 ? -y : y);
-}
-// first digit that may be nonzero, from the bitwise or of magnitudes; NG: none is
-CAPS_DEV int first_digit(unsigned long long any)
-{
-    const int bits = 64 - __clzll((long long)any);
-    return bits == 0 ? NG : bits <= 8 ? 5 : bits <= 16 ? 4 : bits <= 25 ? 3 : bits <= 34 ? 2 : bits <= 43 ? 1 : 0;
-}
-
-// eight numbers (units of 2^-60, |x| < 4) to six 16-byte vectors of FP16 digits
-CAPS_DEV void split8(const long long (&x)[8], uint4 (&d)[ND])
-{
-    const __half2 off = __half2half2(__ushort_as_half(0x6500)); // 1280
-    unsigned w[ND][4];
-#pragma unroll
-    for (int p = 0; p < 4; p++) {
-        unsigned f[2][ND];
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            // round to units of 2^-53 and bias the five low digits by 256, so that they are plain bit fields
-            constexpr long long BIAS = 256LL * (1 + (1LL << 9) + (1LL << 18) + (1LL << 27) + (1LL << 36));
-            const long long t = ((x[2 * p + u] + 64) >> 7) + BIAS;
-#pragma unroll
-            for (int i = 1; i < ND; i++) f[u][i] = (unsigned)(t >> (9 * (5 - i))) & 511u;
-            const int top = (int)(t >> 45);
-            f[u][0] = __half_as_ushort(__int2half_rn(min(max(top, -2047), 2047)));
-        }
-        w[0][p] = f[0][0] | f[1][0] << 16;
-#pragma unroll
-        for (int i = 1; i < ND; i++) {
-            // 0x6400 | u is 1024 + u in FP16
-            const unsigned raw = (f[0][i] | f[1][i] << 16) | 0x64006400u;
-            const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&raw), off);
-            w[i][p] = *reinterpret_cast<const unsigned *>(&h);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < ND; i++) d[i] = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
-}
 
 // the digit products of one 128 x 64 tile, K = 64, of groups G0 .. G1 - 1, accumulator g at tmem + 64 g: NA
 // digits of A (ASTEP bytes apart) and NBD digits of B (one block apart); alo, blo: low descriptor
@@ -1199,33 +1126,54 @@ static size_t fix_first_bytes(int ntask, int n) { return ((size_t)ntask * (fix_n
 
 size_t cholesky_work_bytes(int ntask, int n) { return fix_info_bytes(ntask) + fix_first_bytes(ntask, n) + (size_t)ntask * fix_task_bytes(n); }
 
-static FixWork fix_work(int ntask, int n, void *work)
+FixWork fix_work(int ntask, int n, void *work)
 {
     unsigned char *w = (unsigned char *)work;
     return FixWork{w + fix_info_bytes(ntask) + fix_first_bytes(ntask, n), (FixInfo *)w, (int *)(w + fix_info_bytes(ntask))};
 }
 
-void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, double *logdet, void *work,
-                     cudaStream_t st, bool fixed)
+static int fix_sms()
 {
-    static bool attr = false;
-    static int sms = 148;
-    if (!attr) {
+    static int sms = 0;
+    if (!sms) {
         CK(cudaFuncSetAttribute(k_fix_potf2, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
         CK(cudaFuncSetAttribute(k_fix_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, TR_SMEM));
         CK(cudaFuncSetAttribute(k_fix_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, SY_SMEM));
         int dev = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        attr = true;
     }
+    return sms;
+}
+
+void fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, const int *status, const double *mdiag, const FixWork &wk,
+                 cudaStream_t st)
+{
+    k_fix_convert<<<dim3((n + 7) / 8, ntask), 256, 0, st>>>(ntask, n, A, lda, mstride, status, mdiag, wk.info);
+    COUNT_LAUNCH(1);
+}
+
+void fix_syrk(int ntask, int n, int t0, long long *S, size_t lda, size_t mstride, int *status, const FixWork &wk, cudaStream_t st)
+{
+    // tiles per CTA: about three CTAs per SM where the batch is small, at most 8 tiles
+    const int nbt = (n - t0 + NB - 1) / NB, np = (nbt + 1) / 2;
+    long long tiles = 0;
+    for (int p = 0; p < np; p++) tiles += std::min(2 * p + 2, nbt);
+    const int chunk = (int)std::max(1LL, std::min(8LL, tiles * ntask / (3LL * fix_sms())));
+    int items = 0;
+    for (int p = 0; p < np; p++) items += (std::min(2 * p + 2, nbt) + chunk - 1) / chunk;
+    k_fix_syrk<<<dim3(items, ntask), SY_THREADS, SY_SMEM, st>>>(ntask, n, t0, chunk, S, lda, mstride, status, wk);
+    COUNT_LAUNCH(1);
+}
+
+void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, double *logdet, void *work,
+                     cudaStream_t st, bool fixed)
+{
+    fix_sms();
     const FixWork wk = fix_work(ntask, n, work);
     long long *S = reinterpret_cast<long long *>(A);
     // grid y is at most 65535: every caller's chunk is
-    if (!fixed) {
-        k_fix_convert<<<dim3((n + 7) / 8, ntask), 256, 0, st>>>(ntask, n, A, lda, mstride, status, mdiag, wk.info);
-        COUNT_LAUNCH(1);
-    }
+    if (!fixed) fix_convert(ntask, n, A, lda, mstride, status, mdiag, wk, st);
     for (int k0 = 0; k0 < n; k0 += NB) {
         k_fix_potf2<<<ntask, PF_NT, PF_SMEM, st>>>(ntask, n, k0, S, lda, mstride, status, wk, logdet);
         COUNT_LAUNCH(1);
@@ -1233,15 +1181,7 @@ void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, in
         if (rest <= 0) break;
         k_fix_trsm<<<dim3((rest + 127) / 128, ntask), TR_NT, TR_SMEM, st>>>(ntask, n, k0, S, lda, mstride, status, wk);
         COUNT_LAUNCH(1);
-        // tiles per CTA: about three CTAs per SM where the batch is small, at most 8 tiles
-        const int nbt = (rest + NB - 1) / NB, np = (nbt + 1) / 2;
-        long long tiles = 0;
-        for (int p = 0; p < np; p++) tiles += std::min(2 * p + 2, nbt);
-        const int chunk = (int)std::max(1LL, std::min(8LL, tiles * ntask / (3LL * sms)));
-        int items = 0;
-        for (int p = 0; p < np; p++) items += (std::min(2 * p + 2, nbt) + chunk - 1) / chunk;
-        k_fix_syrk<<<dim3(items, ntask), SY_THREADS, SY_SMEM, st>>>(ntask, n, t0, chunk, S, lda, mstride, status, wk);
-        COUNT_LAUNCH(1);
+        fix_syrk(ntask, n, t0, S, lda, mstride, status, wk, st);
     }
     CK(cudaGetLastError());
 }

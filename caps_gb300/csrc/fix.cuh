@@ -1,0 +1,89 @@
+// fix.cuh -- 64-bit fixed-point matrices as FP16 digit images, shared by the Cholesky factorisation
+// (cholesky.cu, which explains the format) and the square of M (square.cu)
+#pragma once
+#include "common.cuh"
+#include <cuda_fp16.h>
+
+namespace capsgpu {
+
+constexpr int NB = 64;
+constexpr int FQ = 60;                       // fixed point: value = integer 2^-60
+constexpr int ND = 6, NG = 7;                // digits of a factor, accumulators (i + j = 0..6)
+constexpr int SY_G0 = 4;                     // accumulators of a first part, see k_fix_syrk
+constexpr int IMG_BLK = NB * NB * 2;         // bytes of one digit of one 64 x 64 block
+constexpr int FIX_WAIT_ITERS = 1 << 22;      // polls of a bounded mbarrier wait
+
+// per-task workspace: W image, X image (one digit after the other, a spare row block so that a
+// pair of row blocks can always be read), exponents
+__host__ __device__ inline int fix_nbk(int n) { return (n + NB - 1) / NB; }
+__host__ __device__ inline size_t fix_ximg_bytes(int n) { return (size_t)(fix_nbk(n) + 1) * ND * IMG_BLK; }
+__host__ __device__ inline size_t fix_task_bytes(int n) { return (size_t)ND * IMG_BLK + fix_ximg_bytes(n); }
+struct FixInfo { int sexp, wexp; };          // A 2^-sexp is factored; W 2^-wexp is in the image
+// first[task * (nbk + 1) + block]: the first digit of the current panel's X that is not zero in the whole 64-row
+// block (block counted below the diagonal block; NG: none)
+struct FixWork {
+    unsigned char *img;
+    FixInfo *info;
+    int *first;
+    __host__ __device__ unsigned char *wimg(int task, int n) const { return img + (size_t)task * fix_task_bytes(n); }
+    __host__ __device__ unsigned char *ximg(int task, int n) const { return wimg(task, n) + (size_t)ND * IMG_BLK; }
+};
+
+// byte offset of element (row, k) inside one digit of a 64-row block: the operand layout of
+// umma.cuh (8 x 16-byte core matrices), k innermost, 1024 bytes per 8 rows
+CAPS_DEV int img_off(int row, int kcore) { return (row >> 3) * 1024 + kcore * 128 + (row & 7) * 16; }
+
+// ---- digits ----
+// the magnitude of x (units of 2^-60) as digits see it, in units of 2^-53: its bit length bounds the digits
+// that are not zero (k digits hold +-255 (512^k - 1) / 511)
+CAPS_DEV unsigned long long digit_mag(long long x)
+{
+    const long long y = (x + 64) >> 7;
+    return (unsigned long long)(y < 0 ? -y : y);
+}
+// first digit that may be nonzero, from the bitwise or of magnitudes; NG: none is
+CAPS_DEV int first_digit(unsigned long long any)
+{
+    const int bits = 64 - __clzll((long long)any);
+    return bits == 0 ? NG : bits <= 8 ? 5 : bits <= 16 ? 4 : bits <= 25 ? 3 : bits <= 34 ? 2 : bits <= 43 ? 1 : 0;
+}
+
+// eight numbers (units of 2^-60, |x| < 4) to six 16-byte vectors of FP16 digits
+CAPS_DEV void split8(const long long (&x)[8], uint4 (&d)[ND])
+{
+    const __half2 off = __half2half2(__ushort_as_half(0x6500)); // 1280
+    unsigned w[ND][4];
+#pragma unroll
+    for (int p = 0; p < 4; p++) {
+        unsigned f[2][ND];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            // round to units of 2^-53 and bias the five low digits by 256, so that they are plain bit fields
+            constexpr long long BIAS = 256LL * (1 + (1LL << 9) + (1LL << 18) + (1LL << 27) + (1LL << 36));
+            const long long t = ((x[2 * p + u] + 64) >> 7) + BIAS;
+#pragma unroll
+            for (int i = 1; i < ND; i++) f[u][i] = (unsigned)(t >> (9 * (5 - i))) & 511u;
+            const int top = (int)(t >> 45);
+            f[u][0] = __half_as_ushort(__int2half_rn(min(max(top, -2047), 2047)));
+        }
+        w[0][p] = f[0][0] | f[1][0] << 16;
+#pragma unroll
+        for (int i = 1; i < ND; i++) {
+            // 0x6400 | u is 1024 + u in FP16
+            const unsigned raw = (f[0][i] | f[1][i] << 16) | 0x64006400u;
+            const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&raw), off);
+            w[i][p] = *reinterpret_cast<const unsigned *>(&h);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ND; i++) d[i] = make_uint4(w[i][0], w[i][1], w[i][2], w[i][3]);
+}
+
+// cholesky.cu: the parts of a workspace of cholesky_work_bytes; FP64 -> fixed point in place, with the exponents;
+// S -= X X^T over the rows and columns from t0 on, X the 64 columns in the image, first digits in wk.first
+FixWork fix_work(int ntask, int n, void *work);
+void fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, const int *status, const double *mdiag, const FixWork &wk,
+                 cudaStream_t st);
+void fix_syrk(int ntask, int n, int t0, long long *S, size_t lda, size_t mstride, int *status, const FixWork &wk, cudaStream_t st);
+
+} // namespace capsgpu

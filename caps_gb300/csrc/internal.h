@@ -65,9 +65,14 @@ int itab_group_size();
 void launch_itab_grp(const Task *tasks, const int *tlist, const int4 *groups, int ngroups, int ldim, const float4 *KP,
                      const int *KPe, int nu_stride, const float4 *ptabf, int pstride, const void *a12, void *Iout, bool ffe_out,
                      int *status, cudaStream_t st);
-// sphere-sphere: B = 1 - M^2 and (M^2)_ii from A = 1 - M and M_ii (square.cu)
-void launch_square(int ntask, int n, const double *A, size_t lda, size_t mstride, const double *mdiag, double *B,
-                   const int *status, double *mdiag2, cudaStream_t st);
+// sphere-sphere (square.cu): B = 1 - M^2 in fixed point from A = 1 - M (FP64 with M_ii, or fixed point with its exponents
+// in work, see launch_cholesky) for the tasks of status ST_OK; rn: n floats per task; fro: square_nsum sums of
+// squares of M^2 per task.  launch_square_norm: the same sums of M from FP64 A and M_ii
+int square_nsum(int n);
+void launch_square_norm(int ntask, int n, const double *A, size_t lda, size_t mstride, const double *mdiag, const int *status, double *out,
+                        cudaStream_t st);
+void launch_square(int ntask, int n, double *A, size_t lda, size_t mstride, const double *mdiag, double *B, int *status, float *rn, double *fro,
+                   void *work, bool fixed, cudaStream_t st);
 // a_0, a_1, a_2 per distinct m of a chunk (groups), shared by all frequencies
 void launch_a12(const int *group_m, const int *group_lmin, int ngroup, int ldim, const double *lft, void *tab, cudaStream_t st);
 size_t a12_bytes(int ldim, int ngroup);

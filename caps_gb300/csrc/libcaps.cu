@@ -105,7 +105,7 @@ struct Engine {
     cudaStream_t side = nullptr;          // Mie coefficients and scale factors, beside setup and K
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     double *d_lfac = nullptr;
-    DevBuf tasks, coef, partM, partE, K, I, Sa, Sb, uv, A, logdiag, trace, result, status, mie_a, mie_b, xi, eps, lft, xtab, ptab, S32, ptabf, a12, gm, glmin, Saf, Sbf, uvf, part, diag, groups, B, diag2, mwork, a12t, coefF, tlist, groups2, glist2, KP, KPe, hwork, seed, sw64, fro;
+    DevBuf tasks, coef, partM, partE, K, I, Sa, Sb, uv, A, logdiag, trace, result, status, mie_a, mie_b, xi, eps, lft, xtab, ptab, S32, ptabf, a12, gm, glmin, Saf, Sbf, uvf, part, diag, groups, B, diag2, mwork, a12t, coefF, tlist, groups2, glist2, KP, KPe, hwork, seed, sw64, fro, fro2;
     std::vector<double> host_pinned_dummy;
     double timings[6] = {0, 0, 0, 0, 0, 0};
     double timings_cum[6] = {0, 0, 0, 0, 0, 0};
@@ -498,7 +498,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     // by 4 L q-sums per matrix (sweep.cu) instead of the q-sums of every pair
     const bool sweep = ff_elem && sweep_fits(ldim);
     // the FP64 form's dense matrices by the same recurrence in FP64 (sweep64.cu), into fixed point
-    const bool sweep64 = !mixed && O.factor && !O.square && !O.M_out && !hodlr;
+    const bool sweep64 = !mixed && O.factor && !O.M_out && !hodlr;
     // chunk size from free memory.  The budget counts the large work buffers held from earlier
     // batches as free for this one: true while batches keep one shape, each buffer serving the
     // same array again; when the shape (dimension, precision, path) changes they are released
@@ -517,7 +517,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     const size_t mat_bytes = O.square ? 16 : ff_elem ? 4 + 1 : (caps->precision == CAPS_PREC_MIXED ? 12 : 8);
     const size_t dense_bytes = hodlr ? hodlr_work_bytes(ldim, 1)
                              : sweep ? (size_t)dim * dim * 4 + seed_bytes(ldim, 1)
-                             : sweep64 ? (size_t)dim * dim * 8 + seed64_bytes(ldim, 1) + sweep64_work_bytes(ldim, 1)
+                             : sweep64 ? (size_t)dim * dim * (O.square ? 16 : 8) + seed64_bytes(ldim, 1) + sweep64_work_bytes(ldim, 1)
                                      : (size_t)dim * dim * mat_bytes + (size_t)2 * L * L * sizeof(sd)
                                            + (size_t)L * (L + 1) / 2 * 32; // a_0..a_2 table (one row per task)
     const size_t per_task = dense_bytes + (size_t)2 * nu_stride * sizeof(sd)
@@ -741,9 +741,9 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             d_seed = g_eng.seed.get(seed64_bytes(ldim, nt));
             launch_diag64(d_tasks, nt, ldim, d_K, nu_stride, d_lft, d_ptab, pstride, d_Sa, d_Sb, d_uv, d_seed, d_dg, d_status, st);
             CK(cudaEventRecord(g_eng.ev[3], st));
-            launch_stats(nullptr, nt, dim, nullptr, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st);
+            if (!O.square) launch_stats(nullptr, nt, dim, nullptr, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st);
             CK(cudaEventRecord(g_eng.ev[4], st));
-            undecided();
+            if (!O.square) undecided();
             CK(cudaEventRecord(g_eng.ev[5], st));
         } else {
             launch_ptab(d_tasks, nt, d_ptab, pstride, st);
@@ -763,6 +763,17 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
 
         double *d_A = nullptr;
         float *d_S = nullptr;
+        // sphere-sphere: continue with B = 1 - M^2 in place of A.  tr M^2 = |M|^2 comes as nsum partial sums per task, and
+        // the trace rule is applied before the product
+        auto square = [&](const double *d_norm, int nsum) {
+            launch_stats(nullptr, nt, nsum, nullptr, lda, mstride, d_norm, O.mode, d_trace, d_res, d_status, st);
+            double *d_B = (double *)g_eng.B.get((size_t)nt * mstride * sizeof(double));
+            float *d_rn = (float *)g_eng.diag2.get((size_t)nt * dim * sizeof(float));
+            double *d_fro2 = (double *)g_eng.fro2.get((size_t)nt * square_nsum(dim) * sizeof(double));
+            launch_square(nt, dim, d_A, lda, mstride, d_dg, d_B, d_status, d_rn, d_fro2, g_eng.mwork.get(cholesky_work_bytes(nt, dim)), sweep64, st);
+            launch_stats(nullptr, nt, nsum, d_B, lda, mstride, d_norm, O.mode, d_trace, d_res, d_status, st, d_fro2, square_nsum(dim));
+            d_A = d_B;
+        };
         if (hodlr) {
             // (no element phase)
         } else if (ff_elem && sweep) {
@@ -784,19 +795,17 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             launch_sweep64(d_tasks, d_list, nlist, ldim, d_K, nu_stride, d_lft, d_ptab, pstride, d_Sa, d_Sb, d_seed, d_dg,
                            (const int *)d_work, g_eng.sw64.get(sweep64_work_bytes(ldim, nlist)), (long long *)d_A, mstride, d_fro,
                            d_status, st);
-            launch_stats(d_list, nlist, dim, d_A, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st, d_fro, nfro);
+            if (O.square) square(d_fro, nfro);
+            else launch_stats(d_list, nlist, dim, d_A, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st, d_fro, nfro);
         } else {
             d_A = (double *)g_eng.A.get((size_t)nt * mstride * sizeof(double));
             launch_elem(d_tasks, d_list, nlist, ldim, d_I, d_Sa, d_Sb, d_uv, d_A, lda, mstride, d_dg, d_status, st, false);
             if (O.square) {
-                // sphere-sphere: continue with B = 1 - M^2 in place of A
-                double *d_B = (double *)g_eng.B.get((size_t)nt * mstride * sizeof(double));
-                double *d_dg2 = (double *)g_eng.diag2.get((size_t)nt * dim * sizeof(double));
-                launch_square(nt, dim, d_A, lda, mstride, d_dg, d_B, d_status, d_dg2, st);
-                d_A = d_B;
-                d_dg = d_dg2;
-            }
-            if (O.factor) launch_stats(d_list, nlist, dim, d_A, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st);
+                double *d_norm = (double *)g_eng.fro.get((size_t)nt * square_nsum(dim) * sizeof(double));
+                launch_square_norm(nt, dim, d_A, lda, mstride, d_dg, d_status, d_norm, st);
+                square(d_norm, square_nsum(dim));
+            } else if (O.factor)
+                launch_stats(d_list, nlist, dim, d_A, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st);
         }
         CK(cudaEventRecord(g_eng.ev[7], st));
 
@@ -818,7 +827,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         } else if (O.factor) {
             double *d_ld = (double *)g_eng.logdiag.get((size_t)nt * dim * sizeof(double));
             void *d_work = g_eng.mwork.get(cholesky_work_bytes(nt, dim));
-            launch_cholesky(nt, dim, d_A, lda, mstride, d_status, d_dg, d_ld, d_work, st, sweep64);
+            launch_cholesky(nt, dim, d_A, lda, mstride, d_status, d_dg, d_ld, d_work, st, sweep64 || O.square);
             launch_final(nt, dim, d_ld, d_work, d_trace, d_status, d_res, O.mode, st);
         }
         CK(cudaEventRecord(g_eng.ev[8], st));
