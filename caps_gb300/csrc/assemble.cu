@@ -41,14 +41,18 @@ __global__ void k_coef(const int *group_m, int ngroup, int nu_stride, double2 *c
 // ---------------------------------------------------------------------------
 // Mie coefficients per distinct xi
 // ---------------------------------------------------------------------------
-__global__ void k_mie(const double *xi_list, const double *epsm1_list, int nxi, double LbyR, int lmax,
-                      double *lna, double *lnb)
+// Four lanes per l and one warp per CTA: about 3000 FP64 operations per lane in long dependent chains, a warp's operation
+// holds the FP64 pipe for 16 clocks, and four warps of one CTA, a thread per l, took 186 us for lmax = 300 (one or
+// several frequencies), this 68 us.
+__global__ void __launch_bounds__(32) k_mie(const double *xi_list, const double *epsm1_list, int nxi, double LbyR, int lmax,
+                                            double *lna, double *lnb)
 {
-    const int l = blockIdx.x * blockDim.x + threadIdx.x + 1;
+    const int l = blockIdx.x * 8 + (threadIdx.x >> 2) + 1;
     const int ix = blockIdx.y;
-    if (l > lmax || ix >= nxi) return;
+    if (ix >= nxi) return;
     double a, b;
-    mie(LbyR, xi_list[ix], l, epsm1_list[ix], &a, &b);
+    mie(LbyR, xi_list[ix], min(l, lmax), epsm1_list[ix], &a, &b);
+    if (l > lmax || (threadIdx.x & 3)) return;
     lna[(size_t)ix * (lmax + 1) + l] = a;
     lnb[(size_t)ix * (lmax + 1) + l] = b;
 }
@@ -700,10 +704,23 @@ void set_k_nodes(Task &T, double left)
 }
 double k_left(int mu, int s) { return kgrid_left(mu, s); }
 
+// The Mie coefficients and scale factors run beside the K integrals: an SM whose shared memory they left small would
+// take fewer CTAs of the integrals for as long as those last (24 matrices of dimension 2100: K 2.2 ms
+// instead of 0.5), so all of them ask for the same split of the SM's memory
+static void beside_ktab()
+{
+    static bool attr = false;
+    if (attr) return;
+    for (const void *f : {(const void *)k_mie, (const void *)k_scale, (const void *)k_ktab<true>, (const void *)k_ktab<false>})
+        CK(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    attr = true;
+}
+
 void launch_mie(const double *xi, const double *epsm1, int nxi, double LbyR, int lmax, double *lna, double *lnb, cudaStream_t st)
 {
-    dim3 g((lmax + 127) / 128, nxi);
-    k_mie<<<g, 128, 0, st>>>(xi, epsm1, nxi, LbyR, lmax, lna, lnb);
+    beside_ktab();
+    dim3 g((lmax + 7) / 8, nxi);
+    k_mie<<<g, 32, 0, st>>>(xi, epsm1, nxi, LbyR, lmax, lna, lnb);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }
@@ -711,6 +728,7 @@ void launch_mie(const double *xi, const double *epsm1, int nxi, double LbyR, int
 void launch_scale(const Task *tasks, int ntask, int ldim, const double *lna, const double *lnb, int lmax, const double *lfac_tab,
                   sd *Sa, sd *Sb, double2 *uv, cudaStream_t st)
 {
+    beside_ktab();
     dim3 g((ldim + 2 + 127) / 128, ntask);
     k_scale<<<g, 128, 0, st>>>(tasks, ntask, ldim, lna, lnb, lmax, lfac_tab, Sa, Sb, uv);
     COUNT_LAUNCH(1);
@@ -722,6 +740,7 @@ size_t ktab_smem_bytes() { return (size_t)KT_WARPS * (32 * 33 + 64) * sizeof(dou
 void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double2 *coefAB, int nu_stride, const double *lfac_tab,
                  double *partM, int *partE, cudaStream_t st)
 {
+    beside_ktab();
     static bool attr_set = false;
     const size_t sm = ktab_smem_bytes();
     if (!attr_set) {

@@ -552,13 +552,6 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     for (int c0 = 0; c0 < n; c0 += chunk) {
         const int nt = std::min(chunk, n - c0);
         CK(cudaEventRecord(g_eng.ev[0], st));
-        // the Mie coefficients (first chunk) and the scale factors do not feed the quadrature
-        // set-up or the K integrals: they run on a side stream beside them
-        if (c0 == 0) {
-            CK(cudaEventRecord(g_eng.ev_fork, st));
-            CK(cudaStreamWaitEvent(g_eng.side, g_eng.ev_fork, 0));
-            launch_mie(d_xi, d_eps, nxi, caps->LbyR, lmax_mie, d_lna, d_lnb, g_eng.side);
-        }
         // group the chunk's tasks by m: a_0, a_1, a_2 of the q-sums depend on (l1, l2, m) only
         std::map<int, int> gidx;
         std::vector<int> gm, glm;
@@ -599,11 +592,17 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         sd *d_Sb = (sd *)g_eng.Sb.get((size_t)nt * L * sizeof(sd));
         double2 *d_uv = (double2 *)g_eng.uv.get((size_t)nt * L * sizeof(double2));
         CK(cudaEventRecord(g_eng.ev_fork, st)); // the chunk's task table is on the device
-        CK(cudaStreamWaitEvent(g_eng.side, g_eng.ev_fork, 0));
-        launch_scale(d_tasks, nt, ldim, d_lna, d_lnb, lmax_mie, g_eng.d_lfac, d_Sa, d_Sb, d_uv, g_eng.side);
-        CK(cudaEventRecord(g_eng.ev_join, g_eng.side));
         CK(cudaEventRecord(g_eng.ev[1], st));
 
+        // the Mie coefficients (first chunk) and the scale factors do not feed the K integrals: they run on a side
+        // stream beside them, launched after them so that the integrals' CTAs are spread evenly first
+        // (the other way round some SMs got twice as many: 24 matrices of dimension 2100, K 1.2 ms instead of 0.5)
+        auto side = [&]() {
+            CK(cudaStreamWaitEvent(g_eng.side, g_eng.ev_fork, 0));
+            if (c0 == 0) launch_mie(d_xi, d_eps, nxi, caps->LbyR, lmax_mie, d_lna, d_lnb, g_eng.side);
+            launch_scale(d_tasks, nt, ldim, d_lna, d_lnb, lmax_mie, g_eng.d_lfac, d_Sa, d_Sb, d_uv, g_eng.side);
+            CK(cudaEventRecord(g_eng.ev_join, g_eng.side));
+        };
         double *d_pM = (double *)g_eng.partM.get((size_t)nt * 2 * max_warps * nu_stride * sizeof(double));
         int *d_pE = (int *)g_eng.partE.get((size_t)nt * 2 * max_warps * nu_stride * sizeof(int));
         sd *d_K = nullptr;
@@ -614,10 +613,12 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             d_KP = (float4 *)g_eng.KP.get((size_t)nt * nu_stride * sizeof(float4));
             d_KPe = (int *)g_eng.KPe.get((size_t)nt * nu_stride * sizeof(int));
             launch_ktab_ff(is_pr, d_tasks, nt, max_warps, d_coefF, nu_stride, g_eng.d_lfac, (float2 *)d_pM, d_pE, st);
+            side();
             launch_kred_ff(d_tasks, nt, nnu_max, (const float2 *)d_pM, d_pE, max_warps, nu_stride, d_KP, d_KPe, d_status, st);
         } else {
             d_K = (sd *)g_eng.K.get((size_t)nt * 2 * nu_stride * sizeof(sd));
             launch_ktab(is_pr, d_tasks, nt, max_warps, d_coef, nu_stride, g_eng.d_lfac, d_pM, d_pE, st);
+            side();
             launch_kred(d_tasks, nt, nnu_max, d_pM, d_pE, max_warps, nu_stride, d_K, d_status, st);
         }
         CK(cudaEventRecord(g_eng.ev[2], st));

@@ -73,7 +73,7 @@ CAPS_DEV void logIK_half(int n, double x, double rho, double *logI, double *logK
 {
     if (n >= 100) {
         *logK = logK_asymp(n + 0.5, x);
-        if (logI) *logI = logI_asymp(n + 0.5, x);
+        *logI = logI_asymp(n + 0.5, x);
         return;
     }
     const double logx = log(x), invx = 1.0 / x;
@@ -87,7 +87,7 @@ CAPS_DEV void logIK_half(int n, double x, double rho, double *logI, double *logK
     const double pre = -x + 0.5 * (log(PI / 2) - logx) + sc * LN2;
     const double lk = pre + log(k0), lkp = pre + log(k1);
     *logK = lk;
-    if (logI) *logI = -logx - lkp - log1p(exp(lk - lkp - log(rho)));
+    *logI = -logx - lkp - log1p(exp(lk - lkp - log(rho)));
 }
 
 CAPS_DEV double logadd(double a, double b)
@@ -97,28 +97,32 @@ CAPS_DEV double logadd(double a, double b)
     return a > b ? a + log1p(exp(b - a)) : b + log1p(exp(a - b));
 }
 
-// log|a_l|, log|b_l| at chi = xi_/(1+L/R); epsm1 = +inf selects perfect reflectors
+// log|a_l|, log|b_l| at chi = xi_/(1+L/R); epsm1 = +inf selects perfect reflectors.  Four lanes share one l
+// (all 32 lanes of the warp call): lane j of the four takes the functions of order l + 1/2 (j even) or l - 1/2 at chi
+// (j < 2) or, for a metal, at n chi; all four end with the same values.
 CAPS_DEV void mie(double LbyR, double xi_, int l, double epsm1, double *lna, double *lnb)
 {
+    const int j = threadIdx.x & 3;
+    const bool pr = isinf(epsm1); // uniform: one frequency per warp
     const double chi = xi_ / (1 + LbyR);
     const double ln_chi = log(xi_) - log1p(LbyR);
-    double lIp, lKp, lKm;
+    const double ln_n = pr ? 0.0 : log1p(epsm1) / 2, nr = pr ? 1.0 : exp(ln_n);
+    const double x = j < 2 ? chi : nr * chi;
     // I_{l+1/2} / I_{l+3/2} by the continued fraction, I_{l-1/2} / I_{l+1/2} from it
-    const double rho = ratioI(l + 0.5, chi), ratio = (2 * l + 1) / chi + 1.0 / rho;
-    logIK_half(l, chi, rho, &lIp, &lKp);
-    logIK_half(l - 1, chi, ratio, nullptr, &lKm);
-    if (isinf(epsm1)) {
+    const double rho = ratioI(l + 0.5, x), my_ratio = (2 * l + 1) / x + 1.0 / rho;
+    double lI, lK;
+    logIK_half(j & 1 ? l - 1 : l, x, j & 1 ? my_ratio : rho, &lI, &lK);
+    auto of = [&](double v, int k) { return __shfl_sync(0xffffffffu, v, (threadIdx.x & 28) | k); };
+    const double ratio = of(my_ratio, 0), lIp = of(lI, 0), lKp = of(lK, 0), lKm = of(lK, 1);
+    if (pr) {
         *lnb = LOGPI - LN2 + lIp - lKp;
         const double num = LOGPI - LN2 + lIp + log(chi * ratio - l);
         const double den = logadd(log((double)l) + lKp, ln_chi + lKm);
         *lna = num - den;
         return;
     }
-    const double ln_n = log1p(epsm1) / 2, nr = exp(ln_n), ln_l = log((double)l);
-    double lIp_n, lKp_n, lIm_n, lKm_n;
-    const double xn = nr * chi, rho_n = ratioI(l + 0.5, xn), ratio_n = (2 * l + 1) / xn + 1.0 / rho_n;
-    logIK_half(l, xn, rho_n, &lIp_n, &lKp_n);
-    logIK_half(l - 1, xn, ratio_n, &lIm_n, &lKm_n);
+    const double ln_l = log((double)l);
+    const double ratio_n = of(my_ratio, 2), lIp_n = of(lI, 2), lIm_n = of(lI, 3);
     const double ln_gB = lIp_n + lIp + ln_chi + log(nr * ratio_n - ratio);
     const double ln_gC = log(epsm1) + lIp_n + logadd(ln_chi + lKm, ln_l + lKp);
     const double ln_gD = ln_chi + logadd(lIp_n + lKm, ln_n + lKp + lIm_n);
