@@ -380,6 +380,13 @@ __device__ __noinline__ int potf2_limbs(const long long *Sm, size_t lda, int nb,
 // order shows; a block of condition above about 50) or FP32 finds no factor, potf2_limbs takes the
 // block.
 //
+// A block that is near the identity needs no first factor: with |S - 1| < 2^-19 (Frobenius) W0 = 1, E = S - 1
+// as it stands, third order is below 2^-57 and W = 1 - Z; below 2^-33 second order is too.  Two thirds to
+// four fifths of the blocks of a free energy's matrices are such (all but the first few of a
+// matrix), and the blocks of one launch tend to be so together: a launch of such blocks takes about 14 us
+// instead of 40 (factorisation of a free energy at R/L = 100 11.0 -> 9.2 ms, of the 5500 small matrices of
+// a T = 0 energy 6.3 -> 4.3).
+//
 // 512 threads.  The FP32 part runs on the block augmented by the identity in panels of 8 columns (three
 // warps hold a panel's 8 diagonal rows and 24 of the others each; two barriers per panel), so that its
 // code is short: fully unrolled 32 x 32 steps spent most of their time fetching instructions (50 us a
@@ -575,17 +582,19 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
     __shared__ uint64_t sfull[2], drain;
     __shared__ uint32_t tslot;
     __shared__ int s_ok, s_max, s_emax;
+    __shared__ float s_fro[PF_NT / 32];
     __shared__ double slog[2];
-    __shared__ long long sy;
+    __shared__ long long sy[8];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = warp & 3, part = warp >> 2;
     const bool folds = quad < 2;
     const int nb = min(NB, n - k0);
     const long long *Sm = S + (size_t)task * mstride + (size_t)k0 * lda + k0;
     constexpr float Q2F = 0x1p-60f;
     const int er = tid & 63, ek = tid >> 6; // this thread's row and chunk of 8 columns of an image
+    long long *tmp = reinterpret_cast<long long *>(pf_sm + PF_W0); // [64][PP]
+    // the lower triangle (the identity past the matrix), mirrored in shared memory, and |S - 1|^2
     {
-        // the lower triangle (the identity past the matrix), mirrored in shared memory
-        long long x[8], *tmp = reinterpret_cast<long long *>(pf_sm + PF_W0); // [64][PP]
+        long long x[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             const int c = ek * 8 + u;
@@ -597,45 +606,70 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
             umma::mbar_init(&drain, 1);
             s_ok = 1;
             s_max = s_emax = 0;
-            sy = 0;
         }
+        if (tid < 2) slog[tid] = 0.0;
         if (warp == 15) umma::alloc(&tslot, 512);
+        float fro = 0.0f;
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             const int c = ek * 8 + u;
             if (c <= er) {
+                const float e = (float)(x[u] - (er == c ? 1LL << FQ : 0LL)) * Q2F;
+                fro = fmaf(e, e, fro);
                 F[er * PP + c] = (float)x[u] * Q2F;
                 tmp[er * PP + c] = x[u];
                 tmp[c * PP + er] = x[u];
             }
         }
-        __syncthreads();
+        for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
+        if (lane == 0) s_fro[warp] = fro;
+    }
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    float fro = 0.0f;
+    for (int w = 0; w < PF_NT / 32; w++) fro += s_fro[w];
+    fro *= 2.0f; // both triangles (the diagonal counts twice)
+    const bool near1 = fro < 0x1p-38f;     // W0 = 1
+    const bool second = !(fro < 0x1p-66f); // PP^T and P^2 reach the last digit
+    const uint32_t base = umma::smem_u32(pf_sm);
+    const int row = quad * 32 + lane, c0 = part * 16;
+    PfCtx C{sfull, tslot, 0, 0, true};
+    bool ok = true;
+    int wexp = 0;
+    long long v[16];
+    if (near1) {
+        // E = S - 1
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int c = ek * 8 + u;
+            const float e = (float)(tmp[er * PP + c] - (er == c ? 1LL << FQ : 0LL)) * Q2F;
+            F[er * PP + c] = er > c ? e : er == c ? 0.5f * e : 0.0f;
+        }
+        if (folds)
+#pragma unroll
+            for (int c = 0; c < 16; c++) v[c] = tmp[row * PP + c0 + c] - (row == c0 + c ? 1LL << FQ : 0LL);
+    } else {
+        long long x[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) x[u] = tmp[er * PP + ek * 8 + u];
         uint4 d[ND];
         split8(x, d);
 #pragma unroll
         for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(pf_sm + i * IMG_BLK + img_off(er, ek)) = d[i];
-    }
-    if (!pf_factor32(F, X, rinv)) s_ok = 0; // its barriers publish s_ok's first value; the ones below this
-    {
+        if (!pf_factor32(F, X, rinv)) s_ok = 0; // its barriers stand between this and the reads below
         float mx = 0.0f;
 #pragma unroll
         for (int u = 0; u < 8; u++) mx = fmaxf(mx, fabsf(X[er * PP + ek * 8 + u]));
         for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         if (lane == 0) atomicMax(&s_max, __float_as_int(mx)); // non-negative floats order as integers; NaN is large
+        __syncthreads();
+        const float w0max = __int_as_float(s_max);
+        ok = s_ok && w0max < 1e6f; // uniform
+        while (wexp < 24 && w0max > 3.9f * (float)(1 << wexp)) wexp++;
     }
-    umma::fence_before();
-    __syncthreads();
-    umma::fence_after();
-    const float w0max = __int_as_float(s_max);
-    bool ok = s_ok && w0max < 1e6f; // uniform
-    int wexp = 0;
-    while (wexp < 24 && w0max > 3.9f * (float)(1 << wexp)) wexp++;
-    PfCtx C{sfull, tslot, 0, 0, true};
-    if (ok) {
+    if (ok && !near1) {
         const float sc = (float)(1 << 26) / (float)(1 << wexp);
-        const uint32_t base = umma::smem_u32(pf_sm);
         // W0 in place as integers of 27 bits, then its digits, by rows and by columns
 #pragma unroll
         for (int u = 0; u < 8; u++) W27[er * PP + ek * 8 + u] = __float2int_rn(X[er * PP + ek * 8 + u] * sc);
@@ -650,7 +684,6 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
 #pragma unroll
             for (int i = 0; i < 3; i++) *reinterpret_cast<uint4 *>(pf_sm + (t ? PF_WT : PF_W0) + i * IMG_BLK + img_off(er, ek)) = d[i];
         }
-        long long v[16];
         // T = W0 S, in the digits' place afterwards
         pf_product<3, ND>(base + PF_W0, base, v, C);
         if (folds) pf_store(v, pf_sm);
@@ -663,7 +696,6 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
         }
         // E = T W0^T - I; P = F(E) in FP32 in place of L
         pf_product<ND, 3>(base, base + PF_W0, v, C);
-        const int row = quad * 32 + lane, c0 = part * 16;
         if (folds) {
             int mx = 0;
 #pragma unroll
@@ -676,24 +708,30 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
             for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
             if (lane == 0) atomicMax(&s_emax, mx);
         }
+    }
+    if (ok) {
         __syncthreads(); // the MMAs have read T: P's parts take its place (rows high, low, columns high, low)
+        if (second) {
 #pragma unroll
-        for (int t = 0; t < 2; t++) {
-            float x[8];
+            for (int t = 0; t < 2; t++) {
+                float x[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = t ? F[(ek * 8 + u) * PP + er] : F[er * PP + ek * 8 + u];
-            uint4 h, l;
-            split_half(x, h, l);
-            *reinterpret_cast<uint4 *>(pf_sm + (2 * t) * IMG_BLK + img_off(er, ek)) = h;
-            *reinterpret_cast<uint4 *>(pf_sm + (2 * t + 1) * IMG_BLK + img_off(er, ek)) = l;
+                for (int u = 0; u < 8; u++) x[u] = t ? F[(ek * 8 + u) * PP + er] : F[er * PP + ek * 8 + u];
+                uint4 h, l;
+                split_half(x, h, l);
+                *reinterpret_cast<uint4 *>(pf_sm + (2 * t) * IMG_BLK + img_off(er, ek)) = h;
+                *reinterpret_cast<uint4 *>(pf_sm + (2 * t + 1) * IMG_BLK + img_off(er, ek)) = l;
+            }
         }
         const float emax = __int_as_float(s_emax);
         // P P^T and P^2, scaled by 2^36: high high + high low + low high
-        umma::fence_smem_async();
-        umma::fence_before();
-        __syncthreads();
-        umma::fence_after();
-        if (warp == 15) {
+        if (second) {
+            umma::fence_smem_async();
+            umma::fence_before();
+            __syncthreads();
+            umma::fence_after();
+        }
+        if (warp == 15 && second) {
             if (lane == 0) {
                 constexpr uint32_t idesc = umma::idesc_f16(128, 64), hi = umma::desc_hi(1024);
                 const uint32_t ph = umma::desc_lo(base, 128), pl = ph + IMG_BLK / 16;
@@ -712,13 +750,19 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
             }
             __syncwarp();
         } else if (folds) {
-            C.live = C.live && umma::mbar_wait(&sfull[0], C.n0 & 1, FIX_WAIT_ITERS);
-            C.live = __all_sync(0xffffffffu, C.live);
-            umma::fence_after();
+            float gg[16], pp[16];
+#pragma unroll
+            for (int c = 0; c < 16; c++) gg[c] = pp[c] = 0.0f;
+            if (second) {
+                C.live = C.live && umma::mbar_wait(&sfull[0], C.n0 & 1, FIX_WAIT_ITERS);
+                C.live = __all_sync(0xffffffffu, C.live);
+                umma::fence_after();
+                if (C.live) {
+                    umma::ld16(C.tmem + ((uint32_t)(quad * 32) << 16) + c0, gg);
+                    umma::ld16(C.tmem + ((uint32_t)(quad * 32) << 16) + NB + c0, pp);
+                }
+            }
             if (C.live) {
-                float gg[16], pp[16];
-                umma::ld16(C.tmem + ((uint32_t)(quad * 32) << 16) + c0, gg);
-                umma::ld16(C.tmem + ((uint32_t)(quad * 32) << 16) + NB + c0, pp);
                 long long ysum = 0;
 #pragma unroll
                 for (int c = 0; c < 16; c++) {
@@ -732,17 +776,20 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
                     }
                     v[c] = row >= c0 + c ? e - __float2int_rn((g + pp[c]) * 0x1p24f) : 0; // below 2^30 for |E| < 2^-18
                 }
-                if (ysum) atomicAdd(reinterpret_cast<unsigned long long *>(&sy), (unsigned long long)ysum);
-                pf_store(v, pf_sm); // Z's digits; every MMA so far has completed
+                // (64 atomic additions to one word of shared memory took 3 us)
+                for (int o = 16; o > 0; o >>= 1) ysum += __shfl_xor_sync(0xffffffffu, ysum, o);
+                if (lane == 0) sy[part * 2 + quad] = ysum;
+                if (!near1) pf_store(v, pf_sm); // Z's digits; every MMA so far has completed
             }
             umma::fence_before();
         }
-        C.n0++;
+        if (second) C.n0++;
         // W = W0 - Z W0, its digits straight to the image (below 4: the top digit stays below 1024)
-        pf_product<ND, 3>(base, base + PF_WT, v, C);
+        if (!near1) pf_product<ND, 3>(base, base + PF_WT, v, C);
         if (folds) {
 #pragma unroll
-            for (int c = 0; c < 16; c++) v[c] = ((long long)W27[row * PP + c0 + c] << (FQ - 26)) - v[c];
+            for (int c = 0; c < 16; c++)
+                v[c] = (near1 ? (row == c0 + c ? 1LL << FQ : 0LL) : (long long)W27[row * PP + c0 + c] << (FQ - 26)) - v[c];
             if (C.live) pf_store(v, wk.wimg(task, n));
         }
         ok = emax < 0x1p-18f;
@@ -756,7 +803,7 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
     } else if (ok) {
         if (tid == 0) {
             wk.info[task].wexp = wexp;
-            logdet[(size_t)task * fix_nbk(n) + k0 / NB] = (double)sy * 0x1p-60 - (slog[0] + slog[1]);
+            logdet[(size_t)task * fix_nbk(n) + k0 / NB] = (double)(((sy[0] + sy[1]) + (sy[2] + sy[3])) + ((sy[4] + sy[5]) + (sy[6] + sy[7]))) * 0x1p-60 - (slog[0] + slog[1]);
         }
     } else {
         double lg;
