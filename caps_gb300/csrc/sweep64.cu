@@ -177,11 +177,14 @@ __global__ void __launch_bounds__(256) k_sweep64_tab(const Task *tasks, const in
 // contiguous, the order in which k_elem64 reads it)
 constexpr int R64_NT = 256, R64_RING = 4;
 
-// grid nlist * P.  The ring of four rows (TE then TM, L + 2 values each) is in shared memory, or
-// in global memory (ring != nullptr) where it does not fit; one barrier per row.  Rows are a serial chain, so
-// nothing but the ring, three dependent FP64 operations and the barrier stands in it: a thread keeps the
-// coefficients of its first columns in registers, and the next row's seeds and factors are loaded a row
-// ahead (with all of them loaded in the row, 2 us a row; now ROWTIME).
+// grid nlist * P * 2: one polarisation (TE, TM) per CTA, none for the TE of a perfect reflector.  The ring of
+// four rows (L + 2 values each) is in shared memory, or in global memory (ring != nullptr) where it does
+// not fit; one barrier per row.  Rows are a serial chain, so nothing but the ring, three dependent FP64
+// operations and the barrier stands in it: a thread keeps the coefficients of its first columns in
+// registers, and the next row's seeds and factors are loaded a row ahead (with all of them loaded in
+// the row, 2 us a row).  Both polarisations in one CTA hold one SM's FP64 pipe for 2800 clocks per
+// row of 700 columns while others have no matrix (24 matrices of ldim 1050 0.98 ms, one polarisation per CTA 0.52;
+// 4 of ldim 2500 2.4 and 1.3).  A row of ldim 140 takes 0.45 us.
 constexpr int R64_KEEP = 3; // columns per thread with coefficients in registers
 __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *tlist, int nlist, int ldim, int P,
                                                   const sd *__restrict__ rows, const double *__restrict__ tab,
@@ -189,39 +192,34 @@ __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *
 {
     extern __shared__ __align__(16) double r64_sm[];
     const int L = ldim + 2, LP = L + 2;
-    const int b = blockIdx.x / P, q = P - 1 - (int)blockIdx.x % P;
+    const int pol = blockIdx.x & 1, part = blockIdx.x >> 1, b = part / P, q = P - 1 - part % P;
     if (b >= nlist) return;
     const int task = tlist ? tlist[b] : b;
     if (status[task] & ~0xF) return; // no status changes in this launch: uniform
     const Task &T = tasks[task];
+    if (T.is_pr && pol == 0) return;
     const int c = col64(T), r1 = rec64_row(q + 1, P, L);
-    const bool te = !T.is_pr;
-    double *R = ring ? ring + (size_t)blockIdx.x * R64_RING * 2 * LP : r64_sm;
-    auto rowp = [&](int r) { return R + (size_t)((r & 3) * 2) * LP; };
+    double *R = ring ? ring + (size_t)blockIdx.x * R64_RING * LP : r64_sm;
+    auto rowp = [&](int r) { return R + (size_t)(r & 3) * LP; };
     const double *W = tab + (size_t)b * W_FIELDS * L;
     auto F = [&](int f, int w) { return __ldg(W + (size_t)f * L + w); };
     const int *kt = ktab + (size_t)b * L;
-    double *tE = tt + (size_t)b * 2 * L * L, *tT = tE + (size_t)L * L;
+    double *t = tt + ((size_t)b * 2 + pol) * L * L;
     const int tid = threadIdx.x;
     int r = 0;
     if (q > 0) { // the two rows before the range, from their q-sums
         r = rec64_row(q, P, L) + 1;
         for (int i = 0; i < 2; i++) {
             const int rr = r - 2 + i;
-            const sd *src = rows + ((((size_t)b * (P - 1) + q - 1) * 2 + i) * 2) * L;
+            const sd *src = rows + ((((size_t)b * (P - 1) + q - 1) * 2 + i) * 2 + pol) * L;
             double *D = rowp(rr);
-            for (int y = tid; y <= rr; y += R64_NT) {
-                const int k = kt[rr] + kt[y];
-                const double vE = y < c ? 0.0 : sd_scaled(src[y], k), vT = y < c ? 0.0 : sd_scaled(src[L + y], k);
-                D[y] = vE;
-                D[LP + y] = vT;
-            }
+            for (int y = tid; y <= rr; y += R64_NT) D[y] = y < c ? 0.0 : sd_scaled(src[y], kt[rr] + kt[y]);
         }
         __syncthreads();
     }
-    __shared__ double ahead[2][8]; // of the next row: its seeds (W_SEED ..), R1, R2
+    __shared__ double ahead[2][5]; // of the next row: its seeds (W_SEED ..), R1, R2
     auto fetch = [&](int row) {
-        if (tid < 8 && row < L) ahead[row & 1][tid] = F(tid < 6 ? W_SEED + tid : W_R1 + tid - 6, row);
+        if (tid < 5 && row < L) ahead[row & 1][tid] = F(tid < 3 ? W_SEED + 2 * tid + pol : W_R1 + tid - 3, row);
     };
     double cp[R64_KEEP], cm[R64_KEEP];
 #pragma unroll
@@ -238,25 +236,15 @@ __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *
         // rows before the first are never read: y >= c + 1 and y <= r - 2 need r >= 3
         const double *P1 = rowp(r + 3), *P2 = rowp(r + 2); // rows r - 1, r - 2
         const double *sr = ahead[r & 1];
-        const double R1 = sr[6], R2 = sr[7];
+        const double R1 = sr[3], R2 = sr[4];
         auto column = [&](int y, double Cp, double Cm) {
-            double vE = 0.0, vT = 0.0;
+            double v = 0.0;
             if (y >= c) {
-                if (y == r || y == r - 1 || y == c) {
-                    const int k = y == r ? 0 : y == r - 1 ? 2 : 4;
-                    vE = sr[k];
-                    vT = sr[k + 1];
-                } else {
-                    vT = fma(R1, fma(Cp, P1[LP + y + 1], Cm * P1[LP + y - 1]), R2 * P2[LP + y]);
-                    if (te) vE = fma(R1, fma(Cp, P1[y + 1], Cm * P1[y - 1]), R2 * P2[y]);
-                }
+                if (y == r || y == r - 1 || y == c) v = sr[y == r ? 0 : y == r - 1 ? 1 : 2];
+                else v = fma(R1, fma(Cp, P1[y + 1], Cm * P1[y - 1]), R2 * P2[y]);
             }
-            D[LP + y] = vT;
-            tT[(size_t)y * L + r] = vT;
-            if (te) {
-                D[y] = vE;
-                tE[(size_t)y * L + r] = vE;
-            }
+            D[y] = v;
+            t[(size_t)y * L + r] = v;
         };
 #pragma unroll
         for (int i = 0; i < R64_KEEP; i++)
@@ -373,7 +361,7 @@ __global__ void __launch_bounds__(E64_X) k_elem64(const Task *tasks, const int *
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-static size_t r64_ring_bytes(int ldim) { return (size_t)R64_RING * 2 * (ldim + 4) * sizeof(double); }
+static size_t r64_ring_bytes(int ldim) { return (size_t)R64_RING * (ldim + 4) * sizeof(double); }
 static bool r64_ring_fits(int ldim) { return r64_ring_bytes(ldim) <= 220 * 1024; }
 
 size_t seed64_bytes(int ldim, int ntask) { return (size_t)ntask * 2 * SEED_KINDS * (ldim + 2) * sizeof(sd); }
@@ -385,7 +373,7 @@ size_t sweep64_work_bytes(int ldim, int nlist)
 {
     const size_t L = ldim + 2, P = rec64_parts(ldim);
     size_t b = (size_t)nlist * L * (2 * L * sizeof(double) + W_FIELDS * sizeof(double) + (P - 1) * 4 * sizeof(sd) + sizeof(int)) + 512;
-    if (!r64_ring_fits(ldim)) b += (size_t)nlist * P * r64_ring_bytes(ldim);
+    if (!r64_ring_fits(ldim)) b += (size_t)nlist * P * 2 * r64_ring_bytes(ldim);
     return b;
 }
 
@@ -428,7 +416,7 @@ void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, co
     }
     seed64(tasks, tlist, nlist, ldim, P, SEED_D1, SEED_COL, K, nu_stride, lft, ptab, pstride, seed, rows, status, st);
     k_sweep64_tab<<<nlist, 256, 0, st>>>(tasks, tlist, nlist, ldim, (const sd *)seed, Sa, Sb, tab, kt);
-    k_rec64<<<nlist * P, R64_NT, sm, st>>>(tasks, tlist, nlist, ldim, P, rows, tab, kt, tt, status, ring);
+    k_rec64<<<nlist * P * 2, R64_NT, sm, st>>>(tasks, tlist, nlist, ldim, P, rows, tab, kt, tt, status, ring);
     const dim3 g((ldim + E64_X - 1) / E64_X, (ldim + E64_Y - 1) / E64_Y, nlist);
     if (fro) k_elem64<true><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, mdiag, info, A, mstride, fro, status);
     else k_elem64<false><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, mdiag, info, A, mstride, fro, status);
