@@ -9,11 +9,13 @@
 // formed from an exact integer numerator.  One division per pair remains.
 #pragma once
 #include "common.cuh"
+#include <climits>
+#include <type_traits>
 
 namespace capsgpu {
 
 struct QAcc {
-    double s; int e; bool on; int count;
+    double s; int e;
 };
 
 CAPS_DEV void qacc_add(QAcc &A, double mant, int ex)
@@ -72,9 +74,9 @@ CAPS_DEV bool qsum_pair(const Task &T, int l1, int l2, const A012 &A12, const sd
     QAcc aT, aE;
     {
         const sd k0 = KTM[l12];
-        aT = QAcc{k0.m, k0.e, true, 0};
-        if (both) { const sd e0 = KTE[l12]; aE = QAcc{e0.m, e0.e, true, 0}; }
-        else aE = QAcc{0, 0, false, 0};
+        aT = QAcc{k0.m, k0.e};
+        if (both) { const sd e0 = KTE[l12]; aE = QAcc{e0.m, e0.e}; }
+        else aE = QAcc{0, 0};
     }
     double aqm2 = 0, aqm1 = 1; // a_{q-2}, a_{q-1}
     if (qmax >= 1) {
@@ -97,10 +99,12 @@ CAPS_DEV bool qsum_pair(const Task &T, int l1, int l2, const A012 &A12, const sd
         //   X_q = Ap^2 + K1 alpha(p+2) + K2 alpha(p+3), Y_q = K3 alpha(p+4), Z_q = K0 alpha(p+1)
         // (eqs. (26)-(28) with the common factor Ap divided out), and the partial
         // sums carried as S_q = D_q sum_{j<=q} a_j K_j = Z_q S_{q-1} + b_q K_q.
-        // b, D and each S keep their own power-of-two exponent; the reference's
-        // early stop (term 60 e-folds below the q=0 term, three times in a row)
-        // is decided on those exponents, with logarithms only inside the +-2
-        // binade band around the threshold.  One division per pair remains.
+        // b, D and each S keep their own power-of-two exponent.  Four steps at a time: their coefficients
+        // need p alone and only the b, D and S chains are serial, the exponents are set to zero once
+        // per four (a step changes them by 2^102 at most) and the reference's early stop (term 60
+        // e-folds below the q = 0 term, three times in a row) is tested on the exponents of the last
+        // three; terms after it are below 2^-86 of the sum.  One step at a time with a branch for each
+        // of these took 820 clocks a step in a thread of its own, this 450.  One division per pair remains.
         // alpha(x) = N(x)/(4x^2-1) with the integer numerator
         // N(x) = (x-S)(x+S)(x-Dd)(x+Dd), S = l1+l2+1, Dd = l1-l2, formed exactly in int64
         // (|N| < 2^62 for every degree this library accepts) and converted once.
@@ -112,73 +116,83 @@ CAPS_DEV bool qsum_pair(const Task &T, int l1, int l2, const A012 &A12, const sd
         const bool diag = (l1 == l2); // Ap == 0: eq. (30)
         const double Ap2 = diag ? 0.0 : Ap * Ap;
         const double4 *pt = ptab + (diag ? pstride : 0);
-        struct PS { double S; int eS; bool on; int count; double D; int eD; int e0; const sd *K0; };
-        PS P[2] = {{aT.s, aT.e, true, 0, 1.0, 0, 0, KTM + l12}, {aE.s, aE.e, both, 0, 1.0, 0, 0, KTE + l12}};
-        P[0].e0 = KTM[l12].e;
-        if (both) P[1].e0 = KTE[l12].e;
-        const sd *Kp[2] = {KTM, KTE};
+        struct PS { double S; int eS; const sd *K; int e0; };
+        PS P[2] = {{aT.s, aT.e, KTM, KTM[l12].e}, {aE.s, aE.e, KTE, both ? KTE[l12].e : 0}};
         double bm2 = aqm2, bm1 = aqm1, Dq = 1.0, Zprev = 1.0;
         int eb = 0, eD = 0;
         int ip = l12 - 6; // p of q = 3
         double N3 = Nf(ip + 3), N4 = Nf(ip + 4);
-        for (int q = 3; q <= qmax && (P[0].on || P[1].on); q++, ip -= 2) {
-            const double N1 = Nf(ip + 1), N2 = Nf(ip + 2);
-            const double4 k = pt[ip];
-            const double X = fma(k.z, N3, fma(k.y, N2, Ap2));
-            const double Y = k.w * N4;
-            const double Z = k.x * N1;
-            const double b = fma(X, bm1, -(Y * Zprev) * bm2);
-            Dq *= Z;
-            N3 = N1; N4 = N2; Zprev = Z;
-            bm2 = bm1; bm1 = b;
-            {   // exact rescaling of b (with b_{q-1}) and D
-                const int kb = expo(b);
-                if (kb > 300 || (kb < -300 && kb > -1023)) { bm1 = shift2(bm1, -kb); bm2 = shift2(bm2, -kb); eb += kb; }
-                const int kd = expo(Dq);
-                if (kd > 300 || kd < -300) { Dq = shift2(Dq, -kd); eD += kd; }
+        // NS steps; true when the last three terms of every sum are below the bound
+        auto steps = [&](auto ns) -> bool {
+            constexpr int NS = decltype(ns)::value;
+            double X[NS], Y[NS], Z[NS], b[NS];
+            int eDq[NS];
+#pragma unroll
+            for (int i = 0; i < NS; i++) {
+                const int x = ip - 2 * i;
+                const double N1 = Nf(x + 1), N2 = Nf(x + 2);
+                const double4 k = pt[x];
+                X[i] = fma(k.z, N3, fma(k.y, N2, Ap2));
+                Y[i] = k.w * N4;
+                Z[i] = k.x * N1;
+                N3 = N1;
+                N4 = N2;
             }
-            const int eb1 = expo(bm1);
-            const int eDq = expo(Dq) + eD;
+            // exact rescaling of b (with b_{q-1}) and D
+            const int eb1 = expo(bm1), kb = eb1 == -1023 ? 0 : eb1, kd = expo(Dq);
+            bm1 = shift2(bm1, -kb);
+            bm2 = shift2(bm2, -kb);
+            eb += kb;
+            Dq = shift2(Dq, -kd);
+            eD += kd;
+#pragma unroll
+            for (int i = 0; i < NS; i++) {
+                b[i] = fma(X[i], bm1, -(Y[i] * Zprev) * bm2);
+                Dq *= Z[i];
+                eDq[i] = expo(Dq) + eD;
+                Zprev = Z[i];
+                bm2 = bm1;
+                bm1 = b[i];
+            }
+            bool done = NS >= 3;
 #pragma unroll
             for (int pi = 0; pi < 2; pi++) {
+                if (pi && !both) continue;
                 PS &A = P[pi];
-                if (!A.on) continue;
-                const sd Kv = Kp[pi][ip];
-                const double t = bm1 * Kv.m;          // term * D_q / 2^(eb+Ke)
-                const int et = eb + Kv.e;
-                // S_q = Z S_{q-1} + t 2^(et - eS)
-                int d = et - A.eS;
-                const int es = expo(A.S);
-                if (es == -1023) { A.eS = et; d = 0; }
-                else if (d > 64) { A.S = shift2(A.S, -d); A.eS = et; d = 0; }
-                A.S = fma(Z, A.S, shift2(t, d));
+                sd Kv[NS];
+                int top = INT_MIN;
+#pragma unroll
+                for (int i = 0; i < NS; i++) {
+                    Kv[i] = A.K[ip - 2 * i];
+                    top = max(top, eb + Kv[i].e);
+                }
+                // S_q = Z S_{q-1} + b K 2^(eb + Ke - eS)
                 const int ks = expo(A.S);
-                if (ks > 300 || (ks < -300 && ks > -1023)) { A.S = shift2(A.S, -ks); A.eS += ks; }
-                // early stop on |a_q K_q| / |K_0| < e^-60, i.e. log2 ratio < -86.5617; a zero
-                // term counts as below, as log 0 = -inf does in the reference's test
-                {
-                    const int approx = eb1 + eb + Kv.e - eDq - A.e0; // true log2 ratio in (approx-2, approx+2)
-                    bool below;
-                    if (eb1 == -1023) below = true;
-                    else if (approx <= -89) below = true;
-                    else if (approx >= -84) below = false;
-                    else {
-                        // exact test without logarithms: with mantissas in [1,2),
-                        // ratio = 2^approx * (mb mK)/(mD m0) < e^-60  <=>  mb mK < 2^(-60/ln2 - approx) mD m0
-                        const double c = approx == -88 ? 2.710008819393852 : approx == -87 ? 1.355004409696926
-                                       : approx == -86 ? 0.677502204848463 : 0.3387511024242315;
-                        const double mb = shift2(bm1, -eb1), mD = shift2(Dq, -expo(Dq));
-                        below = fabs(mb * Kv.m) < c * fabs(mD * A.K0->m);
-                    }
-                    if (below) { if (++A.count >= 3) { A.on = false; A.D = Dq; A.eD = eD; } }
-                    else A.count = 0;
+                if (ks == -1023) A.eS = top;
+                else {
+                    A.eS += ks;
+                    const int d = top - A.eS > 64 ? top - A.eS : 0; // S that far below the new terms
+                    A.S = shift2(A.S, -ks - d);
+                    A.eS += d;
+                }
+#pragma unroll
+                for (int i = 0; i < NS; i++) {
+                    A.S = fma(Z[i], A.S, b[i] * shift2(Kv[i].m, eb + Kv[i].e - A.eS));
+                    // log2 of the term's ratio to the q = 0 term, to within 2; a zero term counts as below, as log 0 = -inf
+                    // does in the reference's test (60 e-folds are 86.56)
+                    if (i >= NS - 3) done &= expo(b[i]) == -1023 || expo(b[i]) + eb + Kv[i].e - eDq[i] - A.e0 <= -89;
                 }
             }
-        }
+            ip -= 2 * NS;
+            return done;
+        };
+        int q = 3;
+        bool done = false;
+        for (; q + 3 <= qmax && !done; q += 4) done = steps(std::integral_constant<int, 4>());
+        for (; q <= qmax && !done; q++) steps(std::integral_constant<int, 1>());
         for (int pi = 0; pi < 2; pi++) {
             PS &A = P[pi];
-            if (A.on) { A.D = Dq; A.eD = eD; }
-            const sd r = sd_norm(A.S / A.D, A.eS - A.eD);
+            const sd r = sd_norm(A.S / Dq, A.eS - eD);
             if (pi == 0) { aT.s = r.m; aT.e = r.e; } else { aE.s = r.m; aE.e = r.e; }
         }
     }

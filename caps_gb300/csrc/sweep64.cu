@@ -42,16 +42,20 @@ __host__ __device__ inline int rec64_parts(int ldim) { return ldim < 1024 ? 1 : 
 // ---------------------------------------------------------------------------
 // seed[((task * 2 + pol) * SEED_KINDS + kind) * L + w]: the pair (w, w), (w+1, w), (w+2, w) or (w, c);
 // rows[(((b * (P - 1) + q - 1) * 2 + i) * 2 + pol) * L + y]: row(q) - 1 + i of listed task b, y <= row
-// grid (ceil(L / 128) * (2 + 2 (P - 1)), nlist), one pair per thread; kind0 and kind1 first
-__global__ void __launch_bounds__(128) k_seed64(const Task *tasks, const int *tlist, int nlist, int ldim, int P, int kind0, int kind1,
+// grid (ceil(L / 32) * (2 + 2 (P - 1)), nlist), one pair per thread; kind0 and kind1 first.  One warp per CTA: a
+// step of the q recurrence takes about 20 FP64 operations, 16 clocks of the SM's pipe each and warp, so that the
+// warps of one CTA would wait for each other while other SMs have none (free energy at R/L = 20: four warps per
+// CTA 0.68 ms, one 0.55; R/L = 100 3.18 and 3.05)
+constexpr int SEED_NT = 32;
+__global__ void __launch_bounds__(SEED_NT) k_seed64(const Task *tasks, const int *tlist, int nlist, int ldim, int P, int kind0, int kind1,
                                                 const sd *__restrict__ K, int nu_stride, const double *__restrict__ lft,
                                                 const double4 *__restrict__ ptab, int pstride, sd *seed, sd *rows, int *status)
 {
-    const int L = ldim + 2, nbw = (L + 127) / 128;
+    const int L = ldim + 2, nbw = (L + SEED_NT - 1) / SEED_NT;
     if ((int)blockIdx.y >= nlist) return;
     const int task = tlist ? tlist[blockIdx.y] : (int)blockIdx.y;
     const Task &T = tasks[task];
-    const int part = blockIdx.x / nbw, w = ((int)blockIdx.x % nbw) * 128 + threadIdx.x;
+    const int part = blockIdx.x / nbw, w = ((int)blockIdx.x % nbw) * SEED_NT + threadIdx.x;
     if (w >= L) return;
     int a1 = w, a2 = w;
     sd *oT, *oE;
@@ -380,8 +384,8 @@ size_t sweep64_work_bytes(int ldim, int nlist)
 static void seed64(const Task *tasks, const int *tlist, int nlist, int ldim, int P, int k0, int k1, const sd *K, int nu_stride,
                    const double *lft, const double4 *ptab, int pstride, void *seed, sd *rows, int *status, cudaStream_t st)
 {
-    const int nbw = (ldim + 2 + 127) / 128;
-    k_seed64<<<dim3(nbw * (2 + 2 * (P - 1)), nlist), 128, 0, st>>>(tasks, tlist, nlist, ldim, P, k0, k1, K, nu_stride, lft, ptab, pstride,
+    const int nbw = (ldim + 2 + SEED_NT - 1) / SEED_NT;
+    k_seed64<<<dim3(nbw * (2 + 2 * (P - 1)), nlist), SEED_NT, 0, st>>>(tasks, tlist, nlist, ldim, P, k0, k1, K, nu_stride, lft, ptab, pstride,
                                                                   (sd *)seed, rows, status);
     COUNT_LAUNCH(1);
 }
