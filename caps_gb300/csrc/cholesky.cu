@@ -79,23 +79,34 @@ CAPS_DEV void mma_nonzero(uint32_t tmem, uint32_t alo, uint32_t blo, int fa, int
     }
 }
 
-// NC columns of group s of this warp's lanes folded into v: groups come in the order s = 0, 1, ..., 6 and
+// 16 columns of group s of this warp's lanes folded into v: groups come in the order s = s0, ..., 6 and
 // each weighs 2^-9 of the one before, v = 512 v + g up to s = 5 (units of 2^-61; |v| < 2), then
 // units of 2^-60.  One piece of code for all groups: unrolled, its first pass through the instruction cache
-// cost more than the work.
-template <int NC> CAPS_DEV void fold_group(uint32_t taddr, int s, long long (&v)[NC])
+// cost more than the work.  A sum (an integer below 2^25) is read as the bits of g + 1.5 2^23 and the
+// constant taken out at the end; a warp with one of 2^22 or more converts (19 clocks a number and warp where
+// this takes about 7).
+CAPS_DEV void fold_group(uint32_t taddr, int s, int s0, long long (&v)[16])
 {
+    float f[16];
+    unsigned t[16], over = 0;
+    umma::ld16(taddr, f);
 #pragma unroll
-    for (int h = 0; h < NC / 16; h++) {
-        float f[16];
-        umma::ld16(taddr + h * 16, f);
-        if (s < 6) { // uniform
+    for (int c = 0; c < 16; c++) {
+        t[c] = __float_as_uint(f[c] + FX_MAGIC);
+        over |= t[c] ^ 0x4B000000u;
+    }
+    if (__any_sync(0xffffffffu, over >> 23)) {
 #pragma unroll
-            for (int c = 0; c < 16; c++) v[h * 16 + c] = v[h * 16 + c] * 512 + __float2int_rn(f[c]);
-        } else {
+        for (int c = 0; c < 16; c++) t[c] = FX_MBITS + (unsigned)__float2int_rn(f[c]);
+    }
+    if (s < 6) { // uniform
 #pragma unroll
-            for (int c = 0; c < 16; c++) v[h * 16 + c] = (v[h * 16 + c] + ((__float2int_rn(f[c]) + 256) >> 9) + 1) >> 1;
-        }
+        for (int c = 0; c < 16; c++) v[c] = (long long)((unsigned long long)v[c] * 512 + t[c]);
+    } else {
+        unsigned long long k = 0;
+        for (int i = s0; i < 6; i++) k = k * 512 + FX_MBITS;
+#pragma unroll
+        for (int c = 0; c < 16; c++) v[c] = ((long long)((unsigned long long)v[c] - k) + (((int)(t[c] - FX_MBITS) + 256) >> 9) + 1) >> 1;
     }
 }
 
@@ -381,7 +392,8 @@ __device__ __noinline__ int potf2_limbs(const long long *Sm, size_t lda, int nb,
 // block.
 //
 // A block that is near the identity needs no first factor: with |S - 1| < 2^-19 (Frobenius) W0 = 1, E = S - 1
-// as it stands, third order is below 2^-57 and W = 1 - Z; below 2^-33 second order is too.  Two thirds to
+// as it stands, third order is below 2^-57 and W = 1 - Z; below 2^-33 second order is too; up to 2^-10 W0 = 1 - F(S - 1)
+// leaves an E below 2^-19, and no FP32 factor is needed (8 us).  Two thirds to
 // four fifths of the blocks of a free energy's matrices are such (all but the first few of a
 // matrix), and the blocks of one launch tend to be so together: a launch of such blocks takes about 14 us
 // instead of 40 (factorisation of a free energy at R/L = 100 11.0 -> 9.2 ms, of the 5500 small matrices of
@@ -546,7 +558,7 @@ template <int NA, int NBD> CAPS_DEV void pf_product(uint32_t a, uint32_t b, long
                 C.live = __all_sync(0xffffffffu, C.live);
                 umma::fence_after();
             }
-            if (C.live) fold_group(C.tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
+            if (C.live) fold_group(C.tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, 0, v);
         }
         umma::fence_before();
     }
@@ -589,7 +601,6 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
     const bool folds = quad < 2;
     const int nb = min(NB, n - k0);
     const long long *Sm = S + (size_t)task * mstride + (size_t)k0 * lda + k0;
-    constexpr float Q2F = 0x1p-60f;
     const int er = tid & 63, ek = tid >> 6; // this thread's row and chunk of 8 columns of an image
     long long *tmp = reinterpret_cast<long long *>(pf_sm + PF_W0); // [64][PP]
     // the lower triangle (the identity past the matrix), mirrored in shared memory, and |S - 1|^2
@@ -614,9 +625,9 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
         for (int u = 0; u < 8; u++) {
             const int c = ek * 8 + u;
             if (c <= er) {
-                const float e = (float)(x[u] - (er == c ? 1LL << FQ : 0LL)) * Q2F;
+                const float e = fx_value(x[u] - (er == c ? 1LL << FQ : 0LL));
                 fro = fmaf(e, e, fro);
-                F[er * PP + c] = (float)x[u] * Q2F;
+                F[er * PP + c] = e;
                 tmp[er * PP + c] = x[u];
                 tmp[c * PP + er] = x[u];
             }
@@ -643,8 +654,7 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             const int c = ek * 8 + u;
-            const float e = (float)(tmp[er * PP + c] - (er == c ? 1LL << FQ : 0LL)) * Q2F;
-            F[er * PP + c] = er > c ? e : er == c ? 0.5f * e : 0.0f;
+            if (c >= er) F[er * PP + c] = c == er ? 0.5f * F[er * PP + c] : 0.0f;
         }
         if (folds)
 #pragma unroll
@@ -657,7 +667,17 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
         split8(x, d);
 #pragma unroll
         for (int i = 0; i < ND; i++) *reinterpret_cast<uint4 *>(pf_sm + i * IMG_BLK + img_off(er, ek)) = d[i];
-        if (!pf_factor32(F, X, rinv)) s_ok = 0; // its barriers stand between this and the reads below
+        if (fro < 0x1p-20f) {
+            // W0 = 1 - F(S - 1)
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int c = ek * 8 + u;
+                X[er * PP + c] = c > er ? 0.0f : c == er ? 1.0f - 0.5f * F[er * PP + c] : -F[er * PP + c];
+            }
+        } else {
+            if (er >= ek * 8 && er < ek * 8 + 8) F[er * PP + er] += 1.0f;
+            if (!pf_factor32(F, X, rinv)) s_ok = 0; // its barriers stand between this and the reads below
+        }
         float mx = 0.0f;
 #pragma unroll
         for (int u = 0; u < 8; u++) mx = fmaxf(mx, fabsf(X[er * PP + ek * 8 + u]));
@@ -672,7 +692,7 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
         const float sc = (float)(1 << 26) / (float)(1 << wexp);
         // W0 in place as integers of 27 bits, then its digits, by rows and by columns
 #pragma unroll
-        for (int u = 0; u < 8; u++) W27[er * PP + ek * 8 + u] = __float2int_rn(X[er * PP + ek * 8 + u] * sc);
+        for (int u = 0; u < 8; u++) W27[er * PP + ek * 8 + u] = fx_f2i(X[er * PP + ek * 8 + u] * sc);
         __syncthreads();
 #pragma unroll
         for (int t = 0; t < 2; t++) {
@@ -701,7 +721,7 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
 #pragma unroll
             for (int c = 0; c < 16; c++) {
                 v[c] = (v[c] << (2 * wexp)) - (row == c0 + c ? 1LL << FQ : 0LL);
-                const float e = (float)v[c] * Q2F;
+                const float e = fx_value(v[c]);
                 F[row * PP + c0 + c] = row > c0 + c ? e : row == c0 + c ? 0.5f * e : 0.0f;
                 mx = max(mx, __float_as_int(fabsf(e)));
             }
@@ -763,19 +783,23 @@ __global__ void __launch_bounds__(PF_NT, 1) k_fix_potf2(int ntask, int n, int k0
                 }
             }
             if (C.live) {
-                long long ysum = 0;
+                long long ydiag = 0;
+                float gdiag = 0.0f;
 #pragma unroll
                 for (int c = 0; c < 16; c++) {
-                    // Z = F(E) - F(P P^T) - P^2; log(1 + y) = y - y^2 / 2 + y^3 / 3 of Y's diagonal
+                    // Z = F(E) - F(P P^T) - P^2
                     const bool dg = row == c0 + c;
                     const long long e = dg ? v[c] >> 1 : v[c];
                     const float g = dg ? 0.5f * gg[c] : gg[c];
-                    if (dg && row < nb) {
-                        const float y = (float)e * Q2F;
-                        ysum = e - __float2int_rn(g * 0x1p24f + y * y * (0.5f - 0.33333333f * y) * 0x1p60f);
+                    if (dg) {
+                        ydiag = e;
+                        gdiag = g;
                     }
-                    v[c] = row >= c0 + c ? e - __float2int_rn((g + pp[c]) * 0x1p24f) : 0; // below 2^30 for |E| < 2^-18
+                    v[c] = row >= c0 + c ? e - fx_f2i((g + pp[c]) * 0x1p24f) : 0; // below 2^30 for |E| < 2^-18
                 }
+                // log(1 + y) = y - y^2 / 2 + y^3 / 3 of Y's diagonal
+                const float y = fx_value(ydiag);
+                long long ysum = row < nb ? ydiag - fx_f2i(gdiag * 0x1p24f + y * y * (0.5f - 0.33333333f * y) * 0x1p60f) : 0;
                 // (64 atomic additions to one word of shared memory took 3 us)
                 for (int o = 16; o > 0; o >>= 1) ysum += __shfl_xor_sync(0xffffffffu, ysum, o);
                 if (lane == 0) sy[part * 2 + quad] = ysum;
@@ -946,7 +970,7 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
             ok = __all_sync(0xffffffffu, ok);
             umma::fence_after();
         }
-        if (ok && g >= fa) fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
+        if (ok && g >= fa) fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, fa, v);
     }
     const int wexp = wk.info[task].wexp, rb = quad >> 1; // rb: row block of the pair
     {
@@ -1067,7 +1091,7 @@ __global__ void __launch_bounds__(SY_THREADS, 1) k_fix_syrk(int ntask, int n, in
                 umma::fence_after();
 #pragma unroll 1
                 for (int g = max(s0, h ? SY_G0 : 0); g < (h ? NG : SY_G0); g++)
-                    fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, v);
+                    fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, s0, v);
                 umma::fence_before();
                 __syncwarp();
                 if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(&sempty[h])) : "memory");
