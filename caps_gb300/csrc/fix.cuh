@@ -64,6 +64,20 @@ CAPS_DEV float fx_value(long long x)
     return fmaf((float)(int)((x + 0x80000000LL) >> 32), 0x1p-28f, (float)(int)x * 0x1p-60f);
 }
 
+// v in units of 2^-q, rounded, saturated at +-2^62 (integer work only)
+CAPS_DEV long long to_fix(double v, int q, bool &bad)
+{
+    const long long b = __double_as_longlong(v);
+    const int ex = (int)((b >> 52) & 0x7ff);
+    bad |= ex == 0x7ff;
+    const int sh = ex - 1075 + q;
+    long long mnt = (b & 0xfffffffffffffLL) | (1LL << 52);
+    if (sh >= 10) mnt = 1LL << 62;
+    else if (sh >= 0) mnt <<= sh;
+    else mnt = sh < -54 ? 0 : (mnt + (1LL << (-sh - 1))) >> -sh;
+    return b < 0 ? -mnt : mnt;
+}
+
 // eight numbers (units of 2^-60, |x| < 4) to six 16-byte vectors of FP16 digits
 CAPS_DEV void split8(const long long (&x)[8], uint4 (&d)[ND])
 {

@@ -16,7 +16,7 @@
 // their row (J' = dA J costs what J does) and the column factors into tables, 20 operations for
 // the four elements of a pair; conversion to fixed point is integer work.  For a perfectly
 // reflecting plate T_TE = -T_TM, and only T_TM is formed.
-#include "common.cuh"
+#include "fix.cuh"
 #include "internal.h"
 #include "qsum64.cuh"
 #include "umma.cuh"
@@ -261,20 +261,6 @@ __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *
 // ---------------------------------------------------------------------------
 // elements
 // ---------------------------------------------------------------------------
-// v in units of 2^-q, rounded, saturated at +-2^62 (integer work only)
-CAPS_DEV long long to_fix(double v, int q, bool &bad)
-{
-    const long long b = __double_as_longlong(v);
-    const int ex = (int)((b >> 52) & 0x7ff);
-    bad |= ex == 0x7ff;
-    const int sh = ex - 1075 + q;
-    long long mnt = (b & 0xfffffffffffffLL) | (1LL << 52);
-    if (sh >= 10) mnt = 1LL << 62;
-    else if (sh >= 0) mnt <<= sh;
-    else mnt = sh < -54 ? 0 : (mnt + (1LL << (-sh - 1))) >> -sh;
-    return b < 0 ? -mnt : mnt;
-}
-
 // grid (ceil(ldim / E64_X), ceil(ldim / E64_Y), nlist), E64_X threads: thread x (window index 1 ..
 // ldim, a row of 2x2 blocks) walks E64_Y columns y <= x with T and J of the columns y - 1, y, y + 1 in
 // registers; consecutive threads write consecutive rows of the column-major matrix.
