@@ -110,10 +110,10 @@ __global__ void k_diag64(const Task *tasks, int ntask, int ldim, const sd *__res
 // per-window tables
 // ---------------------------------------------------------------------------
 // per listed task and window index: Cp, Cm of the recurrence; R1 = 1 / Cp(w - 1), R2 = -Cm(w - 1) R1
-// of row w; UA = Um dA, VA = -Vp dA, A = m dA and the same with dB; dA, dB; the scaled seeds of row w:
+// of row w; UA = Um dA, VA = -Vp dA, A = m dA and the same with dB; dA, dB; the largest of the six; the scaled seeds of row w:
 // T(w, w), T(w, w - 1), T(w, c), TE and TM each.  tab[(b * W_FIELDS + field) * L + w], so that consecutive lanes read
 // consecutive entries
-enum { W_CP, W_CM, W_R1, W_R2, W_UA, W_VA, W_A, W_UB, W_VB, W_B, W_DA, W_DB, W_SEED, W_FIELDS = W_SEED + 6 };
+enum { W_CP, W_CM, W_R1, W_R2, W_UA, W_VA, W_A, W_UB, W_VB, W_B, W_DA, W_DB, W_MX, W_SEED, W_FIELDS = W_SEED + 7 }; // even
 
 // m 2^e as a double; below the normal range 0, above it infinite
 CAPS_DEV double sd_scaled(sd v, int k)
@@ -161,6 +161,10 @@ __global__ void __launch_bounds__(256) k_sweep64_tab(const Task *tasks, const in
         const double um = (l + 1.0) * cm, vp = l * cp, m = T.m;
         const double dA = sd_scaled(Sa[(size_t)task * L + w], -kw), dB = sd_scaled(Sb[(size_t)task * L + w], -kw);
         double f[W_FIELDS] = {cp, cm, r1, r2, um * dA, -vp * dA, m * dA, um * dB, -vp * dB, m * dB, dA, dB};
+        int top = 0; // by the high words, so that a NaN is largest
+#pragma unroll
+        for (int i = W_UA; i <= W_B; i++) top = max(top, __double2hiint(f[i]) & 0x7fffffff);
+        f[W_MX] = __hiloint2double(top, 0);
 #pragma unroll
         for (int pol = 0; pol < 2; pol++) {
             const sd *sp = seed + (size_t)(task * 2 + pol) * SEED_KINDS * L;
@@ -261,12 +265,18 @@ __global__ void __launch_bounds__(R64_NT) k_rec64(const Task *tasks, const int *
 // ---------------------------------------------------------------------------
 // elements
 // ---------------------------------------------------------------------------
-// grid (ceil(ldim / E64_X), ceil(ldim / E64_Y), nlist), E64_X threads: thread x (window index 1 ..
-// ldim, a row of 2x2 blocks) walks E64_Y columns y <= x with T and J of the columns y - 1, y, y + 1 in
+// grid (ceil(ldim / E64_X), ceil(ldim / ny), nlist), E64_X threads: thread x (window index 1 ..
+// ldim, a row of 2x2 blocks) walks ny columns y <= x with T and J of the columns y - 1, y, y + 1 in
 // registers; consecutive threads write consecutive rows of the column-major matrix.
+//
+// Bound by the FP64 pipe: 18 operations per pair.  Far from the diagonal T is so small that all four
+// elements round to zero (a third of the pairs of a free energy's matrices at R/L = 50); a warp whose pairs all
+// do, by the exponents of T and of the largest factors, stores zeros and forms nothing: 441 matrices of ldim 700
+// 5.0 ms with every element formed and 20 operations, 3.1 so; 24 of ldim 1050 0.62 and 0.34.  Where
+// the sums of squares are wanted, too, every element is formed.
 constexpr int E64_X = 64, E64_Y = 16;
 template <bool FRO>
-__global__ void __launch_bounds__(E64_X) k_elem64(const Task *tasks, const int *tlist, int nlist, int ldim, const double *__restrict__ tt,
+__global__ void __launch_bounds__(E64_X) k_elem64(const Task *tasks, const int *tlist, int nlist, int ldim, int ny, const double *__restrict__ tt,
                                                   const double *__restrict__ tab, const double *__restrict__ mdiag, const int *info,
                                                   long long *A, size_t mstride, double *fro_out, int *status)
 {
@@ -274,67 +284,118 @@ __global__ void __launch_bounds__(E64_X) k_elem64(const Task *tasks, const int *
     const int b = blockIdx.z;
     if (b >= nlist) return;
     const int task = tlist ? tlist[b] : b;
-    const int x = blockIdx.x * E64_X + threadIdx.x + 1, y0 = blockIdx.y * E64_Y + 1;
+    const int x = blockIdx.x * E64_X + threadIdx.x + 1, y0 = blockIdx.y * ny + 1;
     double fro = 0.0;
     if (y0 <= min((int)(blockIdx.x + 1) * E64_X, ldim)) { // uniform: some thread of the block has y0 <= x
         bool bad = false;
-        if (x <= ldim && y0 <= x) {
-            const Task &T = tasks[task];
-            const int mt = T.m;
-            const bool pr = T.is_pr;
-            const double *W = tab + (size_t)b * W_FIELDS * L;
-            auto F = [&](int f, int w) { return __ldg(W + (size_t)f * L + w); };
-            const double *tE = tt + (size_t)b * 2 * L * L, *tT = tE + (size_t)L * L;
-            // T(u, v) for any order of u and v
-            auto TV = [&](const double *t, int u, int v) { return u >= v ? t[(size_t)v * L + u] : t[(size_t)u * L + v]; };
-            const int fq = 60 - info[2 * task];
-            const double dA = F(W_DA, x), dB = F(W_DB, x), mA = F(W_A, x), mB = F(W_B, x);
-            const double UxA = F(W_UA, x), VxA = F(W_VA, x), UxB = F(W_UB, x), VxB = F(W_VB, x);
-            // of column v: T_TM, T_TE at x, and J'_TM = dA(x) J_TM, J'_TE = dB(x) J_TE with
-            // J(x, v) = Um(x) T(x-1, v) - Vp(x) T(x+1, v)
-            struct Col { double T, E, JT, JE; };
-            auto col = [&](int v) {
-                Col q{TV(tT, x, v), 0.0, 0.0, 0.0};
-                q.E = pr ? -q.T : TV(tE, x, v);
-                if (mt > 0) {
-                    const double a = TV(tT, x - 1, v), d = TV(tT, x + 1, v);
-                    q.JT = fma(UxA, a, VxA * d);
-                    q.JE = pr ? -fma(UxB, a, VxB * d) : fma(UxB, TV(tE, x - 1, v), VxB * TV(tE, x + 1, v));
+        const Task &T = tasks[task];
+        const int mt = T.m;
+        const bool pr = T.is_pr;
+        const double *W = tab + (size_t)b * W_FIELDS * L;
+        auto F = [&](int f, int w) { return __ldg(W + (size_t)f * L + w); };
+        const double *tE = tt + (size_t)b * 2 * L * L, *tT = tE + (size_t)L * L;
+        const int xx = min(x, ldim); // lanes past the end repeat the last row's loads
+        // T(u, v) for any order of u and v
+        auto TV = [&](const double *t, int u, int v) { return u >= v ? t[(size_t)v * L + u] : t[(size_t)u * L + v]; };
+        const int fq = 60 - info[2 * task];
+        const long long one = 1LL << fq;
+        long long *Am = A + (size_t)task * mstride + (size_t)2 * (y0 - 1) * n + 2 * (x - 1);
+        auto store = [&](int y, double ee, double mm, double em, double me) {
+            if (y != x) {
+                *reinterpret_cast<longlong2 *>(Am) = make_longlong2(-to_fix(ee, fq, bad), -to_fix(me, fq, bad));
+                *reinterpret_cast<longlong2 *>(Am + n) = make_longlong2(-to_fix(em, fq, bad), -to_fix(mm, fq, bad));
+                if (FRO) fro += 2.0 * (fma(ee, ee, me * me) + fma(mm, mm, em * em));
+            } else {
+                // the diagonal from M_ii, which the trace is taken from too
+                const double dee = mdiag[(size_t)task * n + 2 * (x - 1)], dmm = mdiag[(size_t)task * n + 2 * (x - 1) + 1];
+                *reinterpret_cast<longlong2 *>(Am) = make_longlong2(one - to_fix(dee, fq, bad), -to_fix(me, fq, bad));
+                Am[n + 1] = one - to_fix(dmm, fq, bad);
+                if (FRO) fro += fma(dee, dee, dmm * dmm) + 2.0 * me * me;
+            }
+        };
+        const int y1 = min(y0 + ny - 1, ldim); // uniform; lanes with x < y are idle
+        if (mt == 0) {
+            const double dA = F(W_DA, xx), dB = F(W_DB, xx);
+            for (int y = y0; y <= min(y1, x); y++, Am += 2 * (size_t)n) {
+                if (x > ldim) break;
+                const double t = tT[(size_t)y * L + xx], e = pr ? -t : tE[(size_t)y * L + xx];
+                store(y, dA * F(W_DA, y) * t, -(dB * F(W_DB, y) * e), 0.0, 0.0);
+            }
+        } else {
+            const double mA = F(W_A, xx), mB = F(W_B, xx);
+            const double UxA = F(W_UA, xx), VxA = F(W_VA, xx), UxB = F(W_UB, xx), VxB = F(W_VB, xx);
+            // of column v, with J(x, v) = Um(x) T(x-1, v) - Vp(x) T(x+1, v): J'_TM = dA(x) J_TM, J'_TE = dB(x) J_TE, m dB(x) T_TM and
+            // m dA(x) T_TE
+            struct Col { double JT, JE, mT, mE; };
+            struct Raw { double a, t, d, ea, e, ed; };
+            auto raw = [&](int v) {
+                Raw q{TV(tT, xx - 1, v), TV(tT, xx, v), TV(tT, xx + 1, v), 0.0, 0.0, 0.0};
+                if (!pr) {
+                    q.ea = TV(tE, xx - 1, v);
+                    q.e = TV(tE, xx, v);
+                    q.ed = TV(tE, xx + 1, v);
                 }
                 return q;
             };
-            const int y1 = min(min(y0 + E64_Y - 1, ldim), x);
-            Col cm = col(y0 - 1), c0 = col(y0);
-            long long *Am = A + (size_t)task * mstride + (size_t)2 * (y0 - 1) * n + 2 * (x - 1);
+            auto form = [&](const Raw &q) {
+                Col r;
+                r.JT = fma(UxA, q.a, VxA * q.d);
+                r.mT = mB * q.t;
+                if (pr) {
+                    r.JE = -fma(UxB, q.a, VxB * q.d);
+                    r.mE = -(mA * q.t);
+                } else {
+                    r.JE = fma(UxB, q.ea, VxB * q.ed);
+                    r.mE = mA * q.e;
+                }
+                return r;
+            };
+            // biased exponents: of the largest of a column's values (0: all zero)
+            auto ex = [](double v) { return __double2hiint(v) >> 20 & 0x7ff; };
+            auto top = [&](const Raw &q) { return max(max(max(ex(q.a), ex(q.t)), max(ex(q.d), ex(q.ea))), max(ex(q.e), ex(q.ed))); };
+            const int exr = ex(F(W_MX, xx));
+            Raw qm = raw(y0 - 1), q0 = raw(y0);
+            Col cm{}, c0{};
+            int em = top(qm), e0 = top(q0);
+            bool have = false; // cm and c0 are formed (uniform over the warp)
+            Raw next = raw(y0 + 1);
             for (int y = y0; y <= y1; y++, Am += 2 * (size_t)n) {
-                const Col cp = col(y + 1);
-                double ee, mm, em = 0.0, me = 0.0;
-                if (mt == 0) {
-                    ee = dA * F(W_DA, y) * c0.T;
-                    mm = -(dB * F(W_DB, y) * c0.E);
+                const Raw qp = next;
+                next = raw(min(y + 2, ldim + 1)); // a column ahead, for where few warps hide the loads
+                const int ep = top(qp);
+                const bool act = x <= ldim && y <= x;
+                // five products of three factors, each below 2^(sum of exponents + 3): zero below half a unit of 2^-fq
+                const bool zero = !FRO && y != x && exr + ex(F(W_MX, y)) + max(max(em, e0), ep) - 3 * 1023 + 6 + fq < -1;
+                if (__all_sync(0xffffffffu, !act || zero)) {
+                    if (act) {
+                        *reinterpret_cast<longlong2 *>(Am) = make_longlong2(0, 0);
+                        *reinterpret_cast<longlong2 *>(Am + n) = make_longlong2(0, 0);
+                    }
+                    have = false;
                 } else {
+                    if (!have) {
+                        if (y > y0) { // (rare: the values were dropped)
+                            qm = raw(y - 1);
+                            q0 = raw(y);
+                        }
+                        cm = form(qm);
+                        c0 = form(q0);
+                        have = true;
+                    }
+                    const Col cp = form(qp);
                     // EE = dA dA [B_TM - m^2 T_TE], MM = dB dB [m^2 T_TM - B_TE], B(x, y) = Um(y) J(x, y-1) - Vp(y) J(x, y+1)
+                    // EM = m dA(x) dB(y) [H_TE - J_TM], ME = m dB(x) dA(y) [J_TE - H_TM], H(x, y) = Um(y) T(x, y-1) - Vp(y) T(x, y+1)
                     const double yUA = F(W_UA, y), yVA = F(W_VA, y), yA = F(W_A, y), yUB = F(W_UB, y), yVB = F(W_VB, y), yB = F(W_B, y);
-                    ee = fma(yUA, cm.JT, fma(yVA, cp.JT, -(mA * (yA * c0.E))));
-                    mm = fma(mB, yB * c0.T, -fma(yUB, cm.JE, yVB * cp.JE));
-                    // em = m dA(x) dB(y) [H_TE - J_TM], me = m dB(x) dA(y) [J_TE - H_TM], H(x, y) = Um(y) T(x, y-1) - Vp(y) T(x, y+1)
-                    em = fma(mA, fma(yUB, cm.E, yVB * cp.E), -(yB * c0.JT));
-                    me = fma(-mB, fma(yUA, cm.T, yVA * cp.T), yA * c0.JE);
+                    const double ee = fma(yUA, cm.JT, fma(yVA, cp.JT, -(yA * c0.mE)));
+                    const double mm = fma(yB, c0.mT, -fma(yUB, cm.JE, yVB * cp.JE));
+                    const double me2 = fma(yUA, cm.mT, yVA * cp.mT);
+                    const double eem = fma(yUB, cm.mE, fma(yVB, cp.mE, -(yB * c0.JT))), mee = fma(yA, c0.JE, -me2);
+                    if (act) store(y, ee, mm, eem, mee);
+                    cm = c0;
+                    c0 = cp;
                 }
-                if (y != x) {
-                    *reinterpret_cast<longlong2 *>(Am) = make_longlong2(-to_fix(ee, fq, bad), -to_fix(me, fq, bad));
-                    *reinterpret_cast<longlong2 *>(Am + n) = make_longlong2(-to_fix(em, fq, bad), -to_fix(mm, fq, bad));
-                    if (FRO) fro += 2.0 * (fma(ee, ee, me * me) + fma(mm, mm, em * em));
-                } else {
-                    // the diagonal from M_ii, which the trace is taken from too
-                    const double dee = mdiag[(size_t)task * n + 2 * (x - 1)], dmm = mdiag[(size_t)task * n + 2 * (x - 1) + 1];
-                    const long long one = 1LL << fq;
-                    *reinterpret_cast<longlong2 *>(Am) = make_longlong2(one - to_fix(dee, fq, bad), -to_fix(me, fq, bad));
-                    Am[n + 1] = one - to_fix(dmm, fq, bad);
-                    if (FRO) fro += fma(dee, dee, dmm * dmm) + 2.0 * me * me;
-                }
-                cm = c0;
-                c0 = cp;
+                em = e0;
+                e0 = ep;
             }
         }
         if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status + task, ST_ERR_NONFINITE);
@@ -407,9 +468,13 @@ void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, co
     seed64(tasks, tlist, nlist, ldim, P, SEED_D1, SEED_COL, K, nu_stride, lft, ptab, pstride, seed, rows, status, st);
     k_sweep64_tab<<<nlist, 256, 0, st>>>(tasks, tlist, nlist, ldim, (const sd *)seed, Sa, Sb, tab, kt);
     k_rec64<<<nlist * P * 2, R64_NT, sm, st>>>(tasks, tlist, nlist, ldim, P, rows, tab, kt, tt, status, ring);
-    const dim3 g((ldim + E64_X - 1) / E64_X, (ldim + E64_Y - 1) / E64_Y, nlist);
-    if (fro) k_elem64<true><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, mdiag, info, A, mstride, fro, status);
-    else k_elem64<false><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, mdiag, info, A, mstride, fro, status);
+    // A step to the next column is a chain of loads and 18 operations, 1200 clocks: 4 columns where 16 leave SMs
+    // without a CTA (one matrix of ldim 140 24 us with 16, 9 with 4), elsewhere 4 would be one in twelve more operations
+    // (32 of ldim 350: 93 us).  The elements are the same bits, the sums of squares come in the order of E64_Y.
+    const int nx = (ldim + E64_X - 1) / E64_X, ny = !fro && (long long)nx * ((ldim + E64_Y - 1) / E64_Y) * nlist < 152 ? 4 : E64_Y;
+    const dim3 g(nx, (ldim + ny - 1) / ny, nlist);
+    if (fro) k_elem64<true><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, ny, tt, tab, mdiag, info, A, mstride, fro, status);
+    else k_elem64<false><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, ny, tt, tab, mdiag, info, A, mstride, fro, status);
     COUNT_LAUNCH(3);
     CK(cudaGetLastError());
 }

@@ -53,3 +53,22 @@ def test_ring_in_global_memory():
     c.set_path(cg.PATH_HODLR)
     hodlr = c.logdetD(300.0, 1)
     assert abs(dense - hodlr) <= 1e-10 * max(1.0, abs(hodlr)), (dense, hodlr)
+
+
+@pytest.mark.parametrize("ldim", [16, 17, 64, 65, 130, 260])
+@pytest.mark.parametrize("metal", METALS)
+def test_elements_that_round_to_zero(ldim, metal):
+    """HODLR rules skip elements that round to zero, the dense rules (which need |M|) form every one: the
+    same fixed-point matrix, so the same bits wherever both factor it"""
+    import caps_gb300 as cg
+    xi = np.array([0.2, 2.0, 9.0, 25.0]) * 10
+    m = np.array([1, 0, 4, 2])
+    out = []
+    for alg in (cg.DETALG_LU, cg.DETALG_HODLR):
+        c = cg.Caps(40e-6, 1e-6, ldim=ldim, detalg=alg)
+        if metal:
+            c.set_drude(*metal)
+        out.append(c.logdetD_batch(xi, m))
+    both = (out[0][1] == 3) & (out[1][1] == 3)
+    assert both.sum() >= 2
+    assert (out[0][0][both] == out[1][0][both]).all()
