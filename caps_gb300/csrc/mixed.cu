@@ -301,7 +301,7 @@ constexpr int MT = 64, TRSM_THREADS = 128;
 // to S (with the images, nothing reads it there again: later steps read S only in their own
 // columns, the final sums only its diagonal).
 __global__ void __launch_bounds__(TRSM_THREADS) k_trsm_inv(int ntask, int n, int k0, float *S, size_t sstride, int *status,
-                                                  const float *Winv, double *fro, __half *img64, int blk64, bool store_x)
+                                                  const float *Winv, double *fro, __half *img64, int blk64, bool store_x, unsigned char *nz)
 {
     const int task = blockIdx.y;
     if (task >= ntask || status[task] != ST_FACTOR) return;
@@ -314,14 +314,40 @@ __global__ void __launch_bounds__(TRSM_THREADS) k_trsm_inv(int ntask, int n, int
     const float *Wt = Winv + (size_t)task * MB * MB;
     const int rows = min(MT, n - r0);
     constexpr int NT = TRSM_THREADS;
+    const int nrb64 = pipe_img64_nrb(n);
+    if (img64) {
+        img64 += (((size_t)blk64 * ntask + task) * 2 * nrb64 + blockIdx.x) * PIPE_IMG64_HALVES; // this block's hi part
+        nz += ((size_t)blk64 * ntask + task) * nrb64 + blockIdx.x;
+    }
+    const size_t fslot = (size_t)task * fro_slots(n) + (size_t)(k0 / MB) * (fro_nbr(n) + 1) + 1 + blockIdx.x;
     {
         float w[MB * MB / NT], x[MT * MB / NT];
-#pragma unroll
-        for (int u = 0; u < MB * MB / NT; u++) w[u] = __ldg(Wt + threadIdx.x + NT * u);
+        bool any = false;
 #pragma unroll
         for (int u = 0; u < MT * MB / NT; u++) {
             const int e = threadIdx.x + NT * u, c = e / MT, r = e % MT;
             x[u] = (r < rows && c < nb) ? __ldg(Sm + (size_t)(k0 + c) * n + r0 + r) : 0.0f;
+            any |= !(fabsf(x[u]) < 0x1p-52f);
+        }
+        // entries of S below 2^-52: with |W| < 2 every |X| is below 2^-45, so the image is zero (2^-39), and the squares,
+        // below 2^-89 in all, stay under the last place of a log det of 1e-8, the smallest that is factored
+        any = !img64 || __syncthreads_or(any);
+#pragma unroll
+        for (int u = 0; u < MB * MB / NT; u++) w[u] = __ldg(Wt + threadIdx.x + NT * u);
+        if (!any) {
+#pragma unroll
+            for (int u = 0; u < MB * MB / NT; u++) any |= !(fabsf(w[u]) < 2.0f);
+            if (!__syncthreads_or(any)) {
+                for (int e = threadIdx.x; e < PIPE_IMG64_HALVES / 8; e += NT) {
+                    reinterpret_cast<uint4 *>(img64)[e] = make_uint4(0, 0, 0, 0);
+                    reinterpret_cast<uint4 *>(img64 + (size_t)nrb64 * PIPE_IMG64_HALVES)[e] = make_uint4(0, 0, 0, 0);
+                }
+                if (threadIdx.x == 0) {
+                    *nz = 0;
+                    fro[fslot] = 0.0;
+                }
+                return;
+            }
         }
 #pragma unroll
         for (int u = 0; u < MB * MB / NT; u++) {
@@ -366,6 +392,7 @@ __global__ void __launch_bounds__(TRSM_THREADS) k_trsm_inv(int ntask, int n, int
     }
     SqSum q;
     bool big = false;
+    uint32_t bits = 0;
     // the outputs of column group cg (columns 4 cg .. 4 cg + 3) from its accumulators
     auto emit = [&](const float(&acc)[4][4], int cg) {
 #pragma unroll
@@ -386,8 +413,6 @@ __global__ void __launch_bounds__(TRSM_THREADS) k_trsm_inv(int ntask, int n, int
             // columns 4 cg .. 4 cg + 3 are half of one 16-byte row of a core matrix (the groups
             // 2 w, 2 w + 1 or 14 - 2 w, 15 - 2 w of warp w fill it, its 16 rows two whole core
             // matrices)
-            const int nrb64 = pipe_img64_nrb(n);
-            __half *hi = img64 + (((size_t)blk64 * ntask + task) * 2 * nrb64 + blockIdx.x) * PIPE_IMG64_HALVES;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int r = rg + 16 * i;
@@ -397,10 +422,11 @@ __global__ void __launch_bounds__(TRSM_THREADS) k_trsm_inv(int ntask, int n, int
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         img_split16(acc[i][j], h[j], l[j]);
+                        bits |= h[j] | l[j];
                         big |= !(fabsf(acc[i][j]) < PIPE_IMG_XMAX);
                     }
-                    *reinterpret_cast<uint2 *>(hi + e) = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
-                    *reinterpret_cast<uint2 *>(hi + (size_t)nrb64 * PIPE_IMG64_HALVES + e) =
+                    *reinterpret_cast<uint2 *>(img64 + e) = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+                    *reinterpret_cast<uint2 *>(img64 + (size_t)nrb64 * PIPE_IMG64_HALVES + e) =
                         make_uint2(l[0] | l[1] << 16, l[2] | l[3] << 16);
                 }
             }
@@ -411,7 +437,11 @@ __global__ void __launch_bounds__(TRSM_THREADS) k_trsm_inv(int ntask, int n, int
     if (big) atomicOr(status + task, ST_ERR_RANGE);
     __shared__ double red4[NT / 32];
     const double sq = block_sq<NT / 32>(q, red4);
-    if (threadIdx.x == 0) fro[(size_t)task * fro_slots(n) + (size_t)(k0 / MB) * (fro_nbr(n) + 1) + 1 + blockIdx.x] = sq;
+    const bool some = __syncthreads_or((bits & 0x7fff) != 0);
+    if (threadIdx.x == 0) {
+        fro[fslot] = sq;
+        if (img64) *nz = some;
+    }
 }
 
 // trailing update S_ab -= sum_k Lam_ak Lam_bk over the panel, 64x64 tiles of the
@@ -617,10 +647,15 @@ struct KernelTimer {
 };
 KernelTimer g_kts[KT_KINDS];
 KernelTimer &g_kt = g_kts[KT_SYRK];
+unsigned long long *g_kt_moved = nullptr; // device counter of the image-fed updates' bytes
 } // namespace
 
 void kernel_timer_enable(bool on)
 {
+    if (on) {
+        if (!g_kt_moved) CK(cudaMalloc(&g_kt_moved, sizeof *g_kt_moved));
+        CK(cudaMemset(g_kt_moved, 0, sizeof *g_kt_moved));
+    }
     for (KernelTimer &k : g_kts) {
         k.on = on;
         k.used = 0;
@@ -644,6 +679,12 @@ void kernel_timer_collect(long long nfactored)
         k.used = 0;
         k.per_matrix_bytes.clear();
     }
+    if (g_kt.on) {
+        unsigned long long moved;
+        CK(cudaMemcpy(&moved, g_kt_moved, sizeof moved, cudaMemcpyDeviceToHost));
+        CK(cudaMemset(g_kt_moved, 0, sizeof moved));
+        g_kt.bytes += (double)moved;
+    }
 }
 
 void kernel_timer_stats(int kind, double *ms, double *bytes, long long *launches)
@@ -660,9 +701,13 @@ static size_t mixed_img_offset(int ntask, int n)
 {
     return ((size_t)ntask * (MB * MB * sizeof(float) + fro_slots(n) * sizeof(double)) + 255) / 256 * 256;
 }
+// then (256-byte aligned) the flags of the image blocks and the lists of the updates' CTAs (upd_fill)
+constexpr int MIXED_MAX_SMS = 1024; // an update's CTAs: at most one per SM
+static size_t mixed_nz_offset(int ntask, int n) { return mixed_img_offset(ntask, n) + (size_t)ntask * pipe_img64_bytes(n); }
+static size_t mixed_nz_bytes(int ntask, int n) { return ((size_t)PIPE_IMG64_BLOCKS * ntask * pipe_img64_nrb(n) + 255) / 256 * 256; }
 size_t mixed_work_bytes(int ntask, int n)
 {
-    return mixed_img_offset(ntask, n) + (size_t)ntask * pipe_img64_bytes(n);
+    return mixed_nz_offset(ntask, n) + mixed_nz_bytes(ntask, n) + upd_list_entries(ntask, n, MIXED_MAX_SMS) * sizeof(int2);
 }
 
 void launch_cholesky_mixed(int ntask, int n, const double *A, size_t lda, size_t mstride, int *status, float *S, size_t sstride,
@@ -674,7 +719,10 @@ void launch_cholesky_mixed(int ntask, int n, const double *A, size_t lda, size_t
     float *Winv = (float *)work;
     double *part = (double *)((char *)work + (size_t)ntask * MB * MB * sizeof(float));
     __half *img64 = (__half *)((char *)work + mixed_img_offset(ntask, n));
+    unsigned char *nz = (unsigned char *)work + mixed_nz_offset(ntask, n);
+    int2 *list = (int2 *)(nz + mixed_nz_bytes(ntask, n));
     CK(cudaMemsetAsync(part, 0, (size_t)ntask * fro_slots(n) * sizeof(double), st));
+    CK(cudaMemsetAsync(nz, 0, mixed_nz_bytes(ntask, n), st));
     // convert: A is the FP64 matrix 1 - M and S receives its delta form here; otherwise S
     // already holds it.  mdiag: M_ii in FP64, n per task (tr(A - I) = -tr M).
     // Trailing update: tcgen05 (k_syrk_umma); CAPS_MIXED_MMASYNC=1 selects the mma.sync
@@ -703,6 +751,7 @@ void launch_cholesky_mixed(int ntask, int n, const double *A, size_t lda, size_t
         int dev = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        nsm = std::min(nsm, MIXED_MAX_SMS);
         attr = true;
     }
     // update of S[t0.., t0..cmax) by the panel columns k0 .. k0 + kw - 1: the persistent
@@ -710,17 +759,19 @@ void launch_cholesky_mixed(int ntask, int n, const double *A, size_t lda, size_t
     // UPD_BLOCK the 64 columns t0 .. t0 + 64 (left-looking, inside a half panel), UPD_MID the
     // 256 columns t0 .. t0 + 256 (the first half of a panel onto the second half), UPD_TRAIL
     // the whole trailing matrix
-    enum { UPD_BLOCK, UPD_MID, UPD_TRAIL };
     auto syrk = [&](int k0, int kw, int t0, int cmax, int kind) {
         const int nr = (n - t0 + UM_M - 1) / UM_M;
+        const bool counted = use_img && (kind != UPD_TRAIL || kw == PIPE_IMG_CH * PIPE_IMG_TK);
+        unsigned long long *moved = g_kt.on ? g_kt_moved : nullptr;
         if (g_kt.on) CK(cudaEventRecord(g_kt.next(), st));
         if (no_pipe)
             k_syrk_umma<<<dim3(kind == UPD_BLOCK ? nr : nr * (nr + 1), ntask), UM_THREADS, UM_SMEM, st>>>(
                 ntask, n, k0, kw, t0, cmax, kind == UPD_BLOCK, S, sstride, status);
         else if (kind == UPD_BLOCK && use_img) // from the FP16 images of the half panel's earlier blocks
-            k_syrk_blk<<<std::min(ntask * nr, nsm), BLK_THREADS, BLK_SMEM, st>>>(ntask, n, k0, t0, S, sstride, status, img64);
+            k_syrk_blk<<<std::min(ntask * nr, nsm), BLK_THREADS, BLK_SMEM, st>>>(ntask, n, k0, t0, S, sstride, status, img64, nz, list, moved);
         else if (kind != UPD_TRAIL && use_img) // UPD_MID: row blocks against the two column blocks
-            k_syrk_pair<<<std::min(ntask * nr, nsm), PAIR_THREADS, PAIR_SMEM, st>>>(ntask, n, t0, kw, 1, S, sstride, status, img64);
+            k_syrk_pair<<<std::min(ntask * nr, nsm), PAIR_THREADS, PAIR_SMEM, st>>>(ntask, n, t0, kw, 1, S, sstride, status, img64, nz,
+                                                                                      list, moved);
         else if (kind != UPD_TRAIL) { // the same from S: 128 x 64 tiles, 64-column chunks
             const int ncb = (cmax - t0 + 63) / 64;
             k_syrk_pipe<64, 64><<<std::min(ntask * nr * ncb, nsm), PIPE_THREADS, PIPE_SMEM, st>>>(ntask, n, k0, kw, t0, cmax, ncb, S,
@@ -729,7 +780,7 @@ void launch_cholesky_mixed(int ntask, int n, const double *A, size_t lda, size_t
             const int tw = ntask * pipe_tiles<128>(nr, 0);
             if (use_img && kw == PIPE_IMG_CH * PIPE_IMG_TK) // the panel solves left the panel's images: row-pair items
                 k_syrk_pair<<<std::min(ntask * pair_items(nr), nsm), PAIR_THREADS, PAIR_SMEM, st>>>(ntask, n, t0, kw, 0, S, sstride,
-                                                                                                  status, img64);
+                                                                                                  status, img64, nz, list, moved);
             else
                 k_syrk_pipe<128, 32><<<std::min(tw, nsm), PIPE_THREADS, PIPE_SMEM_WIDE, st>>>(ntask, n, k0, kw, t0, cmax, 0, S,
                                                                                               sstride, status);
@@ -737,9 +788,10 @@ void launch_cholesky_mixed(int ntask, int n, const double *A, size_t lda, size_t
         COUNT_LAUNCH(1);
         if (g_kt.on) {
             CK(cudaEventRecord(g_kt.next(), st));
-            // lower part of the target block read and written in FP32, panel rows read once
+            // lower part of the target block read and written in FP32, panel rows read once; the image-fed updates
+            // count what they do themselves
             const double r = n - t0, w = std::min(cmax, n) - t0;
-            g_kt.per_matrix_bytes.push_back(8.0 * (w * r - w * (w - 1) / 2) + 4.0 * r * kw);
+            g_kt.per_matrix_bytes.push_back(counted ? 0.0 : 8.0 * (w * r - w * (w - 1) / 2) + 4.0 * r * kw);
         }
     };
     if (convert) {
@@ -766,7 +818,7 @@ void launch_cholesky_mixed(int ntask, int n, const double *A, size_t lda, size_t
         dim3 gt((rest + MT - 1) / MT, ntask);
         if (tt.on) CK(cudaEventRecord(tt.next(), st));
         k_trsm_inv<<<gt, TRSM_THREADS, 0, st>>>(ntask, n, k0, S, sstride, status, Winv, part, images ? img64 : nullptr, blk,
-                                                !images);
+                                                !images, nz);
         COUNT_LAUNCH(1);
         if (tt.on) { // the panel's rows below read; written: X (without images) or the FP16 image
             CK(cudaEventRecord(tt.next(), st));

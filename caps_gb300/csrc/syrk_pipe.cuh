@@ -343,14 +343,13 @@ constexpr int PAIR_SMEM = PAIR_STAGES * PAIR_STAGE;                     // 192 K
 
 struct PairTile {
     int task, ra, rb, col0; // rb < 0: one tile
-    bool valid;
 };
 __host__ __device__ inline int pair_items(int nr)
 {
     const int np = nr / 2;
     return np * (np + 1) + ((nr & 1) ? nr : 0);
 }
-__device__ __forceinline__ PairTile pair_tile(int t, int ipt, int nr, int t0, const int *status)
+__device__ __forceinline__ PairTile pair_tile(int t, int ipt, int nr, int t0)
 {
     PairTile T;
     T.task = t / ipt;
@@ -370,21 +369,77 @@ __device__ __forceinline__ PairTile pair_tile(int t, int ipt, int nr, int t0, co
     T.ra = t0 + ra * UM_M;
     T.rb = rb >= 0 ? t0 + rb * UM_M : -1;
     T.col0 = t0 + cj * UM_M;
-    // skip matrices that are not being factored or failed before this launch
-    T.valid = (status[T.task] & ~ST_ERR_WAIT) == ST_FACTOR;
     return T;
 }
 // the middle update's items: item t is row block t mod nr of matrix t / nr against the two
 // column blocks t0 .. t0 + 256 (ra = rb = the rows; rb < 0 when the second block lies past n)
-__device__ __forceinline__ PairTile mid_tile(int t, int nr, int n, int t0, const int *status)
+__device__ __forceinline__ PairTile mid_tile(int t, int nr, int n, int t0)
 {
     PairTile T;
     T.task = t / nr;
     T.ra = t0 + (t - T.task * nr) * UM_M;
     T.rb = t0 + UM_M < n ? T.ra : -1;
     T.col0 = t0;
-    T.valid = (status[T.task] & ~ST_ERR_WAIT) == ST_FACTOR;
     return T;
+}
+
+// ---- what an update has to do ----
+// Entries of the factor fall off so fast away from the diagonal that most 64 x 64 image blocks are exactly zero
+// (below 2^-39, the images' resolution): at R/L = 150 5 % of the trailing update's chunks have two slices that
+// are not, in 12 to 15 % of its items.  The panel solves note which blocks are not zero, nz[((b ntask) + task)
+// pipe_img64_nrb(n) + rb]; a CTA of a persistent update first lists its items (item t to CTA t mod gridDim) that
+// have a chunk to do, with all its threads, and then walks the list.  A chunk left out would have added zeros.
+// (A list for all CTAs by a launch of its own took 4.7 us per update, a third of the updates of six matrices of
+// dimension 6000.)
+enum { UPD_TRAIL, UPD_MID, UPD_BLOCK }; // k_syrk_pair over the trailing matrix, over 256 columns; k_syrk_blk
+__host__ __device__ inline int upd_items(int kind, int nr) { return kind == UPD_TRAIL ? pair_items(nr) : nr; }
+// entries of the lists of all CTAs of one update
+__host__ __device__ inline size_t upd_list_entries(int ntask, int n, int ncta)
+{
+    const int nr = (n + UM_M - 1) / UM_M, p = pair_items(nr);
+    return (size_t)ntask * (p > nr ? p : nr) + 2 * ncta;
+}
+// k0: first column of the panel's part that is applied, t0: first column (and row) updated.  seg[i] = (item, bits of
+// its chunks); *count (zeroed before a barrier) of them in any order, complete after the next barrier.  bytes != nullptr:
+// the bytes of the listed work are added (S read and written, image slices read once per chunk)
+__device__ __forceinline__ void upd_fill(int kind, int ntask, int n, int k0, int t0, const int *status, const unsigned char *nz, int2 *seg, int *count,
+                                         unsigned long long *bytes)
+{
+    const int nr = (n - t0 + UM_M - 1) / UM_M, ipt = upd_items(kind, nr), nrb64 = pipe_img64_nrb(n);
+    const int nch = (t0 - k0) / PIPE_IMG_TK, nitem = ntask * ipt;
+    for (int t = blockIdx.x + threadIdx.x * gridDim.x; t < nitem; t += blockDim.x * gridDim.x) {
+        const int task = t / ipt;
+        // skip matrices that are not being factored or failed before this launch
+        if ((status[task] & ~ST_ERR_WAIT) != ST_FACTOR) continue;
+        const PairTile T = kind == UPD_TRAIL ? pair_tile(t, ipt, nr, t0) : mid_tile(t, nr, n, t0);
+        int mask = 0;
+#pragma unroll 1
+        for (int ch = 0; ch < nch; ch++) {
+            // rows of chunk ch are counted from t1
+            const int blk = (k0 % (PIPE_IMG_CH * PIPE_IMG_TK)) / PIPE_IMG_TK + ch, t1 = k0 + PIPE_IMG_TK * (ch + 1);
+            const unsigned char *f = nz + ((size_t)blk * ntask + task) * nrb64;
+            auto rows = [&](int row0) { return f[(row0 - t1) / 64] | f[(row0 - t1) / 64 + 1]; };
+            int a = rows(T.ra), b = kind == UPD_BLOCK ? f[(t0 - t1) / 64] : rows(T.col0);
+            if (T.rb >= 0) {
+                if (kind == UPD_TRAIL) a |= rows(T.rb);
+                if (kind == UPD_MID) b |= rows(t0 + UM_M);
+            }
+            mask |= (a && b ? 1 : 0) << ch;
+        }
+        if (!mask) continue;
+        seg[atomicAdd(count, 1)] = make_int2(t, mask);
+        if (bytes) {
+            const int tiles = kind == UPD_BLOCK ? 1 : 2 * (T.rb >= 0 ? 2 : 1); // of 128 x 64
+            const int slices = kind == UPD_BLOCK ? 3 : 2 * (T.rb >= 0 ? 3 : 2); // of 64 rows
+            atomicAdd(bytes, tiles * UM_M * 64 * 8ULL + __popc(mask) * slices * 64 * 64 * 4ULL);
+        }
+    }
+}
+// this CTA's part of the lists
+__device__ __forceinline__ int2 *upd_seg(int2 *list, int ntask, int kind, int n, int t0)
+{
+    const int nitem = ntask * upd_items(kind, (n - t0 + UM_M - 1) / UM_M);
+    return list + (size_t)blockIdx.x * ((nitem + gridDim.x - 1) / gridDim.x);
 }
 
 // mid = 0: S[t0.., t0..) -= P P^T over the kw panel columns t0 - kw .. t0 (the start of a panel,
@@ -394,7 +449,8 @@ __device__ __forceinline__ PairTile mid_tile(int t, int nr, int n, int t0, const
 // the stage holds the two column slices and the row slice, and the MMAs take the row slice
 // as A.  Grid = min(items, SMs), PAIR_THREADS threads, PAIR_SMEM bytes of dynamic shared memory.
 __global__ void __launch_bounds__(PAIR_THREADS, 1) k_syrk_pair(int ntask, int n, int t0, int kw, int mid, float *S, size_t sstride,
-                                                               int *status, const __half *img)
+                                                               int *status, const __half *img, const unsigned char *nz, int2 *lists,
+                                                             unsigned long long *bytes)
 {
     constexpr int PA = PAIR_SLICE;
     const int nch = kw / PIPE_IMG_TK;
@@ -404,11 +460,14 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) k_syrk_pair(int ntask, int n,
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nr = (n - t0 + UM_M - 1) / UM_M;
     const int ipt = mid ? nr : pair_items(nr);
-    const int nitem = ntask * ipt;
-    auto item = [&](int t) { return mid ? mid_tile(t, nr, n, t0, status) : pair_tile(t, ipt, nr, t0, status); };
+    const int kind = mid ? UPD_MID : UPD_TRAIL;
+    int2 *list = upd_seg(lists, ntask, kind, n, t0);
+    auto item = [&](int t) { return mid ? mid_tile(t, nr, n, t0) : pair_tile(t, ipt, nr, t0); };
 
+    __shared__ int s_count;
     if (warp == 0) umma::alloc(&tslot, 512);
     if (tid == 0) {
+        s_count = 0;
         for (int i = 0; i < PAIR_STAGES; i++) {
             umma::mbar_init(&full[i], 1);
             umma::mbar_init(&empty[i], 1);
@@ -419,10 +478,13 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) k_syrk_pair(int ntask, int n,
         }
         umma::mbar_init(&drain, 1);
     }
+    __syncthreads();
+    upd_fill(kind, ntask, n, t0 - kw, t0, status, nz, list, &s_count, bytes);
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
     const uint32_t tmem = tslot;
+    const int nitem = s_count;
     const int nrb64 = pipe_img64_nrb(n);
     auto slice = [&](int task, int rblock, int ch) { // hi slice of row block rblock, chunk ch (the lo slice is nrb64 blocks on)
         return img + (((size_t)ch * ntask + task) * 2 * nrb64 + nch - 1 - ch + 2 * rblock) * PIPE_IMG64_HALVES;
@@ -432,9 +494,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) k_syrk_pair(int ntask, int n,
         // ---- epilogue ----
         const int quad = warp & 3, part4 = (warp - 2) >> 2; // four warps per lane quadrant, 32 columns each
         int tt = 0;
-        for (int t = blockIdx.x; t < nitem; t += gridDim.x) {
-            const PairTile T = item(t);
-            if (!T.valid) continue;
+        for (int t = 0; t < nitem; t++) {
+            const PairTile T = item(list[t].x);
             float *Sm = S + (size_t)T.task * sstride;
             const int b = tt & 1, ub = tt >> 1;
             // parts p = 2 h + half: tile h (rows ra, then rb; in the middle update the column
@@ -481,15 +542,16 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) k_syrk_pair(int ntask, int n,
             int it = 0, last[PAIR_STAGES];
             for (int s = 0; s < PAIR_STAGES; s++) last[s] = -1;
             bool ok = true;
-            for (int t = blockIdx.x; ok && t < nitem; t += gridDim.x) {
-                const PairTile T = item(t);
-                if (!T.valid) continue;
+            for (int t = 0; ok && t < nitem; t++) {
+                const int2 e = list[t];
+                const PairTile T = item(e.x);
                 // image row blocks of the three slices: A0, A1 (the item's rows) and B (its
                 // columns); in the middle update the two column blocks and then the rows
                 const int br = (T.ra - t0) / UM_M;
                 const int s0 = mid ? 0 : br, s1 = mid ? 1 : (T.rb - t0) / UM_M, s2 = mid ? br : (T.col0 - t0) / UM_M;
                 const bool two = T.rb >= 0;
-                for (int ch = 0; ch < nch; ch++, it++) {
+                for (int left = e.y; left; left &= left - 1, it++) {
+                    const int ch = __ffs(left) - 1;
                     const int s = it % PAIR_STAGES, use = it / PAIR_STAGES;
                     if (use > 0 && !umma::mbar_wait(&empty[s], (use - 1) & 1, PIPE_WAIT_ITERS)) {
                         ok = false;
@@ -523,13 +585,14 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) k_syrk_pair(int ntask, int n,
             int it = 0, tt = 0;
             constexpr uint32_t idesc = umma::idesc_f16(UM_M, UM_M);
             constexpr uint32_t LBO = 128, SBO = (PIPE_IMG_TK / 8) * 128;
-            for (int t = blockIdx.x; t < nitem; t += gridDim.x) {
-                const PairTile T = item(t);
-                if (!T.valid) continue;
+            for (int t = 0; t < nitem; t++) {
+                const int2 e = list[t];
+                const PairTile T = item(e.x);
                 const int b = tt & 1, ub = tt >> 1, nh = T.rb >= 0 ? 2 : 1;
                 bool ok = ub == 0 || umma::mbar_wait(&tempty[b], (ub - 1) & 1, PIPE_WAIT_ITERS);
                 umma::fence_after();
-                for (int ch = 0; ok && ch < nch; ch++, it++) {
+                for (int left = e.y; left; left &= left - 1, it++) {
+                    if (!ok) break;
                     const int s = it % PAIR_STAGES, use = it / PAIR_STAGES;
                     if (!umma::mbar_wait(&full[s], use & 1, PIPE_WAIT_ITERS)) { ok = false; break; }
                     umma::fence_after();
@@ -543,7 +606,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1) k_syrk_pair(int ntask, int n,
                         for (int ks = 0; ks < PIPE_IMG_TK / 16; ks++) { // K = 16 halves: two core matrices
                             const uint32_t o = ks * 256;
                             umma::mma_f16(acc, umma::desc_kmajor(al + o, LBO, SBO), umma::desc_kmajor(bh + o, LBO, SBO), idesc,
-                                          ch > 0 || ks > 0);
+                                          left != e.y || ks > 0);
                             umma::mma_f16(acc, umma::desc_kmajor(ah + o, LBO, SBO), umma::desc_kmajor(bl + o, LBO, SBO), idesc, 1);
                             umma::mma_f16(acc, umma::desc_kmajor(ah + o, LBO, SBO), umma::desc_kmajor(bh + o, LBO, SBO), idesc, 1);
                         }
@@ -583,7 +646,8 @@ constexpr int BLK_A = UM_M * 64 * 2, BLK_B = 64 * 64 * 2;                 // byt
 constexpr int BLK_STAGE = 2 * (BLK_A + BLK_B);                            // 48 KB
 constexpr int BLK_SMEM = BLK_STAGES * BLK_STAGE;                          // 192 KB
 __global__ void __launch_bounds__(BLK_THREADS, 1) k_syrk_blk(int ntask, int n, int k0, int t0, float *S, size_t sstride, int *status,
-                                                             const __half *img)
+                                                             const __half *img, const unsigned char *nz, int2 *lists,
+                                                             unsigned long long *bytes)
 {
     extern __shared__ __align__(1024) unsigned char blk_sm[];
     __shared__ uint64_t full[BLK_STAGES], empty[BLK_STAGES], tfull[BLK_ACC], tempty[BLK_ACC], drain;
@@ -591,12 +655,13 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) k_syrk_blk(int ntask, int n, i
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cend = min(n, t0 + 64);
     const int nr = (n - t0 + UM_M - 1) / UM_M; // row blocks: tile t -> (task t / nr, row block t mod nr)
-    const int ntile = ntask * nr;
-    const int nchunk = (t0 - k0) / 64;
+    int2 *list = upd_seg(lists, ntask, UPD_BLOCK, n, t0);
     const int nrb64 = pipe_img64_nrb(n);
 
+    __shared__ int s_count;
     if (warp == 0) umma::alloc(&tslot, BLK_ACC * 64);
     if (tid == 0) {
+        s_count = 0;
         for (int i = 0; i < BLK_STAGES; i++) {
             umma::mbar_init(&full[i], 1);
             umma::mbar_init(&empty[i], 1);
@@ -607,12 +672,13 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) k_syrk_blk(int ntask, int n, i
         }
         umma::mbar_init(&drain, 1);
     }
+    __syncthreads();
+    upd_fill(UPD_BLOCK, ntask, n, k0, t0, status, nz, list, &s_count, bytes);
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
     const uint32_t tmem = tslot;
-    // skip matrices that are not being factored or failed before this launch
-    auto valid = [&](int task) { return (status[task] & ~ST_ERR_WAIT) == ST_FACTOR; };
+    const int ntile = s_count;
 
     if (warp >= 2) {
         // ---- epilogue ----
@@ -627,20 +693,15 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) k_syrk_blk(int ntask, int n, i
 #pragma unroll
             for (int j = 0; j < 16; j++) d[j] = j < jm ? src[j * n] : 0.0f;
         };
-        auto next = [&](int t) {
-            while (t < ntile && !valid(t / nr)) t += gridDim.x;
-            return t;
-        };
         int tt = 0;
         float cn[16];
-        int t = next(blockIdx.x);
-        if (t < ntile) load(t, cn);
-        while (t < ntile) {
+        if (ntile > 0) load(list[0].x, cn);
+        for (int i = 0; i < ntile; i++) {
+            const int t = list[i].x;
             float c[16];
 #pragma unroll
             for (int j = 0; j < 16; j++) c[j] = cn[j];
-            const int tn = next(t + gridDim.x);
-            if (tn < ntile) load(tn, cn);
+            if (i + 1 < ntile) load(list[i + 1].x, cn);
             const int task = t / nr, R = t0 + (t - task * nr) * UM_M + quad * 32 + lane, jm = lim(R);
             float *dst = S + (size_t)task * sstride + (size_t)cb * n + R;
             const int b = tt % BLK_ACC, ub = tt / BLK_ACC;
@@ -657,7 +718,6 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) k_syrk_blk(int ntask, int n, i
             umma::fence_before();
             mbar_arrive(&tempty[b]);
             tt++;
-            t = tn;
         }
     } else if (warp == 0) {
         // ---- producer: bulk copies of the images (one thread) ----
@@ -665,10 +725,11 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) k_syrk_blk(int ntask, int n, i
             int it = 0, last[BLK_STAGES];
             for (int s = 0; s < BLK_STAGES; s++) last[s] = -1;
             bool ok = true;
-            for (int t = blockIdx.x; ok && t < ntile; t += gridDim.x) {
-                const int task = t / nr, row0 = t0 + (t - task * nr) * UM_M;
-                if (!valid(task)) continue;
-                for (int ch = 0; ch < nchunk; ch++, it++) {
+            for (int i = 0; ok && i < ntile; i++) {
+                const int2 e = list[i];
+                const int task = e.x / nr, row0 = t0 + (e.x - task * nr) * UM_M;
+                for (int left = e.y; left; left &= left - 1, it++) {
+                    const int ch = __ffs(left) - 1;
                     // chunk ch is the image of block k0 / 64 + ch of the panel, its rows counted
                     // from k0 + 64 (ch + 1)
                     const int t1 = k0 + 64 * (ch + 1), blk = (k0 % (PIPE_IMG_CH * PIPE_IMG_TK)) / 64 + ch;
@@ -701,14 +762,15 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) k_syrk_blk(int ntask, int n, i
             int it = 0, tt = 0;
             constexpr uint32_t idesc = umma::idesc_f16(UM_M, 64);
             constexpr uint32_t LBO = 128, SBO = 8 * 128;
-            for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-                const int task = t / nr;
-                if (!valid(task)) continue;
+            for (int i = 0; i < ntile; i++) {
+                const int2 e = list[i];
+                const int task = e.x / nr;
                 const int b = tt % BLK_ACC, ub = tt / BLK_ACC;
                 bool ok = ub == 0 || umma::mbar_wait(&tempty[b], (ub - 1) & 1, PIPE_WAIT_ITERS);
                 umma::fence_after();
                 const uint32_t acc = tmem + b * 64;
-                for (int ch = 0; ok && ch < nchunk; ch++, it++) {
+                for (int left = e.y; left; left &= left - 1, it++) {
+                    if (!ok) break;
                     const int s = it % BLK_STAGES, use = it / BLK_STAGES;
                     if (!umma::mbar_wait(&full[s], use & 1, PIPE_WAIT_ITERS)) { ok = false; break; }
                     umma::fence_after();
@@ -716,7 +778,7 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) k_syrk_blk(int ntask, int n, i
                     for (int ks = 0; ks < 4; ks++) { // K = 16 halves: two core matrices
                         const uint32_t o = ks * 256;
                         umma::mma_f16(acc, umma::desc_kmajor(al + o, LBO, SBO), umma::desc_kmajor(bh + o, LBO, SBO), idesc,
-                                      ch > 0 || ks > 0);
+                                      left != e.y || ks > 0);
                         umma::mma_f16(acc, umma::desc_kmajor(ah + o, LBO, SBO), umma::desc_kmajor(bl + o, LBO, SBO), idesc, 1);
                         umma::mma_f16(acc, umma::desc_kmajor(ah + o, LBO, SBO), umma::desc_kmajor(bh + o, LBO, SBO), idesc, 1);
                     }
