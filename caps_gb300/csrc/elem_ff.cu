@@ -224,22 +224,23 @@ __global__ void __launch_bounds__(EB) k_diag_ff(const Task *tasks, int ntask, in
 // Mercator when its error bound is below 1e-8 relative; otherwise factorise.  Without
 // partials (part == nullptr) only the trace rule is applied: a matrix it does not decide
 // keeps status 0, to be assembled in full.
-__global__ void k_stats_ff(const int *tlist, int nlist, int ldim, const double *diag, const float *part, int nbx, int mode,
+__global__ void k_stats_ff(const int *tlist, int nlist, int ldim, const double *diag, const float *part, int nsum, int mode,
                            double *trace_out, double *result, int *status)
 {
     if ((int)blockIdx.x >= nlist) return;
     const int task = tlist ? tlist[blockIdx.x] : (int)blockIdx.x;
-    const int n = 2 * ldim, per_b = nbx * (EB / 32);
+    const int n = 2 * ldim, per_b = (ldim + EB - 1) / EB * (EB / 32);
     __shared__ double red[256];
-    if (part && nbx == 0) { // one sum per task (k_sweep_ff)
-        if (threadIdx.x == 0) red[0] = (double)part[task];
-        __syncthreads();
-    } else if (part) {
-        const float *p = part + (size_t)task * ldim * per_b;
+    if (part && mode == 0) { // only the dense rules read |M|
         double s = 0.0;
-        for (int i = threadIdx.x; i < ldim * per_b; i += blockDim.x) {
-            const int b = i / per_b, x = (i % per_b) / (EB / 32);
-            if (x >= b / EB) s += p[i];
+        if (nsum > 0)
+            for (int i = threadIdx.x; i < nsum; i += blockDim.x) s += part[(size_t)task * nsum + i];
+        else {
+            const float *p = part + (size_t)task * ldim * per_b;
+            for (int i = threadIdx.x; i < ldim * per_b; i += blockDim.x) {
+                const int b = i / per_b, x = (i % per_b) / (EB / 32);
+                if (x >= b / EB) s += p[i];
+            }
         }
         red[threadIdx.x] = s;
         __syncthreads();
@@ -261,11 +262,13 @@ __global__ void k_stats_ff(const int *tlist, int nlist, int ldim, const double *
     if (status[task] & ~0xF) { result[task] = NAN; return; }
     if (fabs(tr) < 1e-8) { result[task] = -tr; status[task] = ST_TRACE; return; }
     if (!part) return;
-    const double fro2 = red[0], fro = sqrt(fro2);
-    if (mode == 0 && fro < 1) {
-        const double merc = -tr - fro2 / 2;
-        const double err = fabs(fro2 / 2 + fro + log1p(-fro));
-        if (fabs(err / merc) < 1e-8) { result[task] = merc; status[task] = ST_MERCATOR; return; }
+    if (mode == 0) {
+        const double fro2 = red[0], fro = sqrt(fro2);
+        if (fro < 1) {
+            const double merc = -tr - fro2 / 2;
+            const double err = fabs(fro2 / 2 + fro + log1p(-fro));
+            if (fabs(err / merc) < 1e-8) { result[task] = merc; status[task] = ST_MERCATOR; return; }
+        }
     }
     status[task] = ST_FACTOR;
 }
@@ -303,11 +306,10 @@ void launch_elem_ff(const Task *tasks, const int *tlist, int nlist, int ldim, co
 }
 
 void launch_stats_ff(const int *tlist, int nlist, int ldim, const double *diag, const float *part, int mode, double *trace,
-                     double *result, int *status, cudaStream_t st, bool part_per_task)
+                     double *result, int *status, cudaStream_t st, int nsum)
 {
     if (nlist <= 0) return;
-    k_stats_ff<<<nlist, 256, 0, st>>>(tlist, nlist, ldim, diag, part, part_per_task ? 0 : (ldim + EB - 1) / EB, mode, trace, result,
-                                      status);
+    k_stats_ff<<<nlist, 256, 0, st>>>(tlist, nlist, ldim, diag, part, nsum, mode, trace, result, status);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }

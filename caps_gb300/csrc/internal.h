@@ -105,21 +105,23 @@ void launch_seed_ff(const Task *tasks, const int *tlist, const int4 *groups, int
                     int nu_stride, const float4 *ptabf, int pstride, const void *a12t, int ngroup_all, void *seed, bool band,
                     int *status, cudaStream_t st);
 // M of the listed tasks by the I recurrence from all four seed kinds, straight into the FP32
-// delta matrix, with one sum of squares per task in part[task]; sweep_fits: the window fits the
-// kernel's shared-memory ring
+// delta matrix; sums != nullptr: sweep_nsum sums of squares of M per task; sweep_fits: the window is one that
+// takes the recurrence
 bool sweep_fits(int ldim);
+int sweep_nsum(int ldim);
+size_t sweep_work_bytes(int ldim, int nlist);
 void launch_sweep_ff(const Task *tasks, const int *tlist, int nlist, int ldim, const void *seed, const void *Saf, const void *Sbf,
-                     float *S, size_t sstride, float *part, int *status, cudaStream_t st);
+                     void *work, float *S, size_t sstride, float *sums, int *status, cudaStream_t st);
 // the diagonal of M alone, from the band seeds
 void launch_diag_ff(const Task *tasks, int ntask, int ldim, const void *seed, const void *Saf, const void *Sbf, const float4 *uvf,
                     double *diag, int *status, cudaStream_t st);
 // the listed tasks (tlist, nlist; tlist == nullptr: tasks 0..nlist-1)
 void launch_elem_ff(const Task *tasks, const int *tlist, int nlist, int ldim, const void *Saf, const void *Sbf, const float4 *uvf,
                     const void *I, float *S, size_t sstride, double *diag, float *part, int *status, cudaStream_t st);
-// part == nullptr: the trace rule alone, undecided tasks keep status 0; part_per_task: part holds
-// one sum of squares per task (launch_sweep_ff), otherwise k_elem_ff's per-warp partials
+// part == nullptr: the trace rule alone, undecided tasks keep status 0; nsum > 0: part holds nsum sums of squares per task
+// (launch_sweep_ff), otherwise k_elem_ff's per-warp partials
 void launch_stats_ff(const int *tlist, int nlist, int ldim, const double *diag, const float *part, int mode, double *trace,
-                     double *result, int *status, cudaStream_t st, bool part_per_task = false);
+                     double *result, int *status, cudaStream_t st, int nsum = 0);
 // FP64 form: A (lower triangle, FP64) is converted to fixed point in place and factored; mdiag: M_ii
 // (n per task); logdet: ceil(n / 64) partial sums per task; work: cholesky_work_bytes
 size_t cholesky_work_bytes(int ntask, int n);

@@ -516,7 +516,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     CK(cudaMemGetInfo(&freeb, &totb));
     const size_t mat_bytes = O.square ? 16 : ff_elem ? 4 + 1 : (caps->precision == CAPS_PREC_MIXED ? 12 : 8);
     const size_t dense_bytes = hodlr ? hodlr_work_bytes(ldim, 1)
-                             : sweep ? (size_t)dim * dim * 4 + seed_bytes(ldim, 1)
+                             : sweep ? (size_t)dim * dim * 4 + seed_bytes(ldim, 1) + sweep_work_bytes(ldim, 1)
                              : sweep64 ? (size_t)dim * dim * (O.square ? 16 : 8) + seed64_bytes(ldim, 1) + sweep64_work_bytes(ldim, 1)
                                      : (size_t)dim * dim * mat_bytes + (size_t)2 * L * L * sizeof(sd)
                                            + (size_t)L * (L + 1) / 2 * 32; // a_0..a_2 table (one row per task)
@@ -779,9 +779,11 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             // (no element phase)
         } else if (ff_elem && sweep) {
             d_S = (float *)g_eng.S32.get((size_t)nt * mstride * sizeof(float));
-            float *d_part = (float *)g_eng.part.get((size_t)nt * sizeof(float));
-            launch_sweep_ff(d_tasks, d_list, nlist, ldim, d_seed, d_Saf, d_Sbf, d_S, mstride, d_part, d_status, st);
-            launch_stats_ff(d_list, nlist, ldim, d_dg, d_part, O.mode, d_trace, d_res, d_status, st, true);
+            const int nsum = sweep_nsum(ldim);
+            float *d_part = (float *)g_eng.part.get((size_t)nt * nsum * sizeof(float));
+            launch_sweep_ff(d_tasks, d_list, nlist, ldim, d_seed, d_Saf, d_Sbf, g_eng.sw64.get(sweep_work_bytes(ldim, nlist)), d_S, mstride,
+                            O.mode == 0 ? d_part : nullptr, d_status, st);
+            launch_stats_ff(d_list, nlist, ldim, d_dg, d_part, O.mode, d_trace, d_res, d_status, st, nsum);
         } else if (ff_elem) {
             d_S = (float *)g_eng.S32.get((size_t)nt * mstride * sizeof(float));
             float *d_part = (float *)g_eng.part.get((size_t)nt * elem_ff_part_floats(ldim) * sizeof(float));

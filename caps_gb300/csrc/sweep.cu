@@ -38,14 +38,14 @@
 // (m = 0: EE = dA dA T_TM, MM = -dB dB T_TE).  Um = (l+1) Cm and Vp = l Cp for m >= 1, Cp and Cm
 // the column coefficients of the recurrence, so one pair of tables serves both.
 //
-// k_sweep_ff: one CTA per matrix, warp-specialised.  Producer warps form the rows of T into a
-// ring of four shared-memory rows (both polarisations) and publish each on an mbarrier;
-// consumer warps form the elements of row x once row x + 1 is published, 30 columns per pass
-// of 32 lanes (J of the neighbours by shuffles), and release row x - 1 for reuse, so that
-// they wait only for a producer that falls behind, never for one another.  The elements go
-// straight into the FP32 delta matrix (-M, lower triangle, column-major), with a per-matrix
-// sum of squares for the reference's Mercator bound; the FP64 diagonal comes from the band
-// (k_diag_ff).
+// Two kernels behind a table of coefficients (k_sweep_tab).  k_rec_ff fills T row by row, one CTA per matrix and
+// polarisation; k_elem_sweep forms the elements of all pairs from tiles of T, with the row factors dA, dB
+// folded into the row's coefficients and the column factors into the column's.  The elements go
+// straight into the FP32 delta matrix (-M, lower triangle, column-major), with sums
+// of squares for the reference's Mercator bound where they are wanted; the FP64 diagonal comes from the band
+// (k_diag_ff).  One kernel for both, one CTA per matrix with producer warps for the rows and consumer warps for
+// the elements, was bound by its 10 warps' latencies and by stores 2 n rows apart from lane to lane: 547 matrices of
+// ldim 1050 8.9 ms, now 2.1 (rows) + 4.0 (elements).
 #include "common.cuh"
 #include "ff.cuh"
 #include "internal.h"
@@ -112,13 +112,6 @@ __global__ void __launch_bounds__(128, 7) k_seed_ff(const Task *tasks, const int
 // ---------------------------------------------------------------------------
 // the sweep
 // ---------------------------------------------------------------------------
-constexpr int SW_NT = 320, SW_NW = SW_NT / 32; // threads, warps per CTA
-constexpr int SW_PW = 3, SW_CW = SW_NW - SW_PW;  // producer (recurrence) and consumer (element) warps
-constexpr int SW_CH = 30;                       // output columns of a consumer pass (32 lanes)
-constexpr int SW_RING = 4;                      // rows of T held in shared memory
-constexpr int SW_WAIT_ITERS = 1 << 22;          // polls of a bounded mbarrier wait
-constexpr size_t SW_BYTES_PER_L = SW_RING * 2 * sizeof(float2) + 2 * sizeof(float4) + 2 * sizeof(int);
-
 CAPS_DEV ff ff_sub(ff x, ff y) { return ff_add(x, ff_neg(y)); }
 // x c for c exactly representable in FP32 (small integers)
 CAPS_DEV ff ff_mulf(ff x, float c)
@@ -143,21 +136,22 @@ CAPS_DEV ff ff_dot2(ff a, ff x, ff b, ff y)
     const float t = (p - (s - bb)) + (q - bb);
     return ff_fast2(s, t + (ep + eq));
 }
-// a x + b y + c z, c exactly representable in FP32
-CAPS_DEV ff ff_dot3f(ff a, ff x, ff b, ff y, float c, ff z)
+// FP32 of a x + b y + c z: float-float products and sums, one rounding at the end
+CAPS_DEV float ff_dot3(ff a, ff x, ff b, ff y, ff c, ff z)
 {
-    const float p = a.h * x.h, q = b.h * y.h, u = c * z.h;
+    const float p = a.h * x.h, q = b.h * y.h, u = c.h * z.h;
     float ep = fmaf(a.h, x.h, -p);
     ep = fmaf(a.h, x.l, ep);
     ep = fmaf(a.l, x.h, ep);
     float eq = fmaf(b.h, y.h, -q);
     eq = fmaf(b.h, y.l, eq);
     eq = fmaf(b.l, y.h, eq);
-    float eu = fmaf(c, z.h, -u);
-    eu = fmaf(c, z.l, eu);
+    float eu = fmaf(c.h, z.h, -u);
+    eu = fmaf(c.h, z.l, eu);
+    eu = fmaf(c.l, z.h, eu);
     const float s1 = p + q, b1 = s1 - p, t1 = (p - (s1 - b1)) + (q - b1);
     const float s2 = s1 + u, b2 = s2 - s1, t2 = (s1 - (s2 - b2)) + (u - b2);
-    return ff_fast2(s2, (t1 + t2) + (ep + (eq + eu)));
+    return s2 + ((t1 + t2) + (ep + (eq + eu)));
 }
 
 // 1 / y in float-float: the hardware reciprocal and two corrections (relative error ~2^-48)
@@ -185,249 +179,274 @@ CAPS_DEV int sw_k(const ffe *__restrict__ d0tm, int w, int c)
 // a seed (h + l) 2^e in the frame: times 2^{k1 + k2}
 CAPS_DEV ff sw_seed(const ffe &v, int k12) { return v.h == 0.0f ? ff{0.0f, 0.0f} : ff_shift(ff{v.h, v.l}, v.e + k12); }
 
-// FP32 of (d1 d2 2^e) v: the float-float product d1 d2 unrounded, times v with one rounding
-// (error ~0.5 ulp); below 2^-120 -> 0, non-finite or above 2^125 sets bad
-CAPS_DEV float sw_out(ff d1, ff d2, int e, ff v, bool &bad)
+// FP32 of h 2^e; below 2^-120 -> 0, non-finite or above 2^125 sets bad
+CAPS_DEV float sw_out(float h, int e, bool &bad)
 {
-    const float a = d1.h * d2.h;
-    float ea = fmaf(d1.h, d2.h, -a);
-    ea = fmaf(d1.h, d2.l, ea);
-    ea = fmaf(d1.l, d2.h, ea);
-    const float h = fmaf(a, v.h, fmaf(ea, v.h, a * v.l));
     const int k = fexpo(h);
     if (k == -127) return 0.0f;
     if (k == 128 || k + e > 125) { bad = true; return h; }
     return fshift(h, e);
 }
 
-CAPS_DEV ff ldff(const float2 *p) { const float2 v = *p; return ff{v.x, v.y}; }
+// per listed task and window index w, tab[(b * SWF_FIELDS + field) * L + w]: pairs of float-float numbers --
+// Cp, Cm of the recurrence; R1 = 1 / Cp(w - 1), -R1 Cm(w - 1) of row w; the mantissas of Um dA, -Vp dA; m dA, dA; Um dB, -Vp dB;
+// m dB, dB; the scaled seeds (TE, TM) of row w, T(w, w), T(w, w - 1), T(w, c); the exponents of dA, dB as two
+// integers and, third, a bound of the exponents of the six factors times theirs
+enum { SWF_C, SWF_R, SWF_UA, SWF_A, SWF_UB, SWF_B, SWF_D0, SWF_D1, SWF_COL, SWF_E, SWF_FIELDS };
 
-// bounded wait for phase `parity` of an mbarrier that also gives up once another role has
-// given up (*abort); a wait that runs out sets *abort
-CAPS_DEV bool sw_wait(uint64_t *mbar, uint32_t parity, volatile int *abort)
+// grid nlist, 256 threads
+__global__ void __launch_bounds__(256) k_sweep_tab(const Task *tasks, const int *tlist, int nlist, int ldim, const ffe *__restrict__ seed,
+                                                   const ffe *__restrict__ Saf, const ffe *__restrict__ Sbf, float4 *tab)
 {
-    const uint32_t a = umma::smem_u32(mbar);
-    for (int it = 0; it < SW_WAIT_ITERS; it++) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done)
-                     : "r"(a), "r"(parity)
-                     : "memory");
-        if (done) return true;
-        if ((it & 63) == 63 && *abort) return false;
-    }
-    *abort = 1;
-    return false;
-}
-CAPS_DEV void sw_arrive(uint64_t *mbar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(mbar)) : "memory");
-}
-// barrier of the SW_PW producer warps alone (hardware barrier 1)
-CAPS_DEV void sw_producer_bar() { asm volatile("bar.sync 1, %0;" ::"n"(SW_PW * 32) : "memory"); }
-
-// grid nlist (task tlist[b], or b), SW_NT threads, SW_BYTES_PER_L * L bytes of dynamic shared memory.
-// S receives -M (lower triangle, column-major, leading dimension 2 ldim); part[task] the sum of
-// squares of M (both triangles).  Tasks with an error status are skipped.
-//
-// Warp-specialised: SW_PW producer warps form the rows of T (lane y forms T(r, y) from rows r-1
-// and r-2) into a ring of SW_RING rows and publish each on its slot's "ready" mbarrier; SW_CW
-// consumer warps form the elements of row x once row x + 1 is ready, in passes of 30 columns
-// (32 lanes, the two outer ones repeating the neighbours' edges, J of the neighbours by
-// shuffles), and release row x - 1 on its slot's "free" mbarrier, which the producers wait
-// for before they reuse the slot.  Consumers therefore never wait for one another, only for a
-// producer that falls behind.  Row r also writes T(r, r-1) and T(r, r-2) past the diagonals
-// of rows r-1 and r-2 (index r), so that the consumers read rows x-1, x, x+1 up to column
-// x + 1 directly.  Every wait is bounded; a role that gives up flags the others, and the
-// matrix gets ST_ERR_WAIT.
-__global__ void __launch_bounds__(SW_NT, 2) k_sweep_ff(const Task *tasks, const int *tlist, int nlist, int ldim,
-                                                       const ffe *__restrict__ seed, const ffe *__restrict__ Saf,
-                                                       const ffe *__restrict__ Sbf, float *S, size_t sstride, float *part,
-                                                       int *status)
-{
-    extern __shared__ __align__(16) unsigned char sw_smem[];
-    __shared__ uint64_t rready[SW_RING], rfree[SW_RING];
-    __shared__ int s_abort, s_ok;
-    __shared__ float2 seedrow[2][3][2]; // scaled seeds of the producers' next row: [row parity][D0, D1, COL][TE, TM]
-    __shared__ float red[SW_NW];
-    const int L = ldim + 2, n = 2 * ldim;
+    const int L = ldim + 2;
     if ((int)blockIdx.x >= nlist) return;
     const int task = tlist ? tlist[blockIdx.x] : (int)blockIdx.x;
-    if (status[task] & ~0xF) return; // uniform per block
     const Task &T = tasks[task];
     const int mt = T.m, mm = mt > 0 ? mt : 1, lm1 = T.lmin - 1, c = seed_col(T);
-    float2 *ring = reinterpret_cast<float2 *>(sw_smem);   // [SW_RING][pol][L], pol 1 = TM, 0 = TE
-    float4 *cpm = reinterpret_cast<float4 *>(ring + (size_t)SW_RING * 2 * L); // Cp h, l, Cm h, l
-    float4 *dab = cpm + L;                                                   // dA h, l, dB h, l
-    int *eab = reinterpret_cast<int *>(dab + L);                             // exponents of dA (low 16 bits), dB
-    int *ktab = eab + L;                                                     // k(w) of the scaling
     auto sp = [&](int pol, int kind) { return seed + ((size_t)(task * 2 + pol) * SEED_KINDS + kind) * L; };
-    auto rowp = [&](int r) { return ring + (size_t)((r % SW_RING) * 2) * L; }; // row r (r >= 0): TE at +0, TM at +L
     const ffe *d0tm = sp(1, SEED_D0);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-    // per window index: k(w), then the recurrence's column coefficients and the element factors
-    for (int w = tid; w < L; w += SW_NT) ktab[w] = sw_k(d0tm, w, c);
-    __syncthreads();
-    for (int w = tid; w < L; w += SW_NT) {
-        const int l = lm1 + w, kw = ktab[w];
-        ff cp{0.0f, 0.0f}, cmv{0.0f, 0.0f};
-        if (w >= c && w + 1 < L) cp = ff_shift(ff_from_d((double)(l - mm + 1) / (2.0 * l + 1)), kw - ktab[w + 1]);
-        if (w >= c + 1) cmv = ff_shift(ff_from_d((double)(l + mm) / (2.0 * l + 1)), kw - ktab[w - 1]);
-        cpm[w] = make_float4(cp.h, cp.l, cmv.h, cmv.l);
-        const ffe a = Saf[(size_t)task * L + w], b = Sbf[(size_t)task * L + w];
-        dab[w] = make_float4(a.h, a.l, b.h, b.l);
-        const int ea = a.h == 0.0f ? 0 : min(max(a.e - kw, -30000), 30000);
-        const int eb = b.h == 0.0f ? 0 : min(max(b.e - kw, -30000), 30000);
-        eab[w] = (int)(((unsigned)ea & 0xffffu) | ((unsigned)eb << 16));
-    }
-    if (tid == 0) {
-        for (int i = 0; i < SW_RING; i++) {
-            umma::mbar_init(&rready[i], 1);
-            umma::mbar_init(&rfree[i], SW_CW);
+    auto CP = [&](int w) {
+        const int l = lm1 + w;
+        return w >= c && w + 1 < L ? ff_shift(ff_from_d((double)(l - mm + 1) / (2.0 * l + 1)), sw_k(d0tm, w, c) - sw_k(d0tm, w + 1, c))
+                                   : ff{0.0f, 0.0f};
+    };
+    auto CM = [&](int w) {
+        const int l = lm1 + w;
+        return w >= c + 1 ? ff_shift(ff_from_d((double)(l + mm) / (2.0 * l + 1)), sw_k(d0tm, w, c) - sw_k(d0tm, w - 1, c)) : ff{0.0f, 0.0f};
+    };
+    auto pair = [](ff a, ff b) { return make_float4(a.h, a.l, b.h, b.l); };
+    for (int w = threadIdx.x; w < L; w += blockDim.x) {
+        float4 *t = tab + (size_t)blockIdx.x * SWF_FIELDS * L + w;
+        auto put = [&](int field, float4 v) { t[(size_t)field * L] = v; };
+        const int l = lm1 + w, kw = sw_k(d0tm, w, c);
+        const ff cp = CP(w), cm = CM(w);
+        put(SWF_C, pair(cp, cm));
+        ff r1{0.0f, 0.0f}, r2{0.0f, 0.0f};
+        if (w >= c + 3) {
+            r1 = ff_rcp(CP(w - 1));
+            r2 = ff_neg(ff_mul(r1, CM(w - 1)));
         }
-        s_abort = 0;
+        put(SWF_R, pair(r1, r2));
+        const ff um = ff_mulf(cm, (float)(l + 1)), vp = ff_neg(ff_mulf(cp, (float)l));
+        const ffe a = Saf[(size_t)task * L + w], b = Sbf[(size_t)task * L + w];
+        const ff dA{a.h, a.l}, dB{b.h, b.l};
+        const int ea = a.h == 0.0f ? 0 : min(max(a.e - kw, -30000), 30000), eb = b.h == 0.0f ? 0 : min(max(b.e - kw, -30000), 30000);
+        const float4 f[4] = {pair(ff_mul(um, dA), ff_mul(vp, dA)), pair(ff_mulf(dA, (float)mt), dA), pair(ff_mul(um, dB), ff_mul(vp, dB)),
+                             pair(ff_mulf(dB, (float)mt), dB)};
+        put(SWF_UA, f[0]);
+        put(SWF_A, f[1]);
+        put(SWF_UB, f[2]);
+        put(SWF_B, f[3]);
+        const int xa = max(max(fexpo(f[0].x), fexpo(f[0].z)), max(fexpo(f[1].x), fexpo(f[1].z))) + ea; // not finite: 128
+        const int xb = max(max(fexpo(f[2].x), fexpo(f[2].z)), max(fexpo(f[3].x), fexpo(f[3].z))) + eb;
+        put(SWF_E, make_float4(__int_as_float(ea), __int_as_float(eb), __int_as_float(max(xa, xb)), 0.0f));
+        auto seeds = [&](int kind, int y, int wi) {
+            ff v[2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+            if (y >= c && wi >= 0)
+                for (int pol = 0; pol < 2; pol++) v[pol] = sw_seed(sp(pol, kind)[wi], kw + sw_k(d0tm, y, c));
+            return pair(v[0], v[1]);
+        };
+        put(SWF_D0, seeds(SEED_D0, w, w));
+        put(SWF_D1, seeds(SEED_D1, w - 1, w - 1));
+        put(SWF_COL, seeds(SEED_COL, c, w));
     }
-    __syncthreads();
-    volatile int *abort = &s_abort;
-    const ff zero{0.0f, 0.0f};
-    float fro = 0.0f;
-    bool bad = false;
+}
 
-    if (warp < SW_PW) {
-        // ---- producers: rows of T ----
-        // the seeds of row r (pairs (r, r), (r, r-1), (r, c)), scaled into the frame, into
-        // seedrow[r & 1] by threads 0..5 one row ahead, so that their loads are off the row's path
-        auto fetch_seeds = [&](int r) {
-            if (tid < 6 && r < L) {
-                const int kind = tid >> 1, pol = tid & 1;
-                const int y = kind == 0 ? r : (kind == 1 ? r - 1 : c), wi = kind == 2 ? r : y;
-                const int skind = kind == 0 ? SEED_D0 : (kind == 1 ? SEED_D1 : SEED_COL);
-                ff v = zero;
-                if (y >= c && wi >= 0) v = sw_seed(sp(pol, skind)[wi], ktab[r] + ktab[y]);
-                seedrow[r & 1][kind][pol] = make_float2(v.h, v.l);
+// T(r, y), y <= r, of listed task b at tt[((b * 2 + pol) * L + r) * L + y].  Grid nlist * 2: one polarisation (TE, TM) per CTA,
+// the ring of three rows in shared memory (r and the two before it), one barrier per row; a thread keeps the coefficients of its first
+// columns in registers and the next row's seeds and factors are loaded a row ahead, so that the row's chain
+// is two float-float sums and the barrier.  Bound by that chain and by issue (about 95 instructions per column).
+constexpr int RF_NT = 256, RF_RING = 3, RF_KEEP = 4;
+__global__ void __launch_bounds__(RF_NT) k_rec_ff(const Task *tasks, const int *tlist, int nlist, int ldim, const float4 *__restrict__ tab, float2 *tt,
+                                                  const int *status)
+{
+    extern __shared__ __align__(16) float2 rf_sm[];
+    const int L = ldim + 2;
+    const int pol = blockIdx.x & 1, b = blockIdx.x >> 1, tid = threadIdx.x;
+    if (b >= nlist) return;
+    const int task = tlist ? tlist[b] : b;
+    if (status[task] & ~0xF) return; // no status changes in this launch: uniform
+    const int c = seed_col(tasks[task]);
+    const float4 *W = tab + (size_t)b * SWF_FIELDS * L;
+    float2 *t = tt + ((size_t)b * 2 + pol) * L * L;
+    __shared__ float4 s_r[2];       // of the next row: R1, -R2
+    __shared__ float2 s_seed[2][3]; // and its seeds
+    auto fetch = [&](int row) {
+        if (tid < 4 && row < L) {
+            const float4 v = __ldg(W + (size_t)(tid < 3 ? SWF_D0 + tid : SWF_R) * L + row);
+            if (tid < 3) s_seed[row & 1][tid] = pol ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+            else s_r[row & 1] = v;
+        }
+    };
+    float4 keep[RF_KEEP];
+#pragma unroll
+    for (int i = 0; i < RF_KEEP; i++) keep[i] = tid + i * RF_NT < L ? __ldg(W + (size_t)SWF_C * L + tid + i * RF_NT) : make_float4(0, 0, 0, 0);
+    fetch(0);
+    // rows r, r - 1, r - 2; rows before the first are never read: y >= c + 1 and y <= r - 2 need r >= 3
+    float2 *D = rf_sm, *P1 = rf_sm + L, *P2 = rf_sm + 2 * L;
+    __syncthreads();
+    for (int r = 0; r < L; r++) {
+        fetch(r + 1);
+        const float4 R = s_r[r & 1];
+        const float2 *seeds = s_seed[r & 1];
+        auto column = [&](int y, const float4 &C) {
+            float2 v = make_float2(0.0f, 0.0f);
+            if (y >= c) {
+                if (y == r || y == r - 1 || y == c) v = seeds[y == r ? 0 : y == r - 1 ? 1 : 2];
+                else {
+                    auto ld = [](const float2 &u) { return ff{u.x, u.y}; };
+                    const ff s = ff_dot2(ff{R.x, R.y}, ff_dot2(ff{C.x, C.y}, ld(P1[y + 1]), ff{C.z, C.w}, ld(P1[y - 1])), ff{R.z, R.w}, ld(P2[y]));
+                    v = make_float2(s.h, s.l);
+                }
+            }
+            D[y] = v;
+            t[y] = v;
+        };
+#pragma unroll
+        for (int i = 0; i < RF_KEEP; i++)
+            if (tid + i * RF_NT <= r) column(tid + i * RF_NT, keep[i]);
+        for (int y = tid + RF_KEEP * RF_NT; y <= r; y += RF_NT) column(y, __ldg(W + (size_t)SWF_C * L + y));
+        __syncthreads();
+        float2 *next = P2;
+        P2 = P1;
+        P1 = D;
+        D = next;
+        t += L;
+    }
+}
+
+// Elements from the table.  Grid (ceil(ldim / EL_X), ceil(ldim / EL_Y), nlist), EL_X threads: thread x walks EL_Y columns y <= x of
+// a tile of T in shared memory, with J(x, v) = Um(x) T(x-1, v) - Vp(x) T(x+1, v) of the columns y - 1, y, y + 1 in
+// registers; consecutive threads write consecutive rows of the column-major matrix.  S receives -M; sums (FRO) the sum
+// of squares of M (both triangles), one per block.
+//
+// Pairs whose four elements are all below 2^-62 of the matrix (the FP64 form's last digit; the panel solves take
+// what is below 2^-52 as zero) are stored as zeros where a whole warp's are, unless the sums are wanted.  Bound by
+// issue and shared-memory latency at 11 CTAs per SM (256 instructions per pair); the next column read one step ahead
+// cost more in registers' moves than it hid (4.4 ms against 4.0).
+constexpr int EL_X = 64, EL_Y = 16, EL_LD = EL_Y + 3; // odd row length: consecutive rows in distinct banks
+template <bool FRO>
+__global__ void __launch_bounds__(EL_X) k_elem_sweep(const Task *tasks, const int *tlist, int nlist, int ldim, const float2 *__restrict__ tt,
+                                                     const float4 *__restrict__ tab, float *S, size_t sstride, float *sums, int *status)
+{
+    const int L = ldim + 2, n = 2 * ldim, b = blockIdx.z, tid = threadIdx.x;
+    if (b >= nlist) return;
+    const int task = tlist ? tlist[b] : b;
+    const int X0 = blockIdx.x * EL_X + 1, x = X0 + tid, y0 = blockIdx.y * EL_Y + 1;
+    __shared__ float2 sT[2][EL_X + 2][EL_LD];
+    __shared__ float red[EL_X / 32];
+    float fro = 0.0f;
+    if (y0 <= min(X0 + EL_X - 1, ldim)) { // uniform: the block has elements
+        bool bad = false;
+        const int mt = tasks[task].m;
+        // T(u, v) of rows X0 - 1 .. X0 + EL_X and columns y0 - 1 .. y0 + EL_Y, any order of u and v
+        constexpr int ROWS = EL_X / (EL_Y + 2); // rows at a time
+        const int ti = tid / (EL_Y + 2), tj = tid % (EL_Y + 2), v = min(y0 - 1 + tj, L - 1);
+        if (ti < ROWS) {
+            const float2 *t0 = tt + (size_t)b * 2 * L * L, *t1 = t0 + (size_t)L * L;
+#pragma unroll 4
+            for (int i = ti; i < EL_X + 2; i += ROWS) {
+                const int u = min(X0 - 1 + i, L - 1);
+                const size_t o = u >= v ? (size_t)u * L + v : (size_t)v * L + u;
+                sT[0][i][tj] = t0[o];
+                sT[1][i][tj] = t1[o];
+            }
+        }
+        __syncthreads();
+        const float4 *W = tab + (size_t)b * SWF_FIELDS * L;
+        auto F = [&](int f, int w) { return __ldg(W + (size_t)f * L + w); };
+        auto lo = [](const float4 &v) { return ff{v.x, v.y}; };
+        auto hi = [](const float4 &v) { return ff{v.z, v.w}; };
+        const int xx = min(x, ldim);
+        auto TV = [&](int pol, int i, int v) { const float2 q = sT[pol][tid + i][v - y0 + 1]; return ff{q.x, q.y}; };
+        const float4 xE = F(SWF_E, xx);
+        const int eA = __float_as_int(xE.x), eB = __float_as_int(xE.y), exr = __float_as_int(xE.z);
+        float *Sp = S + (size_t)task * sstride + (size_t)2 * (y0 - 1) * n + 2 * (x - 1);
+        const int y1 = min(y0 + EL_Y - 1, ldim); // uniform; lanes with x < y are idle
+        auto store = [&](int y, float ee, float mm, float em, float me) {
+            *reinterpret_cast<float2 *>(Sp) = make_float2(-ee, -me);
+            if (y != x) {
+                *reinterpret_cast<float2 *>(Sp + n) = make_float2(-em, -mm);
+                if (FRO) fro += 2.0f * (ee * ee + me * me + mm * mm + em * em);
+            } else {
+                Sp[n + 1] = -mm;
+                if (FRO) fro += ee * ee + mm * mm + 2.0f * me * me;
             }
         };
-        fetch_seeds(0);
-        sw_producer_bar();
-        for (int r = 0; r < L; r++) {
-            const int s = r % SW_RING;
-            if (r >= SW_RING) { // slot s held row r - SW_RING: every consumer warp has released it
-                if (tid == 0) s_ok = sw_wait(&rfree[s], (r / SW_RING - 1) & 1, abort) ? 1 : 0;
-                sw_producer_bar();
-                if (!s_ok) break; // uniform over the producer warps
+        if (mt == 0) {
+            const ff dA = hi(F(SWF_A, xx)), dB = hi(F(SWF_B, xx));
+            for (int y = y0; y <= min(y1, x) && x <= ldim; y++, Sp += 2 * (size_t)n) {
+                const float4 yE = F(SWF_E, y);
+                const ff z{0.0f, 0.0f};
+                const ff a = ff_mul(dA, hi(F(SWF_A, y))), bb = ff_mul(dB, hi(F(SWF_B, y)));
+                store(y, sw_out(ff_dot3(a, TV(1, 1, y), z, z, z, z), eA + __float_as_int(yE.x), bad),
+                      sw_out(-ff_dot3(bb, TV(0, 1, y), z, z, z, z), eB + __float_as_int(yE.y), bad), 0.0f, 0.0f);
             }
-            float2 *W = rowp(r);
-            const float2 *P1 = r >= 1 ? rowp(r - 1) : W, *P2 = r >= 2 ? rowp(r - 2) : W;
-            float2 *X1 = const_cast<float2 *>(P1), *X2 = const_cast<float2 *>(P2);
-            // the recurrence of row r divided by its row coefficient: R1 = 1 / Cp(r-1), R2 = R1 Cm(r-1)
-            ff R1 = zero, nR2 = zero;
-            if (r >= c + 3) {
-                const float4 q = cpm[r - 1];
-                R1 = ff_rcp(ff{q.x, q.y});
-                nR2 = ff_neg(ff_mul(R1, ff{q.z, q.w}));
-            }
-            fetch_seeds(r + 1); // read at row r + 1, after the barriers below
-            for (int y = tid; y <= r; y += SW_PW * 32) {
-                ff vT = zero, vE = zero;
-                if (y < c) {
-                } else if (y == r || y == r - 1 || y == c) {
-                    const int kind = y == r ? 0 : (y == r - 1 ? 1 : 2);
-                    const float2 t1 = seedrow[r & 1][kind][1], t0 = seedrow[r & 1][kind][0];
-                    vT = ff{t1.x, t1.y};
-                    vE = ff{t0.x, t0.y};
-                } else {
-                    const float4 q = cpm[y];
-                    const ff Cp{q.x, q.y}, Cm{q.z, q.w};
-                    vT = ff_dot2(R1, ff_dot2(Cp, ldff(P1 + L + y + 1), Cm, ldff(P1 + L + y - 1)), nR2, ldff(P2 + L + y));
-                    vE = ff_dot2(R1, ff_dot2(Cp, ldff(P1 + y + 1), Cm, ldff(P1 + y - 1)), nR2, ldff(P2 + y));
+        } else {
+            const float4 fUA = F(SWF_UA, xx), fUB = F(SWF_UB, xx);
+            const ff UA = lo(fUA), VA = hi(fUA), UB = lo(fUB), VB = hi(fUB), mA = lo(F(SWF_A, xx)), mB = lo(F(SWF_B, xx));
+            // of column v: dA(x) J_TM, dB(x) J_TE, m dB(x) T_TM, m dA(x) T_TE (mantissas)
+            struct Col { ff JT, JE, mT, mE; };
+            struct Raw { ff a, t, d, ea, e, ed; }; // T_TM and T_TE at x - 1, x, x + 1
+            auto raw = [&](int v) { return Raw{TV(1, 0, v), TV(1, 1, v), TV(1, 2, v), TV(0, 0, v), TV(0, 1, v), TV(0, 2, v)}; };
+            auto form = [&](const Raw &q) {
+                return Col{ff_dot2(UA, q.a, VA, q.d), ff_dot2(UB, q.ea, VB, q.ed), ff_mul(mB, q.t), ff_mul(mA, q.e)};
+            };
+            // exponent of the largest of a column's values, from the magnitudes' bits
+            auto top = [&](const Raw &q) {
+                auto m = [](ff x) { return __float_as_int(x.h) & 0x7fffffff; };
+                return (max(max(max(m(q.a), m(q.t)), max(m(q.d), m(q.ea))), max(m(q.e), m(q.ed))) >> 23) - 127;
+            };
+            Col cm{}, c0{};
+            int em_ = top(raw(y0 - 1)), e0_ = top(raw(y0));
+            bool have = false; // cm and c0 are formed (uniform over the warp)
+            for (int y = y0; y <= y1; y++, Sp += 2 * (size_t)n) {
+                const bool act = x <= ldim && y <= x;
+                const float4 yE = F(SWF_E, y);
+                const Raw qp = raw(y + 1);
+                const int ep_ = top(qp);
+                // five products of three factors, each below 2^(sum of exponents + 3)
+                const bool zero = !FRO && y != x && exr + __float_as_int(yE.z) + max(max(em_, e0_), ep_) + 6 < -62;
+                em_ = e0_;
+                e0_ = ep_;
+                if (__all_sync(0xffffffffu, !act || zero)) {
+                    if (act) store(y, 0.0f, 0.0f, 0.0f, 0.0f);
+                    have = false;
+                    continue;
                 }
-                W[L + y] = make_float2(vT.h, vT.l);
-                W[y] = make_float2(vE.h, vE.l);
-                // T(r, r-1) and T(r, r-2) past the diagonals of rows r-1 and r-2
-                if (y == r - 1) { X1[L + r] = make_float2(vT.h, vT.l); X1[r] = make_float2(vE.h, vE.l); }
-                if (y == r - 2) { X2[L + r] = make_float2(vT.h, vT.l); X2[r] = make_float2(vE.h, vE.l); }
+                if (!have) {
+                    cm = form(raw(y - 1));
+                    c0 = form(raw(y));
+                    have = true;
+                }
+                const Col cp = form(qp);
+                // EE = dA dA [B_TM - m^2 T_TE], MM = dB dB [m^2 T_TM - B_TE], B(x, y) = Um(y) J(x, y-1) - Vp(y) J(x, y+1);
+                // EM = m dA(x) dB(y) [H_TE - J_TM], ME = m dB(x) dA(y) [J_TE - H_TM], H(x, y) = Um(y) T(x, y-1) - Vp(y) T(x, y+1)
+                const float4 gUA = F(SWF_UA, y), gUB = F(SWF_UB, y);
+                const ff yUA = lo(gUA), yVA = hi(gUA), yUB = lo(gUB), yVB = hi(gUB), yA = lo(F(SWF_A, y)), yB = lo(F(SWF_B, y));
+                const float ee = ff_dot3(yUA, cm.JT, yVA, cp.JT, ff_neg(yA), c0.mE);
+                const float mm = -ff_dot3(yUB, cm.JE, yVB, cp.JE, ff_neg(yB), c0.mT);
+                const float em = ff_dot3(yUB, cm.mE, yVB, cp.mE, ff_neg(yB), c0.JT);
+                const float me = -ff_dot3(yUA, cm.mT, yVA, cp.mT, ff_neg(yA), c0.JE);
+                const int fA = __float_as_int(yE.x), fB = __float_as_int(yE.y);
+                bool wrong = false;
+                const float oee = sw_out(ee, eA + fA, wrong), omm = sw_out(mm, eB + fB, wrong), oem = sw_out(em, eA + fB, wrong),
+                            ome = sw_out(me, eB + fA, wrong);
+                if (act) {
+                    bad |= wrong;
+                    store(y, oee, omm, oem, ome);
+                }
+                cm = c0;
+                c0 = cp;
             }
-            sw_producer_bar(); // row r complete before the next row reads it, and before it is published
-            if (tid == 0) sw_arrive(&rready[s]);
         }
-    } else {
-        // ---- consumers: elements of rows x = 1 .. ldim ----
-        const int cw = warp - SW_PW;
-        const float m2 = (float)mt * (float)mt; // exact for m < 4096
-        float *Sm = S + (size_t)task * sstride;
-        bool ok = __all_sync(0xffffffffu, sw_wait(&rready[0], 0, abort) && sw_wait(&rready[1], 0, abort));
-        for (int x = 1; ok && x <= ldim; x++) {
-            ok = __all_sync(0xffffffffu, sw_wait(&rready[(x + 1) % SW_RING], ((x + 1) / SW_RING) & 1, abort));
-            if (!ok) break;
-            const float2 *Rm = rowp(x - 1), *R0 = rowp(x), *Rp = rowp(x + 1);
-            const float4 qx = cpm[x], dx = dab[x];
-            const int ex = eab[x];
-            const ff Umx = ff_mulf(ff{qx.z, qx.w}, (float)(lm1 + x + 1)), nVpx = ff_neg(ff_mulf(ff{qx.x, qx.y}, (float)(lm1 + x)));
-            const ff dAx{dx.x, dx.y}, dBx{dx.z, dx.w};
-            const ff mdAx = ff_mulf(dAx, (float)mt), mdBx = ff_mulf(dBx, (float)mt);
-            const int eAx = (int)(short)(ex & 0xffff), eBx = ex >> 16;
-            const int r0 = 2 * (x - 1);
-            for (int k = cw; k * SW_CH <= x; k += SW_CW) {
-                const int y = k * SW_CH - 1 + lane;
-                // J(x, y) = Um(x) T(x-1, y) - Vp(x) T(x+1, y), y in [0, x+1]
-                ff JT = zero, JE = zero;
-                if (mt > 0 && y >= 0 && y <= x + 1) {
-                    JT = ff_dot2(Umx, ldff(Rm + L + y), nVpx, ldff(Rp + L + y));
-                    JE = ff_dot2(Umx, ldff(Rm + y), nVpx, ldff(Rp + y));
-                }
-                const ff JTm{__shfl_up_sync(0xffffffffu, JT.h, 1), __shfl_up_sync(0xffffffffu, JT.l, 1)};
-                const ff JTp{__shfl_down_sync(0xffffffffu, JT.h, 1), __shfl_down_sync(0xffffffffu, JT.l, 1)};
-                const ff JEm{__shfl_up_sync(0xffffffffu, JE.h, 1), __shfl_up_sync(0xffffffffu, JE.l, 1)};
-                const ff JEp{__shfl_down_sync(0xffffffffu, JE.h, 1), __shfl_down_sync(0xffffffffu, JE.l, 1)};
-                if (lane == 0 || lane == 31 || y < 1 || y > x) continue;
-                const float4 dy = dab[y];
-                const int ey = eab[y];
-                const ff dAy{dy.x, dy.y}, dBy{dy.z, dy.w};
-                const int eAy = (int)(short)(ey & 0xffff), eBy = ey >> 16;
-                const ff c1T = ldff(R0 + L + y), c1E = ldff(R0 + y);
-                float ee, mmv, em = 0.0f, me = 0.0f;
-                if (mt == 0) {
-                    ee = sw_out(dAx, dAy, eAx + eAy, c1T, bad);
-                    mmv = sw_out(dBx, dBy, eBx + eBy, ff_neg(c1E), bad);
-                } else {
-                    const float4 qy = cpm[y];
-                    const int ly = lm1 + y;
-                    const ff Umy = ff_mulf(ff{qy.z, qy.w}, (float)(ly + 1)), nVpy = ff_neg(ff_mulf(ff{qy.x, qy.y}, (float)ly));
-                    const ff HT = ff_dot2(Umy, ldff(R0 + L + y - 1), nVpy, ldff(R0 + L + y + 1));
-                    const ff HE = ff_dot2(Umy, ldff(R0 + y - 1), nVpy, ldff(R0 + y + 1));
-                    // EE = dA dA [B_TM - m^2 T_TE], MM = dB dB [m^2 T_TM - B_TE], B(x, y) = Um(y) J(x, y-1) - Vp(y) J(x, y+1)
-                    const ff iEE = ff_dot3f(Umy, JTm, nVpy, JTp, -m2, c1E);
-                    const ff iMM = ff_neg(ff_dot3f(Umy, JEm, nVpy, JEp, -m2, c1T));
-                    ee = sw_out(dAx, dAy, eAx + eAy, iEE, bad);
-                    mmv = sw_out(dBx, dBy, eBx + eBy, iMM, bad);
-                    em = sw_out(mdAx, dBy, eAx + eBy, ff_sub(HE, JT), bad);
-                    me = sw_out(mdBx, dAy, eBx + eAy, ff_sub(JE, HT), bad);
-                }
-                const int c0 = 2 * (y - 1);
-                *reinterpret_cast<float2 *>(Sm + (size_t)c0 * n + r0) = make_float2(-ee, -me);
-                if (y != x) {
-                    *reinterpret_cast<float2 *>(Sm + (size_t)(c0 + 1) * n + r0) = make_float2(-em, -mmv);
-                    fro += 2.0f * (ee * ee + me * me + mmv * mmv + em * em);
-                } else {
-                    Sm[(size_t)(c0 + 1) * n + r0 + 1] = -mmv;
-                    fro += ee * ee + mmv * mmv + 2.0f * me * me;
-                }
-            }
-            __syncwarp();
-            if (lane == 0) sw_arrive(&rfree[(x - 1) % SW_RING]); // row x - 1 is done with
-        }
+        if (__syncthreads_or(bad) && tid == 0) atomicOr(status + task, ST_ERR_NONFINITE);
     }
-    __syncthreads();
-    for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
-    if (lane == 0) red[warp] = fro;
-    const int anybad = __syncthreads_or(bad);
-    if (tid == 0) {
-        float sum = 0.0f;
-        for (int w = 0; w < SW_NW; w++) sum += red[w];
-        part[task] = sum;
-        if (anybad) atomicOr(status + task, ST_ERR_NONFINITE);
-        if (s_abort) atomicOr(status + task, ST_ERR_WAIT);
+    if (FRO) { // per-block sums, added by the statistics kernel in order
+        for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);
+        if ((tid & 31) == 0) red[tid >> 5] = fro;
+        __syncthreads();
+        if (tid == 0) sums[((size_t)task * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = red[0] + red[1];
     }
 }
 
@@ -436,17 +455,17 @@ __global__ void __launch_bounds__(SW_NT, 2) k_sweep_ff(const Task *tasks, const 
 // ---------------------------------------------------------------------------
 size_t seed_bytes(int ldim, int ntask) { return (size_t)ntask * 2 * SEED_KINDS * (ldim + 2) * sizeof(ffe); }
 
-size_t sweep_smem_bytes(int ldim) { return SW_BYTES_PER_L * (size_t)(ldim + 2); }
+static size_t sweep_smem_bytes(int ldim) { return (size_t)RF_RING * (ldim + 2) * sizeof(float2); }
 
-bool sweep_fits(int ldim)
+// windows up to this take the recurrence, larger ones the q-sums of every pair.  The line is that of the tested range
+// (the recurrence has been compared over 1000 rows from its seeds); the ring would fit up to 7000.
+constexpr int SWEEP_MAX = 2230;
+bool sweep_fits(int ldim) { return ldim <= SWEEP_MAX; }
+int sweep_nsum(int ldim) { return ((ldim + EL_X - 1) / EL_X) * ((ldim + EL_Y - 1) / EL_Y); }
+size_t sweep_work_bytes(int ldim, int nlist)
 {
-    static int smax = -1;
-    if (smax < 0) {
-        int dev = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    }
-    return sweep_smem_bytes(ldim) + 256 <= (size_t)smax;
+    const size_t L = ldim + 2;
+    return (size_t)nlist * L * (SWF_FIELDS * sizeof(float4) + 2 * L * sizeof(float2));
 }
 
 void launch_seed_ff(const Task *tasks, const int *tlist, const int4 *groups, int ngroups, int ldim, const float4 *KP, const int *KPe,
@@ -465,18 +484,23 @@ void launch_seed_ff(const Task *tasks, const int *tlist, const int4 *groups, int
 }
 
 void launch_sweep_ff(const Task *tasks, const int *tlist, int nlist, int ldim, const void *seed, const void *Saf, const void *Sbf,
-                     float *S, size_t sstride, float *part, int *status, cudaStream_t st)
+                     void *work, float *S, size_t sstride, float *sums, int *status, cudaStream_t st)
 {
     if (nlist <= 0) return;
     static size_t attr = 0;
-    const size_t smem = sweep_smem_bytes(ldim);
+    const size_t smem = sweep_smem_bytes(ldim), L = ldim + 2;
     if (smem > attr) {
-        CK(cudaFuncSetAttribute(k_sweep_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(cudaFuncSetAttribute(k_rec_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr = smem;
     }
-    k_sweep_ff<<<nlist, SW_NT, smem, st>>>(tasks, tlist, nlist, ldim, (const ffe *)seed, (const ffe *)Saf, (const ffe *)Sbf, S, sstride,
-                                           part, status);
-    COUNT_LAUNCH(1);
+    float4 *tab = (float4 *)work;
+    float2 *tt = (float2 *)(tab + nlist * SWF_FIELDS * L);
+    k_sweep_tab<<<nlist, 256, 0, st>>>(tasks, tlist, nlist, ldim, (const ffe *)seed, (const ffe *)Saf, (const ffe *)Sbf, tab);
+    k_rec_ff<<<nlist * 2, RF_NT, smem, st>>>(tasks, tlist, nlist, ldim, tab, tt, status);
+    const dim3 g((ldim + EL_X - 1) / EL_X, (ldim + EL_Y - 1) / EL_Y, nlist);
+    if (sums) k_elem_sweep<true><<<g, EL_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, S, sstride, sums, status);
+    else k_elem_sweep<false><<<g, EL_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, S, sstride, nullptr, status);
+    COUNT_LAUNCH(3);
     CK(cudaGetLastError());
 }
 
