@@ -100,10 +100,10 @@ void launch_scale_ff(int ntask, int ldim, const sd *Sa, const sd *Sb, const doub
 enum { SEED_D0 = 0, SEED_D1 = 1, SEED_D2 = 2, SEED_COL = 3, SEED_KINDS = 4 };
 size_t seed_bytes(int ldim, int ntask);
 // band: kinds D0 and D2 (what the diagonal of M reads); otherwise D1 and COL (the rest of the
-// recurrence's seeds).  a12t: the per-m tables of launch_a12_mixed (ngroup_all groups)
+// recurrence's seeds) and the rows that its parts start from, into the work of launch_sweep_ff.  a12t: the per-m tables of launch_a12_mixed (ngroup_all groups)
 void launch_seed_ff(const Task *tasks, const int *tlist, const int4 *groups, int ngroups, int ldim, const float4 *KP, const int *KPe,
                     int nu_stride, const float4 *ptabf, int pstride, const void *a12t, int ngroup_all, void *seed, bool band,
-                    int *status, cudaStream_t st);
+                    void *work, int nlist, int *status, cudaStream_t st);
 // M of the listed tasks by the I recurrence from all four seed kinds, straight into the FP32
 // delta matrix; sums != nullptr: sweep_nsum sums of squares of M per task; sweep_fits: the window is one that
 // takes the recurrence

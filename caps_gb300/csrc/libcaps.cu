@@ -694,7 +694,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
                 // the band of q-sums that M_ii reads (l1 - l2 in {0, 2})
                 d_seed = g_eng.seed.get(seed_bytes(ldim, nt));
                 launch_seed_ff(d_tasks, nullptr, d_sub, nsub, ldim, d_KP, d_KPe, nu_stride, d_ptabf, pstride, d_a12t, ngroup, d_seed,
-                               true, d_status, st);
+                               true, nullptr, 0, d_status, st);
                 CK(cudaEventRecord(g_eng.ev[3], st));
                 launch_diag_ff(d_tasks, nt, ldim, d_seed, d_Saf, d_Sbf, d_uvf, d_dg, d_status, st);
                 launch_stats_ff(nullptr, nt, ldim, d_dg, nullptr, O.mode, d_trace, d_res, d_status, st);
@@ -717,7 +717,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
                 CK(cudaEventRecord(g_eng.ev[5], st));
                 if (sweep) // the rest of the recurrence's seeds: l1 - l2 = 1 and the first column
                     launch_seed_ff(d_tasks, d_list, dg2, nlist > 0 ? (int)sub2.size() : 0, ldim, d_KP, d_KPe, nu_stride, d_ptabf, pstride,
-                                   d_a12t, ngroup, d_seed, false, d_status, st);
+                                   d_a12t, ngroup, d_seed, false, g_eng.sw64.get(sweep_work_bytes(ldim, nlist)), nlist, d_status, st);
                 else
                     launch_itab_grp(d_tasks, d_list, dg2, nlist > 0 ? (int)sub2.size() : 0, ldim, d_KP, d_KPe, nu_stride, d_ptabf, pstride,
                                     d_a12, d_I, true, d_status, st);

@@ -61,11 +61,18 @@ CAPS_DEV int seed_col(const Task &T)
     return T.lmin - 1 >= mm ? 0 : 1;
 }
 
+// ranges of rows of T: part q of P forms rows (row(q), row(q + 1)], row(0) = -1, of about equal numbers of pairs; parts
+// q >= 1 start from the q-sums of rows row(q) - 1 and row(q).  The number depends on ldim alone.  Few large
+// matrices leave SMs idle behind the chain of rows: 6 matrices of ldim 3000 take 4.7 ms in one part, 1.05 in five
+__host__ __device__ inline int recf_row(int q, int P, int L) { return q <= 0 ? -1 : q >= P ? L - 1 : (int)(L * sqrt((double)q / P)); }
+__host__ __device__ inline int recf_parts(int ldim) { return ldim <= 2230 ? 1 : ldim / 512; }
+
 // ---------------------------------------------------------------------------
 // seeds: q-sums of the pairs of two kinds per window index w
 // ---------------------------------------------------------------------------
-// grid (2 ceil(L/128), ngroups): the first half of the blocks computes kind0, the second kind1
-// (so that a warp runs sums of one kind and similar length).  groups as in launch_itab_grp; a_0,
+// grid (np ceil(L/128), ngroups): the first block row computes kind0, the second kind1
+// (so that a warp runs sums of one kind and similar length), two more per part q = 1 .. the pairs (row(q) - 1, w) and
+// (row(q), w), rows[((((list entry) (P - 1) + q - 1) * 2 + i) * 2 + pol) * L + w].  groups as in launch_itab_grp; a_0,
 // a_1, a_2 come from the per-m tables (a012f_pair), so no pair table is formed.  seed[((task *
 // 2 + pol) * SEED_KINDS + kind) * L + w] receives the pair's value as float-float with exponent;
 // pairs outside the window are not written (nothing reads them).
@@ -73,13 +80,14 @@ template <int G>
 __global__ void __launch_bounds__(128, 7) k_seed_ff(const Task *tasks, const int *tlist, const int4 *groups, int ngroups, int ldim,
                                                     const float4 *__restrict__ KP, const int *__restrict__ KPe, int nu_stride,
                                                     const float4 *__restrict__ ptabf, int pstride, const A12L *__restrict__ tl,
-                                                    const A12J *__restrict__ tj, int kind0, int kind1, ffe *seed, int *status,
+                                                    const A12J *__restrict__ tj, int kind0, int kind1, ffe *seed, int P, ffe *rows, int *status,
                                                     int stop_bits)
 {
     const int L = ldim + 2, NJ = 2 * L - 1, nbw = (L + 127) / 128;
     const int gi = blockIdx.y;
     if (gi >= ngroups) return;
-    const int kind = (int)blockIdx.x < nbw ? kind0 : kind1;
+    const int bp = (int)blockIdx.x / nbw, kind = bp == 0 ? kind0 : bp == 1 ? kind1 : SEED_KINDS; // SEED_KINDS: a row
+    const int rq = (bp - 2) / 2 + 1, ri = bp & 1;
     const int w = ((int)blockIdx.x % nbw) * 128 + threadIdx.x;
     if (w >= L) return;
     const int4 grp = groups[gi];
@@ -92,9 +100,12 @@ __global__ void __launch_bounds__(128, 7) k_seed_ff(const Task *tasks, const int
     if (kind == SEED_D1) a1 = w + 1;
     else if (kind == SEED_D2) a1 = w + 2;
     else if (kind == SEED_COL) a2 = seed_col(T);
-    if (a1 >= L) return;
+    else if (kind == SEED_KINDS) a1 = recf_row(rq, P, L) - 1 + ri;
+    if (a1 >= L || (kind == SEED_KINDS && w > a1)) return;
     auto store = [&](int g, int pol, float h, float l, int e) {
-        seed[((size_t)(tk[g] * 2 + pol) * SEED_KINDS + kind) * L + w] = ffe{h, l, e, 0};
+        ffe *o = kind == SEED_KINDS ? rows + ((((size_t)(grp.x + g) * (P - 1) + rq - 1) * 2 + ri) * 2 + pol) * L
+                                    : seed + ((size_t)(tk[g] * 2 + pol) * SEED_KINDS + kind) * L;
+        o[w] = ffe{h, l, e, 0};
     };
     const int mm = T.m > 0 ? T.m : 1, l1 = T.lmin - 1 + a1, l2 = T.lmin - 1 + a2;
     if (a1 < a2 || l2 < mm || l2 < T.m || l1 < 1) { // I = 0 for l < m (integration.c:631)
@@ -191,7 +202,7 @@ CAPS_DEV float sw_out(float h, int e, bool &bad)
 // per listed task and window index w, tab[(b * SWF_FIELDS + field) * L + w]: pairs of float-float numbers --
 // Cp, Cm of the recurrence; R1 = 1 / Cp(w - 1), -R1 Cm(w - 1) of row w; the mantissas of Um dA, -Vp dA; m dA, dA; Um dB, -Vp dB;
 // m dB, dB; the scaled seeds (TE, TM) of row w, T(w, w), T(w, w - 1), T(w, c); the exponents of dA, dB as two
-// integers and, third, a bound of the exponents of the six factors times theirs
+// integers, a bound of the exponents of the six factors times theirs, and k(w)
 enum { SWF_C, SWF_R, SWF_UA, SWF_A, SWF_UB, SWF_B, SWF_D0, SWF_D1, SWF_COL, SWF_E, SWF_FIELDS };
 
 // grid nlist, 256 threads
@@ -239,7 +250,7 @@ __global__ void __launch_bounds__(256) k_sweep_tab(const Task *tasks, const int 
         put(SWF_B, f[3]);
         const int xa = max(max(fexpo(f[0].x), fexpo(f[0].z)), max(fexpo(f[1].x), fexpo(f[1].z))) + ea; // not finite: 128
         const int xb = max(max(fexpo(f[2].x), fexpo(f[2].z)), max(fexpo(f[3].x), fexpo(f[3].z))) + eb;
-        put(SWF_E, make_float4(__int_as_float(ea), __int_as_float(eb), __int_as_float(max(xa, xb)), 0.0f));
+        put(SWF_E, make_float4(__int_as_float(ea), __int_as_float(eb), __int_as_float(max(xa, xb)), __int_as_float(kw)));
         auto seeds = [&](int kind, int y, int wi) {
             ff v[2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
             if (y >= c && wi >= 0)
@@ -252,23 +263,24 @@ __global__ void __launch_bounds__(256) k_sweep_tab(const Task *tasks, const int 
     }
 }
 
-// T(r, y), y <= r, of listed task b at tt[((b * 2 + pol) * L + r) * L + y].  Grid nlist * 2: one polarisation (TE, TM) per CTA,
-// the ring of three rows in shared memory (r and the two before it), one barrier per row; a thread keeps the coefficients of its first
+// T(r, y), y <= r, of listed task b at tt[((b * 2 + pol) * L + r) * L + y].  Grid nlist * P * 2: a part of the rows and one
+// polarisation (TE, TM) per CTA, the ring of three rows in shared memory (r and the two before it), one barrier per row; a thread keeps the coefficients of its first
 // columns in registers and the next row's seeds and factors are loaded a row ahead, so that the row's chain
 // is two float-float sums and the barrier.  Bound by that chain and by issue (about 95 instructions per column).
 constexpr int RF_NT = 256, RF_RING = 3, RF_KEEP = 4;
-__global__ void __launch_bounds__(RF_NT) k_rec_ff(const Task *tasks, const int *tlist, int nlist, int ldim, const float4 *__restrict__ tab, float2 *tt,
+__global__ void __launch_bounds__(RF_NT) k_rec_ff(const Task *tasks, const int *tlist, int nlist, int ldim, int P, const ffe *__restrict__ rows,
+                                                  const float4 *__restrict__ tab, float2 *tt,
                                                   const int *status)
 {
     extern __shared__ __align__(16) float2 rf_sm[];
     const int L = ldim + 2;
-    const int pol = blockIdx.x & 1, b = blockIdx.x >> 1, tid = threadIdx.x;
+    const int pol = blockIdx.x & 1, part = blockIdx.x >> 1, b = part / P, q = part % P, tid = threadIdx.x;
     if (b >= nlist) return;
     const int task = tlist ? tlist[b] : b;
     if (status[task] & ~0xF) return; // no status changes in this launch: uniform
-    const int c = seed_col(tasks[task]);
+    const int c = seed_col(tasks[task]), r0 = recf_row(q, P, L) + 1, r1 = recf_row(q + 1, P, L);
     const float4 *W = tab + (size_t)b * SWF_FIELDS * L;
-    float2 *t = tt + ((size_t)b * 2 + pol) * L * L;
+    float2 *t = tt + (((size_t)b * 2 + pol) * L + r0) * L;
     __shared__ float4 s_r[2];       // of the next row: R1, -R2
     __shared__ float2 s_seed[2][3]; // and its seeds
     auto fetch = [&](int row) {
@@ -281,11 +293,21 @@ __global__ void __launch_bounds__(RF_NT) k_rec_ff(const Task *tasks, const int *
     float4 keep[RF_KEEP];
 #pragma unroll
     for (int i = 0; i < RF_KEEP; i++) keep[i] = tid + i * RF_NT < L ? __ldg(W + (size_t)SWF_C * L + tid + i * RF_NT) : make_float4(0, 0, 0, 0);
-    fetch(0);
+    fetch(r0);
     // rows r, r - 1, r - 2; rows before the first are never read: y >= c + 1 and y <= r - 2 need r >= 3
     float2 *D = rf_sm, *P1 = rf_sm + L, *P2 = rf_sm + 2 * L;
+    if (q > 0) // the two rows before the part, from their q-sums
+        for (int i = 0; i < 2; i++) {
+            const int rr = r0 - 2 + i;
+            const ffe *src = rows + ((((size_t)b * (P - 1) + q - 1) * 2 + i) * 2 + pol) * L;
+            const int kr = __float_as_int(__ldg(W + (size_t)SWF_E * L + rr).w);
+            for (int y = tid; y <= rr; y += RF_NT) {
+                const ff v = y < c ? ff{0.0f, 0.0f} : sw_seed(src[y], kr + __float_as_int(__ldg(W + (size_t)SWF_E * L + y).w));
+                (i ? P1 : P2)[y] = make_float2(v.h, v.l);
+            }
+        }
     __syncthreads();
-    for (int r = 0; r < L; r++) {
+    for (int r = r0; r <= r1; r++) {
         fetch(r + 1);
         const float4 R = s_r[r & 1];
         const float2 *seeds = s_seed[r & 1];
@@ -457,28 +479,34 @@ size_t seed_bytes(int ldim, int ntask) { return (size_t)ntask * 2 * SEED_KINDS *
 
 static size_t sweep_smem_bytes(int ldim) { return (size_t)RF_RING * (ldim + 2) * sizeof(float2); }
 
-// windows up to this take the recurrence, larger ones the q-sums of every pair.  The line is that of the tested range
-// (the recurrence has been compared over 1000 rows from its seeds); the ring would fit up to 7000.
-constexpr int SWEEP_MAX = 2230;
+// windows up to this take the recurrence (its ring of rows fits in shared memory), larger ones the q-sums of every pair
+constexpr int SWEEP_MAX = 7000;
 bool sweep_fits(int ldim) { return ldim <= SWEEP_MAX; }
 int sweep_nsum(int ldim) { return ((ldim + EL_X - 1) / EL_X) * ((ldim + EL_Y - 1) / EL_Y); }
 size_t sweep_work_bytes(int ldim, int nlist)
 {
     const size_t L = ldim + 2;
-    return (size_t)nlist * L * (SWF_FIELDS * sizeof(float4) + 2 * L * sizeof(float2));
+    return (size_t)nlist * L * (SWF_FIELDS * sizeof(float4) + 2 * L * sizeof(float2) + (recf_parts(ldim) - 1) * 4 * sizeof(ffe));
+}
+static ffe *sweep_rows(void *work, int ldim, int nlist)
+{
+    const size_t L = ldim + 2;
+    return (ffe *)((char *)work + (size_t)nlist * L * (SWF_FIELDS * sizeof(float4) + 2 * L * sizeof(float2)));
 }
 
 void launch_seed_ff(const Task *tasks, const int *tlist, const int4 *groups, int ngroups, int ldim, const float4 *KP, const int *KPe,
                     int nu_stride, const float4 *ptabf, int pstride, const void *a12t, int ngroup_all, void *seed, bool band,
-                    int *status, cudaStream_t st)
+                    void *work, int nlist, int *status, cudaStream_t st)
 {
     if (ngroups <= 0) return;
     const int L = ldim + 2;
     const A12L *tl = (const A12L *)a12t;
     const A12J *tj = (const A12J *)((const char *)a12t + (size_t)L * ngroup_all * sizeof(A12L));
-    dim3 g(2 * ((L + 127) / 128), ngroups);
+    const int P = band ? 1 : recf_parts(ldim);
+    dim3 g(2 * P * ((L + 127) / 128), ngroups);
     k_seed_ff<3><<<g, 128, 0, st>>>(tasks, tlist, groups, ngroups, ldim, KP, KPe, nu_stride, ptabf, pstride, tl, tj,
-                                    band ? SEED_D0 : SEED_D1, band ? SEED_D2 : SEED_COL, (ffe *)seed, status, QSUM_FF_STOP_BITS);
+                                    band ? SEED_D0 : SEED_D1, band ? SEED_D2 : SEED_COL, (ffe *)seed, P, P > 1 ? sweep_rows(work, ldim, nlist) : nullptr,
+                                    status, QSUM_FF_STOP_BITS);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }
@@ -496,7 +524,8 @@ void launch_sweep_ff(const Task *tasks, const int *tlist, int nlist, int ldim, c
     float4 *tab = (float4 *)work;
     float2 *tt = (float2 *)(tab + nlist * SWF_FIELDS * L);
     k_sweep_tab<<<nlist, 256, 0, st>>>(tasks, tlist, nlist, ldim, (const ffe *)seed, (const ffe *)Saf, (const ffe *)Sbf, tab);
-    k_rec_ff<<<nlist * 2, RF_NT, smem, st>>>(tasks, tlist, nlist, ldim, tab, tt, status);
+    const int P = recf_parts(ldim);
+    k_rec_ff<<<nlist * P * 2, RF_NT, smem, st>>>(tasks, tlist, nlist, ldim, P, sweep_rows(work, ldim, nlist), tab, tt, status);
     const dim3 g((ldim + EL_X - 1) / EL_X, (ldim + EL_Y - 1) / EL_Y, nlist);
     if (sums) k_elem_sweep<true><<<g, EL_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, S, sstride, sums, status);
     else k_elem_sweep<false><<<g, EL_X, 0, st>>>(tasks, tlist, nlist, ldim, tt, tab, S, sstride, nullptr, status);
