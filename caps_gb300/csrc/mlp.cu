@@ -39,7 +39,7 @@ static_assert(SH1 % 4 == 0 && SX % 4 == 0, "vector loads of four samples");
 
 // forward (and optionally backward) of the samples [blockIdx.x*per, ...); y == nullptr: inference only.
 // Bound by latency (2600 samples: 163 CTAs of one batch): one sample after the other with a thread per neuron took
-// 150 us, 16 at once take 24 (loss, gradient and prediction of 2600 samples, copies included: 0.378 -> 0.121 ms).
+// 150 us, 16 at once take 24 (loss, gradient and prediction of 2600 samples, copies included: 0.378 -> 0.095 ms).
 __global__ void __launch_bounds__(MLP_NT) k_mlp_fwdbwd(const float *__restrict__ P, const float *__restrict__ X, const float *__restrict__ Y,
                                                        int n, int per, float *out, float *gpart, float *lpart)
 {
@@ -261,7 +261,8 @@ using namespace capsgpu;
 
 struct caps_mlp {
     float *P = nullptr, *G = nullptr, *M1 = nullptr, *M2 = nullptr, *loss = nullptr;
-    float *X = nullptr, *Y = nullptr, *out = nullptr, *gpart = nullptr, *lpart = nullptr;
+    float *X = nullptr, *Y = nullptr, *out = nullptr, *gpart = nullptr, *lpart = nullptr; // Y behind X
+    float *host = nullptr; // pinned: samples on the way in, gradient and loss or predictions on the way out
     size_t cap = 0, blk_cap = 0;
     int t = 0;
 };
@@ -269,13 +270,32 @@ struct caps_mlp {
 static void mlp_reserve(caps_mlp_t *m, size_t n)
 {
     if (n > m->cap) {
-        if (m->X) { CK(cudaFree(m->X)); CK(cudaFree(m->Y)); CK(cudaFree(m->out)); }
-        m->cap = std::max(n, (size_t)1024);
-        CK(cudaMalloc(&m->X, m->cap * NIN * sizeof(float)));
-        CK(cudaMalloc(&m->Y, m->cap * sizeof(float)));
+        if (m->X) { CK(cudaFree(m->X)); CK(cudaFree(m->out)); CK(cudaFreeHost(m->host)); }
+        m->cap = std::max(n, (size_t)2048);
+        CK(cudaMalloc(&m->X, m->cap * (NIN + 1) * sizeof(float)));
         CK(cudaMalloc(&m->out, m->cap * sizeof(float)));
+        CK(cudaMallocHost(&m->host, m->cap * (NIN + 1) * sizeof(float)));
     }
 }
+
+// n samples and (y != nullptr) their values to the device, by one copy from pinned memory: six pageable copies, each
+// with a synchronisation, were half of the time of a loss, gradient and prediction of 2600 samples (121 us; 95 so)
+static void mlp_upload(caps_mlp_t *m, const float *X, const float *y, int n)
+{
+    mlp_reserve(m, n);
+    const size_t nx = (size_t)n * NIN, ny = y ? n : 0;
+    std::copy(X, X + nx, m->host);
+    if (y) std::copy(y, y + n, m->host + nx);
+    m->Y = m->X + nx;
+    CK(cudaMemcpyAsync(m->X, m->host, (nx + ny) * sizeof(float), cudaMemcpyHostToDevice, 0));
+}
+// count floats back through pinned memory; returns when they are there
+static void mlp_download(caps_mlp_t *m, const float *src, size_t count)
+{
+    CK(cudaMemcpyAsync(m->host, src, count * sizeof(float), cudaMemcpyDeviceToHost, 0));
+    CK(cudaStreamSynchronize(0));
+}
+static_assert(NPARAM + 1 <= 2048 * (NIN + 1), "gradient and loss fit the pinned buffer");
 
 static int mlp_blocks(int n, int *per)
 {
@@ -313,10 +333,10 @@ extern "C" caps_mlp_t *caps_mlp_create(unsigned seed)
     init(OFF_W3, HN, HN * HN);
     init(OFF_W4, HN, HN);
     CK(cudaMalloc(&m->P, NPARAM * sizeof(float)));
-    CK(cudaMalloc(&m->G, NPARAM * sizeof(float)));
+    CK(cudaMalloc(&m->G, (NPARAM + 1) * sizeof(float))); // the loss behind it
+    m->loss = m->G + NPARAM;
     CK(cudaMalloc(&m->M1, NPARAM * sizeof(float)));
     CK(cudaMalloc(&m->M2, NPARAM * sizeof(float)));
-    CK(cudaMalloc(&m->loss, sizeof(float)));
     CK(cudaMemcpy(m->P, p.data(), NPARAM * sizeof(float), cudaMemcpyHostToDevice));
     CK(cudaMemset(m->M1, 0, NPARAM * sizeof(float)));
     CK(cudaMemset(m->M2, 0, NPARAM * sizeof(float)));
@@ -331,45 +351,33 @@ extern "C" caps_mlp_t *caps_mlp_create(unsigned seed)
 extern "C" void caps_mlp_free(caps_mlp_t *m)
 {
     if (!m) return;
-    for (float *p : {m->P, m->G, m->M1, m->M2, m->loss, m->X, m->Y, m->out, m->gpart, m->lpart})
+    for (float *p : {m->P, m->G, m->M1, m->M2, m->X, m->out, m->gpart, m->lpart})
         if (p) CK(cudaFree(p));
+    if (m->host) CK(cudaFreeHost(m->host));
     delete m;
 }
 
 extern "C" void caps_mlp_get_params(caps_mlp_t *m, float *out) { CK(cudaMemcpy(out, m->P, NPARAM * sizeof(float), cudaMemcpyDeviceToHost)); }
 extern "C" void caps_mlp_set_params(caps_mlp_t *m, const float *in) { CK(cudaMemcpy(m->P, in, NPARAM * sizeof(float), cudaMemcpyHostToDevice)); }
 
-static double mlp_fwdbwd(caps_mlp_t *m, int n)
+extern "C" double caps_mlp_loss_grad(caps_mlp_t *m, const float *X, const float *y, int n, float *grad)
 {
+    mlp_upload(m, X, y, n);
     int per;
     const int nblk = mlp_blocks(n, &per);
     mlp_reserve_blocks(m, nblk);
     k_mlp_fwdbwd<<<nblk, MLP_NT, MLP_SMEM>>>(m->P, m->X, m->Y, n, per, nullptr, m->gpart, m->lpart);
-    COUNT_LAUNCH(1);
     k_mlp_reduce<<<MLP_RED_GRID, 256>>>(m->gpart, m->lpart, nblk, m->G, m->loss, n);
-    COUNT_LAUNCH(1);
+    COUNT_LAUNCH(2);
     CK(cudaGetLastError());
-    float l;
-    CK(cudaMemcpy(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
-    return l;
-}
-
-extern "C" double caps_mlp_loss_grad(caps_mlp_t *m, const float *X, const float *y, int n, float *grad)
-{
-    mlp_reserve(m, n);
-    CK(cudaMemcpy(m->X, X, (size_t)n * NIN * sizeof(float), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(m->Y, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice));
-    const double l = mlp_fwdbwd(m, n);
-    if (grad) CK(cudaMemcpy(grad, m->G, NPARAM * sizeof(float), cudaMemcpyDeviceToHost));
-    return l;
+    mlp_download(m, m->G, NPARAM + 1);
+    if (grad) std::copy(m->host, m->host + NPARAM, grad);
+    return m->host[NPARAM];
 }
 
 extern "C" double caps_mlp_train(caps_mlp_t *m, const float *X, const float *y, int n, int epochs, float lr)
 {
-    mlp_reserve(m, n);
-    CK(cudaMemcpy(m->X, X, (size_t)n * NIN * sizeof(float), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(m->Y, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice));
-    double l = 0;
+    mlp_upload(m, X, y, n);
     int per;
     const int nblk = mlp_blocks(n, &per);
     mlp_reserve_blocks(m, nblk);
@@ -382,23 +390,21 @@ extern "C" double caps_mlp_train(caps_mlp_t *m, const float *X, const float *y, 
         COUNT_LAUNCH(3);
     }
     CK(cudaGetLastError());
-    float lf;
-    CK(cudaMemcpy(&lf, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
-    l = lf;
-    return l;
+    mlp_download(m, m->loss, 1);
+    return epochs > 0 ? m->host[0] : 0.0;
 }
 
 extern "C" void caps_mlp_predict(caps_mlp_t *m, const float *X, int n, float *y)
 {
     if (n <= 0) return;
-    mlp_reserve(m, n);
-    CK(cudaMemcpy(m->X, X, (size_t)n * NIN * sizeof(float), cudaMemcpyHostToDevice));
+    mlp_upload(m, X, nullptr, n);
     int per;
     const int nblk = mlp_blocks(n, &per);
     k_mlp_fwdbwd<<<nblk, MLP_NT, MLP_SMEM>>>(m->P, m->X, nullptr, n, per, m->out, nullptr, nullptr);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
-    CK(cudaMemcpy(y, m->out, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost));
+    mlp_download(m, m->out, n);
+    std::copy(m->host, m->host + n, y);
 }
 
 // features of one (geometry, material, xi_, m): the normalisation the network is trained with.
