@@ -502,10 +502,7 @@ __global__ void k_a12_mix(const int *group_m, const int *group_lmin, const int *
     tab[(size_t)g * npair + pid] = r;
 }
 
-// grid (ceil(npair/128), nlist) or, for the band, (ceil(2L/128), nlist); block row y handles
-// task tlist[y] (tlist == nullptr: task y).  BAND computes only the pairs that the
-// diagonal of M reads (l1 - l2 in {0, 2}), each with the sum the full kernel forms.
-template <bool BAND>
+// grid (ceil(npair/128), nlist); block row y handles task tlist[y] (tlist == nullptr: task y)
 __global__ void __launch_bounds__(128) k_itab(const Task *tasks, const int *tlist, int nlist, int ldim, const sd *K, int nu_stride,
                                               const double *__restrict__ lft, const double2 *__restrict__ xtab,
                                               const double4 *__restrict__ ptab, int pstride, sd *I, int *status,
@@ -516,24 +513,13 @@ __global__ void __launch_bounds__(128) k_itab(const Task *tasks, const int *tlis
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if ((int)blockIdx.y >= nlist) return;
     const int task = tlist ? tlist[blockIdx.y] : (int)blockIdx.y;
-    long long pid;
-    int a1, a2;
-    if (BAND) {
-        // thread 2 a2 + d owns the pair (a2 + 2 d, a2)
-        if (tid >= 2LL * L) return;
-        a2 = (int)(tid >> 1);
-        a1 = a2 + 2 * (int)(tid & 1);
-        if (a1 >= L) return;
-        pid = (long long)a1 * (a1 + 1) / 2 + a2;
-    } else {
-        if (tid >= npair) return;
-        pid = tid;
-        // pair index -> (a1 >= a2)
-        a1 = (int)((sqrt(8.0 * (double)pid + 1.0) - 1.0) * 0.5);
-        while ((long long)(a1 + 1) * (a1 + 2) / 2 <= pid) a1++;
-        while ((long long)a1 * (a1 + 1) / 2 > pid) a1--;
-        a2 = (int)(pid - (long long)a1 * (a1 + 1) / 2);
-    }
+    if (tid >= npair) return;
+    const long long pid = tid;
+    // pair index -> (a1 >= a2)
+    int a1 = (int)((sqrt(8.0 * (double)pid + 1.0) - 1.0) * 0.5);
+    while ((long long)(a1 + 1) * (a1 + 2) / 2 <= pid) a1++;
+    while ((long long)a1 * (a1 + 1) / 2 > pid) a1--;
+    const int a2 = (int)(pid - (long long)a1 * (a1 + 1) / 2);
 
     const Task &T = tasks[task];
     const int l1 = T.lmin - 1 + a1, l2 = T.lmin - 1 + a2;
@@ -569,16 +555,13 @@ __global__ void k_tables(const double *lfac_tab, double *lft, int nlf, double2 *
 
 // A = 1 - M (lower triangle); mdiag receives M_ii itself, so that the trace keeps its
 // relative precision when M_ii is far below the unit diagonal of A.  Grid (ceil(ldim/128),
-// ldim, nlist), block z on task tlist[z] (tlist == nullptr: task z).  DIAG: grid
-// (ceil(ldim/128), 1, nlist), M_ii alone into mdiag (A untouched), from the band of I
-// values that k_itab<true> leaves; the same arithmetic as the full assembly.
-template <bool DIAG>
+// ldim, nlist), block z on task tlist[z] (tlist == nullptr: task z).
 __global__ void k_elem(const Task *tasks, const int *tlist, int nlist, int ldim, const sd *I, const sd *Sa, const sd *Sb,
                        const double2 *uv, double *A, size_t lda, size_t mat_stride, double *mdiag, int *status)
 {
     const int L = ldim + 2;
     const int a = blockIdx.x * blockDim.x + threadIdx.x; // row block
-    const int b = DIAG ? a : (int)blockIdx.y;           // column block
+    const int b = blockIdx.y;                            // column block
     if (a >= ldim || b > a || (int)blockIdx.z >= nlist) return;
     const int task = tlist ? tlist[blockIdx.z] : (int)blockIdx.z;
     const Task &T = tasks[task];
@@ -592,14 +575,7 @@ __global__ void k_elem(const Task *tasks, const int *tlist, int nlist, int ldim,
     // (consecutive x) read consecutive entries
     auto Iv = [&](int p, int x, int y) { return (p ? ITM : ITE)[(size_t)y * L + x]; };
     sd EE, MM, EM, ME;
-    elem_block<DIAG>(T.m, i1, i2, sa1, sa2, sb1, sb2, uv1, uv2, Iv, EE, MM, EM, ME);
-    if (DIAG) {
-        const double ee = sd_to_double(EE), mm = sd_to_double(MM);
-        if (!isfinite(ee) || !isfinite(mm)) atomicOr(status + task, ST_ERR_NONFINITE);
-        mdiag[(size_t)task * 2 * ldim + 2 * a] = ee;
-        mdiag[(size_t)task * 2 * ldim + 2 * a + 1] = mm;
-        return;
-    }
+    elem_block<false>(T.m, i1, i2, sa1, sa2, sb1, sb2, uv1, uv2, Iv, EE, MM, EM, ME);
     double *Am = A + (size_t)task * mat_stride;
     const int r0 = 2 * a, c0 = 2 * b;
     const double ee = sd_to_double(EE), mm = sd_to_double(MM), me = sd_to_double(ME), em = sd_to_double(EM);
@@ -856,33 +832,22 @@ void launch_ptab(const Task *tasks, int ntask, double4 *ptab, int pstride, cudaS
 }
 
 void launch_itab(const Task *tasks, const int *tlist, int nlist, int ldim, const sd *K, int nu_stride, const double *lft,
-                 const double2 *xtab, const double4 *ptab, int pstride, sd *I, int *status, cudaStream_t st, const void *a12,
-                 bool band)
+                 const double2 *xtab, const double4 *ptab, int pstride, sd *I, int *status, cudaStream_t st, const void *a12)
 {
     if (nlist <= 0) return;
     const long long L = ldim + 2, npair = L * (L + 1) / 2;
-    dim3 g((unsigned)(((band ? 2 * L : npair) + 127) / 128), nlist);
-    if (band)
-        k_itab<true><<<g, 128, 0, st>>>(tasks, tlist, nlist, ldim, K, nu_stride, lft, xtab, ptab, pstride, I, status,
-                                        (const A012 *)a12);
-    else
-        k_itab<false><<<g, 128, 0, st>>>(tasks, tlist, nlist, ldim, K, nu_stride, lft, xtab, ptab, pstride, I, status,
-                                         (const A012 *)a12);
+    dim3 g((unsigned)((npair + 127) / 128), nlist);
+    k_itab<<<g, 128, 0, st>>>(tasks, tlist, nlist, ldim, K, nu_stride, lft, xtab, ptab, pstride, I, status, (const A012 *)a12);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }
 
 void launch_elem(const Task *tasks, const int *tlist, int nlist, int ldim, const sd *I, const sd *Sa, const sd *Sb, const double2 *uv,
-                 double *A, size_t lda, size_t mat_stride, double *mdiag, int *status, cudaStream_t st, bool diag_only)
+                 double *A, size_t lda, size_t mat_stride, double *mdiag, int *status, cudaStream_t st)
 {
     if (nlist <= 0) return;
-    if (diag_only) {
-        dim3 g((ldim + 127) / 128, 1, nlist);
-        k_elem<true><<<g, 128, 0, st>>>(tasks, tlist, nlist, ldim, I, Sa, Sb, uv, A, lda, mat_stride, mdiag, status);
-    } else {
-        dim3 g((ldim + 127) / 128, ldim, nlist);
-        k_elem<false><<<g, 128, 0, st>>>(tasks, tlist, nlist, ldim, I, Sa, Sb, uv, A, lda, mat_stride, mdiag, status);
-    }
+    dim3 g((ldim + 127) / 128, ldim, nlist);
+    k_elem<<<g, 128, 0, st>>>(tasks, tlist, nlist, ldim, I, Sa, Sb, uv, A, lda, mat_stride, mdiag, status);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }

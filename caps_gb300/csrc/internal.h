@@ -50,12 +50,11 @@ void launch_kred_ff(const Task *tasks, int ntask, int max_nnu, const float2 *par
                     float4 *KP, int *KPe, int *status, cudaStream_t st);
 void launch_tables(const double *lfac_tab, double *lft, int nlf, double2 *xtab, int nx, cudaStream_t st);
 struct ffe;
-// FP64 q-sums of the listed tasks (tlist, nlist; tlist == nullptr: tasks 0..nlist-1); band:
-// only the pairs the diagonal reads.  The p tables come first (launch_ptab).
+// FP64 q-sums of the listed tasks (tlist, nlist; tlist == nullptr: tasks 0..nlist-1).  The p tables come first
+// (launch_ptab).
 void launch_ptab(const Task *tasks, int ntask, double4 *ptab, int pstride, cudaStream_t st);
 void launch_itab(const Task *tasks, const int *tlist, int nlist, int ldim, const sd *K, int nu_stride, const double *lft,
-                 const double2 *xtab, const double4 *ptab, int pstride, sd *I, int *status, cudaStream_t st, const void *a12,
-                 bool band);
+                 const double2 *xtab, const double4 *ptab, int pstride, sd *I, int *status, cudaStream_t st, const void *a12);
 // float-float q recurrence tables once per distinct m (group_m), row g per group
 void launch_ptab_groups(const int *group_m, int ngroup, float4 *ptabf, int pstride, cudaStream_t st);
 // mixed form: q-sums of every pair with one a_q recurrence per (pair, subgroup of same-m tasks)
@@ -82,9 +81,9 @@ size_t a12_tab_bytes(int ldim, int ngroup);
 // 0..nlist-1, nlist < 0: all)
 void launch_a12_mixed(const int *group_m, const int *group_lmin, int ngroup, int ldim, const double *lft, void *tab, void *work,
                       cudaStream_t st, bool tabs = true, const int *glist = nullptr, int nlist = -1);
-// elements of the listed tasks into A = 1 - M and M_ii; diag_only: M_ii alone (from the band)
+// elements of the listed tasks into A = 1 - M and M_ii
 void launch_elem(const Task *tasks, const int *tlist, int nlist, int ldim, const sd *I, const sd *Sa, const sd *Sb, const double2 *uv,
-                 double *A, size_t lda, size_t mat_stride, double *mdiag, int *status, cudaStream_t st, bool diag_only);
+                 double *A, size_t lda, size_t mat_stride, double *mdiag, int *status, cudaStream_t st);
 // shortcut decision of the listed tasks; A == nullptr: the trace rule alone, undecided tasks keep status 0
 void launch_stats(const int *tlist, int nlist, int n, const double *A, size_t lda, size_t mat_stride, const double *mdiag, int mode,
                   double *trace, double *result, int *status, cudaStream_t st, const double *fro = nullptr, int nfro = 0);

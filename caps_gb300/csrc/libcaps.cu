@@ -650,7 +650,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         // diagonal first, as kernel_logdet does (matrix.c:62-82): the band of the q-sums that
         // M_ii reads, M_ii, and the rule.  Only the matrices it leaves undecided are summed
         // and assembled in full.
-        const bool diag_first = O.factor && !O.square && !O.M_out && (ff_elem || caps->precision != CAPS_PREC_MIXED);
+        const bool diag_first = ff_elem; // mixed form, dense
         auto undecided = [&]() {
             std::vector<int> hs(nt);
             d2h(hs.data(), d_status, nt * sizeof(int), st);
@@ -748,17 +748,9 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             CK(cudaEventRecord(g_eng.ev[5], st));
         } else {
             launch_ptab(d_tasks, nt, d_ptab, pstride, st);
-            if (diag_first) {
-                launch_itab(d_tasks, nullptr, nt, ldim, d_K, nu_stride, d_lft, d_xtab, d_ptab, pstride, d_I, d_status, st, d_a12, true);
-                CK(cudaEventRecord(g_eng.ev[3], st));
-                launch_elem(d_tasks, nullptr, nt, ldim, d_I, d_Sa, d_Sb, d_uv, nullptr, lda, mstride, d_dg, d_status, st, true);
-                launch_stats(nullptr, nt, dim, nullptr, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st);
-                CK(cudaEventRecord(g_eng.ev[4], st));
-                undecided();
-                CK(cudaEventRecord(g_eng.ev[5], st));
-            } else
-                for (int k = 3; k <= 5; k++) CK(cudaEventRecord(g_eng.ev[k], st));
-            launch_itab(d_tasks, d_list, nlist, ldim, d_K, nu_stride, d_lft, d_xtab, d_ptab, pstride, d_I, d_status, st, d_a12, false);
+            // M itself is wanted
+            for (int k = 3; k <= 5; k++) CK(cudaEventRecord(g_eng.ev[k], st));
+            launch_itab(d_tasks, nullptr, nt, ldim, d_K, nu_stride, d_lft, d_xtab, d_ptab, pstride, d_I, d_status, st, d_a12);
         }
         CK(cudaEventRecord(g_eng.ev[6], st));
 
@@ -802,7 +794,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             else launch_stats(d_list, nlist, dim, d_A, lda, mstride, d_dg, O.mode, d_trace, d_res, d_status, st, d_fro, nfro);
         } else {
             d_A = (double *)g_eng.A.get((size_t)nt * mstride * sizeof(double));
-            launch_elem(d_tasks, d_list, nlist, ldim, d_I, d_Sa, d_Sb, d_uv, d_A, lda, mstride, d_dg, d_status, st, false);
+            launch_elem(d_tasks, d_list, nlist, ldim, d_I, d_Sa, d_Sb, d_uv, d_A, lda, mstride, d_dg, d_status, st);
             if (O.square) {
                 double *d_norm = (double *)g_eng.fro.get((size_t)nt * square_nsum(dim) * sizeof(double));
                 launch_square_norm(nt, dim, d_A, lda, mstride, d_dg, d_status, d_norm, st);

@@ -50,7 +50,6 @@
 #include "ff.cuh"
 #include "internal.h"
 #include "qsum_ff.cuh"
-#include "umma.cuh"
 
 namespace capsgpu {
 

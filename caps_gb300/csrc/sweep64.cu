@@ -19,7 +19,6 @@
 #include "fix.cuh"
 #include "internal.h"
 #include "qsum64.cuh"
-#include "umma.cuh"
 
 namespace capsgpu {
 
@@ -87,7 +86,7 @@ __global__ void __launch_bounds__(SEED_NT) k_seed64(const Task *tasks, const int
     *oE = rE;
 }
 
-// M_ii alone, from the band seeds (the arithmetic of k_elem<true>); grid (ceil(ldim / 128), ntask)
+// M_ii alone, from the band seeds (the arithmetic of the full assembly); grid (ceil(ldim / 128), ntask)
 __global__ void k_diag64(const Task *tasks, int ntask, int ldim, const sd *__restrict__ seed, const sd *Sa, const sd *Sb, const double2 *uv,
                          double *mdiag, int *status)
 {
