@@ -342,7 +342,7 @@ double caps_gpu_fp32_peak(void);
  * fragment the pool).  No counterpart in the reference.  All scratch lives in
  * one fixed 32 MiB file-scope device array (held on every GPU that loads the
  * library until exit); no cudaMalloc/cudaFree or allocating library call is made.
- * Limits: ldim <= 512, lmin+ldim <= 2048, <= 256 K-quadrature panels; larger
+ * Limits: ldim <= 512, lmin+ldim <= 2048, <= 4096 K-quadrature nodes; larger
  * cases return a negative code with a message (caps_noalloc_last_error(), per
  * host thread).  The first call on a device resolves the array's address
  * (cudaGetSymbolAddress) and uploads constant tables: make it before any stream

@@ -72,3 +72,15 @@ def test_elements_that_round_to_zero(ldim, metal):
     both = (out[0][1] == 3) & (out[1][1] == 3)
     assert both.sum() >= 2
     assert (out[0][0][both] == out[1][0][both]).all()
+
+
+def test_ring_beyond_shared_memory():
+    """one row of one polarisation no longer fits shared memory four times: against HODLR as above"""
+    import caps_gb300 as cg
+    c = cg.Caps(900e-6, 1e-6, ldim=7100)
+    c.set_drude(9.0, 0.0)
+    c.set_path(cg.PATH_DENSE)
+    dense = c.logdetD(900.0, 1)
+    c.set_path(cg.PATH_HODLR)
+    hodlr = c.logdetD(900.0, 1)
+    assert abs(dense - hodlr) <= 1e-10 * max(1.0, abs(hodlr)), (dense, hodlr)
