@@ -119,41 +119,49 @@ template <bool PR> CAPS_DEV void k_node(const Task &T, int j, const double *lfac
     WTE = f * rTE;
 }
 
-// one warp per CTA, so that a small batch's warps spread over the SMs and their FP64 pipes (24
-// matrices of dimension 2100: eight warps per CTA 1.54 ms, one 0.99)
+// An FP64 operation of a warp holds its scheduler's unit for 64 clocks, so a warp per 32 nodes takes 5 x 64 clocks per
+// degree however few warps there are.  Two warps share the 32 nodes: one runs the recurrence (3 operations) into
+// one buffer of 16 degrees while the other folds the buffer before (2: a polarisation per half warp).  One pair per
+// CTA, so that a small batch's pairs spread over the SMs (24 matrices of dimension 2100: eight warps per CTA 1.54 ms,
+// one 0.99, fewer nodes 0.50, two warps per 32 nodes 0.37; a T = 0 energy, which fills the SMs, 2.06 and 1.66),
+// and little shared memory, so that a large batch's CTAs and the Mie coefficients' beside them are all resident.
 constexpr int KT_WARPS = 1, KT_ALIGN = 16;
+constexpr int KT_BUF = KT_ALIGN * 33;                                               // doubles of a buffer
+static size_t ktab64_smem_bytes() { return (size_t)(2 * KT_BUF + 64) * sizeof(double); }
 
 template <bool PR>
-__global__ void __launch_bounds__(KT_WARPS * 32)
+__global__ void __launch_bounds__(64)
 k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lfac_tab, double *partM, int *partE, int max_warps)
 {
     extern __shared__ double smem[];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double *buf = smem + wib * (32 * 33);                    // [32][33]
-    double *wTM = smem + KT_WARPS * 32 * 33 + wib * 64;      // [32]
-    double *wTE = wTM + 32;                                  // [32]
-    int *rowE = (int *)(smem + KT_WARPS * (32 * 33 + 64)) + wib * 32;
+    __shared__ int bufE[2];
+    const int lane = threadIdx.x & 31;
+    const bool folds = threadIdx.x >= 32;
+    double *wTM = smem + 2 * KT_BUF, *wTE = wTM + 32; // [32]
 
     const int task = blockIdx.y;
     const Task T = tasks[task];
-    const int warp = blockIdx.x * KT_WARPS + wib;
+    const int warp = blockIdx.x;
     if (warp * 32 >= T.nnode) return;
     const bool valid = warp * 32 + lane < T.nnode;
-    double x = 1.0, WTM = 0.0, WTE = 0.0;
+    double x = 1.0;
     int E = -(1 << 29);
-    if (valid) k_node<PR>(T, warp * 32 + lane, lfac_tab, x, E, WTM, WTE);
-    wTM[lane] = WTM;
-    wTE[lane] = WTE;
-
+    if (!folds) {
+        double WTM = 0.0, WTE = 0.0;
+        if (valid) k_node<PR>(T, warp * 32 + lane, lfac_tab, x, E, WTM, WTE);
+        wTM[lane] = WTM;
+        wTE[lane] = WTE;
+    }
     double pp = 0.0, pc = valid ? 1.0 : 0.0;
     const int nnu = T.nu_max - T.mu + 1;
     const double2 *ab = coefAB + (size_t)T.mgroup * nu_stride;
     const size_t pTM = ((size_t)(task * 2 + 1) * max_warps + warp) * nu_stride;
     const size_t pTE = ((size_t)(task * 2 + 0) * max_warps + warp) * nu_stride;
 
-    for (int base = 0; base < nnu; base += 32) {
-        const int rows = min(32, nnu - base);
-        for (int half = 0; half < 32; half += KT_ALIGN) {
+    for (int base = 0; base < nnu + KT_ALIGN; base += KT_ALIGN) {
+        const int b = base / KT_ALIGN & 1;
+        if (!folds && base < nnu) {
+            double *buf = smem + b * KT_BUF;
             // the lane values aligned to the largest of the warp, for KT_ALIGN degrees at once: a value
             // grows by (A x)^16 < 2^900 meanwhile (x < 2^50), and one that starts 2^1000 below stays below
             const int ex = (int)((__double_as_longlong(pc) >> 52) & 0x7ff), k = ex ? ex - 1023 : 0;
@@ -162,36 +170,35 @@ k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lf
             E += k;
             const int emax = __reduce_max_sync(0xffffffffu, ex ? E : -(1 << 29));
             const int d = max(E - emax, -1023);
-            if (lane < KT_ALIGN) rowE[half + lane] = emax;
+            if (lane == 0) bufE[b] = emax;
 #pragma unroll
             for (int r = 0; r < KT_ALIGN; r++) {
-                if (half + r < rows) { // uniform
-                    buf[(half + r) * 33 + lane] = shift2(pc, d);
-                    const double2 c = __ldg(ab + base + half + r);
+                if (base + r < nnu) { // uniform
+                    buf[r * 33 + lane] = shift2(pc, d);
+                    const double2 c = __ldg(ab + base + r);
                     const double pn = fma(c.x * x, pc, -c.y * pp);
                     pp = pc;
                     pc = pn;
                 }
             }
         }
-        __syncwarp();
-        if (lane < rows) {
-            double sM[2] = {0.0, 0.0}, sE[2] = {0.0, 0.0}; // two chains each: the additions' latency
-            const double *row = buf + lane * 33;
+        const int row = base - KT_ALIGN + (lane & 15), upper = lane >> 4; // of the buffer before
+        if (folds && base > 0) {
+            // lanes 0..15 TM, 16..31 TE; a perfect reflector's TM alone: nodes 0..15 and 16..31
+            const double *v0 = smem + (b ^ 1) * KT_BUF + (lane & 15) * 33 + (PR ? upper * 16 : 0);
+            const double *w = PR ? wTM + upper * 16 : upper ? wTE : wTM;
+            double s[2] = {0.0, 0.0}; // two chains: the additions' latency
 #pragma unroll 8
-            for (int l = 0; l < 32; l++) {
-                const double v = row[l];
-                sM[l & 1] = fma(v, wTM[l], sM[l & 1]);
-                if (!PR) sE[l & 1] = fma(v, wTE[l], sE[l & 1]);
-            }
-            partM[pTM + base + lane] = sM[0] + sM[1];
-            partE[pTM + base + lane] = rowE[lane];
-            if (!PR) {
-                partM[pTE + base + lane] = sE[0] + sE[1];
-                partE[pTE + base + lane] = rowE[lane];
+            for (int l = 0; l < (PR ? 16 : 32); l++) s[l & 1] = fma(v0[l], w[l], s[l & 1]);
+            double sum = s[0] + s[1];
+            if (PR) sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+            if (row < nnu && (!PR || !upper)) {
+                const size_t o = upper ? pTE + row : pTM + row;
+                partM[o] = sum;
+                partE[o] = bufE[b ^ 1];
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -718,15 +725,15 @@ void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const dou
 {
     beside_ktab();
     static bool attr_set = false;
-    const size_t sm = ktab_smem_bytes();
+    const size_t sm = ktab64_smem_bytes();
     if (!attr_set) {
         CK(cudaFuncSetAttribute(k_ktab<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         CK(cudaFuncSetAttribute(k_ktab<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         attr_set = true;
     }
-    dim3 g((max_warps + KT_WARPS - 1) / KT_WARPS, ntask);
-    if (pr) k_ktab<true><<<g, KT_WARPS * 32, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
-    else k_ktab<false><<<g, KT_WARPS * 32, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
+    dim3 g(max_warps, ntask);
+    if (pr) k_ktab<true><<<g, 64, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
+    else k_ktab<false><<<g, 64, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }
