@@ -488,7 +488,9 @@ def main():
         "time_to_E_s": tte,
         "E": E, "E_reference": ref["E"] if ref else None, "E_rel_err": err,
         "phases_ms_per_step": {k: v / args.steps for k, v in zip(["setup_mie", "K", "I", "elements", "factor", "total"], ph)},
-        "roofline": ({"bound": "fp64", "kernel": "FP64 Cholesky (potf2+trsm+syrk), n^3/3 flops per factored matrix",
+        "roofline": ({"bound": "fp64", "kernel": "Cholesky of the FP64 form (64-bit fixed point, digit products on the tensor cores), "
+                                                      "n^3/3 flops per factored matrix against the FP64 pipe that it does without: a fraction "
+                                                      "above 1 is what FP64 arithmetic could not reach",
                       "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
                       "frac": achieved / fp64_peak if achieved else None,
                       "peak_source": "measured live: DFMA-chain probe kernel (caps_gpu_fp64_peak); MEASURED_PEAKS.json has no FP64 figure",
@@ -500,8 +502,8 @@ def main():
                                 "the whole trailing matrix (row-pair items sharing the column slice) and for the middle "
                                 "update of each panel (its first half onto the second half's 256 columns), k_syrk_blk for "
                                 "the left-looking block updates, all fed by bulk copies of the panel images that the panel "
-                                "solves write; algorithmic bytes = target block read + written once (FP32) and the panel "
-                                "rows read once (4 bytes per entry), per factored matrix",
+                                "solves write, over the items whose image blocks are not zero; algorithmic bytes = the tiles of "
+                                "S that those items read + write (FP32), counted by the kernels",
                       "achieved": syrk_gbs, "peak": hbm_peak, "unit": "GB/s",
                       "frac": syrk_gbs / hbm_peak if syrk_gbs else None,
                       "traffic": syrk_bytes / syrk_n * SYRK_DRAM_PER_ALGORITHMIC if syrk_n else None,
@@ -509,9 +511,9 @@ def main():
                       "launches": syrk_n, "avg_launch_ms": syrk_ms / syrk_n if syrk_n else None,
                       "algorithmic_bytes_per_launch": syrk_bytes / syrk_n if syrk_n else None,
                       "traffic_source": "DRAM bytes per algorithmic byte over all 32 update launches of the factorisation "
-                                        "of 24 matrices of this workload in one ncu capture (trailing updates 0.84, middle "
-                                        "updates 0.73, block updates 0.78: the images just written by the panel solves are "
-                                        "partly read from L2), times this run's algorithmic bytes per launch",
+                                        "of 24 matrices of this workload with every tile updated, in one ncu capture (trailing "
+                                        "updates 0.84, middle updates 0.73, block updates 0.78), times this run's algorithmic "
+                                        "bytes per launch",
                       "fp32_accurate_tflops_factorisation": achieved,
                       "panel_kernels": panel_kernels or None,
                       "panel_kernels_note": "the panel solve is bytes-bound like the update (its rate against the same peak); "
@@ -523,12 +525,12 @@ def main():
             "bound": "HBM for the trailing update; the panel solve streams the panel, the diagonal block is latency-bound",
             "evidence": "roofline and panel_kernels above; ncu captures of k_syrk_pair and k_syrk_blk on a 24-matrix case"},
         "assembly_kernel": None if args.precision == "fp64" else {
-            "kernel": "k_sweep_ff (I table by the three-term Legendre recurrence from 4L seed q-sums, fused with "
-                      "the elements, straight into the FP32 delta matrix)",
+            "kernel": "k_rec_ff and k_elem_sweep (I table by the three-term Legendre recurrence from 4L seed q-sums; "
+                      "elements from its tiles, straight into the FP32 delta matrix)",
             "phase_share_of_step": (ph[2] + ph[3]) / ph[5] if ph[5] else None,
-            "bound": "latency: float-float dependency chains (producer and consumer warps on mbarriers, 20 warps "
-                     "per SM); FP32 work, DRAM idle",
-            "evidence": "ncu capture of k_sweep_ff on 48 matrices of this workload"},
+            "bound": "issue and latency: the rows' chain of float-float sums and a barrier per row; 256 instructions per "
+                     "pair of the elements at 48 % issue",
+            "evidence": "ncu capture of both kernels on 40 matrices of this workload"},
         "cpu_baseline": cpu,
         "autotune": autotune,
         "learned_training": train_info,

@@ -401,7 +401,7 @@ __host__ __device__ inline size_t upd_list_entries(int ntask, int n, int ncta)
 }
 // k0: first column of the panel's part that is applied, t0: first column (and row) updated.  seg[i] = (item, bits of
 // its chunks); *count (zeroed before a barrier) of them in any order, complete after the next barrier.  bytes != nullptr:
-// the bytes of the listed work are added (S read and written, image slices read once per chunk)
+// the bytes of the listed tiles of S, read and written, are added (the images come from L2 mostly and are not counted)
 __device__ __forceinline__ void upd_fill(int kind, int ntask, int n, int k0, int t0, const int *status, const unsigned char *nz, int2 *seg, int *count,
                                          unsigned long long *bytes)
 {
@@ -430,8 +430,7 @@ __device__ __forceinline__ void upd_fill(int kind, int ntask, int n, int k0, int
         seg[atomicAdd(count, 1)] = make_int2(t, mask);
         if (bytes) {
             const int tiles = kind == UPD_BLOCK ? 1 : 2 * (T.rb >= 0 ? 2 : 1); // of 128 x 64
-            const int slices = kind == UPD_BLOCK ? 3 : 2 * (T.rb >= 0 ? 3 : 2); // of 64 rows
-            atomicAdd(bytes, tiles * UM_M * 64 * 8ULL + __popc(mask) * slices * 64 * 64 * 4ULL);
+            atomicAdd(bytes, tiles * UM_M * 64 * 8ULL);
         }
     }
 }
