@@ -13,20 +13,21 @@ constexpr int SY_G0 = 4;                     // accumulators of a first part, se
 constexpr int IMG_BLK = NB * NB * 2;         // bytes of one digit of one 64 x 64 block
 constexpr int FIX_WAIT_ITERS = 1 << 22;      // polls of a bounded mbarrier wait
 
-// per-task workspace: W image, X image (one digit after the other, a spare row block so that a
-// pair of row blocks can always be read), exponents
+// per-task workspace: W image, two X images (panels alternate; one digit after the other, a spare row block so
+// that a pair of row blocks can always be read), exponents
 __host__ __device__ inline int fix_nbk(int n) { return (n + NB - 1) / NB; }
 __host__ __device__ inline size_t fix_ximg_bytes(int n) { return (size_t)(fix_nbk(n) + 1) * ND * IMG_BLK; }
-__host__ __device__ inline size_t fix_task_bytes(int n) { return (size_t)ND * IMG_BLK + fix_ximg_bytes(n); }
+__host__ __device__ inline size_t fix_task_bytes(int n) { return (size_t)ND * IMG_BLK + 2 * fix_ximg_bytes(n); }
 struct FixInfo { int sexp, wexp; };          // A 2^-sexp is factored; W 2^-wexp is in the image
-// first[task * (nbk + 1) + block]: the first digit of the current panel's X that is not zero in the whole 64-row
+// first[task * (nbk + 1) + block] (one table per image): the first digit of the panel's X that is not zero in the whole 64-row
 // block (block counted below the diagonal block; NG: none)
 struct FixWork {
     unsigned char *img;
     FixInfo *info;
     int *first;
+    int par; // the image in use
     __host__ __device__ unsigned char *wimg(int task, int n) const { return img + (size_t)task * fix_task_bytes(n); }
-    __host__ __device__ unsigned char *ximg(int task, int n) const { return wimg(task, n) + (size_t)ND * IMG_BLK; }
+    __host__ __device__ unsigned char *ximg(int task, int n) const { return wimg(task, n) + (size_t)ND * IMG_BLK + par * fix_ximg_bytes(n); }
 };
 
 // byte offset of element (row, k) inside one digit of a 64-row block: the operand layout of
@@ -114,10 +115,12 @@ CAPS_DEV void split8(const long long (&x)[8], uint4 (&d)[ND])
 }
 
 // cholesky.cu: the parts of a workspace of cholesky_work_bytes; FP64 -> fixed point in place, with the exponents;
-// S -= X X^T over the rows and columns from t0 on, X the 64 columns in the image, first digits in wk.first
+// S -= X X^T over the rows and columns from t0 on, X the 64 columns in the image, first digits in wk.first; column
+// blocks j0 .. j1 - 1 of it
 FixWork fix_work(int ntask, int n, void *work);
 void fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, const int *status, const double *mdiag, const FixWork &wk,
                  cudaStream_t st);
-void fix_syrk(int ntask, int n, int t0, long long *S, size_t lda, size_t mstride, int *status, const FixWork &wk, cudaStream_t st);
+void fix_syrk(int ntask, int n, int t0, long long *S, size_t lda, size_t mstride, int *status, const FixWork &wk, cudaStream_t st,
+              int j0 = 0, int j1 = 1 << 30);
 
 } // namespace capsgpu

@@ -125,7 +125,12 @@ void launch_stats_ff(const int *tlist, int nlist, int ldim, const double *diag, 
 // (n per task); logdet: ceil(n / 64) partial sums per task; work: cholesky_work_bytes
 size_t cholesky_work_bytes(int ntask, int n);
 void launch_cholesky(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, double *logdet,
-                     void *work, cudaStream_t st, bool fixed = false);
+                     void *work, cudaStream_t st, bool fixed = false, const struct TwoStreams *two = nullptr);
+// a stream of high priority and events for work beside the caller's stream
+struct TwoStreams {
+    cudaStream_t stream;
+    cudaEvent_t ev[3];
+};
 // fixed: the matrix is in fixed point already (units 2^(sexp - 60), launch_sweep64), its exponents
 // written by launch_fix_scale: two ints per task at the start of the workspace, sexp the first
 void launch_fix_scale(const int *tlist, int nlist, int n, const double *mdiag, void *work, cudaStream_t st);

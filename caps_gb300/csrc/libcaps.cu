@@ -104,6 +104,7 @@ struct Engine {
     cudaStream_t own = nullptr, user = nullptr;
     cudaStream_t side = nullptr;          // Mie coefficients and scale factors, beside setup and K
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    TwoStreams two{};                     // diagonal blocks and panels of the FP64 form's Cholesky, beside its updates
     double *d_lfac = nullptr;
     DevBuf tasks, coef, partM, partE, K, I, Sa, Sb, uv, A, logdiag, trace, result, status, mie_a, mie_b, xi, eps, lft, xtab, ptab, S32, ptabf, a12, gm, glmin, Saf, Sbf, uvf, part, diag, groups, B, diag2, mwork, a12t, coefF, tlist, groups2, glist2, KP, KPe, hwork, seed, sw64, fro, fro2;
     std::vector<double> host_pinned_dummy;
@@ -141,6 +142,10 @@ static void engine_init()
     CK(cudaGetDevice(&g_eng.device));
     CK(cudaStreamCreateWithFlags(&g_eng.own, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&g_eng.side, cudaStreamNonBlocking));
+    int least = 0, greatest = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    CK(cudaStreamCreateWithPriority(&g_eng.two.stream, cudaStreamNonBlocking, greatest));
+    for (cudaEvent_t &e : g_eng.two.ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&g_eng.ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&g_eng.ev_join, cudaEventDisableTiming));
     std::call_once(g_tab_once, init_host_tables);
@@ -822,7 +827,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
         } else if (O.factor) {
             double *d_ld = (double *)g_eng.logdiag.get((size_t)nt * dim * sizeof(double));
             void *d_work = g_eng.mwork.get(cholesky_work_bytes(nt, dim));
-            launch_cholesky(nt, dim, d_A, lda, mstride, d_status, d_dg, d_ld, d_work, st, sweep64 || O.square);
+            launch_cholesky(nt, dim, d_A, lda, mstride, d_status, d_dg, d_ld, d_work, st, sweep64 || O.square, &g_eng.two);
             launch_final(nt, dim, d_ld, d_work, d_trace, d_status, d_res, O.mode, st);
         }
         CK(cudaEventRecord(g_eng.ev[8], st));

@@ -56,3 +56,22 @@ def test_small_entries(scale):
         tr = np.trace(M)
         want = -tr if tr < 1e-8 else np.linalg.slogdet(np.eye(2 * ldim) - M)[1]
         assert abs(v - want) <= 1e-10 * abs(want) + 3e-14, (xi, m, v, want)
+
+
+@pytest.mark.parametrize("ldim", [255, 256, 257, 288, 330])
+@pytest.mark.parametrize("count", [1, 3, 170])
+def test_updates_beside_panels(ldim, count):
+    """both sides of the dimension (512) from which the rest of an update runs beside the next panel, for few and for
+    many matrices, against LU of the oracle's M; the bar of the suite"""
+    import caps_gb300 as cg
+    from oracle import binding as ob
+    R, L = 45e-6, 1e-6
+    c = cg.Caps(R, L, ldim=ldim)
+    xi = np.linspace(0.5, 30.0, count)
+    got, status = c.logdetD_batch(xi, np.full(count, 1))
+    assert (status < 16).all()
+    for k in {0, count // 3, count - 1}:
+        M = ob.M_dense(R, L, ldim, float(xi[k]), 1)
+        want = np.linalg.slogdet(np.eye(2 * ldim) - M)[1]
+        assert abs(got[k] - want) <= 1e-10 * max(1.0, abs(want)), (k, got[k], want)
+        assert got[k] == c.logdetD(xi[k], 1)
