@@ -96,8 +96,8 @@ __global__ void k_to_delta32(int ntask, int n, const double *A, size_t lda, size
 
 // diagonal block in delta form, one CTA of 256 threads per matrix; also writes W =
 // (I + Lam_kk)^{-1} (lower triangular, MB x MB per task, stored transposed) for the panel solve and
-// the block's share of ||Lam||_F^2.  The factorisation runs in 16-column sub-panels (warp-level
-// diagonal block, substitution below it, rank-16 update of the rest); the updates take the
+// the block's share of ||Lam||_F^2.  The factorisation runs in 16-column sub-panels (three
+// warps with the diagonal block and a third of the rows below each, rank-16 update of the rest); the updates take the
 // entries (i, c) of the trailing triangle from a list of the whole triangle ordered by column
 // (last column first), so that each sub-panel's entries are a prefix of it and the 256
 // threads share them evenly (consecutive threads: consecutive rows of one column, T rows 65
@@ -107,7 +107,8 @@ __global__ void k_to_delta32(int ntask, int n, const double *A, size_t lda, size
 // triangle with half the diagonal, and W = 1 - Lam + Lam^2 leave out third order, below 2^-39, where FP32 entries of
 // that size have units of 2^-37, and the log det's correction takes up what is left of the diagonal's.  About
 // half of the blocks at R/L = 400 and most at R/L = 150 are such; a launch of them takes 15 us instead of 33 (6 matrices
-// of dimension 6000: 3.1 -> 2.4 ms in all).
+// of dimension 6000: 3.1 -> 2.4 ms in all; 2.1 since a sub-panel's rows below go with its diagonal block instead of by
+// a forward substitution, one thread per row, after it).
 __global__ void __launch_bounds__(256) k_potf2_w(int ntask, int n, int k0, float *S, size_t sstride, int *status, float *Winv,
                                                  double *fro)
 {
@@ -115,7 +116,6 @@ __global__ void __launch_bounds__(256) k_potf2_w(int ntask, int n, int k0, float
     if (task >= ntask || status[task] != ST_FACTOR) return;
     __shared__ float T[MB][MB + 1];
     __shared__ float W[MB][MB + 1];
-    __shared__ float colj[MB];
     __shared__ float Yb[3][16][17]; // blocks of the blockwise inverse in progress
     __shared__ double red8[8];
     // the entries (i, c), 1 <= c <= i <= 63, as i | c << 8, columns 63, 62, ..., 1, rows
@@ -174,25 +174,26 @@ __global__ void __launch_bounds__(256) k_potf2_w(int ntask, int n, int k0, float
         }
         __syncthreads();
     }
-    // blocked in 16-column sub-panels: (a) the sub-panel's diagonal block by warp 0 (lane i
-    // holds its row i in registers, column entries broadcast by shuffles), (b) the rows below it
-    // by forward substitution, one thread per row, (c) the rank-16 update of the rest of the
-    // triangle from the tail of the entry list; three barriers per sub-panel
+    // blocked in 16-column sub-panels: (a) the sub-panel by three warps, each with the 16 rows of its diagonal
+    // block and 16 of the rows below (a lane holds a row in registers, column entries broadcast by shuffles),
+    // (b) the rank-16 update of the rest of the triangle from the tail of the entry list; two barriers per sub-panel
     constexpr int PB = 16;
     for (int o = near0 ? nb : 0; o < nb; o += PB) {
         const int w = min(PB, nb - o);
-        if (tid < 32) {
+        if (tid < 96) {
             // every lane also keeps the sub-panel's future pivots dd[c] (pivot - 1), updated
             // with the same fma and order as lane c's own diagonal entry: the shuffles of the
             // update bring l_cj to every lane, so no pivot is broadcast, and the step's chain is
             // one shuffle, an fma, an add, a reciprocal square root and a product
-            const int i = tid;
+            const int i = tid & 31, row = i < PB ? o + i : o + i + (tid >> 5) * PB;
+            const bool below = i >= PB, live = below ? row < nb : i < w;
             float t[PB], dd[PB];
 #pragma unroll
             for (int k = 0; k < PB; k++) {
-                t[k] = (i < w && k <= i) ? T[o + i][o + k] : 0.0f;
+                t[k] = (live && k <= i) ? T[row][o + k] : 0.0f;
                 dd[k] = k < w ? T[o + k][o + k] : 0.0f;
             }
+            asm volatile("bar.sync 1, 96;" ::: "memory"); // the three warps have read the diagonal block
 #pragma unroll
             for (int j = 0; j < PB; j++) {
                 if (j < w) { // uniform
@@ -204,41 +205,22 @@ __global__ void __launch_bounds__(256) k_potf2_w(int ntask, int n, int k0, float
                 const float inv = __frsqrt_rn(fmaxf(one_d, 1e-30f));
                 if (i > j) t[j] *= inv;
                 else if (i == j) t[j] = d * inv * __frcp_rn(1.0f + inv);
-                if (i == 0) colj[o + j] = inv;
                 const float cj = t[j];
 #pragma unroll
                 for (int c = j + 1; c < PB; c++) {
                     const float v = __shfl_sync(0xffffffffu, cj, c); // column j of row c
-                    if (i >= c && i < w) t[c] = fmaf(-cj, v, t[c]);
+                    if (i >= c && live) t[c] = fmaf(-cj, v, t[c]);
                     dd[c] = fmaf(-v, v, dd[c]);
                 }
                 }
             }
+            if (live && (below || tid < 32))
 #pragma unroll
-            for (int k = 0; k < PB; k++)
-                if (i < w && k <= i) T[o + i][o + k] = t[k];
+                for (int k = 0; k < PB; k++)
+                    if (k <= i) T[row][o + k] = t[k];
         }
         __syncthreads();
         const int c0 = o + w;
-        if (tid < nb - c0) {
-            const int r = c0 + tid;
-            float x[PB];
-#pragma unroll
-            for (int k = 0; k < PB; k++) x[k] = k < w ? T[r][o + k] : 0.0f;
-#pragma unroll
-            for (int k = 0; k < PB; k++) {
-                if (k < w) {
-                    float a = x[k];
-#pragma unroll
-                    for (int j = 0; j < k; j++) a = fmaf(-x[j], T[o + k][o + j], a);
-                    x[k] = a * colj[o + k];
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < PB; k++)
-                if (k < w) T[r][o + k] = x[k];
-        }
-        __syncthreads();
         if (c0 < nb) {
             // the entries (i, c), c0 <= c <= i, are the first (MB - c0)(MB - c0 + 1) / 2 of the list
             const int cnt = (MB - c0) * (MB - c0 + 1) / 2;
