@@ -125,7 +125,7 @@ template <bool PR> CAPS_DEV void k_node(const Task &T, int j, const double *lfac
 // CTA, so that a small batch's pairs spread over the SMs (24 matrices of dimension 2100: eight warps per CTA 1.54 ms,
 // one 0.99, fewer nodes 0.50, two warps per 32 nodes 0.37; a T = 0 energy, which fills the SMs, 2.06 and 1.66),
 // and little shared memory, so that a large batch's CTAs and the Mie coefficients' beside them are all resident.
-constexpr int KT_WARPS = 1, KT_ALIGN = 16;
+constexpr int KT_ALIGN = 16;
 constexpr int KT_BUF = KT_ALIGN * 33;                                               // doubles of a buffer
 static size_t ktab64_smem_bytes() { return (size_t)(2 * KT_BUF + 64) * sizeof(double); }
 
@@ -209,33 +209,43 @@ k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lf
 // the sums do not cancel; the upward recurrence (dominant solution) loses at most a bit
 // per step to its subtraction.  The node weights are still formed once per node in FP64.
 // Partials: float-float (h, l) times 2^partE.
-template <bool PR>
-__global__ void __launch_bounds__(KT_WARPS * 32)
+//
+// PAIR: as in k_ktab two warps share 32 nodes, one with the recurrence and one with the folding of the 32 degrees before,
+// where schedulers would have no more than one warp (6 matrices of dimension 6000: 1.31 ms with one warp, 0.85 with
+// two); a large batch has warps enough, and the second one and its buffer only take room (993 matrices of
+// dimension 2100: 2.02 ms with one, 2.65 with two).  The values are the same bits.
+constexpr int KTF_PAIR_MAX = 608; // groups of 32 nodes, one per scheduler
+template <bool PR, bool PAIR>
+__global__ void __launch_bounds__(PAIR ? 64 : 32)
 k_ktab_ff(const Task *tasks, const float4 *coefF, int nu_stride, const double *lfac_tab, float2 *partF, int *partE, int max_warps)
 {
     extern __shared__ double smem[];
-    const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float2 *buf = reinterpret_cast<float2 *>(smem + wib * (32 * 33));      // [32][33]
-    float2 *wTM = reinterpret_cast<float2 *>(smem + KT_WARPS * 32 * 33 + wib * 64); // [32]
-    float2 *wTE = wTM + 32;                                                          // [32]
-    int *rowE = (int *)(smem + KT_WARPS * (32 * 33 + 64)) + wib * 32;
+    const int lane = threadIdx.x & 31;
+    constexpr int NBUF = PAIR ? 2 : 1;
+    const bool recurs = !PAIR || threadIdx.x < 32, folds = !PAIR || threadIdx.x >= 32;
+    float2 *bufs = reinterpret_cast<float2 *>(smem);          // [NBUF][32][33]
+    float2 *wTM = bufs + NBUF * 32 * 33, *wTE = wTM + 32;     // [32]
+    int *rowEs = reinterpret_cast<int *>(wTE + 32);           // [NBUF][32]
 
     const int task = blockIdx.y;
     const Task T = tasks[task];
-    const int warp = blockIdx.x * KT_WARPS + wib;
+    const int warp = blockIdx.x;
     if (warp * 32 >= T.nnode) return;
     const bool valid = warp * 32 + lane < T.nnode;
-    ff x{1.0f, 0.0f}, WTM{0.0f, 0.0f}, WTE{0.0f, 0.0f};
+    ff x{1.0f, 0.0f};
     int E = -(1 << 29);
-    if (valid) {
-        double xd, tm, te;
-        k_node<PR>(T, warp * 32 + lane, lfac_tab, xd, E, tm, te);
-        x = ff_from_d(xd);
-        WTM = ff_from_d(tm);
-        WTE = ff_from_d(te);
+    if (recurs) {
+        ff WTM{0.0f, 0.0f}, WTE{0.0f, 0.0f};
+        if (valid) {
+            double xd, tm, te;
+            k_node<PR>(T, warp * 32 + lane, lfac_tab, xd, E, tm, te);
+            x = ff_from_d(xd);
+            WTM = ff_from_d(tm);
+            WTE = ff_from_d(te);
+        }
+        wTM[lane] = make_float2(WTM.h, WTM.l);
+        wTE[lane] = make_float2(WTE.h, WTE.l);
     }
-    wTM[lane] = make_float2(WTM.h, WTM.l);
-    wTE[lane] = make_float2(WTE.h, WTE.l);
 
     ff pp{0.0f, 0.0f}, pc{valid ? 1.0f : 0.0f, 0.0f};
     const int nnu = T.nu_max - T.mu + 1;
@@ -243,30 +253,39 @@ k_ktab_ff(const Task *tasks, const float4 *coefF, int nu_stride, const double *l
     const size_t pTM = ((size_t)(task * 2 + 1) * max_warps + warp) * nu_stride;
     const size_t pTE = ((size_t)(task * 2 + 0) * max_warps + warp) * nu_stride;
 
-    for (int base = 0; base < nnu; base += 32) {
-        const int rows = min(32, nnu - base);
-        for (int r = 0; r < rows; r++) {
-            const int e = (pc.h != 0.0f) ? fexpo(pc.h) + E : -(1 << 29);
-            const int emax = __reduce_max_sync(0xffffffffu, e);
-            // align to the warp maximum by one multiply with 2^(E - emax) (0 below 2^-126; the
-            // clamp at 2^127 only matters for a zero value, which stays zero)
-            const float p2 = __uint_as_float((unsigned)min(max(127 + E - emax, 0), 254) << 23);
-            const ff v{pc.h * p2, pc.l * p2};
-            buf[r * 33 + lane] = make_float2(v.h, v.l);
-            if (lane == 0) rowE[r] = emax;
-            const float4 c = __ldg(ab + base + r);
-            const ff pn = ff_add(ff_mul(ff_mul(ff{c.x, c.y}, x), pc), ff_neg(ff_mul(ff{c.z, c.w}, pp)));
-            pp = pc;
-            pc = pn;
-            if (fabsf(pc.h) > 0x1p40f) { pc = ff_shift(pc, -40); pp = ff_shift(pp, -40); E += 40; }
+    float4 c = __ldg(ab);
+    for (int base = 0; base < nnu + (PAIR ? 32 : 0); base += 32) {
+        const int b = PAIR ? (base >> 5) & 1 : 0;
+        if (recurs && base < nnu) {
+            const int rows = min(32, nnu - base);
+            float2 *buf = bufs + b * 32 * 33;
+            int *rowE = rowEs + b * 32;
+            for (int r = 0; r < rows; r++) {
+                const float4 next = __ldg(ab + min(base + r + 1, nnu - 1));
+                const int e = (pc.h != 0.0f) ? fexpo(pc.h) + E : -(1 << 29);
+                const int emax = __reduce_max_sync(0xffffffffu, e);
+                // align to the warp maximum by one multiply with 2^(E - emax) (0 below 2^-126; the
+                // clamp at 2^127 only matters for a zero value, which stays zero)
+                const float p2 = __uint_as_float((unsigned)min(max(127 + E - emax, 0), 254) << 23);
+                const ff v{pc.h * p2, pc.l * p2};
+                buf[r * 33 + lane] = make_float2(v.h, v.l);
+                if (lane == 0) rowE[r] = emax;
+                const ff pn = ff_add(ff_mul(ff_mul(ff{c.x, c.y}, x), pc), ff_neg(ff_mul(ff{c.z, c.w}, pp)));
+                pp = pc;
+                pc = pn;
+                if (fabsf(pc.h) > 0x1p40f) { pc = ff_shift(pc, -40); pp = ff_shift(pp, -40); E += 40; }
+                c = next;
+            }
         }
-        __syncwarp();
-        if (lane < rows) {
+        if (!PAIR) __syncwarp();
+        const int row = base - (PAIR ? 32 : 0) + lane, bf = PAIR ? b ^ 1 : 0; // the buffer before
+        if (folds && row >= lane && row < nnu) {
             ff sTM{0.0f, 0.0f}, sTE{0.0f, 0.0f};
-            const float2 *row = buf + lane * 33;
+            const float2 *v0 = bufs + bf * 32 * 33 + lane * 33;
+            const int e = rowEs[bf * 32 + lane];
 #pragma unroll 8
             for (int l = 0; l < 32; l++) {
-                const float2 v = row[l];
+                const float2 v = v0[l];
                 const float2 wm = wTM[l];
                 sTM = ff_add(sTM, ff_mul(ff{v.x, v.y}, ff{wm.x, wm.y}));
                 if (!PR) {
@@ -274,14 +293,15 @@ k_ktab_ff(const Task *tasks, const float4 *coefF, int nu_stride, const double *l
                     sTE = ff_add(sTE, ff_mul(ff{v.x, v.y}, ff{we.x, we.y}));
                 }
             }
-            partF[pTM + base + lane] = make_float2(sTM.h, sTM.l);
-            partE[pTM + base + lane] = rowE[lane];
+            partF[pTM + row] = make_float2(sTM.h, sTM.l);
+            partE[pTM + row] = e;
             if (!PR) {
-                partF[pTE + base + lane] = make_float2(sTE.h, sTE.l);
-                partE[pTE + base + lane] = rowE[lane];
+                partF[pTE + row] = make_float2(sTE.h, sTE.l);
+                partE[pTE + row] = e;
             }
         }
-        __syncwarp();
+        if (PAIR) __syncthreads();
+        else __syncwarp();
     }
 }
 
@@ -718,7 +738,7 @@ void launch_scale(const Task *tasks, int ntask, int ldim, const double *lna, con
     CK(cudaGetLastError());
 }
 
-size_t ktab_smem_bytes() { return (size_t)KT_WARPS * (32 * 33 + 64) * sizeof(double) + KT_WARPS * 32 * sizeof(int); }
+static size_t ktab_ff_smem_bytes(bool pair) { return (size_t)((pair ? 2 : 1) * 32 * 33 + 64) * sizeof(float2) + (pair ? 64 : 32) * sizeof(int); }
 
 void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double2 *coefAB, int nu_stride, const double *lfac_tab,
                  double *partM, int *partE, cudaStream_t st)
@@ -807,16 +827,13 @@ void launch_ptab_groups(const int *group_m, int ngroup, float4 *ptabf, int pstri
 void launch_ktab_ff(bool pr, const Task *tasks, int ntask, int max_warps, const float4 *coefF, int nu_stride, const double *lfac_tab,
                     float2 *partF, int *partE, cudaStream_t st)
 {
-    static bool attr_set = false;
-    const size_t sm = ktab_smem_bytes();
-    if (!attr_set) {
-        CK(cudaFuncSetAttribute(k_ktab_ff<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        CK(cudaFuncSetAttribute(k_ktab_ff<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        attr_set = true;
-    }
-    dim3 g((max_warps + KT_WARPS - 1) / KT_WARPS, ntask);
-    if (pr) k_ktab_ff<true><<<g, KT_WARPS * 32, sm, st>>>(tasks, coefF, nu_stride, lfac_tab, partF, partE, max_warps);
-    else k_ktab_ff<false><<<g, KT_WARPS * 32, sm, st>>>(tasks, coefF, nu_stride, lfac_tab, partF, partE, max_warps);
+    // (both buffers stay below the 48 KB that need no attribute)
+    const bool pair = (long long)ntask * max_warps <= KTF_PAIR_MAX;
+    const size_t sm = ktab_ff_smem_bytes(pair);
+    const dim3 g(max_warps, ntask);
+    auto run = [&](auto f) { f<<<g, pair ? 64 : 32, sm, st>>>(tasks, coefF, nu_stride, lfac_tab, partF, partE, max_warps); };
+    if (pr) pair ? run(k_ktab_ff<true, true>) : run(k_ktab_ff<true, false>);
+    else pair ? run(k_ktab_ff<false, true>) : run(k_ktab_ff<false, false>);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }

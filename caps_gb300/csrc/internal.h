@@ -36,7 +36,6 @@ void launch_coef(const int *group_m, int ngroup, int nu_stride, double2 *coefAB,
 void launch_mie(const double *xi, const double *epsm1, int nxi, double LbyR, int lmax, double *lna, double *lnb, cudaStream_t st);
 void launch_scale(const Task *tasks, int ntask, int ldim, const double *lna, const double *lnb, int lmax, const double *lfac_tab,
                   sd *Sa, sd *Sb, double2 *uv, cudaStream_t st);
-size_t ktab_smem_bytes();
 void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double2 *coefAB, int nu_stride, const double *lfac_tab,
                  double *partM, int *partE, cudaStream_t st);
 void launch_kred(const Task *tasks, int ntask, int max_nnu, const double *partM, const int *partE, int max_warps, int nu_stride,

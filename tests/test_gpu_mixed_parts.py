@@ -22,3 +22,19 @@ def test_parts(ldim, metal):
         out.append(c.logdetD_batch(xi, m))
     assert (out[0][1] < 16).all() and (out[1][1] < 16).all()
     assert (np.abs(out[0][0] - out[1][0]) <= 5e-8 * np.maximum(1.0, np.abs(out[0][0]))).all()
+
+
+@pytest.mark.parametrize("metal", [None, (9.0, 0.035)])
+def test_nodes_by_one_warp_or_two(metal):
+    """the K integrals of few matrices share 32 nodes between two warps, those of many do not: the same bits"""
+    import caps_gb300 as cg
+    c = cg.Caps(30e-6, 1e-6, ldim=60)
+    if metal:
+        c.set_drude(*metal)
+    c.set_precision(cg.PREC_MIXED)
+    xi, m = np.linspace(1.0, 40.0, 500), np.arange(500) % 7
+    many, status = c.logdetD_batch(xi, m)
+    assert (status < 16).all()
+    for k in (0, 3, 250, 499):
+        one, _ = c.logdetD_batch(xi[k:k + 1], m[k:k + 1])
+        assert one[0] == many[k]
