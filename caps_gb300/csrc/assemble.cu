@@ -84,7 +84,7 @@ __global__ void k_scale(const Task *tasks, int ntask, int ldim, const double *ln
 // ---------------------------------------------------------------------------
 // One warp owns 32 nodes.  Each lane runs the degree recurrence of P_nu^mu at its node; at every
 // degree the warp aligns the lane values to the warp-maximum binary exponent and parks them in
-// shared memory; every 32 degrees lane r folds row r with the node weights (times the Fresnel
+// shared memory; every 16 degrees (mixed form: 32) lane r folds row r with the node weights (times the Fresnel
 // coefficient of each node) into the partial K sum of degree nu0+r.
 //
 // FP64 form: 5 FP64 operations per node and degree at two per clock and SM; the nodes of kgrid.cuh
@@ -131,10 +131,10 @@ static size_t ktab64_smem_bytes() { return (size_t)(2 * KT_BUF + 64) * sizeof(do
 
 template <bool PR>
 __global__ void __launch_bounds__(64)
-k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lfac_tab, double *partM, int *partE, int max_warps)
+k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lfac_tab, double *partM, int *partE, int max_warps, int *status)
 {
     extern __shared__ double smem[];
-    __shared__ int bufE[2];
+    __shared__ int bufE[2][KT_ALIGN];
     const int lane = threadIdx.x & 31;
     const bool folds = threadIdx.x >= 32;
     double *wTM = smem + 2 * KT_BUF, *wTE = wTM + 32; // [32]
@@ -158,29 +158,44 @@ k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lf
     const size_t pTM = ((size_t)(task * 2 + 1) * max_warps + warp) * nu_stride;
     const size_t pTE = ((size_t)(task * 2 + 0) * max_warps + warp) * nu_stride;
 
+    // the lane values of NS degrees from base + r0 on, aligned to the largest of the warp at the first of them
+    auto degrees = [&](auto ns, int base, int r0, double *buf, int *rowE) {
+        constexpr int NS = decltype(ns)::value;
+        const int ex = (int)((__double_as_longlong(pc) >> 52) & 0x7ff), k = ex ? ex - 1023 : 0;
+        if (ex == 0x7ff) atomicOr(status + task, ST_ERR_NONFINITE); // (shifted below as if it were finite)
+        pc = shift2(pc, -k);
+        pp = shift2(pp, -k);
+        E += k;
+        const int emax = __reduce_max_sync(0xffffffffu, ex ? E : -(1 << 29));
+        const int d = max(E - emax, -1023);
+        if (lane < NS) rowE[r0 + lane] = emax;
+#pragma unroll
+        for (int r = 0; r < NS; r++) {
+            if (base + r0 + r < nnu) { // uniform
+                buf[(r0 + r) * 33 + lane] = shift2(pc, d);
+                const double2 c = __ldg(ab + base + r0 + r);
+                const double pn = fma(c.x * x, pc, -c.y * pp);
+                pp = pc;
+                pc = pn;
+            }
+        }
+    };
+    // A value grows by A x < 2^grow per degree (A is largest at the first) and starts below 2; 16 degrees share an
+    // alignment where that stays below 2^900, else 4 or each has its own.  A task's nodes reach x = nu_max / (2 xi_)
+    // or so, so that only xi_ below 1e-7 (large m) or 1e-11 (small m) take the shorter steps.  A value that starts 2^1000
+    // below the largest of the warp stays negligible.  Values are shifted by powers of two: the same bits either way.
+    const int grow = 34 - __clz(2 * T.mu + 1) + __reduce_max_sync(0xffffffffu, expo(x));
     for (int base = 0; base < nnu + KT_ALIGN; base += KT_ALIGN) {
         const int b = base / KT_ALIGN & 1;
         if (!folds && base < nnu) {
             double *buf = smem + b * KT_BUF;
-            // the lane values aligned to the largest of the warp, for KT_ALIGN degrees at once: a value
-            // grows by (A x)^16 < 2^900 meanwhile (x < 2^50), and one that starts 2^1000 below stays below
-            const int ex = (int)((__double_as_longlong(pc) >> 52) & 0x7ff), k = ex ? ex - 1023 : 0;
-            pc = shift2(pc, -k);
-            pp = shift2(pp, -k);
-            E += k;
-            const int emax = __reduce_max_sync(0xffffffffu, ex ? E : -(1 << 29));
-            const int d = max(E - emax, -1023);
-            if (lane == 0) bufE[b] = emax;
-#pragma unroll
-            for (int r = 0; r < KT_ALIGN; r++) {
-                if (base + r < nnu) { // uniform
-                    buf[r * 33 + lane] = shift2(pc, d);
-                    const double2 c = __ldg(ab + base + r);
-                    const double pn = fma(c.x * x, pc, -c.y * pp);
-                    pp = pc;
-                    pc = pn;
-                }
-            }
+            if (grow <= 56) degrees(std::integral_constant<int, KT_ALIGN>(), base, 0, buf, bufE[b]);
+            else if (grow <= 225)
+#pragma unroll 1
+                for (int r0 = 0; r0 < KT_ALIGN; r0 += 4) degrees(std::integral_constant<int, 4>(), base, r0, buf, bufE[b]);
+            else
+#pragma unroll 1
+                for (int r0 = 0; r0 < KT_ALIGN; r0++) degrees(std::integral_constant<int, 1>(), base, r0, buf, bufE[b]);
         }
         const int row = base - KT_ALIGN + (lane & 15), upper = lane >> 4; // of the buffer before
         if (folds && base > 0) {
@@ -195,7 +210,7 @@ k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lf
             if (row < nnu && (!PR || !upper)) {
                 const size_t o = upper ? pTE + row : pTM + row;
                 partM[o] = sum;
-                partE[o] = bufE[b ^ 1];
+                partE[o] = bufE[b ^ 1][lane & 15];
             }
         }
         __syncthreads();
@@ -741,7 +756,7 @@ void launch_scale(const Task *tasks, int ntask, int ldim, const double *lna, con
 static size_t ktab_ff_smem_bytes(bool pair) { return (size_t)((pair ? 2 : 1) * 32 * 33 + 64) * sizeof(float2) + (pair ? 64 : 32) * sizeof(int); }
 
 void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double2 *coefAB, int nu_stride, const double *lfac_tab,
-                 double *partM, int *partE, cudaStream_t st)
+                 double *partM, int *partE, int *status, cudaStream_t st)
 {
     beside_ktab();
     static bool attr_set = false;
@@ -752,8 +767,8 @@ void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const dou
         attr_set = true;
     }
     dim3 g(max_warps, ntask);
-    if (pr) k_ktab<true><<<g, 64, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
-    else k_ktab<false><<<g, 64, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps);
+    if (pr) k_ktab<true><<<g, 64, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps, status);
+    else k_ktab<false><<<g, 64, sm, st>>>(tasks, coefAB, nu_stride, lfac_tab, partM, partE, max_warps, status);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
 }

@@ -37,7 +37,7 @@ void launch_mie(const double *xi, const double *epsm1, int nxi, double LbyR, int
 void launch_scale(const Task *tasks, int ntask, int ldim, const double *lna, const double *lnb, int lmax, const double *lfac_tab,
                   sd *Sa, sd *Sb, double2 *uv, cudaStream_t st);
 void launch_ktab(bool pr, const Task *tasks, int ntask, int max_warps, const double2 *coefAB, int nu_stride, const double *lfac_tab,
-                 double *partM, int *partE, cudaStream_t st);
+                 double *partM, int *partE, int *status, cudaStream_t st);
 void launch_kred(const Task *tasks, int ntask, int max_nnu, const double *partM, const int *partE, int max_warps, int nu_stride,
                  sd *K, int *status, cudaStream_t st);
 // mixed form: the K integrals in float-float

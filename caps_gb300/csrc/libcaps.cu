@@ -622,7 +622,7 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
             launch_kred_ff(d_tasks, nt, nnu_max, (const float2 *)d_pM, d_pE, max_warps, nu_stride, d_KP, d_KPe, d_status, st);
         } else {
             d_K = (sd *)g_eng.K.get((size_t)nt * 2 * nu_stride * sizeof(sd));
-            launch_ktab(is_pr, d_tasks, nt, max_warps, d_coef, nu_stride, g_eng.d_lfac, d_pM, d_pE, st);
+            launch_ktab(is_pr, d_tasks, nt, max_warps, d_coef, nu_stride, g_eng.d_lfac, d_pM, d_pE, d_status, st);
             side();
             launch_kred(d_tasks, nt, nnu_max, d_pM, d_pE, max_warps, nu_stride, d_K, d_status, st);
         }

@@ -182,7 +182,7 @@ extern "C" int caps_logdetD_noalloc(caps_t *self, double xi_, int m, double *log
     NA_CK(cudaMemcpyAsync(d_gm, &gm_h[0], sizeof(int), cudaMemcpyHostToDevice, st));
     NA_CK(cudaMemcpyAsync(d_glm, &gm_h[1], sizeof(int), cudaMemcpyHostToDevice, st));
     launch_coef(d_gm, 1, nu_stride, d_coef, nullptr, st);
-    launch_ktab(T.is_pr != 0, d_task, 1, max_warps, d_coef, nu_stride, g_lfac_ptr[dev], d_pM, d_pE, st);
+    launch_ktab(T.is_pr != 0, d_task, 1, max_warps, d_coef, nu_stride, g_lfac_ptr[dev], d_pM, d_pE, d_status, st);
     launch_kred(d_task, 1, nnu, d_pM, d_pE, max_warps, nu_stride, d_K, d_status, st);
     launch_a12(d_gm, d_glm, 1, ldim, d_lft, d_a12, st);
     launch_ptab(d_task, 1, d_ptab, pstride, st);
