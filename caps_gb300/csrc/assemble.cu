@@ -687,8 +687,11 @@ __global__ void __launch_bounds__(ST_NT) k_stats(const int *tlist, int nlist, in
     for (int w = 0; w < (int)blockDim.x / 32; w++) all.add(rs[w], rc[w]);
     const double t = all.s + all.c;
     trace_out[task] = t;
-    if (status[task] & ~0xF) { result[task] = NAN; return; }
+    // (an entry of 2 or more is noted as a pivot that is not positive; the rules that need none come first)
+    const int st = status[task];
+    if (st & ~(0xF | ST_ERR_PIVOT)) { result[task] = NAN; return; }
     if (fabs(t) < 1e-8) { result[task] = -t; status[task] = ST_TRACE; return; }
+    if (st & ST_ERR_PIVOT) { result[task] = NAN; return; }
     if (!A) return;
     if (mode == 0) {
         double fro2 = 0.0;

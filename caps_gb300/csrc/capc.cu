@@ -384,7 +384,8 @@ __global__ void __launch_bounds__(CE_X) k_capc_elem(int ntask, int n, const sd *
         const sd *S = T, *KQ = T + n, *W = T + 3 * n + 1;
         const bool type = task & 1;
         const int fq = FQ - info[2 * task];
-        bool bad = false;
+        const long long one = fq >= 0 ? 1LL << fq : 0;
+        int err = 0;
         if (r < n) {
             const sd Sr = S[r], Wr = W[r];
             // m 2^e of products of three mantissas in [0.5, 1)
@@ -399,17 +400,17 @@ __global__ void __launch_bounds__(CE_X) k_capc_elem(int ntask, int n, const sd *
                     const sd Wc = W[c];
                     M = U + V + val(Wr.m * Wc.m, Wr.e + Wc.e);
                 }
-                A[(size_t)task * mstride + (size_t)c * n + r] = -to_fix(M, fq, bad);
+                A[(size_t)task * mstride + (size_t)c * n + r] = -to_fix(M, fq, err);
                 fro = fma(M, M, fro);
             }
             fro *= 2.0;
             if (r >= c0 && r < c0 + CE_Y) {
                 const double M = mdiag[(size_t)task * n + r];
-                A[(size_t)task * mstride + (size_t)r * n + r] = (1LL << fq) - to_fix(M, fq, bad);
+                A[(size_t)task * mstride + (size_t)r * n + r] = one - to_fix(M, fq, err);
                 fro = fma(M, M, fro);
             }
         }
-        if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status + task, ST_ERR_NONFINITE);
+        if (err) atomicOr(status + task, err);
     }
     __shared__ double red[CE_X / 32];
     for (int o = 16; o > 0; o >>= 1) fro += __shfl_xor_sync(0xffffffffu, fro, o);

@@ -24,6 +24,12 @@
 // k_fix_syrk (S -= X X^T).  log det A = 2 sum_j log L_jj.  A non-positive pivot marks the task
 // (ST_ERR_PIVOT) and its result becomes NaN; nothing traps.  A matrix whose diagonal exceeds 2
 // (M with large negative diagonal entries) is scaled by a power of four on conversion.
+//
+// A matrix that is not positive definite keeps none of these bounds, and integers that wrap could end as
+// positive pivots.  So what the bounds say is checked, and a matrix that breaks them is marked like one with a
+// non-positive pivot: entries below 2 (on conversion, in the panel solve and in potf2_limbs), and the squares of
+// a row of the factor, summed over all panels so far in FP32, below 2 (FIX_ROW).  While both hold nothing wraps,
+// and the pivots are what they are.
 #include "common.cuh"
 #include "fix.cuh"
 #include "internal.h"
@@ -114,7 +120,9 @@ CAPS_DEV void fold_group(uint32_t taddr, int s, int s0, long long (&v)[16])
 // FP64 -> fixed point, in place (lower triangle)
 // ---------------------------------------------------------------------------
 // scale exponent of a matrix whose largest diagonal entry is mx: none below 2, else a power of four
-CAPS_DEV int fix_sexp(double mx) { return mx >= 2.0 ? min(2 * ((ilogb(mx) + 2) / 2), 400) : 0; }
+CAPS_DEV int fix_sexp(double mx) { return mx >= 2.0 ? 2 * ((min(ilogb(mx), 1023) + 2) / 2) : 0; }
+// a diagonal entry is below 2, and so are the squares of a row of the factor; their FP32 sum stays below this
+constexpr float FIX_ROW = 2.25f;
 
 // for producers that write fixed point themselves: the exponents alone, one warp per task
 __global__ void k_fix_scale(const int *tlist, int nlist, int n, const double *mdiag, FixInfo *info)
@@ -129,11 +137,11 @@ __global__ void k_fix_scale(const int *tlist, int nlist, int n, const double *md
 }
 
 // grid (ceil(n / 8), ntask), 256 threads: 8 columns per block
-__global__ void __launch_bounds__(256) k_fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, const int *status,
+__global__ void __launch_bounds__(256) k_fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, int *status,
                                                      const double *mdiag, FixInfo *info)
 {
     const int task = blockIdx.y;
-    if (task >= ntask || status[task] != ST_FACTOR) return;
+    if (task >= ntask || (status[task] & 0xF) != ST_FACTOR) return; // error bits may be set by this launch: not read
     __shared__ double red[8];
     double mx = 0.0;
     for (int i = threadIdx.x; i < n; i += 256) mx = fmax(mx, 1.0 - mdiag[(size_t)task * n + i]);
@@ -144,13 +152,16 @@ __global__ void __launch_bounds__(256) k_fix_convert(int ntask, int n, double *A
     const int sexp = fix_sexp(mx);
     if (blockIdx.x == 0 && threadIdx.x == 0) info[task].sexp = sexp;
     const double sc = ldexp(1.0, FQ - sexp);
+    bool over = false;
     for (int c = blockIdx.x * 8; c < min(n, (int)blockIdx.x * 8 + 8); c++) {
         double *col = A + (size_t)task * mstride + (size_t)c * lda;
         for (int r = c + threadIdx.x; r < n; r += 256) {
-            const double v = fmin(fmax(col[r] * sc, -0x1.fp61), 0x1.fp61);
+            const double x = col[r] * sc, v = fmin(fmax(x, -0x1.fp61), 0x1.fp61);
+            over |= !(fabs(x) < 0x1p61);
             reinterpret_cast<long long *>(col)[r] = __double2ll_rn(v);
         }
     }
+    if (over) atomicOr(status + task, ST_ERR_PIVOT);
 }
 
 // ---------------------------------------------------------------------------
@@ -216,7 +227,10 @@ __device__ __noinline__ int potf2_limbs(const long long *Sm, size_t lda, int nb,
     __shared__ long long piv[NB], inv[NB];
     __shared__ int invk[NB];
     __shared__ double slog[2];
+    __shared__ float rown[NB]; // squares of each row's entries so far
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    bool bad = false;
+    if (tid < NB) rown[tid] = 0.0f;
     __syncthreads(); // the shared memory is free
     {
         long long v[NB * NB / PF_NT];
@@ -229,11 +243,11 @@ __device__ __noinline__ int potf2_limbs(const long long *Sm, size_t lda, int nb,
         for (int u = 0; u < NB * NB / PF_NT; u++) {
             const int e = tid + PF_NT * u, c = e >> 6, r = e & 63;
             T[r * PP + c] = v[u];
+            bad |= v[u] >= 1LL << (FQ + 1) || v[u] <= -(1LL << (FQ + 1));
         }
     }
     __syncthreads();
     int2 *Lm = reinterpret_cast<int2 *>(T);
-    bool bad = false;
     constexpr int PB = 16;
 #pragma unroll 1
     for (int o = 0; o < NB; o += PB) {
@@ -247,6 +261,8 @@ __device__ __noinline__ int potf2_limbs(const long long *Sm, size_t lda, int nb,
                 b[c] = 0;
             }
             asm volatile("bar.sync 1, 96;" ::: "memory"); // the three warps have read the diagonal rows
+            const bool mine = live && (warp == 0 || lane >= 16);
+            float sq = 0.0f;
 #pragma unroll
             for (int j = 0; j < PB; j++) {
                 const long long sj = s[j] + ((b[j] + (1 << 29)) >> 30);
@@ -261,7 +277,11 @@ __device__ __noinline__ int potf2_limbs(const long long *Sm, size_t lda, int nb,
                 const long long ll = (long long)sl.x * rl.x, bb = (long long)sl.y * rl.x + (long long)sl.x * rl.y + (ll >> 30);
                 const long long x = (((long long)sl.y * rl.y) << k) + (k < 30 ? bb >> (30 - k) : bb << (k - 30));
                 const int2 xl = limbs(x);
-                if (live && row > o + j && (warp == 0 || lane >= 16)) Lm[row * PP + o + j] = xl;
+                if (mine && row > o + j) {
+                    const float xf = (float)sj * 0x1p-60f * ((float)r * 0x1p-60f) * ldexpf(1.0f, k);
+                    sq = fmaf(xf, xf, sq);
+                    Lm[row * PP + o + j] = xl;
+                }
                 const int nh = -xl.y, nl = -xl.x;
 #pragma unroll
                 for (int c = j + 1; c < PB; c++) {
@@ -270,6 +290,11 @@ __device__ __noinline__ int potf2_limbs(const long long *Sm, size_t lda, int nb,
                     b[c] += (long long)nh * cl;
                     b[c] += (long long)nl * ch;
                 }
+            }
+            if (mine) {
+                sq += rown[row];
+                rown[row] = sq;
+                bad |= !(sq < FIX_ROW);
             }
         }
         __syncthreads();
@@ -899,6 +924,7 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
     extern __shared__ __align__(1024) unsigned char tr_sm[];
     __shared__ uint64_t wfull, gfull[2];
     __shared__ uint32_t tslot, s_any[2][3]; // or of the magnitudes' low and high words: S, X of both row blocks
+    __shared__ float s_rn[4][128];          // squares of X, 16 columns each
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row0 = k0 + NB + blockIdx.x * 128;
     int *first = wk.first + (size_t)task * (fix_nbk(n) + 1) + blockIdx.x * 2;
@@ -921,6 +947,7 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
         __syncthreads();
         if ((s_any[0][0] | s_any[1][0]) == 0) { // S has no digit here: X = 0
             if (tid < 2) first[tid] = NG;
+            if (k0 == 0 && tid < 128 && R < n) wk.rn[(size_t)task * n + R] = 0.0f;
             return;
         }
         if (warp == 0) umma::alloc(&tslot, 512);
@@ -961,6 +988,7 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
         __syncwarp();
     }
     const int quad = warp & 3, part = warp >> 2;
+    bool over = s_any[1][0] >> 22; // an entry of S is 2 or more (2^54 units of 2^-53)
     long long v[16];
 #pragma unroll
     for (int c = 0; c < 16; c++) v[c] = 0;
@@ -972,15 +1000,30 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
             umma::fence_after();
         }
         if (ok && g >= fa) fold_group(tmem + ((uint32_t)(quad * 32) << 16) + g * NB + part * 16, g, fa, v);
+        if (g == 0 && fa == 0) {
+            // The fold holds sums below 4.  Of X 2^-wexp, below sqrt 2, the later groups are at most 1.01 (64 products of
+            // top digits, 1023 at most, with second ones, 256), so the first is below 2.75, and a sum with such a first group
+            // is below 4.  Without top digits of S the sum is below 64 * 2^-8 * 4 = 1
+#pragma unroll
+            for (int c = 0; c < 16; c++) over |= (unsigned)v[c] - (FX_MBITS - (11 << 14)) > 2u * (11 << 14);
+        }
     }
     const int wexp = wk.info[task].wexp, rb = quad >> 1; // rb: row block of the pair
     {
+        if (wexp) // uniform
+#pragma unroll
+            for (int c = 0; c < 16; c++) over |= (unsigned long long)(v[c] + (1LL << (FQ + 1 - wexp))) >> (FQ + 2 - wexp) != 0;
         unsigned long long any = 0;
+        float sq = 0.0f;
 #pragma unroll
         for (int c = 0; c < 16; c++) {
             v[c] <<= wexp;
             any |= digit_mag(v[c]);
+            // in units of 2^-20, |X| < 2
+            const float f = __int_as_float((int)FX_MBITS + ((int)(v[c] >> 32) >> 8)) - FX_MAGIC;
+            sq = fmaf(f, f, sq);
         }
+        s_rn[part][quad * 32 + lane] = sq;
         const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)any), hi = __reduce_or_sync(0xffffffffu, (unsigned)(any >> 32));
         if (lane == 0 && (lo | hi)) {
             atomicOr(&s_any[0][1 + rb], lo);
@@ -990,6 +1033,13 @@ __global__ void __launch_bounds__(TR_NT) k_fix_trsm(int ntask, int n, int k0, co
     umma::fence_before();
     __syncthreads();
     if (tid < 2) first[tid] = first_digit((unsigned long long)s_any[1][1 + tid] << 32 | s_any[0][1 + tid]);
+    if (tid < 128 && row0 + tid < n) {
+        float *t = wk.rn + (size_t)task * n + row0 + tid;
+        const float s = fmaf((s_rn[0][tid] + s_rn[1][tid]) + (s_rn[2][tid] + s_rn[3][tid]), 0x1p-40f, k0 ? *t : 0.0f);
+        *t = s;
+        over |= s > FIX_ROW || (s_any[1][1] | s_any[1][2]) >> 22;
+    }
+    if (over) atomicOr(status + task, ST_ERR_PIVOT);
     if (ok) {
         const int r = quad * 32 + lane, blk = blockIdx.x * 2 + rb; // row block below the diagonal block
         // digits that are zero in both blocks of the pair are not read
@@ -1193,16 +1243,20 @@ __global__ void k_final(int ntask, int n, const double *logdet, const FixInfo *i
     result[task] = ld;
 }
 
-// the exponents first (launch_fix_scale), then the digit table, then the images
+// the exponents first (launch_fix_scale), then the digit table, the rows' squares, the images
 static size_t fix_info_bytes(int ntask) { return ((size_t)ntask * sizeof(FixInfo) + 255) & ~(size_t)255; }
 static size_t fix_first_bytes(int ntask, int n) { return ((size_t)2 * ntask * (fix_nbk(n) + 1) * sizeof(int) + 255) & ~(size_t)255; }
+static size_t fix_rn_bytes(int ntask, int n) { return ((size_t)ntask * n * sizeof(float) + 255) & ~(size_t)255; }
 
-size_t cholesky_work_bytes(int ntask, int n) { return fix_info_bytes(ntask) + fix_first_bytes(ntask, n) + (size_t)ntask * fix_task_bytes(n); }
+size_t cholesky_work_bytes(int ntask, int n)
+{
+    return fix_info_bytes(ntask) + fix_first_bytes(ntask, n) + fix_rn_bytes(ntask, n) + (size_t)ntask * fix_task_bytes(n);
+}
 
 FixWork fix_work(int ntask, int n, void *work)
 {
-    unsigned char *w = (unsigned char *)work;
-    return FixWork{w + fix_info_bytes(ntask) + fix_first_bytes(ntask, n), (FixInfo *)w, (int *)(w + fix_info_bytes(ntask)), 0};
+    unsigned char *w = (unsigned char *)work, *first = w + fix_info_bytes(ntask), *rn = first + fix_first_bytes(ntask, n);
+    return FixWork{rn + fix_rn_bytes(ntask, n), (FixInfo *)w, (int *)first, (float *)rn, 0};
 }
 
 static int fix_sms()
@@ -1219,7 +1273,7 @@ static int fix_sms()
     return sms;
 }
 
-void fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, const int *status, const double *mdiag, const FixWork &wk,
+void fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, const FixWork &wk,
                  cudaStream_t st)
 {
     k_fix_convert<<<dim3((n + 7) / 8, ntask), 256, 0, st>>>(ntask, n, A, lda, mstride, status, mdiag, wk.info);

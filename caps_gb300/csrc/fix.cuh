@@ -21,10 +21,12 @@ __host__ __device__ inline size_t fix_task_bytes(int n) { return (size_t)ND * IM
 struct FixInfo { int sexp, wexp; };          // A 2^-sexp is factored; W 2^-wexp is in the image
 // first[task * (nbk + 1) + block] (one table per image): the first digit of the panel's X that is not zero in the whole 64-row
 // block (block counted below the diagonal block; NG: none)
+// rn[task * n + row]: squares of a row's part of the factor so far
 struct FixWork {
     unsigned char *img;
     FixInfo *info;
     int *first;
+    float *rn;
     int par; // the image in use
     __host__ __device__ unsigned char *wimg(int task, int n) const { return img + (size_t)task * fix_task_bytes(n); }
     __host__ __device__ unsigned char *ximg(int task, int n) const { return wimg(task, n) + (size_t)ND * IMG_BLK + par * fix_ximg_bytes(n); }
@@ -65,13 +67,14 @@ CAPS_DEV float fx_value(long long x)
     return fmaf((float)(int)((x + 0x80000000LL) >> 32), 0x1p-28f, (float)(int)x * 0x1p-60f);
 }
 
-// v in units of 2^-q, rounded, saturated at +-2^62 (integer work only)
-CAPS_DEV long long to_fix(double v, int q, bool &bad)
+// v in units of 2^-q, rounded, saturated at +-2^62 (integer work only).  err: status bits; a matrix whose diagonal is
+// below 2 and that has an entry of 2 or more is not positive definite
+CAPS_DEV long long to_fix(double v, int q, int &err)
 {
     const long long b = __double_as_longlong(v);
     const int ex = (int)((b >> 52) & 0x7ff);
-    bad |= ex == 0x7ff;
     const int sh = ex - 1075 + q;
+    if (sh >= 9) err |= ex == 0x7ff ? ST_ERR_NONFINITE : ST_ERR_PIVOT; // |v| >= 2^61 units
     long long mnt = (b & 0xfffffffffffffLL) | (1LL << 52);
     if (sh >= 10) mnt = 1LL << 62;
     else if (sh >= 0) mnt <<= sh;
@@ -118,7 +121,7 @@ CAPS_DEV void split8(const long long (&x)[8], uint4 (&d)[ND])
 // S -= X X^T over the rows and columns from t0 on, X the 64 columns in the image, first digits in wk.first; column
 // blocks j0 .. j1 - 1 of it
 FixWork fix_work(int ntask, int n, void *work);
-void fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, const int *status, const double *mdiag, const FixWork &wk,
+void fix_convert(int ntask, int n, double *A, size_t lda, size_t mstride, int *status, const double *mdiag, const FixWork &wk,
                  cudaStream_t st);
 void fix_syrk(int ntask, int n, int t0, long long *S, size_t lda, size_t mstride, int *status, const FixWork &wk, cudaStream_t st,
               int j0 = 0, int j1 = 1 << 30);

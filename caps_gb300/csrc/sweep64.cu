@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(E64_X) k_elem64(const Task *tasks, const int *
     const int x = blockIdx.x * E64_X + threadIdx.x + 1, y0 = blockIdx.y * ny + 1;
     double fro = 0.0;
     if (y0 <= min((int)(blockIdx.x + 1) * E64_X, ldim)) { // uniform: some thread of the block has y0 <= x
-        bool bad = false;
+        int err = 0;
         const Task &T = tasks[task];
         const int mt = T.m;
         const bool pr = T.is_pr;
@@ -297,18 +297,18 @@ __global__ void __launch_bounds__(E64_X) k_elem64(const Task *tasks, const int *
         // T(u, v) for any order of u and v
         auto TV = [&](const double *t, int u, int v) { return u >= v ? t[(size_t)v * L + u] : t[(size_t)u * L + v]; };
         const int fq = 60 - info[2 * task];
-        const long long one = 1LL << fq;
+        const long long one = fq >= 0 ? 1LL << fq : 0;
         long long *Am = A + (size_t)task * mstride + (size_t)2 * (y0 - 1) * n + 2 * (x - 1);
         auto store = [&](int y, double ee, double mm, double em, double me) {
             if (y != x) {
-                *reinterpret_cast<longlong2 *>(Am) = make_longlong2(-to_fix(ee, fq, bad), -to_fix(me, fq, bad));
-                *reinterpret_cast<longlong2 *>(Am + n) = make_longlong2(-to_fix(em, fq, bad), -to_fix(mm, fq, bad));
+                *reinterpret_cast<longlong2 *>(Am) = make_longlong2(-to_fix(ee, fq, err), -to_fix(me, fq, err));
+                *reinterpret_cast<longlong2 *>(Am + n) = make_longlong2(-to_fix(em, fq, err), -to_fix(mm, fq, err));
                 if (FRO) fro += 2.0 * (fma(ee, ee, me * me) + fma(mm, mm, em * em));
             } else {
                 // the diagonal from M_ii, which the trace is taken from too
                 const double dee = mdiag[(size_t)task * n + 2 * (x - 1)], dmm = mdiag[(size_t)task * n + 2 * (x - 1) + 1];
-                *reinterpret_cast<longlong2 *>(Am) = make_longlong2(one - to_fix(dee, fq, bad), -to_fix(me, fq, bad));
-                Am[n + 1] = one - to_fix(dmm, fq, bad);
+                *reinterpret_cast<longlong2 *>(Am) = make_longlong2(one - to_fix(dee, fq, err), -to_fix(me, fq, err));
+                Am[n + 1] = one - to_fix(dmm, fq, err);
                 if (FRO) fro += fma(dee, dee, dmm * dmm) + 2.0 * me * me;
             }
         };
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(E64_X) k_elem64(const Task *tasks, const int *
                 e0 = ep;
             }
         }
-        if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status + task, ST_ERR_NONFINITE);
+        if (err) atomicOr(status + task, err);
     }
     if (FRO) { // per-block sums, added by the statistics kernel in order
         __shared__ double red[E64_X / 32];
