@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <random>
 #include <vector>
 
@@ -262,7 +263,6 @@ using namespace capsgpu;
 struct caps_mlp {
     float *P = nullptr, *G = nullptr, *M1 = nullptr, *M2 = nullptr, *loss = nullptr;
     float *X = nullptr, *Y = nullptr, *out = nullptr, *gpart = nullptr, *lpart = nullptr; // Y behind X
-    float *host = nullptr; // pinned: samples on the way in, gradient and loss or predictions on the way out
     size_t cap = 0, blk_cap = 0;
     int t = 0;
 };
@@ -270,32 +270,57 @@ struct caps_mlp {
 static void mlp_reserve(caps_mlp_t *m, size_t n)
 {
     if (n > m->cap) {
-        if (m->X) { CK(cudaFree(m->X)); CK(cudaFree(m->out)); CK(cudaFreeHost(m->host)); }
+        if (m->X) { CK(cudaFree(m->X)); CK(cudaFree(m->out)); }
         m->cap = std::max(n, (size_t)2048);
         CK(cudaMalloc(&m->X, m->cap * (NIN + 1) * sizeof(float)));
         CK(cudaMalloc(&m->out, m->cap * sizeof(float)));
-        CK(cudaMallocHost(&m->host, m->cap * (NIN + 1) * sizeof(float)));
     }
 }
 
-// n samples and (y != nullptr) their values to the device, by one copy from pinned memory: six pageable copies, each
-// with a synchronisation, were half of the time of a loss, gradient and prediction of 2600 samples (121 us; 95 so)
+// Pinned memory that samples, gradients and predictions pass through, one block for all networks: taken by the first
+// network that is made, given back with the last.  Six pageable copies, each with a synchronisation, were half of the
+// time of a loss, gradient and prediction of 2600 samples (121 us; 95 so); a block per network, taken at its
+// first call, cost that call up to 110 us (a new network's first loss, gradient and prediction 322 us, 211 so; the other
+// 110 are its device memory).  A call holds
+// the lock while its data are in the block; what does not fit goes by pageable copies.
+static constexpr size_t MLP_STAGE = 16384 * (NIN + 1); // floats
+static_assert(NPARAM + 1 <= MLP_STAGE, "gradient and loss fit");
+static struct {
+    std::mutex mu;
+    float *p = nullptr;
+    int users = 0;
+} g_stage;
+
+static void stage_enter()
+{
+    std::lock_guard<std::mutex> lk(g_stage.mu);
+    if (g_stage.users++ == 0) CK(cudaMallocHost(&g_stage.p, MLP_STAGE * sizeof(float)));
+}
+static void stage_leave()
+{
+    std::lock_guard<std::mutex> lk(g_stage.mu);
+    if (--g_stage.users == 0) {
+        CK(cudaFreeHost(g_stage.p));
+        g_stage.p = nullptr;
+    }
+}
+
+// n samples and (y != nullptr) their values to the device, by one copy; the caller holds the lock and synchronises before
+// it lets go
 static void mlp_upload(caps_mlp_t *m, const float *X, const float *y, int n)
 {
     mlp_reserve(m, n);
     const size_t nx = (size_t)n * NIN, ny = y ? n : 0;
-    std::copy(X, X + nx, m->host);
-    if (y) std::copy(y, y + n, m->host + nx);
     m->Y = m->X + nx;
-    CK(cudaMemcpyAsync(m->X, m->host, (nx + ny) * sizeof(float), cudaMemcpyHostToDevice, 0));
+    if (nx + ny > MLP_STAGE) {
+        CK(cudaMemcpy(m->X, X, nx * sizeof(float), cudaMemcpyHostToDevice));
+        if (y) CK(cudaMemcpy(m->Y, y, ny * sizeof(float), cudaMemcpyHostToDevice));
+        return;
+    }
+    std::copy(X, X + nx, g_stage.p);
+    if (y) std::copy(y, y + ny, g_stage.p + nx);
+    CK(cudaMemcpyAsync(m->X, g_stage.p, (nx + ny) * sizeof(float), cudaMemcpyHostToDevice, 0));
 }
-// count floats back through pinned memory; returns when they are there
-static void mlp_download(caps_mlp_t *m, const float *src, size_t count)
-{
-    CK(cudaMemcpyAsync(m->host, src, count * sizeof(float), cudaMemcpyDeviceToHost, 0));
-    CK(cudaStreamSynchronize(0));
-}
-static_assert(NPARAM + 1 <= 2048 * (NIN + 1), "gradient and loss fit the pinned buffer");
 
 static int mlp_blocks(int n, int *per)
 {
@@ -322,6 +347,7 @@ extern "C" int caps_mlp_nparams(void) { return NPARAM; }
 extern "C" caps_mlp_t *caps_mlp_create(unsigned seed)
 {
     caps_mlp_t *m = new caps_mlp_t();
+    stage_enter();
     std::vector<float> p(NPARAM, 0.0f);
     std::mt19937 rng(seed);
     auto init = [&](int off, int fan_in, int count) {
@@ -353,7 +379,7 @@ extern "C" void caps_mlp_free(caps_mlp_t *m)
     if (!m) return;
     for (float *p : {m->P, m->G, m->M1, m->M2, m->X, m->out, m->gpart, m->lpart})
         if (p) CK(cudaFree(p));
-    if (m->host) CK(cudaFreeHost(m->host));
+    stage_leave();
     delete m;
 }
 
@@ -362,6 +388,7 @@ extern "C" void caps_mlp_set_params(caps_mlp_t *m, const float *in) { CK(cudaMem
 
 extern "C" double caps_mlp_loss_grad(caps_mlp_t *m, const float *X, const float *y, int n, float *grad)
 {
+    std::lock_guard<std::mutex> lk(g_stage.mu);
     mlp_upload(m, X, y, n);
     int per;
     const int nblk = mlp_blocks(n, &per);
@@ -370,14 +397,20 @@ extern "C" double caps_mlp_loss_grad(caps_mlp_t *m, const float *X, const float 
     k_mlp_reduce<<<MLP_RED_GRID, 256>>>(m->gpart, m->lpart, nblk, m->G, m->loss, n);
     COUNT_LAUNCH(2);
     CK(cudaGetLastError());
-    mlp_download(m, m->G, NPARAM + 1);
-    if (grad) std::copy(m->host, m->host + NPARAM, grad);
-    return m->host[NPARAM];
+    // gradient and loss lie one after the other
+    CK(cudaMemcpyAsync(g_stage.p, m->G, (NPARAM + 1) * sizeof(float), cudaMemcpyDeviceToHost, 0));
+    CK(cudaStreamSynchronize(0));
+    if (grad) std::copy(g_stage.p, g_stage.p + NPARAM, grad);
+    return g_stage.p[NPARAM];
 }
 
 extern "C" double caps_mlp_train(caps_mlp_t *m, const float *X, const float *y, int n, int epochs, float lr)
 {
-    mlp_upload(m, X, y, n);
+    {
+        std::lock_guard<std::mutex> lk(g_stage.mu);
+        mlp_upload(m, X, y, n);
+        CK(cudaStreamSynchronize(0)); // other networks may use the block during the epochs
+    }
     int per;
     const int nblk = mlp_blocks(n, &per);
     mlp_reserve_blocks(m, nblk);
@@ -390,21 +423,28 @@ extern "C" double caps_mlp_train(caps_mlp_t *m, const float *X, const float *y, 
         COUNT_LAUNCH(3);
     }
     CK(cudaGetLastError());
-    mlp_download(m, m->loss, 1);
-    return epochs > 0 ? m->host[0] : 0.0;
+    float loss;
+    CK(cudaMemcpy(&loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
+    return epochs > 0 ? loss : 0.0;
 }
 
 extern "C" void caps_mlp_predict(caps_mlp_t *m, const float *X, int n, float *y)
 {
     if (n <= 0) return;
+    std::lock_guard<std::mutex> lk(g_stage.mu);
     mlp_upload(m, X, nullptr, n);
     int per;
     const int nblk = mlp_blocks(n, &per);
     k_mlp_fwdbwd<<<nblk, MLP_NT, MLP_SMEM>>>(m->P, m->X, nullptr, n, per, m->out, nullptr, nullptr);
     COUNT_LAUNCH(1);
     CK(cudaGetLastError());
-    mlp_download(m, m->out, n);
-    std::copy(m->host, m->host + n, y);
+    if ((size_t)n > MLP_STAGE) {
+        CK(cudaMemcpy(y, m->out, n * sizeof(float), cudaMemcpyDeviceToHost));
+        return;
+    }
+    CK(cudaMemcpyAsync(g_stage.p, m->out, n * sizeof(float), cudaMemcpyDeviceToHost, 0));
+    CK(cudaStreamSynchronize(0));
+    std::copy(g_stage.p, g_stage.p + n, y);
 }
 
 // features of one (geometry, material, xi_, m): the normalisation the network is trained with.
