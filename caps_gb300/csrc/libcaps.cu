@@ -484,15 +484,29 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     for (auto &T : tasks) nnu_max = std::max(nnu_max, T.nu_max - T.mu + 1);
     const int nu_stride = (nnu_max + 31) / 32 * 32;
 
+    // memory for a chunk: 0.7 of the free device memory, the large work buffers held from earlier batches counted as free
+    // (they serve this batch, or are released below)
+    DevBuf *const large[] = {&g_eng.A, &g_eng.I, &g_eng.partM, &g_eng.partE, &g_eng.S32, &g_eng.a12, &g_eng.part, &g_eng.B,
+                             &g_eng.hwork, &g_eng.seed, &g_eng.mwork, &g_eng.sw64};
+    auto budget = [&]() {
+        size_t bytes = 0, total = 0;
+        CK(cudaMemGetInfo(&bytes, &total));
+        for (const DevBuf *b : large) bytes += b->bytes;
+        return (size_t)(0.70 * (double)bytes);
+    };
+    // of one task, whatever the path
+    const size_t task_bytes = (size_t)2 * nu_stride * sizeof(sd) + (size_t)nu_stride * sizeof(double2) + (size_t)3 * L * sizeof(sd)
+                            + (size_t)dim * 8 + (size_t)2 * ((max_nodes + 31) / 32) * nu_stride * 12 // partial K sums per warp
+                            + (size_t)(4 * (caps->ldim + 4096)) * sizeof(double4);                    // p tables
+    const size_t sweep64_task = (size_t)dim * dim * (O.square ? 16 : 8) + seed64_bytes(ldim, 1) + sweep64_work_bytes(ldim, 1);
+
     // HODLR semantics: the HODLR path (elements on demand) where it applies; the FP64 form
     // takes it from CAPS_HODLR_AUTO_DIM on, the mixed form from CAPS_HODLR_AUTO_DIM_MIXED on
     const bool mixed = caps->precision == CAPS_PREC_MIXED;
     auto auto_hodlr = [&]() {
         if (mixed) return dim >= CAPS_HODLR_AUTO_DIM_MIXED;
         if (dim < CAPS_HODLR_LOW_MEM_DIM || dim >= CAPS_HODLR_AUTO_DIM) return dim >= CAPS_HODLR_AUTO_DIM;
-        size_t f = 0, t = 0;
-        CK(cudaMemGetInfo(&f, &t));
-        return (size_t)dim * dim * 8 + cholesky_work_bytes(1, dim) > (f + g_eng.A.bytes + g_eng.hwork.bytes) / 2;
+        return task_bytes + sweep64_task + cholesky_work_bytes(1, dim) > budget();
     };
     const bool hodlr = O.factor && !O.square && !O.M_out && !O.force_dense && caps->detalg == DETALG_HODLR &&
                        (caps->path == CAPS_PATH_HODLR || (caps->path == CAPS_PATH_AUTO && auto_hodlr()));
@@ -504,36 +518,25 @@ static int run_batch(caps_t *caps, const double *xi_, const int *ms, int n, doub
     const bool sweep = ff_elem && sweep_fits(ldim);
     // the FP64 form's dense matrices by the same recurrence in FP64 (sweep64.cu), into fixed point
     const bool sweep64 = !mixed && O.factor && !O.M_out && !hodlr;
-    // chunk size from free memory.  The budget counts the large work buffers held from earlier
-    // batches as free for this one: true while batches keep one shape, each buffer serving the
+    // chunk size from the budget.  While batches keep one shape each held buffer serves the
     // same array again; when the shape (dimension, precision, path) changes they are released
     // first, since a buffer the new path does not use would stay held beside the new ones
     // (every batch ends synchronised with the device, so none is in use)
     const uint64_t shape = ((uint64_t)dim << 16) | (uint64_t)mixed | (uint64_t)hodlr << 1 | (uint64_t)sweep << 2 |
                            (uint64_t)ff_elem << 3 | (uint64_t)O.square << 4 | (uint64_t)(O.M_out != nullptr) << 5 | (uint64_t)O.factor << 6 | (uint64_t)sweep64 << 7;
     if (g_eng.shape != shape) {
-        for (DevBuf *b : {&g_eng.A, &g_eng.I, &g_eng.partM, &g_eng.partE, &g_eng.S32, &g_eng.a12, &g_eng.part, &g_eng.B,
-                          &g_eng.hwork, &g_eng.seed, &g_eng.mwork, &g_eng.sw64})
-            b->release();
+        for (DevBuf *b : large) b->release();
         g_eng.shape = shape;
     }
-    size_t freeb = 0, totb = 0;
-    CK(cudaMemGetInfo(&freeb, &totb));
     const size_t mat_bytes = O.square ? 16 : ff_elem ? 4 + 1 : (caps->precision == CAPS_PREC_MIXED ? 12 : 8);
     const size_t dense_bytes = hodlr ? hodlr_work_bytes(ldim, 1)
                              : sweep ? (size_t)dim * dim * 4 + seed_bytes(ldim, 1) + sweep_work_bytes(ldim, 1)
-                             : sweep64 ? (size_t)dim * dim * (O.square ? 16 : 8) + seed64_bytes(ldim, 1) + sweep64_work_bytes(ldim, 1)
+                             : sweep64 ? sweep64_task
                                      : (size_t)dim * dim * mat_bytes + (size_t)2 * L * L * sizeof(sd)
                                            + (size_t)L * (L + 1) / 2 * 32; // a_0..a_2 table (one row per task)
-    const size_t per_task = dense_bytes + (size_t)2 * nu_stride * sizeof(sd)
-                          + (size_t)nu_stride * sizeof(double2) + (size_t)3 * L * sizeof(sd) + (size_t)dim * 8
-                          + (size_t)2 * ((max_nodes + 31) / 32) * nu_stride * 12 // partial K sums per warp
-                          + (size_t)(4 * (caps->ldim + 4096)) * sizeof(double4) // p tables
-                          + (hodlr ? 0 : mixed && !O.square ? mixed_work_bytes(1, dim) : cholesky_work_bytes(1, dim)); // diagonal-block inverses, panel images
-    size_t budget = (size_t)(0.70 * (double)(freeb + g_eng.A.bytes + g_eng.I.bytes + g_eng.partM.bytes + g_eng.partE.bytes + g_eng.S32.bytes
-                                             + g_eng.a12.bytes + g_eng.part.bytes + g_eng.B.bytes + g_eng.hwork.bytes
-                                             + g_eng.seed.bytes + g_eng.mwork.bytes + g_eng.sw64.bytes));
-    int chunk = (int)std::max<size_t>(1, std::min<size_t>(budget / per_task, 65535));
+    const size_t per_task = task_bytes + dense_bytes // and diagonal-block inverses, panel images:
+                          + (hodlr ? 0 : mixed && !O.square ? mixed_work_bytes(1, dim) : cholesky_work_bytes(1, dim));
+    int chunk = (int)std::max<size_t>(1, std::min<size_t>(budget() / per_task, 65535));
     chunk = std::min(chunk, n);
 
     // Mie table for all distinct xi at once

@@ -195,8 +195,9 @@ int caps_gpu_set_precision(caps_t *self, int precision);
 /* determinant path of an FP64 caps object with DETALG_HODLR (the default): a HODLR
  * factorisation with the elements evaluated on demand (src/libhodlr, matrix.c:125-147) or the
  * dense batched Cholesky with the same result rules.  Automatic: HODLR from dimension
- * CAPS_HODLR_AUTO_DIM on, and from CAPS_HODLR_LOW_MEM_DIM on where half the free device memory
- * does not hold one dense matrix.  Measured on the GB300, ms for 4 matrices (dense, HODLR):
+ * CAPS_HODLR_AUTO_DIM on, and from CAPS_HODLR_LOW_MEM_DIM on where 0.7 of the free device
+ * memory (the library's own work buffers counted as free) does not hold one dense matrix and its workspace, about
+ * 12 bytes per entry.  Measured on the GB300, ms for 4 matrices (dense, HODLR):
  * dimension 5000 26, 397; 8000 64, 581; 12000 163, 1116; 20000 628, 1652; dense grows with the
  * third power of the dimension, HODLR with less than the second, so they meet near 32000.  The mixed form takes HODLR only when asked (CAPS_PATH_HODLR or the
  * autotuner); its sampled elements then come from the float-float q-sums, its compression and
