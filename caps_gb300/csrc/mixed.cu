@@ -679,13 +679,19 @@ struct KernelTimer {
 KernelTimer g_kts[KT_KINDS];
 KernelTimer &g_kt = g_kts[KT_SYRK];
 unsigned long long *g_kt_moved = nullptr; // device counter of the image-fed updates' bytes
+// cudaMemset is asynchronous, and nothing orders it before kernels of a non-blocking stream but a wait
+void kt_clear_moved()
+{
+    CK(cudaMemset(g_kt_moved, 0, sizeof *g_kt_moved));
+    CK(cudaStreamSynchronize(0));
+}
 } // namespace
 
 void kernel_timer_enable(bool on)
 {
     if (on) {
         if (!g_kt_moved) CK(cudaMalloc(&g_kt_moved, sizeof *g_kt_moved));
-        CK(cudaMemset(g_kt_moved, 0, sizeof *g_kt_moved));
+        kt_clear_moved();
     }
     for (KernelTimer &k : g_kts) {
         k.on = on;
@@ -713,7 +719,7 @@ void kernel_timer_collect(long long nfactored)
     if (g_kt.on) {
         unsigned long long moved;
         CK(cudaMemcpy(&moved, g_kt_moved, sizeof moved, cudaMemcpyDeviceToHost));
-        CK(cudaMemset(g_kt_moved, 0, sizeof moved));
+        kt_clear_moved();
         g_kt.bytes += (double)moved;
     }
 }
