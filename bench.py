@@ -204,13 +204,6 @@ def run_reference(args, dist, rank, world):
     print(json.dumps(line), flush=True)
 
 
-# DRAM bytes per algorithmic byte of the updates (k_syrk_pair and k_syrk_blk, all 32 update
-# launches of the factorisation), from one ncu capture of 24 factored matrices of this
-# workload: below 1 because the FP16 panel images that the panel solves have just written are
-# partly still in L2 when the updates read them; nothing is read twice
-SYRK_DRAM_PER_ALGORITHMIC = 0.79
-
-
 def measured_hbm_peak():
     """HBM copy bandwidth of the GB300s (GB/s) from MEASURED_PEAKS.json, else the fallback"""
     p = os.path.join(os.path.dirname(os.path.abspath(__file__)), "MEASURED_PEAKS.json")
@@ -506,14 +499,13 @@ def main():
                                 "S that those items read + write (FP32), counted by the kernels",
                       "achieved": syrk_gbs, "peak": hbm_peak, "unit": "GB/s",
                       "frac": syrk_gbs / hbm_peak if syrk_gbs else None,
-                      "traffic": syrk_bytes / syrk_n * SYRK_DRAM_PER_ALGORITHMIC if syrk_n else None,
+                      "traffic": None,
                       "peak_source": hbm_src,
                       "launches": syrk_n, "avg_launch_ms": syrk_ms / syrk_n if syrk_n else None,
                       "algorithmic_bytes_per_launch": syrk_bytes / syrk_n if syrk_n else None,
-                      "traffic_source": "DRAM bytes per algorithmic byte over all 32 update launches of the factorisation "
-                                        "of 24 matrices of this workload with every tile updated, in one ncu capture (trailing "
-                                        "updates 0.84, middle updates 0.73, block updates 0.78), times this run's algorithmic "
-                                        "bytes per launch",
+                      "traffic_source": "not measured at this size: ncu starts each launch with a clean L2 and ends it before "
+                                        "the stores leave L2 (42 matrices of this workload: 1.05 DRAM bytes read and none "
+                                        "written per byte counted here, about half of them panel images)",
                       "fp32_accurate_tflops_factorisation": achieved,
                       "panel_kernels": panel_kernels or None,
                       "panel_kernels_note": "the panel solve is bytes-bound like the update (its rate against the same peak); "
