@@ -229,7 +229,6 @@ k_ktab(const Task *tasks, const double2 *coefAB, int nu_stride, const double *lf
 // where schedulers would have no more than one warp (6 matrices of dimension 6000: 1.31 ms with one warp, 0.85 with
 // two); a large batch has warps enough, and the second one and its buffer only take room (993 matrices of
 // dimension 2100: 2.02 ms with one, 2.65 with two).  The values are the same bits.
-constexpr int KTF_PAIR_MAX = 608; // groups of 32 nodes, one per scheduler
 template <bool PR, bool PAIR>
 __global__ void __launch_bounds__(PAIR ? 64 : 32)
 k_ktab_ff(const Task *tasks, const float4 *coefF, int nu_stride, const double *lfac_tab, float2 *partF, int *partE, int max_warps)
@@ -846,7 +845,7 @@ void launch_ktab_ff(bool pr, const Task *tasks, int ntask, int max_warps, const 
                     float2 *partF, int *partE, cudaStream_t st)
 {
     // (both buffers stay below the 48 KB that need no attribute)
-    const bool pair = (long long)ntask * max_warps <= KTF_PAIR_MAX;
+    const bool pair = (long long)ntask * max_warps <= 4 * device_sms(); // schedulers
     const size_t sm = ktab_ff_smem_bytes(pair);
     const dim3 g(max_warps, ntask);
     auto run = [&](auto f) { f<<<g, pair ? 64 : 32, sm, st>>>(tasks, coefF, nu_stride, lfac_tab, partF, partE, max_warps); };

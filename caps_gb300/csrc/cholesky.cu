@@ -1266,9 +1266,7 @@ static int fix_sms()
         CK(cudaFuncSetAttribute(k_fix_potf2, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
         CK(cudaFuncSetAttribute(k_fix_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, TR_SMEM));
         CK(cudaFuncSetAttribute(k_fix_syrk, cudaFuncAttributeMaxDynamicSharedMemorySize, SY_SMEM));
-        int dev = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        sms = device_sms();
     }
     return sms;
 }

@@ -25,6 +25,7 @@ namespace capsgpu {
 // counters of kernel launches and host<->device bytes since the last reset
 struct Counters { long long launches = 0, h2d = 0, d2h = 0, nfactor = 0, nmat = 0; double factor_flops = 0; };
 extern Counters g_counters;
+int device_sms(); // multiprocessors of the current device
 #define COUNT_LAUNCH(n) (::capsgpu::g_counters.launches += (n))
 
 // quadrature nodes of K (kgrid.cuh) into a task whose other fields are set; k_left: their left end,

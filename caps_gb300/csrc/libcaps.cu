@@ -43,6 +43,13 @@ Counters g_counters;
     fprintf(stderr, "libcaps_gb300: CUDA failure at %s:%d: %s\n", file, line, what);
     abort();
 }
+int device_sms()
+{
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return sms;
+}
 } // namespace capsgpu
 
 extern "C" const char *caps_gpu_last_error(void) { return g_last_error.c_str(); }

@@ -470,7 +470,8 @@ void launch_sweep64(const Task *tasks, const int *tlist, int nlist, int ldim, co
     // A step to the next column is a chain of loads and 18 operations, 1200 clocks: 4 columns where 16 leave SMs
     // without a CTA (one matrix of ldim 140 24 us with 16, 9 with 4), elsewhere 4 would be one in twelve more operations
     // (32 of ldim 350: 93 us).  The elements are the same bits, the sums of squares come in the order of E64_Y.
-    const int nx = (ldim + E64_X - 1) / E64_X, ny = !fro && (long long)nx * ((ldim + E64_Y - 1) / E64_Y) * nlist < 152 ? 4 : E64_Y;
+    const int nx = (ldim + E64_X - 1) / E64_X;
+    const int ny = !fro && (long long)nx * ((ldim + E64_Y - 1) / E64_Y) * nlist < device_sms() ? 4 : E64_Y;
     const dim3 g(nx, (ldim + ny - 1) / ny, nlist);
     if (fro) k_elem64<true><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, ny, tt, tab, mdiag, info, A, mstride, fro, status);
     else k_elem64<false><<<g, E64_X, 0, st>>>(tasks, tlist, nlist, ldim, ny, tt, tab, mdiag, info, A, mstride, fro, status);
