@@ -61,10 +61,13 @@ CAPS_DEV int seed_col(const Task &T)
 }
 
 // ranges of rows of T: part q of P forms rows (row(q), row(q + 1)], row(0) = -1, of about equal numbers of pairs; parts
-// q >= 1 start from the q-sums of rows row(q) - 1 and row(q).  The number depends on ldim alone.  Few large
-// matrices leave SMs idle behind the chain of rows: 6 matrices of ldim 3000 take 4.7 ms in one part, 1.05 in five
+// q >= 1 start from the q-sums of rows row(q) - 1 and row(q).  The number depends on ldim alone, so that a matrix has the
+// same value in every batch.  Few matrices leave SMs idle behind the chain of rows; parts of 512 rows against one part, ms of
+// seeds, table and elements: ldim 1050, 1 matrix 0.77 -> 0.55, 6 0.86 -> 0.63, 48 1.30 -> 1.12, 547 6.42 -> 6.40; 1500, 1
+// 1.23 -> 0.81, 48 2.20 -> 1.81, 200 4.80 -> 4.73; 2000, 1 1.90 -> 0.91, 48 3.40 -> 2.44, 150 6.27 -> 5.95; 3000, 6
+// 5.22 -> 1.58.  No batch loses, so the line is where there is a second part
 __host__ __device__ inline int recf_row(int q, int P, int L) { return q <= 0 ? -1 : q >= P ? L - 1 : (int)(L * sqrt((double)q / P)); }
-__host__ __device__ inline int recf_parts(int ldim) { return ldim <= 2230 ? 1 : ldim / 512; }
+__host__ __device__ inline int recf_parts(int ldim) { return ldim < 1024 ? 1 : ldim / 512; }
 
 // ---------------------------------------------------------------------------
 // seeds: q-sums of the pairs of two kinds per window index w
