@@ -8,7 +8,8 @@
 // integers in units of 2^-60 (an FP64 number near 1 has units of 2^-53), and the FP64 pipe --
 // two fused multiply-adds per clock and SM on this GPU, 1.05 TFLOP/s in all -- is left out:
 //
-//  * products with 64 columns (panel solve, trailing update) run on the tensor cores.  A factor x
+//  * products with 64 columns (panel solve, trailing update) run on the tensor cores, split into exact
+//    products of digits (Ozaki's scheme, with a common scale instead of one per row).  A factor x
 //    is split into six signed 9-bit digits, x = sum_i d_i 2^(-8-9i), exact as FP16; the MMAs
 //    (kind::f16, FP32 accumulators) form sum_k d_i(k) d_j(k) as exact integers in one accumulator
 //    per i + j = 0..6, and the epilogue adds the accumulators up as 64-bit integers.  Digit

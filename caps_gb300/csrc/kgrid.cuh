@@ -14,9 +14,10 @@
 //   u = c log(1 + e^{w / c})
 // makes it decay like e^{(k+1) w / c}, k = mu + 1 - 2s, on the left and is linear on the right; its
 // poles lie at w = +- i pi c.  The Fresnel coefficients are singular at x = +- i sqrt(eps), at a
-// distance d = sqrt(2 alpha (1 + sqrt(1 + eps))) from the real u axis: d >= 4 keeps the error below
-// e^{-2 pi d / h} = 6e-19 and takes c = 1.5; closer ones are resolved in log u, c = 8 h, since their
-// angle is at least pi / 4.
+// distance d = sqrt(2 alpha (1 + sqrt(1 + eps))) from the real u axis, where the integrand may have grown by
+// e^{d^2/2}: the error is about e^{-2 pi d / h + d^2 / 2}, 2e-15 at d = 4 (in 40 digits 3.5e-15 for nu = mu, K_TM, the largest
+// seen, 4e-16 for K_TE), the end of the range d >= 4 that dominates, with c = 1.5; closer ones are resolved in log u,
+// c = 8 h, since their angle is at least pi / 4.
 //
 // The range: on the left the lowest degree's integrand, at most p (log y + (1 - y^2) / 2) below its
 // peak in log at u = sqrt(2 p) y, p = k + 1 (exact for x - 1 << 1, an upper bound otherwise); on

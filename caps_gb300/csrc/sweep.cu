@@ -1,5 +1,6 @@
 // sweep.cu -- the mixed form's round-trip matrix from a band of q-sums and a three-term
-// recurrence of the I integrals, with the elements formed as the rows of the table appear.
+// recurrence of the I integrals: a kernel that fills the table of I row by row and one that forms
+// the elements from its tiles.
 //
 // The q-sum of every (l1, l2) pair (integration.c:491-609) costs O(l) terms, O(ldim^3) per
 // matrix.  The I integrals also obey the three-term recurrence of the associated Legendre

@@ -8,12 +8,12 @@
 // moving away from the diagonal; against q-sums of every pair log det changes by 1e-13 relative
 // at most (tests/test_gpu_sweep64.py), the size of the q-sums' own rounding.
 //
-// Two kernels, both bound by the FP64 pipe (two operations per clock and SM).  k_rec64 fills the
-// table T row by row, 4 operations per entry and polarisation, one CTA per matrix and range of
-// rows: a range but the first starts from the q-sums of two whole rows, and the number of ranges
-// depends on ldim alone, so that a matrix has the same value in every batch.  k_elem64 forms
-// the elements of all pairs at once: the row factors dA, dB are folded into the coefficients of
-// their row (J' = dA J costs what J does) and the column factors into tables, 20 operations for
+// Two kernels behind the seeds and a table of coefficients, both bound by the FP64 pipe (two operations per clock and
+// SM).  k_rec64 fills the table T row by row, 4 operations per entry and polarisation, one CTA per
+// matrix, range of rows and polarisation: a range but the first starts from the q-sums of two whole
+// rows, and the number of ranges depends on ldim alone, so that a matrix has the same value in every
+// batch.  k_elem64 forms the elements of all pairs at once: the row factors dA, dB are folded into the
+// coefficients of their row (J' = dA J costs what J does) and the column factors into tables, 18 operations for
 // the four elements of a pair; conversion to fixed point is integer work.  For a perfectly
 // reflecting plate T_TE = -T_TM, and only T_TM is formed.
 #include "fix.cuh"
