@@ -426,9 +426,10 @@ int capc_batch(double R, double d, int n, const double *q, int nq, char DN, int 
     std::lock_guard<std::mutex> lk(g_capc_mu);
     const size_t mstride = (size_t)n * n;
     const int ts = tab_stride(n);
-    // chunks of at most ~4 GB of matrices and 16384 wave numbers (grid z = 2 per q)
-    const int chunk = (int)std::max<size_t>(
-        1, std::min<size_t>(std::min<size_t>((size_t)nq, 16384), ((size_t)4 << 30) / (2 * mstride * sizeof(double))));
+    // chunks of at most 4 GB of matrices, 4 GB of the factorisation's workspace (250 KB for the smallest matrices) and
+    // 16384 wave numbers (grid z = 2 per q)
+    const int chunk = (int)std::max<size_t>(1, std::min({(size_t)nq, (size_t)16384, ((size_t)4 << 30) / (2 * mstride * sizeof(double)),
+                                                         ((size_t)4 << 30) / cholesky_work_bytes(2, n)}));
     const int rs = raw_stride(n);
     const dim3 ge((n + CE_X - 1) / CE_X, (n + CE_Y - 1) / CE_Y);
     const int nfro = ge.x * ge.y;
